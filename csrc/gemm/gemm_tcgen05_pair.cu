@@ -9,7 +9,7 @@
 // (cluster rank 0) issues every tcgen05.mma for the pair; the accumulator of each CTA's 128 rows lives in that
 // CTA's own tensor memory, 2 x 256 columns, so epilogue and main loop overlap.
 //
-// Roles per CTA (256 threads; warps 6-7 only work in the all-gather mode, see below): warp 0 lane 0 issues TMA loads (cp.async.bulk.tensor with cta_group::2 and no
+// Roles per CTA (256 threads; warps 6-7 only work in the all-gather mode, see below): warp 0 issues TMA loads (cp.async.bulk.tensor with cta_group::2 and no
 // multicast: both CTAs signal the LEADER's "full" barrier); warp 1 owns tensor memory and, in the leader, issues
 // the MMAs and commits them to both CTAs' barriers; warps 2-5 read the accumulator with tcgen05.ld and store C.
 // Every mbarrier wait is bounded and checks the pair's abort flags; on a give-up all roles fall through to the
@@ -153,6 +153,18 @@ __device__ __forceinline__ void UmmaPairF8(uint32_t tmemD, uint64_t descA, uint6
         : "memory");
 }
 
+// The four instructions of one stage; each consumes 32 bytes of K (16 16-bit or 32 8-bit elements): +2 in descriptor units.
+template <bool FP8>
+__device__ __forceinline__ void IssueStage(uint32_t tmemD, uint64_t descA, uint64_t descB, uint32_t idesc, bool accumulate)
+{
+#pragma unroll
+    for (int k = 0; k < GEMM_BK / GEMM_UMMA_K; ++k) {
+        const uint32_t acc = k != 0 || accumulate ? 1u : 0u;
+        if (FP8) UmmaPairF8(tmemD, descA + static_cast<uint64_t>(k * 2), descB + static_cast<uint64_t>(k * 2), idesc, acc);
+        else UmmaPairF16(tmemD, descA + static_cast<uint64_t>(k * 2), descB + static_cast<uint64_t>(k * 2), idesc, acc);
+    }
+}
+
 // Arrives on `bar` in BOTH CTAs of the pair once every MMA issued so far has finished.
 __device__ __forceinline__ void UmmaCommitPair(uint64_t *bar)
 {
@@ -198,6 +210,12 @@ __device__ __forceinline__ bool WaitBar(uint64_t *bar, uint32_t parity, PairStat
             }
         }
     }
+}
+
+// The same by a whole warp, with one verdict for all lanes.
+__device__ __forceinline__ bool WaitBarWarp(uint64_t *bar, uint32_t parity, PairState *st, uint32_t peerAbortAddr, uint64_t budgetNs)
+{
+    return __all_sync(0xffffffffu, WaitBar(bar, parity, st, peerAbortAddr, budgetNs)) != 0;
 }
 
 __device__ __forceinline__ uint32_t PackPair(float lo, float hi, bool bf16)
@@ -438,89 +456,88 @@ __device__ void PairBody(const GemmArgs &a)
 
     if (warp == 0) {
         // ---- TMA producer: this CTA's 128 rows of A and its half of the B tile ---------------------------------
-        if (lane == 0) {
-            uint32_t stage = 0, phase = 0;
-            for (int t = pair; t < totalTiles && st->abortFlag == 0; t += nPairs) {
-                const PairTile tc = TileOf(a, tileBase + tileSign * t, mTiles, rank, ranks, gt);
-                const int mLocal = tc.mLocalPair * 2 + static_cast<int>(ctaRank);        // this CTA's 128-row block in the shard
-                const bool remoteA = a.mode == GEMM_ALL_GATHER && tc.shard != rank;
-                const CUtensorMap *mapA = (a.mode == GEMM_ALL_GATHER && !remoteA) ? &a.tmapALocal : &a.tmapA;
-                // grouped: a block starts wherever its group's rows start; rows past the group's end belong to the
-                // next group (or are filled with zeros past the end of A) and are computed but never stored
-                const int rowA = a.mode == GEMM_GROUPED ? tc.row0 + static_cast<int>(ctaRank) * GEMM_BM
-                                 : (a.mode == GEMM_ALL_GATHER && !remoteA) ? mLocal * GEMM_BM
-                                                                           : tc.mTile * 2 * GEMM_BM + static_cast<int>(ctaRank) * GEMM_BM;
-                const int rowB = tc.rowB0 + tc.nBlock * GEMM_BN + static_cast<int>(ctaRank) * (GEMM_BN / 2);
-                bool broke = false;
-                for (int kb = 0; kb < a.kBlocks; ++kb) {
-                    if (!WaitBar(&st->empty[stage], phase ^ 1u, st, peerAbortAddr, budgetNs)) {
+        uint32_t stage = 0, phase = 0;
+        for (int t = pair; t < totalTiles && __all_sync(0xffffffffu, st->abortFlag == 0); t += nPairs) {
+            const PairTile tc = TileOf(a, tileBase + tileSign * t, mTiles, rank, ranks, gt);
+            const int mLocal = tc.mLocalPair * 2 + static_cast<int>(ctaRank);        // this CTA's 128-row block in the shard
+            const bool remoteA = a.mode == GEMM_ALL_GATHER && tc.shard != rank;
+            const CUtensorMap *mapA = (a.mode == GEMM_ALL_GATHER && !remoteA) ? &a.tmapALocal : &a.tmapA;
+            // grouped: a block starts wherever its group's rows start; rows past the group's end belong to the
+            // next group (or are filled with zeros past the end of A) and are computed but never stored
+            const int rowA = a.mode == GEMM_GROUPED ? tc.row0 + static_cast<int>(ctaRank) * GEMM_BM
+                             : (a.mode == GEMM_ALL_GATHER && !remoteA) ? mLocal * GEMM_BM
+                                                                       : tc.mTile * 2 * GEMM_BM + static_cast<int>(ctaRank) * GEMM_BM;
+            const int rowB = tc.rowB0 + tc.nBlock * GEMM_BN + static_cast<int>(ctaRank) * (GEMM_BN / 2);
+            bool broke = false;
+            for (int kb = 0; kb < a.kBlocks; ++kb) {
+                if (!WaitBarWarp(&st->empty[stage], phase ^ 1u, st, peerAbortAddr, budgetNs)) {
+                    broke = true;
+                    break;
+                }
+                if (remoteA && kb % a.kBlocksPerChunk == 0) {
+                    const int piece = mLocal * a.kChunks + kb / a.kBlocksPerChunk;
+                    const int64_t slot = FLAG_PLANE_A + static_cast<int64_t>(tc.shard) * a.flagStride + piece;
+                    bool landed = true;
+                    if (lane == 0) landed = WaitFlagGE(w, FlagSlot(a.comm, rank, slot), 1, tc.shard, slot);
+                    if (!__all_sync(0xffffffffu, landed)) {
+                        st->abortFlag = 1;
                         broke = true;
                         break;
                     }
-                    if (remoteA && kb % a.kBlocksPerChunk == 0) {
-                        const int piece = mLocal * a.kChunks + kb / a.kBlocksPerChunk;
-                        const int64_t slot = FLAG_PLANE_A + static_cast<int64_t>(tc.shard) * a.flagStride + piece;
-                        if (!WaitFlagGE(w, FlagSlot(a.comm, rank, slot), 1, tc.shard, slot)) {
-                            st->abortFlag = 1;
-                            broke = true;
-                            break;
-                        }
-                        fence_proxy_async();   // the rows were written by a peer's stores, TMA reads them next
-                    }
+                    __syncwarp();          // the rows lane 0 acquired are there for the lane that issues
+                    fence_proxy_async();   // the rows were written by a peer's stores, TMA reads them next
+                }
+                if (ElectOne()) {
                     uint8_t *sa = stageBase + stage * GEMM_PAIR_STAGE_BYTES;
                     uint8_t *sb = sa + GEMM_STAGE_A_BYTES;
                     if (leader) MbarExpectTx(&st->full[stage], 2 * GEMM_PAIR_STAGE_BYTES);
                     TmaLoadPair2D(sa, mapA, kb * kPerStage, rowA, &st->full[stage]);
                     TmaLoadPair2D(sb, &a.tmapB, kb * kPerStage, rowB, &st->full[stage]);
-                    if (++stage == GEMM_PAIR_STAGES) {
-                        stage = 0;
-                        phase ^= 1u;
-                    }
                 }
-                if (broke) break;
+                if (++stage == GEMM_PAIR_STAGES) {
+                    stage = 0;
+                    phase ^= 1u;
+                }
             }
+            if (broke) break;
         }
     } else if (warp == 1) {
-        // ---- MMA issuer: the leader's lane 0 drives the tensor cores of both SMs ---------------------------------
-        if (leader && lane == 0) {
+        // ---- MMA issuer: one elected lane of the leader drives the tensor cores of both SMs -----------------------
+        if (leader) {
             const uint32_t idesc = fp8 ? MakeInstrDescFp8(a.fp8Format) : MakeInstrDesc(bf16);
+            const uint64_t descA0 = MakeSmemDesc(SmemAddr(stageBase));
+            const uint64_t descB0 = MakeSmemDesc(SmemAddr(stageBase) + GEMM_STAGE_A_BYTES);
             uint32_t stage = 0, phase = 0;
             int iter = 0;
-            for (int t = pair; t < totalTiles && st->abortFlag == 0; t += nPairs, ++iter) {
+            for (int t = pair; t < totalTiles && __all_sync(0xffffffffu, st->abortFlag == 0); t += nPairs, ++iter) {
                 const int acc = iter & 1;
                 const uint32_t accPhase = (iter >> 1) & 1;
-                if (!WaitBar(&st->tmemEmpty[acc], accPhase ^ 1u, st, peerAbortAddr, budgetNs)) break;
+                if (!WaitBarWarp(&st->tmemEmpty[acc], accPhase ^ 1u, st, peerAbortAddr, budgetNs)) break;
                 TcFenceAfter();
                 const uint32_t tmemD = tmemBase + static_cast<uint32_t>(acc) * GEMM_BN;
                 bool broke = false;
                 for (int kb = 0; kb < a.kBlocks; ++kb) {
-                    if (!WaitBar(&st->full[stage], phase, st, peerAbortAddr, budgetNs)) {
+                    if (!WaitBarWarp(&st->full[stage], phase, st, peerAbortAddr, budgetNs)) {
                         broke = true;
                         break;
                     }
                     TcFenceAfter();
-                    const uint32_t sa = SmemAddr(stageBase + stage * GEMM_PAIR_STAGE_BYTES);
-                    const uint64_t descA = MakeSmemDesc(sa);
-                    const uint64_t descB = MakeSmemDesc(sa + GEMM_STAGE_A_BYTES);
-#pragma unroll
-                    for (int k = 0; k < GEMM_BK / GEMM_UMMA_K; ++k) {
-                        // each instruction consumes 32 bytes of K (16 16-bit or 32 8-bit elements): +2 in descriptor units
-                        if (fp8) {
-                            UmmaPairF8(tmemD, descA + static_cast<uint64_t>(k * 2), descB + static_cast<uint64_t>(k * 2), idesc,
-                                       (kb | k) != 0 ? 1u : 0u);
-                        } else {
-                            UmmaPairF16(tmemD, descA + static_cast<uint64_t>(k * 2), descB + static_cast<uint64_t>(k * 2), idesc,
-                                        (kb | k) != 0 ? 1u : 0u);
-                        }
+                    if (ElectOne()) {
+                        const uint64_t descA = descA0 + static_cast<uint64_t>(stage * (GEMM_PAIR_STAGE_BYTES >> 4));
+                        const uint64_t descB = descB0 + static_cast<uint64_t>(stage * (GEMM_PAIR_STAGE_BYTES >> 4));
+                        // the kind is decided once per group: a branch between the four instructions costs as much issue
+                        // time as the instructions themselves
+                        if (fp8) IssueStage<true>(tmemD, descA, descB, idesc, kb != 0);
+                        else IssueStage<false>(tmemD, descA, descB, idesc, kb != 0);
+                        UmmaCommitPair(&st->empty[stage]);    // both CTAs may refill the stage once these MMAs have read it
                     }
-                    UmmaCommitPair(&st->empty[stage]);    // both CTAs may refill the stage once these MMAs have read it
                     if (++stage == GEMM_PAIR_STAGES) {
                         stage = 0;
                         phase ^= 1u;
                     }
                 }
                 if (broke) break;
-                UmmaCommitPair(&st->tmemFull[acc]);
+                if (ElectOne()) UmmaCommitPair(&st->tmemFull[acc]);
             }
         }
     } else if (warp >= 6) {
