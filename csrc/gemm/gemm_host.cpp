@@ -343,10 +343,10 @@ int TileXRMatmulFp8BlockScaled(const void *a, const float *scaleA, const void *b
     const int pairs = std::max(1, std::min<int>(pairTiles, static_cast<int>(EnvLong("TILEXR_GEMM_CTAS", sms)) / 2));
     static std::once_flag once;
     std::call_once(once, [] {
-        cudaFuncSetAttribute(GemmFp8BlockKernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(GEMM_FP8_BLOCK_SMEM_BYTES));
+        cudaFuncSetAttribute(GemmFp8BlockKernel(GEMM_PLAIN), cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(GEMM_FP8_BLOCK_SMEM_BYTES));
     });
     void *params[] = {&g};
-    const cudaError_t e = cudaLaunchKernel(GemmFp8BlockKernel(), dim3(2 * pairs), dim3(GEMM_FP8_BLOCK_THREADS), params, GEMM_FP8_BLOCK_SMEM_BYTES,
+    const cudaError_t e = cudaLaunchKernel(GemmFp8BlockKernel(GEMM_PLAIN), dim3(2 * pairs), dim3(GEMM_FP8_BLOCK_THREADS), params, GEMM_FP8_BLOCK_SMEM_BYTES,
                                            static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) {
         TILEXR_LOG(ERROR) << "block-scaled fp8 matmul launch failed: " << cudaGetErrorString(e);
@@ -543,17 +543,20 @@ int TileXRMatmulReduceScatter(const void *a, const void *b, void *partialStaging
 
 // ---- block-scaled fp8 with the collectives of a tensor-parallel layer ----------------------------------------------------
 
-static const KernelEntry &GemmFp8BlockEntry()
+static const KernelEntry &GemmFp8BlockEntry(int mode)
 {
-    static const KernelEntry e = {GemmFp8BlockKernel(), GemmFp8BlockKernelEmulated(), sizeof(GemmBlockArgs), "TileXRGemmFp8BlockScaled"};
-    return e;
+    static const KernelEntry gather = {GemmFp8BlockKernel(GEMM_ALL_GATHER), GemmFp8BlockKernelEmulated(GEMM_ALL_GATHER), sizeof(GemmBlockArgs),
+                                       "TileXRGemmFp8BlockScaled (all-gather)"};
+    static const KernelEntry scatter = {GemmFp8BlockKernel(GEMM_REDUCE_SCATTER), GemmFp8BlockKernelEmulated(GEMM_REDUCE_SCATTER),
+                                        sizeof(GemmBlockArgs), "TileXRGemmFp8BlockScaled (reduce-scatter)"};
+    return mode == GEMM_ALL_GATHER ? gather : scatter;
 }
 
-static int Fp8BlockFusedGrid(TileXRCommPtr comm, const TileXRCommArgs *hostArgs, unsigned *grid)
+static int Fp8BlockFusedGrid(TileXRCommPtr comm, const TileXRCommArgs *hostArgs, int mode, unsigned *grid)
 {
     const int ranksPerDevice = (hostArgs->extraFlag & TILEXR_FLAG_EMULATED) ? hostArgs->rankSize : 1;
     unsigned maxGrid = 0;
-    int ret = MaxCooperativeGrid(comm, GemmFp8BlockEntry(), GEMM_FP8_BLOCK_THREADS, GEMM_FP8_BLOCK_SMEM_BYTES, ranksPerDevice, &maxGrid);
+    int ret = MaxCooperativeGrid(comm, GemmFp8BlockEntry(mode), GEMM_FP8_BLOCK_THREADS, GEMM_FP8_BLOCK_SMEM_BYTES, ranksPerDevice, &maxGrid);
     if (ret != TILEXR_SUCCESS) return ret;
     maxGrid &= ~1u;
     if (maxGrid < 2) {
@@ -642,14 +645,14 @@ int TileXRAllGatherMatmulFp8Block(const void *aShard, const float *scaleAShard, 
     g.sHandle = sHandle;
     g.sOffset = sOffset;
     unsigned grid = 0;
-    ret = Fp8BlockFusedGrid(comm, hostArgs, &grid);
+    ret = Fp8BlockFusedGrid(comm, hostArgs, g.mode, &grid);
     if (ret != TILEXR_SUCCESS) return ret;
     int64_t magic = 0;
     ret = TileXRCommNextMagic(comm, &magic);
     if (ret != TILEXR_SUCCESS) return ret;
     g.magic = magic;
     LaunchConfig cfg{grid, GEMM_FP8_BLOCK_THREADS, GEMM_FP8_BLOCK_SMEM_BYTES, true};
-    return LaunchKernel(comm, GemmFp8BlockEntry(), &g, cfg, stream);
+    return LaunchKernel(comm, GemmFp8BlockEntry(g.mode), &g, cfg, stream);
 }
 
 int TileXRMatmulReduceScatterFp8Block(const void *a, const float *scaleA, const void *b, const float *scaleB, void *partialStaging, void *out,
@@ -690,14 +693,14 @@ int TileXRMatmulReduceScatterFp8Block(const void *a, const float *scaleA, const 
     g.outHandle = handle;
     g.outOffset = offset;
     unsigned grid = 0;
-    ret = Fp8BlockFusedGrid(comm, hostArgs, &grid);
+    ret = Fp8BlockFusedGrid(comm, hostArgs, g.mode, &grid);
     if (ret != TILEXR_SUCCESS) return ret;
     int64_t magic = 0;
     ret = TileXRCommNextMagic(comm, &magic);
     if (ret != TILEXR_SUCCESS) return ret;
     g.magic = magic;
     LaunchConfig cfg{grid, GEMM_FP8_BLOCK_THREADS, GEMM_FP8_BLOCK_SMEM_BYTES, true};
-    return LaunchKernel(comm, GemmFp8BlockEntry(), &g, cfg, stream);
+    return LaunchKernel(comm, GemmFp8BlockEntry(g.mode), &g, cfg, stream);
 }
 
 } // extern "C"

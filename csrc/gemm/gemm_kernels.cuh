@@ -112,8 +112,8 @@ struct GemmBlockArgs {
     int32_t shardRows, blocksPerShard, flagStride;
 };
 
-const void *GemmFp8BlockKernel();
-const void *GemmFp8BlockKernelEmulated();
+const void *GemmFp8BlockKernel(int mode);            // a kernel per GemmMode (plain, all-gather, reduce-scatter)
+const void *GemmFp8BlockKernelEmulated(int mode);    // all-gather, reduce-scatter
 const void *GemmKernelSingle();
 const void *GemmKernelEmulated();
 const void *GemmPairKernel();

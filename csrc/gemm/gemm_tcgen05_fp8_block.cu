@@ -11,16 +11,20 @@
 // cores already work on the next block.  A stage of the TMA ring is exactly one block of K (128 bytes per row),
 // so the main loop alternates two scratch accumulators:
 //
-//   tensor memory   4 x 128 columns: scratch (p, h) receives, for blocks of K of parity p, the 128 columns
-//                   {h*64..h*64+63} u {128+h*64..128+h*64+63} of the pair's 256 x 256 tile (with cta_group::2 each
-//                   CTA supplies half of B's rows); two blocks of K are in flight for each half;
+//   tensor memory   2 x 256 columns: scratch p receives the pair's 256 x 256 tile for blocks of K of parity p (with
+//                   cta_group::2 each CTA supplies half of B's rows: columns 0-127 and 128-255);
 //   warp 0          TMA producer (this CTA's 128 rows of A and 128 rows of B per block of K, no multicast);
-//   warp 1          tensor-memory owner; in the leader CTA it issues two N = 128 instructions groups per block of K;
+//   warp 1          tensor-memory owner; in the leader CTA it issues four N = 256 instructions per block of K (two groups
+//                   of N = 128 cost twice the issue time and left the tensor cores waiting for instructions);
 //   warps 2-3       idle: they complete the first warpgroup, which hands most of its registers to the others
 //                   (setmaxnreg), because the promoters keep a quarter of the tile each in registers;
 //   warps 4-7, 8-11 promoters of the two column halves: tcgen05.ld, scale, fused multiply-add into 128 fp32
-//                   registers per thread (one row of the CTA's 128, 128 columns), release the scratch buffer;
-//                   at the end of a tile they round to the output type and store through a swizzled staging tile.
+//                   registers per thread (one row of the CTA's 128, 128 columns), release the scratch buffer as soon
+//                   as its last column is in registers; at the end of a tile they round to the output type and store.
+//
+// What bounds a block of K: the four instructions take 513 clocks and the fold of the 256 columns 390 (its 264 of
+// multiply-adds and the tensor-memory reads beside them), both measured alone on one SM at a time; a scratch goes round
+// through instruction, commit, fold and release, two of them in flight.
 //
 // Fused with the collectives of a tensor-parallel layer (mode of GemmBlockArgs):
 //
@@ -55,9 +59,9 @@ using namespace tilexr;
 namespace {
 
 constexpr uint32_t FB_TMEM_COLS = 512;
-constexpr int FB_SCRATCH = 4;               // scratch accumulators: two blocks of K in flight for each half of the tile
+constexpr int FB_SCRATCH = 2;               // scratch accumulators of 256 columns: two blocks of K in flight
 constexpr uint32_t FB_PEER_BIT_MASK = 0xFEFFFFFFu;
-constexpr int FB_HALF_N = GEMM_BN / 2;       // columns of one scratch accumulator
+constexpr int FB_HALF_N = GEMM_BN / 2;       // columns of one promoter group = one 128-wide block of the weight's scales
 constexpr int FB_MAX_KB = 256;               // blocks of K whose weight scales fit the shared-memory copy (K up to 32768)
 constexpr int FB_FLAG_PLANE_A = TILEXR_FLAG_DATA_BASE;    // all-gather: piece (source rank, 128-row block) has landed
 constexpr int FB_FLAG_PLANE_B = TILEXR_FLAG_ACK_BASE;     // reduce-scatter: partial tile (source rank, tile) has landed
@@ -67,7 +71,7 @@ __device__ __forceinline__ void FbMultimemSt(uint8_t *p, const Vec16 &v)
     asm volatile("multimem.st.relaxed.sys.global.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 
-// `bytes` (a multiple of 16) from local memory to `dst`, four vectors per thread in flight (the pushing warps live on the 88 registers of the first warpgroup); `multicast` stores through
+// `bytes` (a multiple of 16) from local memory to `dst`, four vectors per thread in flight (the pushing warps live on the 80 registers of the first warpgroup); `multicast` stores through
 // an NVLink multicast address (every rank's copy at once).
 __device__ __forceinline__ void FbPush(uint8_t *dst, const uint8_t *src, uint64_t bytes, int lane, int lanes, bool multicast)
 {
@@ -95,7 +99,7 @@ struct BlockState {
     uint64_t full[GEMM_FP8_BLOCK_STAGES];       // leader: both CTAs' loads of a stage have landed
     uint64_t empty[GEMM_FP8_BLOCK_STAGES];      // each CTA: the MMAs that read this stage have finished
     uint64_t scratchFull[FB_SCRATCH];      // each CTA: scratch s holds the product of one block of K
-    uint64_t scratchEmpty[FB_SCRATCH];     // leader: the eight promoter warps of scratch s (four per CTA) have read it
+    uint64_t scratchEmpty[FB_SCRATCH];     // leader: the sixteen promoter warps of the pair have read scratch s
     uint32_t tmemBase;
     volatile int abortFlag;
     uint32_t epoch;                        // fused modes: the epoch of this launch (kept here, not in every thread's registers)
@@ -153,11 +157,11 @@ __device__ __forceinline__ uint64_t FbSmemDesc(uint32_t smemAddr)
     return d;
 }
 
-// kind::f8f6f4, D fp32, A and B K-major, M = 256 rows over the pair, N = 128.
+// kind::f8f6f4, D fp32, A and B K-major, M = 256 rows over the pair, N = 256.
 __device__ __forceinline__ uint32_t FbInstrDesc(int fp8Format)
 {
     const uint32_t fmt = fp8Format == 2 ? 1u : 0u;
-    return (1u << 4) | (fmt << 7) | (fmt << 10) | (static_cast<uint32_t>(FB_HALF_N >> 3) << 17) |
+    return (1u << 4) | (fmt << 7) | (fmt << 10) | (static_cast<uint32_t>(GEMM_BN >> 3) << 17) |
            (static_cast<uint32_t>((2 * GEMM_BM) >> 4) << 24);
 }
 
@@ -182,20 +186,25 @@ __device__ __forceinline__ void FbCommitPair(uint64_t *bar)
                  ::"r"(SmemAddr(bar)), "h"(mask) : "memory");
 }
 
-__device__ __forceinline__ void FbTmemLoad32(uint32_t taddr, uint32_t *r)
+__device__ __forceinline__ void FbTmemLoad16(uint32_t taddr, uint32_t *r)
 {
     asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr)
         : "memory");
 }
-__device__ __forceinline__ void FbTmemLoadWait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// Waits for the loads in flight.  `r` goes through the statement: nothing else would keep the compiler from moving
+// arithmetic on a load's registers in front of the wait.
+__device__ __forceinline__ void FbTmemLoadWait16(uint32_t *r)
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]),
+                   "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+                 :
+                 : "memory");
+}
 
 __device__ __forceinline__ bool FbWaitBar(uint64_t *bar, uint32_t parity, BlockState *st, uint32_t peerAbortAddr, uint64_t budgetNs)
 {
@@ -218,6 +227,12 @@ __device__ __forceinline__ bool FbWaitBar(uint64_t *bar, uint32_t parity, BlockS
             }
         }
     }
+}
+
+// The same by a whole warp, with one verdict for all lanes.
+__device__ __forceinline__ bool FbWaitBarWarp(uint64_t *bar, uint32_t parity, BlockState *st, uint32_t peerAbortAddr, uint64_t budgetNs)
+{
+    return __all_sync(0xffffffffu, FbWaitBar(bar, parity, st, peerAbortAddr, budgetNs)) != 0;
 }
 
 // Bounded acquire of a flag by one thread that has no Waiter of its own (the promoters are short of registers).
@@ -276,8 +291,10 @@ __device__ __forceinline__ void FbTileOf(const GemmBlockArgs &a, int t, int mTil
 }
 
 // Twelve warps start with 168 registers each (the most a block of this size can have); the first warpgroup then
-// shrinks to 88 and the two promoter warpgroups grow to 200, so that 128 accumulators and two 32-register
-// tensor-memory reads fit without spilling.
+// shrinks to 80 and the two promoter warpgroups grow to 208 (128 x 80 + 256 x 208 of the 384 x 168 registers of the launch),
+// so that 128 accumulators and two 16-register tensor-memory reads fit.
+// One kernel per mode: with the collectives' code in it the plain kernel spilled inside the fold (8192^3: 511 us with it, 474 us without).
+template <int MODE>
 __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
 {
     extern __shared__ uint8_t smemRaw[];
@@ -290,7 +307,7 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
     const int lane = threadIdx.x & 31;
     const uint32_t ctaRank = FbCtaRank();
     const bool leader = ctaRank == 0;
-    const bool fused = a.mode != GEMM_PLAIN;
+    constexpr bool fused = MODE != GEMM_PLAIN;
     const uint32_t peerAbortAddr = FbMapToCta(SmemAddr(const_cast<int *>(&st->abortFlag)), ctaRank ^ 1u);
 
     // The promoters have no register to spare for values that only the prologue, the TMA lane and the epilogue need: the
@@ -305,7 +322,7 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
         if (threadIdx.x == 0) st->epoch = w.epoch;
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             a.comm->dfx[TILEXR_DFX_MAGIC] = w.epoch;
-            a.comm->dfx[TILEXR_DFX_OP] = a.mode == GEMM_ALL_GATHER ? TILEXR_OP_ALL_GATHER_MATMUL : TILEXR_OP_MATMUL_REDUCE_SCATTER;
+            a.comm->dfx[TILEXR_DFX_OP] = MODE == GEMM_ALL_GATHER ? TILEXR_OP_ALL_GATHER_MATMUL : TILEXR_OP_MATMUL_REDUCE_SCATTER;
             a.comm->dfx[TILEXR_DFX_RUN_STATUS] = TILEXR_RUN_STARTED;
         }
         bool g = true;
@@ -322,7 +339,7 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
         }
         for (int h = 0; h < FB_SCRATCH; ++h) {
             MbarInit(&st->scratchFull[h], 1);     // one commit
-            MbarInit(&st->scratchEmpty[h], 8);    // four promoter warps in each of the two CTAs
+            MbarInit(&st->scratchEmpty[h], 16);   // eight promoter warps in each of the two CTAs
         }
         st->abortFlag = ok ? 0 : 1;
         MbarInitFence();
@@ -348,86 +365,82 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
 
     if (warp < 4) {
     // the first warpgroup gives registers away (all four warps execute this together) and then splits into its roles
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 88;" ::: "memory");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 80;" ::: "memory");
     if (warp == 0) {
-        // ---- TMA producer -----------------------------------------------------------------------------------------
-        if (lane == 0) {
-            const uint64_t budgetNs = fused ? a.comm->waitTimeoutNs : 4000000000ull;
-            const int rank = fused ? a.comm->rank : 0;
-            Waiter w{fused ? a.comm : nullptr, st->epoch, static_cast<int32_t>(blockIdx.x), TILEXR_DEV_OK, 0};
-            uint32_t stage = 0, phase = 0;
-            for (int t = pair; t < totalTiles && st->abortFlag == 0; t += nPairs) {
-                int mTile, nBlock;
-                FbTileOf(a, t, mTiles, rank, &mTile, &nBlock);
-                const int rowA = mTile * 2 * GEMM_BM + static_cast<int>(ctaRank) * GEMM_BM;
-                const int rowB = nBlock * GEMM_BN + static_cast<int>(ctaRank) * (GEMM_BN / 2);
-                if (a.mode == GEMM_ALL_GATHER) {
-                    // this CTA's 128 rows of the gathered A: wait until their owner has written them here
-                    const int block = rowA / GEMM_BM;
-                    const int shard = block / a.blocksPerShard;
-                    const int64_t slot = FB_FLAG_PLANE_A + static_cast<int64_t>(shard) * a.flagStride + (block - shard * a.blocksPerShard);
-                    if (!WaitFlagGE(w, FlagSlot(a.comm, rank, slot), 1, shard, slot)) {
-                        st->abortFlag = 1;
-                        break;
-                    }
-                    fence_proxy_async();       // the rows were written by generic-proxy stores, TMA reads them next
+        // ---- TMA producer (the warp runs whole and elects a lane to issue, see ElectOne) ----------------------------
+        const uint64_t budgetNs = fused ? a.comm->waitTimeoutNs : 4000000000ull;
+        const int rank = fused ? a.comm->rank : 0;
+        Waiter w{fused ? a.comm : nullptr, st->epoch, static_cast<int32_t>(blockIdx.x), TILEXR_DEV_OK, 0};
+        uint32_t stage = 0, phase = 0;
+        for (int t = pair; t < totalTiles && __all_sync(0xffffffffu, st->abortFlag == 0); t += nPairs) {
+            int mTile, nBlock;
+            FbTileOf(a, t, mTiles, rank, &mTile, &nBlock);
+            const int rowA = mTile * 2 * GEMM_BM + static_cast<int>(ctaRank) * GEMM_BM;
+            const int rowB = nBlock * GEMM_BN + static_cast<int>(ctaRank) * (GEMM_BN / 2);
+            if (MODE == GEMM_ALL_GATHER) {
+                // this CTA's 128 rows of the gathered A: wait until their owner has written them here
+                const int block = rowA / GEMM_BM;
+                const int shard = block / a.blocksPerShard;
+                const int64_t slot = FB_FLAG_PLANE_A + static_cast<int64_t>(shard) * a.flagStride + (block - shard * a.blocksPerShard);
+                bool landed = true;
+                if (lane == 0) landed = WaitFlagGE(w, FlagSlot(a.comm, rank, slot), 1, shard, slot);
+                if (!__all_sync(0xffffffffu, landed)) {
+                    st->abortFlag = 1;
+                    break;
                 }
-                bool broke = false;
-                for (int kb = 0; kb < a.kBlocks; ++kb) {
-                    if (!FbWaitBar(&st->empty[stage], phase ^ 1u, st, peerAbortAddr, budgetNs)) {
-                        broke = true;
-                        break;
-                    }
+                __syncwarp();              // the rows lane 0 acquired are there for the lane that issues
+                fence_proxy_async();       // the rows were written by generic-proxy stores, TMA reads them next
+            }
+            bool broke = false;
+            for (int kb = 0; kb < a.kBlocks; ++kb) {
+                if (!FbWaitBarWarp(&st->empty[stage], phase ^ 1u, st, peerAbortAddr, budgetNs)) {
+                    broke = true;
+                    break;
+                }
+                if (ElectOne()) {
                     uint8_t *sa = stageBase + stage * GEMM_PAIR_STAGE_BYTES;
                     uint8_t *sb = sa + GEMM_STAGE_A_BYTES;
                     if (leader) MbarExpectTx(&st->full[stage], 2 * GEMM_PAIR_STAGE_BYTES);
                     FbTmaLoad(sa, &a.tmapA, kb * 128, rowA, &st->full[stage]);       // x in bytes = elements: a multiple of 128
                     FbTmaLoad(sb, &a.tmapB, kb * 128, rowB, &st->full[stage]);
-                    if (++stage == GEMM_FP8_BLOCK_STAGES) {
-                        stage = 0;
-                        phase ^= 1u;
-                    }
                 }
-                if (broke) break;
+                if (++stage == GEMM_FP8_BLOCK_STAGES) {
+                    stage = 0;
+                    phase ^= 1u;
+                }
             }
+            if (broke) break;
         }
     } else if (warp == 1) {
-        // ---- MMA issuer: per block of K, one N = 128 group into each scratch accumulator ----------------------------
-        if (leader && lane == 0) {
+        // ---- MMA issuer: per block of K, four N = 256 instructions into the scratch of its parity --------------------
+        if (leader) {
             const uint64_t budgetNs = fused ? a.comm->waitTimeoutNs : 4000000000ull;
             const uint32_t idesc = FbInstrDesc(a.fp8Format);
+            const uint64_t descA0 = FbSmemDesc(SmemAddr(stageBase));
+            const uint64_t descB0 = FbSmemDesc(SmemAddr(stageBase) + GEMM_STAGE_A_BYTES);
             uint32_t stage = 0, phase = 0;
-            uint32_t sPhase = 0;                   // bit s: parity of the next wait on scratchEmpty[s]
-            int kbAll = 0;                         // blocks of K issued so far, over all tiles: scratch buffers alternate with it
-            for (int t = pair; t < totalTiles && st->abortFlag == 0; t += nPairs) {
+            uint32_t kbAll = 0;                    // blocks of K issued so far, over all tiles: the scratch buffers alternate with it
+            for (int t = pair; t < totalTiles && __all_sync(0xffffffffu, st->abortFlag == 0); t += nPairs) {
                 bool broke = false;
-                for (int kb = 0; kb < a.kBlocks && !broke; ++kb, ++kbAll) {
-                    if (!FbWaitBar(&st->full[stage], phase, st, peerAbortAddr, budgetNs)) {
+                for (int kb = 0; kb < a.kBlocks; ++kb, ++kbAll) {
+                    const uint32_t p = kbAll & 1u;
+                    if (!FbWaitBarWarp(&st->full[stage], phase, st, peerAbortAddr, budgetNs) ||
+                        !FbWaitBarWarp(&st->scratchEmpty[p], ((kbAll >> 1) & 1u) ^ 1u, st, peerAbortAddr, budgetNs)) {
                         broke = true;
                         break;
                     }
-                    const uint32_t sa = SmemAddr(stageBase + stage * GEMM_PAIR_STAGE_BYTES);
-                    const uint64_t descA = FbSmemDesc(sa);
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const int sIdx = (kbAll & 1) * 2 + h;
-                        if (!FbWaitBar(&st->scratchEmpty[sIdx], ((sPhase >> sIdx) & 1u) ^ 1u, st, peerAbortAddr, budgetNs)) {
-                            broke = true;
-                            break;
-                        }
-                        sPhase ^= 1u << sIdx;
-                        FbFenceAfter();
-                        // rows h*64 .. h*64+63 of this CTA's 128 rows of B (and the same rows of the other CTA's half)
-                        const uint64_t descB = FbSmemDesc(sa + GEMM_STAGE_A_BYTES + static_cast<uint32_t>(h) * 64u * 128u);
-                        const uint32_t tmemD = tmemBase + static_cast<uint32_t>(sIdx) * FB_HALF_N;
+                    FbFenceAfter();
+                    if (ElectOne()) {
+                        const uint64_t descA = descA0 + static_cast<uint64_t>(stage * (GEMM_PAIR_STAGE_BYTES >> 4));
+                        const uint64_t descB = descB0 + static_cast<uint64_t>(stage * (GEMM_PAIR_STAGE_BYTES >> 4));
+                        const uint32_t tmemD = tmemBase + p * GEMM_BN;
 #pragma unroll
                         for (int k = 0; k < 4; ++k) {       // 32 elements of K (32 bytes) per instruction: +2 descriptor units
                             FbUmma(tmemD, descA + static_cast<uint64_t>(k * 2), descB + static_cast<uint64_t>(k * 2), idesc, k != 0 ? 1u : 0u);
                         }
-                        FbCommitPair(&st->scratchFull[sIdx]);
+                        FbCommitPair(&st->scratchFull[p]);
+                        FbCommitPair(&st->empty[stage]);
                     }
-                    if (broke) break;
-                    FbCommitPair(&st->empty[stage]);
                     if (++stage == GEMM_FP8_BLOCK_STAGES) {
                         stage = 0;
                         phase ^= 1u;
@@ -436,7 +449,7 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
                 if (broke) break;
             }
         }
-    } else if (a.mode == GEMM_ALL_GATHER && ok) {
+    } else if (MODE == GEMM_ALL_GATHER && ok) {
         // ---- warps 2-3: write this rank's shard, rows and scales, into every rank's staging buffers -------------------
         const int pt2 = static_cast<int>(threadIdx.x) - 64;           // 0..63
         const int rank = a.comm->rank, ranks = a.comm->rankSize;
@@ -473,20 +486,17 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
         }
     }
     } else {
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 200;" ::: "memory");
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 208;" ::: "memory");
         // ---- promoters: warps 4-7 own column half 0, warps 8-11 half 1; TMEM lanes 32 * (warp % 4) .. + 31 --------------
         const int quad = warp & 3;
         const int h = (warp - 4) >> 2;
         const int myRow = quad * 32 + lane;                       // row of this CTA's 128-row sub-tile
         const int pt = static_cast<int>(threadIdx.x) - 128;       // 0..255 among the promoter threads
-        __shared__ int sGot[8];
         __shared__ int sExit;
         __shared__ float sScaleB[2 * FB_MAX_KB];
-        uint32_t fPhase = 0;                       // bit p: parity of the next wait on this half's scratch buffer p
-        int kbAll = 0;
+        uint32_t kbAll = 0;                        // as the issuer counts it: scratch kbAll & 1, its (kbAll >> 1)-th use
         const int KB = a.kBlocks;
-        const bool vec4 = (KB & 3) == 0;           // rows of the scale tables are 16-byte aligned: four blocks per load
-        const bool gathered = a.mode == GEMM_ALL_GATHER;
+        const bool gathered = MODE == GEMM_ALL_GATHER;
         const uint64_t budgetNs = fused ? a.comm->waitTimeoutNs : 4000000000ull;
         for (int t = pair; t < totalTiles; t += nPairs) {
             int mTile, nBlock;
@@ -495,7 +505,7 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
             const int64_t gRow = row0 + myRow;
             const bool rowValid = gRow < a.M;
             const float *saRow = a.scaleA + (rowValid ? gRow : 0) * KB;
-            // scale blocks of B for the two 64-column groups of this scratch accumulator
+            // scale blocks of B for the two column halves
             const int nb0 = min(nBlock * 2, a.scaleBRows - 1);
             const int nb1 = min(nBlock * 2 + 1, a.scaleBRows - 1);
             const float *sb0 = a.scaleB + static_cast<int64_t>(nb0) * KB;
@@ -504,8 +514,8 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
 #pragma unroll
             for (int j = 0; j < FB_HALF_N; ++j) acc[j] = 0.f;
             // The weight's scales of this tile (two rows of the table) go to shared memory once per tile; the activation
-            // scales of the thread's row travel four blocks of K at a time and one group ahead of their use, so that
-            // their latency (an L2 round trip, longer than one block's work) never shows.
+            // scale of the thread's row is fetched two blocks of K ahead of its use, so that its latency (an L2 round
+            // trip where it is not in L1, about one block's work) does not show.
             asm volatile("bar.sync 1, 256;" ::: "memory");          // the previous tile's readers are done with sScaleB
             for (int i = pt; i < 2 * KB && i < 2 * FB_MAX_KB; i += 256) {
                 sScaleB[i] = __ldg((i < KB ? sb0 + i : sb1 + (i - KB)));
@@ -522,67 +532,38 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
             }
             asm volatile("bar.sync 1, 256;" ::: "memory");
             const bool bInSmem = KB <= FB_MAX_KB;
-            float4 curA = make_float4(0.f, 0.f, 0.f, 0.f), nxtA = curA;
-            auto loadGroup = [&](int kb0, float4 &ga) {
-                if (!rowValid) {
-                    ga = make_float4(0.f, 0.f, 0.f, 0.f);
-                } else if (gathered) {
-                    // written during this launch: through L2, never through the read-only path
-                    if (vec4) {
-                        ga = __ldcg(reinterpret_cast<const float4 *>(saRow + kb0));
-                    } else {
-                        ga = make_float4(__ldcg(saRow + min(kb0, KB - 1)), __ldcg(saRow + min(kb0 + 1, KB - 1)), __ldcg(saRow + min(kb0 + 2, KB - 1)),
-                                         __ldcg(saRow + min(kb0 + 3, KB - 1)));
-                    }
-                } else if (vec4) {
-                    ga = __ldg(reinterpret_cast<const float4 *>(saRow + kb0));
-                } else {
-                    ga = make_float4(__ldg(saRow + min(kb0, KB - 1)), __ldg(saRow + min(kb0 + 1, KB - 1)), __ldg(saRow + min(kb0 + 2, KB - 1)),
-                                     __ldg(saRow + min(kb0 + 3, KB - 1)));
-                }
-            };
-            loadGroup(0, curA);
-            bool alive = true;
+            // written during this launch in the all-gather mode: through L2, never through the read-only path
+            auto loadA = [&](int kb) { return !rowValid ? 0.f : gathered ? __ldcg(saRow + min(kb, KB - 1)) : __ldg(saRow + min(kb, KB - 1)); };
+            float sa0 = loadA(0), sa1 = loadA(1);
+            const float *sbHalf = h == 0 ? sb0 : sb1;
+            const float *sbShared = sScaleB + h * KB;
             for (int kb = 0; kb < KB; ++kb) {
-                const int q = kb & 3;
-                if (q == 0 && kb + 4 < KB) loadGroup(kb + 4, nxtA);
-                const float saq = q == 0 ? curA.x : q == 1 ? curA.y : q == 2 ? curA.z : curA.w;
-                const int p = kbAll & 1;
-                const int sIdx = p * 2 + h;
+                const float f = sa0 * (bInSmem ? sbShared[kb] : __ldg(sbHalf + kb));
+                sa0 = sa1;
+                sa1 = loadA(kb + 2);
+                const uint32_t p = kbAll & 1u;
+                if (!FbWaitBarWarp(&st->scratchFull[p], (kbAll >> 1) & 1u, st, peerAbortAddr, budgetNs)) break;
                 ++kbAll;
-                bool got = true;
-                if (lane == 0) {
-                    got = FbWaitBar(&st->scratchFull[sIdx], (fPhase >> p) & 1u, st, peerAbortAddr, budgetNs);
-                    sGot[warp - 4] = got ? 1 : 0;
-                }
-                __syncwarp();
-                if (sGot[warp - 4] == 0) {
-                    alive = false;
-                    break;
-                }
-                __syncwarp();
-                fPhase ^= 1u << p;
                 FbFenceAfter();
-                const float f0 = saq * (bInSmem ? sScaleB[kb] : __ldg(sb0 + kb));
-                const float f1 = saq * (bInSmem ? sScaleB[KB + kb] : __ldg(sb1 + kb));
+                const uint32_t taddr = tmemBase + (static_cast<uint32_t>(quad * 32) << 16) + p * GEMM_BN + static_cast<uint32_t>(h * FB_HALF_N);
+                // Sixteen columns at a time, the next ones on their way while these are folded (8192^3: 8 columns 538 us,
+                // 16 columns 523 us, 32 columns 565 us, before the modes had kernels of their own).
+                uint32_t r[2][16];
+                FbTmemLoad16(taddr, r[0]);
 #pragma unroll
-                for (int cc = 0; cc < 4; cc += 2) {
-                    uint32_t r0[32], r1[32];
-                    const uint32_t taddr = tmemBase + (static_cast<uint32_t>(quad * 32) << 16) + static_cast<uint32_t>(sIdx * FB_HALF_N + cc * 32);
-                    FbTmemLoad32(taddr, r0);
-                    FbTmemLoad32(taddr + 32, r1);
-                    FbTmemLoadWait();
-                    const float f = cc < 2 ? f0 : f1;
+                for (int cc = 0; cc < 8; ++cc) {
+                    FbTmemLoadWait16(r[cc & 1]);
+                    if (cc < 7) {
+                        FbTmemLoad16(taddr + (cc + 1) * 16, r[(cc + 1) & 1]);
+                    } else {
+                        // the half is in registers: the issuer may overwrite it two blocks of K from now
+                        FbFenceBefore();
+                        __syncwarp();
+                        if (lane == 0) FbArriveCluster(SmemAddr(&st->scratchEmpty[p]) & FB_PEER_BIT_MASK);
+                    }
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) acc[cc * 32 + j] = fmaf(__uint_as_float(r0[j]), f, acc[cc * 32 + j]);
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) acc[(cc + 1) * 32 + j] = fmaf(__uint_as_float(r1[j]), f, acc[(cc + 1) * 32 + j]);
+                    for (int j = 0; j < 16; ++j) acc[cc * 16 + j] = fmaf(__uint_as_float(r[cc & 1][j]), f, acc[cc * 16 + j]);
                 }
-                // the scratch accumulator is read out: the MMA lane may overwrite it two blocks of K from now
-                FbFenceBefore();
-                __syncwarp();
-                if (lane == 0) FbArriveCluster(SmemAddr(&st->scratchEmpty[sIdx]) & FB_PEER_BIT_MASK);
-                if (q == 3) curA = nxtA;
             }
             // All eight promoter warps of the CTA arrive here whether or not their waits succeeded, and leave the tile
             // loop together: the store below uses block-wide barriers, which a lone warp must never reach.
@@ -590,22 +571,30 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
             if (pt == 0) sExit = (st->abortFlag != 0) ? 1 : 0;
             asm volatile("bar.sync 1, 256;" ::: "memory");
             if (sExit != 0) break;
-            (void)alive;
-            // ---- store the tile: the two groups take turns with the staging tile, everybody stores ---------------------
-            int rowsValid = static_cast<int>(max(static_cast<int64_t>(0), min(static_cast<int64_t>(GEMM_BM), a.M - row0)));
-            uint8_t *rowBase = a.c + static_cast<uint64_t>(row0) * a.N * 2;
-            int owner = 0, tileLocal = 0;
-            if (a.mode == GEMM_REDUCE_SCATTER) {
-                // the partial tile goes into the row owner's staging slot for this rank
-                const int block = static_cast<int>(row0 / GEMM_BM);
-                owner = block / a.blocksPerShard;
-                const int localBlock = block - owner * a.blocksPerShard;
-                tileLocal = localBlock * a.nBlocks + nBlock;
-                rowBase = a.comm->registryPtr->regions[a.outHandle].peerBase[owner] + a.outOffset +
-                          (static_cast<uint64_t>(a.comm->rank) * a.shardRows + static_cast<uint64_t>(localBlock) * GEMM_BM) * a.N * 2;
-                rowsValid = GEMM_BM;
-            }
             const int col0 = nBlock * GEMM_BN;
+            if (MODE != GEMM_REDUCE_SCATTER) {
+                // Local memory: every thread stores its 256 bytes of a row straight from registers, without the two trips
+                // of the tile through shared memory and their barriers (the issuer has only two blocks of K of work ahead).
+                if (rowValid) {
+                    uint8_t *rowPtr = a.c + (static_cast<uint64_t>(gRow) * a.N + col0 + h * FB_HALF_N) * 2;
+#pragma unroll
+                    for (int v = 0; v < 16; ++v) {
+                        if (col0 + h * FB_HALF_N + v * 8 < a.N) {
+                            st_vec16(rowPtr + v * 16, Vec16{FbPackPair(acc[8 * v], acc[8 * v + 1], bf16), FbPackPair(acc[8 * v + 2], acc[8 * v + 3], bf16),
+                                                            FbPackPair(acc[8 * v + 4], acc[8 * v + 5], bf16), FbPackPair(acc[8 * v + 6], acc[8 * v + 7], bf16)});
+                        }
+                    }
+                }
+                continue;
+            }
+            // ---- the partial tile goes into the row owner's staging slot for this rank, behind NVLink: through a swizzled
+            // staging tile, so that every warp store covers whole row pieces; the two groups take turns with it ----------
+            const int block = static_cast<int>(row0 / GEMM_BM);
+            const int owner = block / a.blocksPerShard;
+            const int localBlock = block - owner * a.blocksPerShard;
+            const int tileLocal = localBlock * a.nBlocks + nBlock;
+            uint8_t *rowBase = a.comm->registryPtr->regions[a.outHandle].peerBase[owner] + a.outOffset +
+                               (static_cast<uint64_t>(a.comm->rank) * a.shardRows + static_cast<uint64_t>(localBlock) * GEMM_BM) * a.N * 2;
 #pragma unroll 1
             for (int pass = 0; pass < 2; ++pass) {
                 if (h == pass) {
@@ -623,16 +612,15 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
                     const int idx = pt + k * 256;
                     const int rr = idx >> 4;
                     const int ch = idx & 15;
-                    // chunk ch of scratch `pass`: columns pass*64 + ch*8 (first group) or 128 + pass*64 + (ch-8)*8
-                    const int col = col0 + (ch < 8 ? pass * 64 + ch * 8 : 128 + pass * 64 + (ch - 8) * 8);
-                    if (rr < rowsValid && col < a.N) {
+                    const int col = col0 + pass * FB_HALF_N + ch * 8;
+                    if (col < a.N) {
                         const uint4 v = *reinterpret_cast<const uint4 *>(stageC + rr * 256 + ((ch ^ (rr & 15)) * 16));
                         st_vec16(rowBase + static_cast<uint64_t>(rr) * a.N * 2 + static_cast<uint64_t>(col) * 2, Vec16{v.x, v.y, v.z, v.w});
                     }
                 }
                 asm volatile("bar.sync 1, 256;" ::: "memory");
             }
-            if (a.mode == GEMM_REDUCE_SCATTER && pt == 0) {
+            if (pt == 0) {
                 // all 256 promoter threads have stored (the barrier above): order their stores, then tell the owner
                 fence_acq_rel_sys();
                 st_relaxed_sys_u64(FlagSlot(a.comm, owner, FB_FLAG_PLANE_B + static_cast<int64_t>(a.comm->rank) * a.flagStride + tileLocal),
@@ -640,7 +628,7 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
             }
         }
         // ---- reduce-scatter: add the partial tiles of the output tiles this CTA owns, in rank order ---------------------
-        if (a.mode == GEMM_REDUCE_SCATTER) {
+        if (MODE == GEMM_REDUCE_SCATTER) {
             const int owned = a.blocksPerShard * a.nBlocks;
             const int rank = a.comm->rank, ranks = a.comm->rankSize;
             const uint32_t epoch = st->epoch;
@@ -723,15 +711,26 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
     }
 }
 
+template <int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_FP8_BLOCK_THREADS, 1)
-TileXRGemmFp8BlockScaled(const __grid_constant__ GemmBlockArgs a) { FbBody(a); }
+TileXRGemmFp8BlockScaled(const __grid_constant__ GemmBlockArgs a) { FbBody<MODE>(a); }
 // Emulated worlds: one argument block per rank in global memory, rank = blockIdx.y.
+template <int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_FP8_BLOCK_THREADS, 1)
-TileXRGemmFp8BlockScaled_emulated(const GemmBlockArgs *perRank) { FbBody(perRank[blockIdx.y]); }
+TileXRGemmFp8BlockScaled_emulated(const GemmBlockArgs *perRank) { FbBody<MODE>(perRank[blockIdx.y]); }
 
 } // namespace
 
-const void *GemmFp8BlockKernel() { return reinterpret_cast<const void *>(&TileXRGemmFp8BlockScaled); }
-const void *GemmFp8BlockKernelEmulated() { return reinterpret_cast<const void *>(&TileXRGemmFp8BlockScaled_emulated); }
+const void *GemmFp8BlockKernel(int mode)
+{
+    return mode == GEMM_ALL_GATHER       ? reinterpret_cast<const void *>(&TileXRGemmFp8BlockScaled<GEMM_ALL_GATHER>)
+           : mode == GEMM_REDUCE_SCATTER ? reinterpret_cast<const void *>(&TileXRGemmFp8BlockScaled<GEMM_REDUCE_SCATTER>)
+                                         : reinterpret_cast<const void *>(&TileXRGemmFp8BlockScaled<GEMM_PLAIN>);
+}
+const void *GemmFp8BlockKernelEmulated(int mode)
+{
+    return mode == GEMM_ALL_GATHER ? reinterpret_cast<const void *>(&TileXRGemmFp8BlockScaled_emulated<GEMM_ALL_GATHER>)
+                                   : reinterpret_cast<const void *>(&TileXRGemmFp8BlockScaled_emulated<GEMM_REDUCE_SCATTER>);
+}
 
 } // namespace TileXR
