@@ -634,6 +634,8 @@ int TileXRAllGatherMatmulFp8Block(const void *aShard, const float *scaleAShard, 
     }
     ret = MakeMap8(&g.tmapA, aStaging, m, k, GEMM_BM);
     if (ret != TILEXR_SUCCESS) return ret;
+    ret = MakeMap8(&g.tmapALocal, aShard, shardRows, k, GEMM_BM);
+    if (ret != TILEXR_SUCCESS) return ret;
     g.scaleA = scaleStaging;
     g.c = static_cast<uint8_t *>(c);
     g.mode = GEMM_ALL_GATHER;

@@ -85,6 +85,7 @@ constexpr size_t GEMM_FP8_BLOCK_SMEM_BYTES = 1024 /* alignment slack */ + GEMM_F
 
 struct GemmBlockArgs {
     CUtensorMap tmapA;        // A [M, K] 8-bit, box 128 rows x 128 bytes
+    CUtensorMap tmapALocal;   // all-gather: this rank's shard [shardRows, K]
     CUtensorMap tmapB;        // B [N, K] 8-bit, box 128 rows x 128 bytes
     const float *scaleA;      // [M, K / 128]
     const float *scaleB;      // [scaleBRows, K / 128], one row per 128 rows of B
@@ -99,7 +100,8 @@ struct GemmBlockArgs {
     int32_t fp8Format;        // 1 = e4m3, 2 = e5m2
     // Fused modes (GemmMode).  ALL_GATHER: tmapA and scaleA describe THIS rank's staging buffers ([R * shardRows, K] rows,
     // [R * shardRows, K / 128] scales, both registered on every rank); every rank writes its shard and the shard's
-    // scales into all of them while the tiles are computed, and a tile starts when the flag of its 128 rows is up.
+    // scales into all of them while the tiles are computed, and a tile of a peer's rows starts when the flag of its 128
+    // rows is up (its own rows are read from the shard).
     // REDUCE_SCATTER: every 128 x 256 partial tile is stored into the row owner's partial staging buffer
     // ([R, shardRows, N] 16-bit, registered) and the owner adds the R partials in rank order into c [shardRows, N].
     int32_t mode;

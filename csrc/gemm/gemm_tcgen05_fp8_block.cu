@@ -32,9 +32,11 @@
 //                   scales) into all ranks' staging buffers, 128 rows at a time, and raise the piece's flag: through
 //                   the NVLink multicast alias of the staging buffer where the runtime has one (multimem.st: one
 //                   store, the switch replicates it), else with one store per peer.  No SM is set aside for
-//                   communication.  The TMA lane of a CTA acquires the flag of its 128 rows before the first load of a
+//                   communication.  The TMA warp of a CTA acquires the flag of its 128 rows before the first load of a
 //                   tile (TMA then reads LOCAL memory, without multicast); each promoter warp acquires it before it
-//                   reads the rows' scales.  Every rank walks the shards starting with its own.
+//                   reads the rows' scales.  Every rank walks the shards starting with its own, whose rows and scales it
+//                   reads where they are: waiting for its own copy of them cost 90 us at 2048 x 4096 on one rank.  That
+//                   copy is made last, in slices of all CTAs, since nobody waits for it.
 //   GEMM -> reduce-scatter    the promoters store their 128 x 256 partial tile into the row owner's staging slot and
 //                   raise the tile's flag; when a CTA has run out of tiles its promoters add, in rank order, the
 //                   R partial tiles of the output tiles it owns.  Every rank starts with the rows of the next rank
@@ -377,13 +379,15 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
             FbTileOf(a, t, mTiles, rank, &mTile, &nBlock);
             const int rowA = mTile * 2 * GEMM_BM + static_cast<int>(ctaRank) * GEMM_BM;
             const int rowB = nBlock * GEMM_BN + static_cast<int>(ctaRank) * (GEMM_BN / 2);
+            bool own = false;              // the rows are this rank's shard
             if (MODE == GEMM_ALL_GATHER) {
                 // this CTA's 128 rows of the gathered A: wait until their owner has written them here
                 const int block = rowA / GEMM_BM;
                 const int shard = block / a.blocksPerShard;
                 const int64_t slot = FB_FLAG_PLANE_A + static_cast<int64_t>(shard) * a.flagStride + (block - shard * a.blocksPerShard);
                 bool landed = true;
-                if (lane == 0) landed = WaitFlagGE(w, FlagSlot(a.comm, rank, slot), 1, shard, slot);
+                own = shard == rank;
+                if (lane == 0 && !own) landed = WaitFlagGE(w, FlagSlot(a.comm, rank, slot), 1, shard, slot);
                 if (!__all_sync(0xffffffffu, landed)) {
                     st->abortFlag = 1;
                     break;
@@ -391,6 +395,8 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
                 __syncwarp();              // the rows lane 0 acquired are there for the lane that issues
                 fence_proxy_async();       // the rows were written by generic-proxy stores, TMA reads them next
             }
+            const CUtensorMap *mapA = own ? &a.tmapALocal : &a.tmapA;
+            const int yA = own ? rowA - rank * a.shardRows : rowA;
             bool broke = false;
             for (int kb = 0; kb < a.kBlocks; ++kb) {
                 if (!FbWaitBarWarp(&st->empty[stage], phase ^ 1u, st, peerAbortAddr, budgetNs)) {
@@ -401,7 +407,7 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
                     uint8_t *sa = stageBase + stage * GEMM_PAIR_STAGE_BYTES;
                     uint8_t *sb = sa + GEMM_STAGE_A_BYTES;
                     if (leader) MbarExpectTx(&st->full[stage], 2 * GEMM_PAIR_STAGE_BYTES);
-                    FbTmaLoad(sa, &a.tmapA, kb * 128, rowA, &st->full[stage]);       // x in bytes = elements: a multiple of 128
+                    FbTmaLoad(sa, mapA, kb * 128, yA, &st->full[stage]);       // x in bytes = elements: a multiple of 128
                     FbTmaLoad(sb, &a.tmapB, kb * 128, rowB, &st->full[stage]);
                 }
                 if (++stage == GEMM_FP8_BLOCK_STAGES) {
@@ -459,12 +465,12 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
         uint8_t *mcScales = reg->regions[a.sHandle].mcBase;
         const bool multicast = ranks > 1 && mcRows != nullptr && mcScales != nullptr;
         const int pieces = a.blocksPerShard;
-        const int items = multicast ? pieces : ranks * pieces;
+        const int items = multicast ? pieces : (ranks - 1) * pieces;
         const uint64_t rowBytes = static_cast<uint64_t>(a.K);
         const uint64_t scaleRowBytes = static_cast<uint64_t>(a.kBlocks) * 4;
         for (int it = blockIdx.x; it < items; it += gridDim.x) {
             const int piece = it % pieces;
-            const int peer = (rank - it / pieces + ranks) % ranks;          // itself first, then rank-1 (which needs it next), ...
+            const int peer = (rank - 1 - it / pieces + ranks) % ranks;      // rank-1 needs it first
             const uint64_t srcRow = static_cast<uint64_t>(piece) * GEMM_BM;
             const uint64_t dstRow = static_cast<uint64_t>(rank) * a.shardRows + srcRow;
             uint8_t *rowsTo = (multicast ? mcRows : reg->regions[a.aHandle].peerBase[peer]) + a.aOffset + dstRow * rowBytes;
@@ -483,6 +489,18 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
                 }
             }
             asm volatile("bar.sync 2, 64;" ::: "memory");
+        }
+        if (!multicast) {
+            // the caller finds all rows in its staging buffers, its own among them: a slice of them per CTA, no flags
+            auto slice = [&](uint8_t *dst, const uint8_t *src, uint64_t bytes) {
+                const uint64_t per = ((bytes / 16 + gridDim.x - 1) / gridDim.x) * 16;
+                const uint64_t b0 = min(bytes, per * blockIdx.x);
+                FbPush(dst + b0, src + b0, min(bytes - b0, per), pt2, 64, false);
+            };
+            const uint64_t myRow = static_cast<uint64_t>(rank) * a.shardRows;
+            slice(reg->regions[a.aHandle].peerBase[rank] + a.aOffset + myRow * rowBytes, a.aLocal, a.shardRows * rowBytes);
+            slice(reg->regions[a.sHandle].peerBase[rank] + a.sOffset + myRow * scaleRowBytes, reinterpret_cast<const uint8_t *>(a.scaleALocal),
+                  a.shardRows * scaleRowBytes);
         }
     }
     } else {
@@ -505,6 +523,11 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
             const int64_t gRow = row0 + myRow;
             const bool rowValid = gRow < a.M;
             const float *saRow = a.scaleA + (rowValid ? gRow : 0) * KB;
+            bool wait = gathered;                  // the scales of these rows come from a peer during this launch
+            if (gathered && row0 / a.shardRows == a.comm->rank) {
+                saRow = a.scaleALocal + (gRow - static_cast<int64_t>(a.comm->rank) * a.shardRows) * KB;
+                wait = false;
+            }
             // scale blocks of B for the two column halves
             const int nb0 = min(nBlock * 2, a.scaleBRows - 1);
             const int nb1 = min(nBlock * 2 + 1, a.scaleBRows - 1);
@@ -520,7 +543,7 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
             for (int i = pt; i < 2 * KB && i < 2 * FB_MAX_KB; i += 256) {
                 sScaleB[i] = __ldg((i < KB ? sb0 + i : sb1 + (i - KB)));
             }
-            if (gathered) {
+            if (wait) {
                 // the scales of these 128 rows were written by their owner during this launch: acquire the rows' flag first
                 if (lane == 0) {
                     const int block = static_cast<int>(row0 / GEMM_BM);
