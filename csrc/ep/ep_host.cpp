@@ -772,6 +772,24 @@ int TileXRFp8Quant1x128(const void *x, int64_t rows, int64_t h, TileXRDataType d
     return LaunchFp8Quant1x128(x, rows, h, dtype == TILEXR_DATA_TYPE_BFP16, yOut, scalesOut, stream);
 }
 
+int TileXRSwiglu(const void *gateUp, int64_t rows, int64_t f, TileXRDataType dtype, void *yOut, TileXRStream stream)
+{
+    if (gateUp == nullptr || yOut == nullptr || rows <= 0 || f <= 0 || f % 8 != 0 || f > INT32_MAX || !HalfType(dtype)) {
+        return TILEXR_ERROR_PARA_CHECK_FAIL;
+    }
+    return LaunchSwiglu(gateUp, rows, f, dtype == TILEXR_DATA_TYPE_BFP16, yOut, nullptr, stream);
+}
+
+int TileXRSwigluFp8Quant1x128(const void *gateUp, int64_t rows, int64_t f, TileXRDataType dtype, void *yOut, float *scalesOut,
+                              TileXRStream stream)
+{
+    if (gateUp == nullptr || yOut == nullptr || scalesOut == nullptr || rows <= 0 || f <= 0 || f % 128 != 0 || f > INT32_MAX ||
+        !HalfType(dtype)) {
+        return TILEXR_ERROR_PARA_CHECK_FAIL;
+    }
+    return LaunchSwiglu(gateUp, rows, f, dtype == TILEXR_DATA_TYPE_BFP16, yOut, scalesOut, stream);
+}
+
 int TileXRFp8Dequant1x128(const void *y, const float *scales, int64_t rows, int64_t h, TileXRDataType dtype, void *xOut,
                           TileXRStream stream)
 {

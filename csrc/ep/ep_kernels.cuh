@@ -156,6 +156,8 @@ const KernelEntry &EpCombineKernelEntry();
 
 // Plain (non communicating) kernels, launched directly.
 int LaunchRoutingTopK(const RoutingArgs &args, void *stream);
+// rows [gate | up] -> silu(gate) * up; with `scales` quantised to e4m3 per 128 elements (f % 128 == 0), else f % 8 == 0
+int LaunchSwiglu(const void *gateUp, int64_t rows, int64_t f, bool bf16, void *y, float *scales, void *stream);
 int LaunchFp8Quant1x128(const void *x, int64_t rows, int64_t h, bool bf16, void *y, float *scales, void *stream);
 int LaunchFp8Dequant1x128(const void *y, const float *scales, int64_t rows, int64_t h, bool bf16, void *x, void *stream);
 int LaunchMxfp8Quant(const void *x, int64_t rows, int64_t h, bool bf16, bool e5m2, void *y, uint8_t *scales, void *stream);

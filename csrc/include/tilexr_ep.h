@@ -190,6 +190,11 @@ int TileXRMoeRoutingTopK(const float *gateLogits, const float *selectionBias, in
 // Block-scaled fp8: y = e4m3(x / s), s = max(amax over 128 elements, 1e-4) / 448, scales fp32 [rows, h/128].
 int TileXRFp8Quant1x128(const void *x, int64_t rows, int64_t h, TXR_DT dtype, void *yOut, float *scalesOut,
                         TileXRStream stream);
+// gateUp [rows, 2 * f] with the gate columns first: y[rows, f] = silu(gate) * up, computed in fp32 and rounded to `dtype`
+// (f a multiple of 8), or that result quantised as TileXRFp8Quant1x128 does (f a multiple of 128) without its trip through memory.
+int TileXRSwiglu(const void *gateUp, int64_t rows, int64_t f, TXR_DT dtype, void *yOut, TileXRStream stream);
+int TileXRSwigluFp8Quant1x128(const void *gateUp, int64_t rows, int64_t f, TXR_DT dtype, void *yOut, float *scalesOut,
+                              TileXRStream stream);
 int TileXRFp8Dequant1x128(const void *y, const float *scales, int64_t rows, int64_t h, TXR_DT dtype, void *xOut,
                           TileXRStream stream);
 // MXFP8 (OCP microscaling): 32-element blocks, shared E8M0 exponent, e4m3 or e5m2 elements

@@ -559,6 +559,29 @@ py::tuple Fp8Quant(const at::Tensor &x)
     return py::make_tuple(y, s);
 }
 
+at::Tensor Swiglu(const at::Tensor &gateUp)
+{
+    TORCH_CHECK(gateUp.is_cuda() && gateUp.dim() == 2 && gateUp.is_contiguous() && gateUp.size(1) % 2 == 0,
+                "gate_up must be a contiguous [rows, 2 * f] CUDA tensor");
+    const int64_t f = gateUp.size(1) / 2;
+    at::Tensor y = at::empty({gateUp.size(0), f}, gateUp.options());
+    Check(TileXRSwiglu(gateUp.data_ptr(), gateUp.size(0), f, ToDtype(gateUp.scalar_type()), y.data_ptr(), StreamOf(gateUp)), "TileXRSwiglu");
+    return y;
+}
+
+py::tuple SwigluFp8Quant(const at::Tensor &gateUp)
+{
+    TORCH_CHECK(gateUp.is_cuda() && gateUp.dim() == 2 && gateUp.is_contiguous() && gateUp.size(1) % 256 == 0,
+                "gate_up must be a contiguous [rows, 2 * f] CUDA tensor with f a multiple of 128");
+    const int64_t f = gateUp.size(1) / 2;
+    at::Tensor y = at::empty({gateUp.size(0), f}, gateUp.options().dtype(at::kFloat8_e4m3fn));
+    at::Tensor s = at::empty({gateUp.size(0), f / 128}, gateUp.options().dtype(at::kFloat));
+    Check(TileXRSwigluFp8Quant1x128(gateUp.data_ptr(), gateUp.size(0), f, ToDtype(gateUp.scalar_type()), y.data_ptr(), s.data_ptr<float>(),
+                                    StreamOf(gateUp)),
+          "TileXRSwigluFp8Quant1x128");
+    return py::make_tuple(y, s);
+}
+
 at::Tensor Fp8Dequant(const at::Tensor &y, const at::Tensor &scales, at::ScalarType dtype)
 {
     TORCH_CHECK(y.is_cuda() && y.dim() == 2 && y.is_contiguous() && scales.is_contiguous(), "bad fp8 input");
@@ -710,6 +733,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m)
     m.def("routing_topk", &RoutingTopK, py::arg("gate_logits"), py::arg("selection_bias") = py::none(), py::arg("top_k") = 1,
           py::arg("score_func") = 0, py::arg("renormalize") = true, py::arg("routed_scale") = 1.0);
     m.def("fp8_quant_1x128", &Fp8Quant);
+    m.def("swiglu", &Swiglu);
+    m.def("swiglu_fp8_quant_1x128", &SwigluFp8Quant);
     m.def("fp8_dequant_1x128", &Fp8Dequant);
     m.def("mxfp8_quant", &Mxfp8Quant, py::arg("x"), py::arg("e5m2") = false);
     m.def("mxfp8_dequant", &Mxfp8Dequant);

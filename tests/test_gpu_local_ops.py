@@ -1,0 +1,60 @@
+"""Elementwise kernels beside the GEMMs and the exchange, against plain PyTorch at the edges of their tiling."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def txr():
+    import tilexr_b200 as t
+
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    return t
+
+
+def _gate_up(rows, f, dtype, seed=3):
+    g = torch.Generator().manual_seed(seed)
+    x = (torch.randn(rows, 2 * f, generator=g) * 3.0).to(dtype).cuda()
+    x[0, 0], x[0, f] = float("inf"), 2.0          # an infinite gate, a zero, a NaN, a row of zeros
+    x[-1, 1], x[-1, f + 2] = 0.0, float("nan")
+    if rows > 2:
+        x[1] = 0.0
+    return x
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,f", [(1, 8), (3, 24), (33, 40), (257, 128), (1000, 7168)])
+def test_swiglu_matches_the_unfused_form(txr, rows, f, dtype):
+    x = _gate_up(rows, f, dtype)
+    want = (torch.nn.functional.silu(x[:, :f].float()) * x[:, f:].float()).to(dtype)
+    got = txr.quant.swiglu(x)
+    assert got.shape == want.shape and got.dtype == dtype
+    # both round an fp32 value once; the fp32 values may differ in their last bits (exp, the order of * and /), which moves
+    # a rounding by one unit in the last place at most
+    ulp = torch.finfo(dtype).eps
+    finite = torch.isfinite(want)
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
+    diff = (got.float() - want.float()).abs()
+    assert (diff[finite] <= ulp * want.float().abs()[finite] + torch.finfo(dtype).smallest_normal * ulp).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,f", [(1, 128), (3, 384), (31, 896), (1000, 7168)])
+def test_swiglu_fp8_quant_is_the_quantised_swiglu(txr, rows, f, dtype):
+    x = _gate_up(rows, f, dtype)
+    q, s = txr.quant.swiglu_fp8_quant_1x128(x)
+    want_q, want_s = txr.quant.fp8_quant_1x128(txr.quant.swiglu(x))
+    assert torch.equal(q.view(torch.uint8), want_q.view(torch.uint8)) and torch.equal(s, want_s)
+
+
+@pytest.mark.parametrize("rows,h", [(1, 128), (5, 128), (7, 384), (33, 640)])
+def test_fp8_quant_rows_that_do_not_fill_a_warp(txr, rows, h):
+    """A 128-element block is eight threads, wherever its row starts in the launch."""
+    from tilexr_b200.utils import oracle
+
+    x = (torch.randn(rows, h, generator=torch.Generator().manual_seed(rows)) * 5).to(torch.bfloat16)
+    q, s = txr.quant.fp8_quant_1x128(x.cuda())
+    want_q, want_s = oracle.fp8_quant_1x128_ref(x)
+    assert torch.equal(s.cpu(), want_s) and torch.equal(q.cpu().view(torch.uint8), want_q.view(torch.uint8))

@@ -82,8 +82,18 @@ class SequenceParallelMLP(torch.nn.Module):
             gu = self.ops.all_gather_matmul_fp8_block(self.comm, qx, sx, self.stage_rows, self.stage_scales, self.w13, self.s13, cfg.dtype)
         else:
             gu = self.ops.all_gather_matmul(self.comm, x_shard, self.w13, self.stage_rows)
-        act = (torch.nn.functional.silu(gu[:, :self.f_loc].float()) * gu[:, self.f_loc:].float()).to(cfg.dtype)
+        # one pass over the product where the kernels apply; other devices, types and injected quantisers take the plain form
+        native = gu.is_cuda and gu.dtype == cfg.dtype and cfg.dtype in (torch.float16, torch.bfloat16) and self.f_loc % 8 == 0
+        fused_quant = getattr(self.quant, "swiglu_fp8_quant_1x128", None) if native and cfg.fp8_block else None
+        if fused_quant is not None:
+            qa, sa = fused_quant(gu)
+        elif native and not cfg.fp8_block:
+            from ..ops.quant import swiglu
+            act = swiglu(gu)
+        else:
+            act = (torch.nn.functional.silu(gu[:, :self.f_loc].float()) * gu[:, self.f_loc:].float()).to(cfg.dtype)
         if cfg.fp8_block:
-            qa, sa = self.quant.fp8_quant_1x128(act)
+            if fused_quant is None:
+                qa, sa = self.quant.fp8_quant_1x128(act)
             return self.ops.matmul_reduce_scatter_fp8_block(self.comm, qa, sa, self.w2, self.s2, self.stage_out, cfg.dtype)
         return self.ops.matmul_reduce_scatter(self.comm, act, self.w2, self.stage_out)

@@ -16,6 +16,16 @@ def fp8_quant_1x128(x: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
     return _C.fp8_quant_1x128(x.contiguous())
 
 
+def swiglu(gate_up: torch.Tensor) -> torch.Tensor:
+    """``silu(gate) * up`` of ``gate_up`` [rows, 2 * f] (gate columns first; f a multiple of 8), computed in fp32."""
+    return _C.swiglu(gate_up.contiguous())
+
+
+def swiglu_fp8_quant_1x128(gate_up: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
+    """:func:`fp8_quant_1x128` of :func:`swiglu` (f a multiple of 128) in one pass."""
+    return _C.swiglu_fp8_quant_1x128(gate_up.contiguous())
+
+
 def fp8_dequant_1x128(y: torch.Tensor, scales: torch.Tensor, dtype=torch.bfloat16) -> torch.Tensor:
     return _C.fp8_dequant_1x128(y, scales, dtype)
 
