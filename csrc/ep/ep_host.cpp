@@ -336,7 +336,9 @@ int TileXRMoeEpDispatchFused(const TileXREpDispatchParams *p, TileXRCommPtr comm
     // ranks) and the column split of the send side both want the parallelism; blocks may own no token.
     const int64_t capBlocks = std::min<int64_t>(EP_COUNT_FLAG_SLOT - 1, std::max<int64_t>(1, EnvLong("TILEXR_EP_BLOCKS", 296)));
     const int64_t minBlocks = std::min<int64_t>(capBlocks, std::max<int64_t>(1, EnvLong("TILEXR_EP_MIN_BLOCKS", 32)));
-    const int64_t wantBlocks = std::max<int64_t>(minBlocks, std::min<int64_t>((p->bs + 15) / 16, capBlocks));
+    // Four tokens to a block until the cap: a warp per quarter of a row.  With sixteen to a block 1009 tokens sat on 64 of the
+    // 148 SMs, and 4096 tokens left 40 of the 296 places empty.
+    const int64_t wantBlocks = std::max<int64_t>(minBlocks, std::min<int64_t>((p->bs + 3) / 4, capBlocks));
     unsigned grid = static_cast<unsigned>(wantBlocks);
     unsigned gridCap = 0;
     uint32_t tokensPerBlock = 0;
@@ -390,6 +392,7 @@ int TileXRMoeEpDispatchFused(const TileXREpDispatchParams *p, TileXRCommPtr comm
     a.expertTokenNumsOut = p->expertTokenNumsOut;
     a.sendCountsOut = p->sendCountsOut;
     a.recvTotalOut = p->recvTotalOut;
+    a.laneCountOut = p->tpRecvCountsOut;
     a.comm = reinterpret_cast<CommArgs *>(c.devArgs);
     a.bs = static_cast<int32_t>(p->bs);
     a.h = static_cast<int32_t>(p->h);
@@ -619,7 +622,7 @@ int TileXRMoeEpDispatchMemoryV2(void *x, int32_t *expertIds, void *scales, bool 
     p.maxRecvRows = bs * c.rankSize * std::min<int64_t>(topK, moeExpertNum / std::max<int64_t>(1, c.rankSize / T - sharedExpertRankNum));
     p.tpWorldSize = T;
     p.tpRankId = tpRankId;
-    p.tpRecvCountsOut = tpRecvCountsOut;
+    p.tpRecvCountsOut = T > 1 ? tpRecvCountsOut : nullptr;
     p.expertScales = static_cast<const float *>(expertScales);
     p.expandScalesOut = static_cast<float *>(expandScalesOut);
     p.expandXOut = expandXOut;

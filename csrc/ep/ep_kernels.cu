@@ -134,17 +134,15 @@ __device__ __forceinline__ void RouteTokenN(const float *logits, const float *bi
                 bestScore = score[j];
             }
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-            const int oe = __shfl_xor_sync(0xffffffffu, bestE, o);
-            const float os = __shfl_xor_sync(0xffffffffu, bestScore, o);
-            if (ob > best || (ob == best && oe < bestE)) {
-                best = ob;
-                bestE = oe;
-                bestScore = os;
-            }
-        }
+        // The lanes' maxima are compared as integers of the same order (a zero of either sign is one value; a lane without
+        // a candidate, whose scores are NaN, minus infinity or used up, has the smallest key): two warp reductions and a
+        // shuffle per pick instead of fifteen shuffles.
+        const uint32_t bits = __float_as_uint(best + 0.f);
+        const uint32_t key = bestE == 0x7fffffff ? 0u : (bits & 0x80000000u) != 0 ? ~bits : bits | 0x80000000u;
+        const uint32_t top = __reduce_max_sync(0xffffffffu, key);
+        bestE = static_cast<int>(__reduce_min_sync(0xffffffffu, key == top ? static_cast<uint32_t>(bestE) : 0x7fffffffu));
+        bestScore = __shfl_sync(0xffffffffu, bestScore, bestE & 31);
+        if (top == 0u) bestScore = 0.f;
         if ((bestE & 31) == lane) {
 #pragma unroll
             for (int j = 0; j < PER_LANE; ++j) {
@@ -201,6 +199,7 @@ struct DispatchSmem {
     int32_t *total;         // [E] routes of all sources per expert
     int32_t *dstRow;        // [E] first row, at the owner, of (expert, this source)
     float *scaleStage;      // [EP_WARPS][64]
+    int32_t *colPrefix;     // [E + 1] routes of all sources to the columns before e
 };
 
 __device__ __forceinline__ DispatchSmem CarveSmem(uint8_t *base, int numExperts, int routesPerBlock)
@@ -213,6 +212,7 @@ __device__ __forceinline__ DispatchSmem CarveSmem(uint8_t *base, int numExperts,
     s.total = s.blockBase + numExperts;
     s.dstRow = s.total + numExperts;
     s.scaleStage = reinterpret_cast<float *>(s.dstRow + numExperts);
+    s.colPrefix = reinterpret_cast<int32_t *>(s.scaleStage + EP_WARPS * 64);
     return s;
 }
 
@@ -291,6 +291,9 @@ __device__ void EpDispatchBody(const EpDispatchArgs &a)
     const int units = (C + 1 + 2) / 3;           // 16-byte units of one source's counts: C counts and its block count
     const uint8_t *llMine = LlHalf(comm, rank, epoch);
     __shared__ int sIsLast;
+    // A world of one rank: every row's final place is this rank's own output, so rows, scales and tuples are stored there
+    // at once; nothing passes through the window and nobody has to be waited for.
+    const bool solo = R == 1;
 
     const int t0 = min(a.bs, static_cast<int>(blockIdx.x * a.tokensPerBlock));
     const int t1 = min(a.bs, t0 + static_cast<int>(a.tokensPerBlock));
@@ -425,18 +428,30 @@ __device__ void EpDispatchBody(const EpDispatchArgs &a)
         ok = BlockBroadcastOk(got) && ok;
     }
     if (ok) {
+        if (warp == 0) {
+            int carry = 0;
+            for (int base = 0; base < C; base += 32) {
+                int v = base + lane < C ? sm.total[base + lane] : 0;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int u = __shfl_up_sync(0xffffffffu, v, o);
+                    if (lane >= o) v += u;
+                }
+                v += carry;
+                if (base + lane < C) sm.colPrefix[base + lane + 1] = v;
+                carry = __shfl_sync(0xffffffffu, v, 31);
+            }
+            if (lane == 0) sm.colPrefix[0] = 0;
+        }
+        __syncthreads();
         for (int e = tid; e < C; e += blockDim.x) {
-            const int first = EpRankFirstCol(a.topo, EpColRank(a.topo, e));
-            int row = sm.hist[e];
-            for (int p = first; p < e; ++p) row += sm.total[p];
-            sm.dstRow[e] = row;
+            sm.dstRow[e] = sm.hist[e] + sm.colPrefix[e] - sm.colPrefix[EpRankFirstCol(a.topo, EpColRank(a.topo, e))];
         }
         // Every rank sees the same counts, so every rank reaches the same verdict on overflow.
         bool fits = true;
         if (tid < R) {
-            int64_t rows = 0;
             const int firstCol = EpRankFirstCol(a.topo, tid);
-            for (int e = firstCol; e < firstCol + EpRankCols(a.topo, tid); ++e) rows += sm.total[e];
+            const int64_t rows = sm.colPrefix[firstCol + EpRankCols(a.topo, tid)] - sm.colPrefix[firstCol];
             fits = rows <= static_cast<int64_t>(a.maxRecvRows);
             if (!fits) RaiseFailure(w, TILEXR_DEV_BAD_ARGUMENT, tid, 0, a.maxRecvRows, static_cast<uint64_t>(rows));
         }
@@ -458,6 +473,11 @@ __device__ void EpDispatchBody(const EpDispatchArgs &a)
         const int iters = (chunks + 31) / 32;
         // A block with few tokens (small batches) cuts every token into column ranges for several warps.
         const int parts = nTok > 0 ? max(1, min(min(8, iters), static_cast<int>(EP_WARPS) / nTok)) : 1;
+        // where the scales of row `rr` go at the destination whose window half is `half`
+        auto scaleRow = [&](unsigned long long half, uint32_t rr) {
+            return (solo ? reinterpret_cast<uint8_t *>(a.dynamicScalesOut) : reinterpret_cast<uint8_t *>(half) + a.win.scalesOff) +
+                   static_cast<uint64_t>(rr) * a.win.scaleRowBytes;
+        };
         for (int item = warp; item < nTok * parts; item += EP_WARPS) {
             const int i = item / parts;
             const int part = item % parts;
@@ -473,7 +493,10 @@ __device__ void EpDispatchBody(const EpDispatchArgs &a)
                     const int dst = EpColRank(a.topo, e);
                     myRow = static_cast<uint32_t>(sm.dstRow[e] + sm.blockBase[e] + sm.routeRank[i * KR + lane]);
                     uint8_t *half = DataHalf(comm, dst, epoch);
-                    uint8_t *payload = a.zeroCopy
+                    // rows for this rank's own experts go to the output directly (the receive step skips their payload)
+                    uint8_t *payload = dst == rank
+                                           ? a.expandXOut + static_cast<uint64_t>(myRow) * a.win.rowBytes
+                                       : a.zeroCopy
                                            ? comm->registryPtr->regions[a.outHandle].peerBase[dst] + a.outOffset +
                                                  static_cast<uint64_t>(myRow) * a.win.rowBytes
                                            : half + a.win.payloadOff + static_cast<uint64_t>(myRow) * a.win.rowBytes;
@@ -513,7 +536,7 @@ __device__ void EpDispatchBody(const EpDispatchArgs &a)
                     const int k = __ffs(m) - 1;
                     m &= m - 1;
                     uint8_t *p = reinterpret_cast<uint8_t *>(__shfl_sync(0xffffffffu, myPayload, k));
-                    uint8_t *half = reinterpret_cast<uint8_t *>(__shfl_sync(0xffffffffu, myHalf, k));
+                    const unsigned long long half = __shfl_sync(0xffffffffu, myHalf, k);
                     const uint32_t rr = __shfl_sync(0xffffffffu, myRow, k);
                     const int e = __shfl_sync(0xffffffffu, myExpert, k);
                     const float *sc = (a.quantScales != nullptr && e >= a.topo.sharedRanks)
@@ -534,8 +557,9 @@ __device__ void EpDispatchBody(const EpDispatchArgs &a)
                         amax = WarpMax(amax);
                         if (amax > 0.f) inv = 127.0f / amax;
                         if (part == 0 && lane == 0) {
-                            st_vec16(half + a.win.scalesOff + static_cast<uint64_t>(rr) * a.win.scaleRowBytes,
-                                     Vec16{__float_as_uint(amax > 0.f ? amax / 127.0f : 1.0f), 0u, 0u, 0u});
+                            const float scale = amax > 0.f ? amax / 127.0f : 1.0f;
+                            if (solo) a.dynamicScalesOut[rr] = scale;              // a 16-byte cell in the window, one fp32 in the output
+                            else st_vec16(scaleRow(half, rr), Vec16{__float_as_uint(scale), 0u, 0u, 0u});
                         }
                     }
                     for (int it = part; it < iters; it += parts) {
@@ -592,9 +616,7 @@ __device__ void EpDispatchBody(const EpDispatchArgs &a)
                         sv.z = __shfl_sync(0xffffffffu, word, 16);
                         sv.w = __shfl_sync(0xffffffffu, word, 24);
                         if ((payloadRoutes >> lane) & 1u) {
-                            st_vec16(reinterpret_cast<uint8_t *>(myHalf) + a.win.scalesOff +
-                                         static_cast<uint64_t>(myRow) * a.win.scaleRowBytes + it * 16,
-                                     sv);
+                            st_vec16(scaleRow(myHalf, myRow) + it * 16, sv);
                         }
                         Vec16 q;
                         if (mxE5m2) {
@@ -631,9 +653,7 @@ __device__ void EpDispatchBody(const EpDispatchArgs &a)
                     sv.z = __float_as_uint(__shfl_sync(0xffffffffu, scale, 16));
                     sv.w = __float_as_uint(__shfl_sync(0xffffffffu, scale, 24));
                     if ((payloadRoutes >> lane) & 1u) {
-                        st_vec16(reinterpret_cast<uint8_t *>(myHalf) + a.win.scalesOff +
-                                     static_cast<uint64_t>(myRow) * a.win.scaleRowBytes + it * 16,
-                                 sv);
+                        st_vec16(scaleRow(myHalf, myRow) + it * 16, sv);
                     }
                     Vec16 q;
                     q.x = Fp8x4(f[0] * inv, f[1] * inv, f[2] * inv, f[3] * inv);
@@ -661,21 +681,29 @@ __device__ void EpDispatchBody(const EpDispatchArgs &a)
                 }
             }
             if (myExpert >= 0 && part == 0) {
-                st_vec16(reinterpret_cast<uint8_t *>(myHalf) + a.win.assistOff + static_cast<uint64_t>(myRow) * 16,
+                st_vec16((solo ? reinterpret_cast<uint8_t *>(a.assistOut) : reinterpret_cast<uint8_t *>(myHalf) + a.win.assistOff) +
+                             static_cast<uint64_t>(myRow) * 16,
                          Vec16{static_cast<uint32_t>(rank), static_cast<uint32_t>(t), static_cast<uint32_t>(lane),
                                static_cast<uint32_t>(lane < K ? myExpert - a.topo.sharedRanks : lane - K)});   // routed expert id, or shared expert id
                 const int64_t route = static_cast<int64_t>(t) * K + lane;
                 const float wgt = lane >= K ? 1.0f
                                   : a.gateLogits != nullptr ? a.topkWeightsOut[route]
                                                             : (a.expertScales != nullptr ? a.expertScales[route] : 1.0f);
-                *reinterpret_cast<uint2 *>(reinterpret_cast<uint8_t *>(myHalf) + a.win.extOff + static_cast<uint64_t>(myRow) * 8) =
-                    make_uint2(myLink, __float_as_uint(wgt));
+                if (solo) {
+                    if (a.assistExtOut != nullptr) {
+                        *reinterpret_cast<uint2 *>(a.assistExtOut + static_cast<int64_t>(myRow) * 2) = make_uint2(myLink, __float_as_uint(wgt));
+                    }
+                    if (a.expandScalesOut != nullptr) a.expandScalesOut[myRow] = wgt;
+                } else {
+                    *reinterpret_cast<uint2 *>(reinterpret_cast<uint8_t *>(myHalf) + a.win.extOff + static_cast<uint64_t>(myRow) * 8) =
+                        make_uint2(myLink, __float_as_uint(wgt));
+                }
             }
             __syncwarp();
         }
     }
     __syncthreads();
-    if (ok && tid < R) {
+    if (ok && !solo && tid < R) {
         SetFlag(FlagSlot(comm, tid, TILEXR_FLAG_OP_BASE + static_cast<int64_t>(rank) * TILEXR_FLAGS_PER_PAIR + blockIdx.x), epoch, 1);
     }
     PerfStageEnd(perf, TILEXR_PERF_LOCAL_INPUT_TO_IPC, static_cast<uint64_t>(nRoutes) * a.win.rowBytes);
@@ -685,7 +713,7 @@ __device__ void EpDispatchBody(const EpDispatchArgs &a)
     {
         // every thread polls its share of the (source, block) flags; a source's block count came with its counts
         bool got = true;
-        if (ok) {
+        if (ok && !solo) {
             for (int s = 0; s < R && got; ++s) {
                 const int64_t base = TILEXR_FLAG_OP_BASE + static_cast<int64_t>(s) * TILEXR_FLAGS_PER_PAIR;
                 const int blocksOfS = min(srcBlocks[s], static_cast<int>(EP_COUNT_FLAG_SLOT));
@@ -701,8 +729,7 @@ __device__ void EpDispatchBody(const EpDispatchArgs &a)
     if (ok) {
         const int firstLocal = EpRankFirstCol(a.topo, rank);
         const int localCols = EpRankCols(a.topo, rank);
-        int64_t rows = 0;
-        for (int e = firstLocal; e < firstLocal + localCols; ++e) rows += sm.total[e];
+        const int64_t rows = solo ? 0 : sm.colPrefix[firstLocal + localCols] - sm.colPrefix[firstLocal];      // rows to take out of the window
         // Rows are dealt out to blocks in chunks of one row per thread.  Per chunk: (a) a thread per row copies
         // the tuple, link and weight and notes the head rows that have followers; (b) a thread per 16 bytes
         // copies the scales of the rows that arrived with a payload; (c) without zero-copy a warp per row moves
@@ -748,6 +775,7 @@ __device__ void EpDispatchBody(const EpDispatchArgs &a)
                 for (int i = warp; i < chunkRows; i += EP_WARPS) {
                     const int64_t r = base + i;
                     if ((reinterpret_cast<const uint2 *>(winExt + r * 8)->x & EP_LINK_FOLLOWER) != 0) continue;
+                    if (*reinterpret_cast<const int32_t *>(myHalf + a.win.assistOff + r * 16) == rank) continue;     // own token: already there
                     CopyLanes(a.expandXOut + r * a.win.rowBytes, winPayload + r * a.win.rowBytes, a.win.rowBytes, lane, 32);
                 }
             }
@@ -802,7 +830,7 @@ __device__ void EpDispatchBody(const EpDispatchArgs &a)
             }
             __syncthreads();
         }
-        if (blockIdx.x == 0) {
+        if (blockIdx.x == (solo ? G - 1 : 0)) {      // alone, the block with the fewest tokens
             // cumulative counts in (local expert, source) order: an inclusive scan of E_local * R numbers
             const int n = localCols * R;
             __syncthreads();
@@ -834,6 +862,7 @@ __device__ void EpDispatchBody(const EpDispatchArgs &a)
                                                ? static_cast<int64_t>(sm.total[firstLocal + le])
                                                : static_cast<int64_t>(sm.hist[le * R + R - 1]);
             }
+            if (tid == 0 && a.laneCountOut != nullptr) *a.laneCountOut = 0;
             if (tid == 0 && a.recvTotalOut != nullptr) *a.recvTotalOut = n > 0 ? sm.hist[n - 1] : 0;
         }
     }
@@ -1417,7 +1446,7 @@ const KernelEntry &EpCombineKernelEntry() { return TileXREpCombineKernelEntry; }
 
 size_t EpDispatchSmemBytes(int numExperts, int routesPerBlock)
 {
-    return static_cast<size_t>(routesPerBlock) * 8 + static_cast<size_t>(numExperts) * 16 + EP_WARPS * 64 * sizeof(float);
+    return static_cast<size_t>(routesPerBlock) * 8 + static_cast<size_t>(numExperts) * 20 + 4 + EP_WARPS * 64 * sizeof(float);
 }
 
 int LaunchRoutingTopK(const RoutingArgs &args, void *stream)

@@ -81,6 +81,7 @@ struct EpDispatchArgs {
     int64_t *expertTokenNumsOut;
     int32_t *sendCountsOut;
     int32_t *recvTotalOut;
+    int32_t *laneCountOut;           // the caller's count per tensor-parallel lane where there is one lane: set to zero; or null
     CommArgs *comm;
     int64_t magic;
     EpDispatchWindow win;

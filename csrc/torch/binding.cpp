@@ -410,12 +410,12 @@ py::tuple EpDispatch(const CommPtr &c, const at::Tensor &x, const c10::optional<
     at::Tensor routeRows = at::empty({bs, topK * T + sharedExpertNum}, i32);
     at::Tensor assistExt = at::empty({maxRecvRows, 2}, i32);
     at::Tensor expandScales = at::empty({maxRecvRows}, x.options().dtype(at::kFloat));
-    at::Tensor tpRecvCounts = at::zeros({T}, i32);
+    at::Tensor tpRecvCounts = at::empty({T}, i32);
     TileXREpDispatchParams p;
     std::memset(&p, 0, sizeof(p));
     p.tpWorldSize = T;
     p.tpRankId = c->rank() % T;
-    p.tpRecvCountsOut = T > 1 ? tpRecvCounts.data_ptr<int32_t>() : nullptr;
+    p.tpRecvCountsOut = tpRecvCounts.data_ptr<int32_t>();
     p.x = x.data_ptr();
     if (expertIds.has_value() && expertIds->defined()) {
         TORCH_CHECK(expertIds->scalar_type() == at::kInt && expertIds->is_contiguous(), "expert_ids must be contiguous int32");

@@ -465,3 +465,52 @@ def test_ep_with_tensor_parallel_groups(txr, dedup):
         got = ys[r].cpu().float()
         assert torch.allclose(got, want, rtol=2e-2, atol=2e-2), (got - want).abs().max()
     world.destroy()
+
+
+@pytest.mark.parametrize("quant_mode", ["none", "fp8", "mxfp8", "int8"])
+@pytest.mark.parametrize("tokens,experts,top_k", [(1, 8, 2), (17, 40, 8), (300, 256, 4), (1009, 5, 3)])
+def test_dispatch_of_a_single_rank_stores_rows_at_their_place(txr, tokens, experts, top_k, quant_mode):
+    """One rank: rows, scales and tuples go to the outputs without the window.  Expert ids with inactive routes, an active
+    mask, more capacity than rows; blocks without tokens at the smallest batch."""
+    from conftest import free_port
+
+    ep, quant = txr.ep, txr.quant
+    h = 512
+    g = torch.Generator().manual_seed(tokens)
+    x = (torch.randn(tokens, h, generator=g) * 2).to(torch.bfloat16).cuda()
+    ids = torch.stack([torch.randperm(experts, generator=g)[:top_k] for _ in range(tokens)]).to(torch.int32)
+    ids[0, top_k - 1] = -1
+    mask = torch.rand(tokens, generator=g) > 0.2
+    mask[0] = True
+    weights = torch.rand(tokens, top_k, generator=g)
+    mode = {"none": ep.QUANT_NONE, "fp8": ep.QUANT_FP8_1X128, "mxfp8": ep.QUANT_MXFP8_E4M3, "int8": ep.QUANT_DYNAMIC_INT8}[quant_mode]
+    comm = txr.init_process(0, 1, comm_id=f"127.0.0.1:{free_port()}", buffer_mb=64, device=0)
+    try:
+        for _ in range(2):        # the second launch finds what the first one left in the control block
+            d = ep.dispatch(comm, x, num_experts=experts, top_k=top_k, expert_ids=ids.cuda(), expert_scales=weights.cuda(), active_mask=mask.cuda(),
+                            quant_mode=mode, max_recv_rows=tokens * top_k + 3)
+            torch.cuda.synchronize()
+            assert comm.device_status() == 0
+        active = (ids >= 0) & mask[:, None]
+        flat = torch.where(active, ids, torch.full_like(ids, experts)).reshape(-1).long()
+        order = torch.sort(flat, stable=True).indices[:int(active.sum())]
+        token, slot, n = order // top_k, order % top_k, order.numel()
+        assert int(d.recv_total) == n and d.tp_recv_counts.tolist() == [0]
+        assert torch.equal(d.assist[:n].cpu(), torch.stack((torch.zeros_like(token), token, slot, flat[order]), 1).int())
+        assert torch.equal(d.expert_token_nums.cpu(), torch.bincount(flat[order], minlength=experts)[:experts])
+        assert torch.equal(d.expand_scales[:n].cpu(), weights.reshape(-1)[order])
+        rows = torch.full((tokens * top_k,), -1, dtype=torch.int32)
+        rows[order] = torch.arange(n, dtype=torch.int32)
+        assert torch.equal(d.route_rows.cpu().reshape(-1), rows)
+        sent = x[token.cuda()]
+        if quant_mode == "none":
+            assert torch.equal(d.expand_x[:n], sent)
+        elif quant_mode == "int8":
+            amax = sent.float().abs().amax(dim=1, keepdim=True)
+            want = torch.round(sent.float() * (torch.full_like(amax, 127.0) / amax)).clamp(-128, 127).to(torch.int8)
+            assert torch.equal(d.expand_x[:n], want) and torch.equal(d.dynamic_scales[:n], (amax / torch.full_like(amax, 127.0)).squeeze(1))
+        else:
+            want, scales = quant.fp8_quant_1x128(sent) if quant_mode == "fp8" else quant.mxfp8_quant(sent)
+            assert torch.equal(d.expand_x[:n].view(torch.uint8), want.view(torch.uint8)) and torch.equal(d.dynamic_scales[:n], scales)
+    finally:
+        comm.destroy()
