@@ -824,6 +824,23 @@ int TileXRMxfp8Dequant(const void *y, const uint8_t *scales, int64_t rows, int64
                               stream);
 }
 
+int TileXRMoeEpCombineBackward(const void *g, const float *weights, const void *rows, const int32_t *assist, const int32_t *rowCount,
+                               int64_t capacity, int64_t h, int64_t slots, int64_t wideCols, TileXRDataType dtype, void *gradRowsOut,
+                               void *wideOut, TileXRStream stream)
+{
+    if (g == nullptr || weights == nullptr || assist == nullptr || rowCount == nullptr || gradRowsOut == nullptr || capacity <= 0 || h <= 0 ||
+        h % 8 != 0 || h > INT32_MAX || !HalfType(dtype) || (rows != nullptr && wideOut == nullptr)) {
+        return TILEXR_ERROR_PARA_CHECK_FAIL;
+    }
+    if (rows != nullptr && (slots <= 0 || wideCols % 8 != 0 || wideCols < 2 * slots || wideCols > INT32_MAX)) return TILEXR_ERROR_PARA_CHECK_FAIL;
+    if (((reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(rows) | reinterpret_cast<uintptr_t>(gradRowsOut) |
+          reinterpret_cast<uintptr_t>(wideOut)) & 15u) != 0) {
+        return TILEXR_ERROR_PARA_CHECK_FAIL;
+    }
+    return LaunchCombineBackward(g, weights, rows, assist, rowCount, capacity, h, dtype == TILEXR_DATA_TYPE_BFP16, static_cast<int>(slots),
+                                 static_cast<int>(wideCols), gradRowsOut, wideOut, stream);
+}
+
 int TileXRRmsNorm(const void *x, void *residualInOut, const void *gamma, float eps, int64_t rows, int64_t h,
                   TileXRDataType dtype, void *yOut, TileXRStream stream)
 {

@@ -159,6 +159,8 @@ const KernelEntry &EpCombineKernelEntry();
 int LaunchRoutingTopK(const RoutingArgs &args, void *stream);
 // rows [gate | up] -> silu(gate) * up; with `scales` quantised to e4m3 per 128 elements (f % 128 == 0), else f % 8 == 0
 int LaunchSwiglu(const void *gateUp, int64_t rows, int64_t f, bool bf16, void *y, float *scales, void *stream);
+int LaunchCombineBackward(const void *g, const float *weights, const void *rows, const int32_t *assist, const int32_t *rowCount, int64_t capacity,
+                          int64_t h, bool bf16, int slots, int wideCols, void *gradRows, void *wide, void *stream);
 int LaunchFp8Quant1x128(const void *x, int64_t rows, int64_t h, bool bf16, void *y, float *scales, void *stream);
 int LaunchFp8Dequant1x128(const void *y, const float *scales, int64_t rows, int64_t h, bool bf16, void *x, void *stream);
 int LaunchMxfp8Quant(const void *x, int64_t rows, int64_t h, bool bf16, bool e5m2, void *y, uint8_t *scales, void *stream);

@@ -203,6 +203,13 @@ int TileXRMxfp8Quant(const void *x, int64_t rows, int64_t h, TXR_DT dtype, TXR_D
                      TileXRStream stream);
 int TileXRMxfp8Dequant(const void *y, const uint8_t *scales, int64_t rows, int64_t h, TXR_DT fp8Type, TXR_DT dtype,
                        void *xOut, TileXRStream stream);
+// Backward of a weighted combine, over the rows a dispatch of the output gradient delivered (`g` [capacity, h], its row weights,
+// assist tuples and *rowCount): gradRows[r] = weights[r] * g[r]; with `rows` (the expert rows the combine summed) also
+// <g[r], rows[r]> as a (high, low) bf16 pair in columns 2 s and 2 s + 1 of wide[r] ([capacity, wideCols] bf16, the other columns zero),
+// s the slot of the row's tuple, clamped to [0, slots).  Rows from *rowCount on get a zero gradient and leave `wide` alone.
+int TileXRMoeEpCombineBackward(const void *g, const float *weights, const void *rows, const int32_t *assist, const int32_t *rowCount,
+                               int64_t capacity, int64_t h, int64_t slots, int64_t wideCols, TXR_DT dtype, void *gradRowsOut, void *wideOut,
+                               TileXRStream stream);
 // RMSNorm: y = x * rsqrt(mean(x^2) + eps) * gamma, optionally x += residual first (and the sum is written back).
 int TileXRRmsNorm(const void *x, void *residualInOut, const void *gamma, float eps, int64_t rows, int64_t h, TXR_DT dtype,
                   void *yOut, TileXRStream stream);

@@ -534,6 +534,33 @@ at::Tensor EpCombine(const CommPtr &c, const at::Tensor &expertOut, const at::Te
     return y;
 }
 
+// (grad_rows, wide | None), see TileXRMoeEpCombineBackward
+py::tuple EpCombineBackward(const at::Tensor &g, const at::Tensor &weights, const c10::optional<at::Tensor> &rows, const at::Tensor &assist,
+                            const at::Tensor &rowCount, int64_t slots, int64_t wideCols)
+{
+    TORCH_CHECK(g.is_cuda() && g.dim() == 2 && g.is_contiguous(), "g must be a contiguous 2-D CUDA tensor");
+    const int64_t capacity = g.size(0), h = g.size(1);
+    TORCH_CHECK(weights.is_cuda() && weights.scalar_type() == at::kFloat && weights.is_contiguous() && weights.numel() >= capacity &&
+                    assist.is_cuda() && assist.scalar_type() == at::kInt && assist.is_contiguous() && assist.numel() >= capacity * 4 &&
+                    rowCount.is_cuda() && rowCount.scalar_type() == at::kInt && rowCount.numel() == 1,
+                "weights fp32 [rows], assist int32 [rows, 4] and the row count int32 [1] of the dispatch");
+    const bool dots = rows.has_value() && rows->defined();
+    TORCH_CHECK(!dots || (rows->is_cuda() && rows->is_contiguous() && rows->sizes() == g.sizes() && rows->scalar_type() == g.scalar_type()),
+                "rows must be contiguous and like g");
+    at::Tensor grad = at::empty_like(g);
+    at::Tensor wide = dots ? at::empty({capacity, wideCols}, g.options().dtype(at::kBFloat16)) : at::Tensor();
+    Keep(g);
+    Keep(weights);
+    Keep(rows);
+    Keep(assist);
+    Keep(rowCount);
+    Check(TileXRMoeEpCombineBackward(g.data_ptr(), weights.data_ptr<float>(), PtrOrNull(rows), assist.data_ptr<int32_t>(),
+                                     rowCount.data_ptr<int32_t>(), capacity, h, slots, wideCols, ToDtype(g.scalar_type()), grad.data_ptr(),
+                                     dots ? wide.data_ptr() : nullptr, StreamOf(g)),
+          "TileXRMoeEpCombineBackward");
+    return py::make_tuple(grad, dots ? py::cast(wide) : py::none());
+}
+
 py::tuple RoutingTopK(const at::Tensor &logits, const c10::optional<at::Tensor> &bias, int64_t topK, int64_t scoreFunc,
                       bool renormalize, double routedScale)
 {
@@ -732,6 +759,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m)
           py::arg("tp_world_size") = 1);
     m.def("routing_topk", &RoutingTopK, py::arg("gate_logits"), py::arg("selection_bias") = py::none(), py::arg("top_k") = 1,
           py::arg("score_func") = 0, py::arg("renormalize") = true, py::arg("routed_scale") = 1.0);
+    m.def("ep_combine_backward", &EpCombineBackward);
     m.def("fp8_quant_1x128", &Fp8Quant);
     m.def("swiglu", &Swiglu);
     m.def("swiglu_fp8_quant_1x128", &SwigluFp8Quant);

@@ -58,3 +58,23 @@ def test_fp8_quant_rows_that_do_not_fill_a_warp(txr, rows, h):
     q, s = txr.quant.fp8_quant_1x128(x.cuda())
     want_q, want_s = oracle.fp8_quant_1x128_ref(x)
     assert torch.equal(s.cpu(), want_s) and torch.equal(q.cpu().view(torch.uint8), want_q.view(torch.uint8))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,h", [(1, 128), (3, 128), (9, 384), (130, 7168)])
+def test_fp8_dequant_at_the_edges_of_a_launch(txr, rows, h, dtype):
+    x = (torch.randn(rows, h, generator=torch.Generator().manual_seed(h)) * 4).to(dtype).cuda()
+    q, s = txr.quant.fp8_quant_1x128(x)
+    got = txr.quant.fp8_dequant_1x128(q, s, dtype)
+    assert torch.equal(got, (q.float().view(rows, -1, 128) * s[:, :, None]).view(rows, h).to(dtype))
+
+
+@pytest.mark.parametrize("e5m2", [False, True])
+@pytest.mark.parametrize("rows,h", [(1, 8), (3, 40), (5, 33), (7, 100), (130, 4096)])
+def test_mxfp8_dequant_rows_of_any_length(txr, rows, h, e5m2):
+    """Rows of a multiple of eight elements take eight at a time, the others one; a row may end inside its last block."""
+    x = (torch.randn(rows, h, generator=torch.Generator().manual_seed(h)) * 4).to(torch.bfloat16).cuda()
+    q, s = txr.quant.mxfp8_quant(x, e5m2)
+    got = txr.quant.mxfp8_dequant(q, s)
+    scale = torch.exp2(s.float() - 127).repeat_interleave(32, dim=1)[:, :h]
+    assert torch.equal(got, (q.float() * scale).to(torch.bfloat16))

@@ -92,3 +92,37 @@ def test_dispatcher_backward_matches_dense_moe():
         assert torch.allclose(gl, logits.grad, rtol=5e-2, atol=2e-2), (gl - logits.grad).abs().max()
     finally:
         comm.destroy()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("tokens,hidden,top_k,capacity", [(1, 8, 1, 1), (5, 264, 3, 19), (130, 1032, 8, 1040)])
+def test_combine_backward_rows_match_the_unfused_form(tokens, hidden, top_k, capacity, dtype):
+    """Row gradients and gate-weight dot products of one pass against plain PyTorch, with rows nobody uses at the end."""
+    import dataclasses
+
+    from tilexr_b200.ops import ep
+
+    gen = torch.Generator().manual_seed(tokens)
+    n = tokens * top_k
+    g = torch.randn(capacity, hidden, generator=gen).to(dtype).cuda()
+    out = torch.randn(capacity, hidden, generator=gen).to(dtype).cuda()
+    w = torch.rand(capacity, generator=gen).cuda()
+    assist = torch.zeros(capacity, 4, dtype=torch.int32)
+    assist[:, 2] = torch.arange(capacity) % top_k
+    d = ep.DispatchResult(**{f.name: None for f in dataclasses.fields(ep.DispatchResult) if f.default is dataclasses.MISSING})
+    d.expand_x, d.expand_scales, d.assist = g, w, assist.cuda()
+    d.recv_total = torch.tensor([n], dtype=torch.int32, device="cuda")
+    width = max(16, (2 * top_k + 7) // 8 * 8)
+    grad, wide = ep.combine_backward_rows(d, out, top_k, width)
+    want = (g[:n].float() * w[:n, None]).to(dtype)
+    assert torch.equal(grad[:n], want) and not grad[n:].any()
+    dots = (g[:n].double() * out[:n].double()).sum(dim=1)
+    cols = (2 * assist[:n, 2].long().cuda())[:, None]
+    got = wide[:n].double().gather(1, cols) + wide[:n].double().gather(1, cols + 1)
+    # the pair keeps 16 bits of the fp32 sum, whose own error is below hidden * 2^-24 of the sum of magnitudes
+    bound = dots.abs() * 2.0 ** -15 + (g[:n].double() * out[:n].double()).abs().sum(dim=1) * hidden * 2.0 ** -24
+    assert ((got.squeeze(1) - dots).abs() <= bound).all()
+    rest = wide[:n].clone().scatter_(1, cols, 0).scatter_(1, cols + 1, 0)
+    assert not rest.any()
+    only_grad, none = ep.combine_backward_rows(d, None, top_k, width)
+    assert none is None and torch.equal(only_grad, grad)

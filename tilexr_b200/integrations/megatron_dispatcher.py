@@ -92,20 +92,27 @@ class _Unpermute(torch.autograd.Function):
                                expert_ids=owner._ids, expert_scales=probs, quant_mode=_ep.QUANT_NONE,
                                max_recv_rows=d.expand_x.shape[0], dedup=False, tp_world_size=owner.tp_world_size)
         rows = d.expand_x.shape[0]
-        grad_out = (g.expand_x.float() * g.expand_scales[:rows].unsqueeze(1)).to(expert_out.dtype)
+        # <grad_y[token], out[row]> per row, placed at column k of a 2K-wide row as a (high, low) bf16 pair, summed at
+        # the origin with unit weights: column k of the result is the dot product of route (token, k)
+        K = owner.top_k * owner.tp_world_size
+        width = max(256, (2 * K + 7) // 8 * 8)           # rows of at least 512 bytes, the width the kernels are tuned for
+        want_probs = ctx.needs_input_grad[1]
+        fused = None
+        if isinstance(g, _ep.DispatchResult) and g.expand_x.dtype == expert_out.dtype:
+            fused = _ep.combine_backward_rows(g, expert_out if want_probs else None, K, width)
+        grad_out = fused[0] if fused is not None else (g.expand_x.float() * g.expand_scales[:rows].unsqueeze(1)).to(expert_out.dtype)
         grad_probs = None
-        if ctx.needs_input_grad[1]:
-            # <grad_y[token], out[row]> per row, placed at column k of a 2K-wide row as a (high, low) bf16 pair, summed at
-            # the origin with unit weights: column k of the result is the dot product of route (token, k)
-            K = owner.top_k * owner.tp_world_size
-            width = max(256, (2 * K + 7) // 8 * 8)       # rows of at least 512 bytes, the width the kernels are tuned for
-            dots = (g.expand_x.float() * expert_out.float()).sum(dim=1)
-            high = dots.to(torch.bfloat16)
-            low = (dots - high.float()).to(torch.bfloat16)
-            slot = g.assist[:, 2].long().clamp(0, K - 1)
-            wide = torch.zeros(rows, width, dtype=torch.bfloat16, device=dots.device)
-            wide.scatter_(1, (2 * slot).unsqueeze(1), high.unsqueeze(1))
-            wide.scatter_(1, (2 * slot + 1).unsqueeze(1), low.unsqueeze(1))
+        if want_probs:
+            if fused is not None:
+                wide = fused[1]
+            else:
+                dots = (g.expand_x.float() * expert_out.float()).sum(dim=1)
+                high = dots.to(torch.bfloat16)
+                low = (dots - high.float()).to(torch.bfloat16)
+                slot = g.assist[:, 2].long().clamp(0, K - 1)
+                wide = torch.zeros(rows, width, dtype=torch.bfloat16, device=dots.device)
+                wide.scatter_(1, (2 * slot).unsqueeze(1), high.unsqueeze(1))
+                wide.scatter_(1, (2 * slot + 1).unsqueeze(1), low.unsqueeze(1))
             back = owner.ops.combine(owner.comm, wide, dataclasses.replace(g, dedup=False), expert_scales=None).float()
             per_slot = back[:, 0:2 * K:2] + back[:, 1:2 * K:2]
             # tensor-parallel lanes hold slices of one route: their dot products add up

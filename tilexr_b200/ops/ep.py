@@ -90,3 +90,18 @@ def combine(comm, expert_out: torch.Tensor, d: DispatchResult, *, expert_scales:
     return _C.ep_combine(comm, expert_out, d.assist, d.send_counts, d.topk_ids, expert_scales, active_mask, shared_expert_x,
                          d.bs, d.top_k, d.num_experts, y_out, d.route_rows, d.assist_ext, d.dedup, d.shared_expert_num,
                          d.shared_expert_rank_num, d.tp_world_size)
+
+
+def combine_backward_rows(g: DispatchResult, expert_rows: Optional[torch.Tensor], slots: int, wide_cols: int):
+    """Over the output gradient ``g`` brought back to the expert rows: ``(grad_rows, wide)`` with ``grad_rows = weight * g`` per
+    row and, where ``expert_rows`` is given, ``<g, expert row>`` as a (high, low) bf16 pair in columns ``2 * slot`` and
+    ``2 * slot + 1`` of ``wide`` [rows, wide_cols] (else None).  One pass on the device; None where the kernel does not take the
+    tensors (other devices or types)."""
+    rows = g.expand_x
+    if not rows.is_cuda or rows.dtype not in (torch.float16, torch.bfloat16) or rows.shape[0] == 0:
+        return None
+    if expert_rows is not None:
+        expert_rows = expert_rows.contiguous()
+        if expert_rows.dtype != rows.dtype or expert_rows.shape != rows.shape or expert_rows.data_ptr() % 16 != 0:
+            return None
+    return _C.ep_combine_backward(rows, g.expand_scales, expert_rows, g.assist, g.recv_total, slots, wide_cols)
