@@ -127,6 +127,72 @@ void FillTiling(GemmArgs *g, int64_t m, int64_t n, int64_t k)
     g->kBlocks = static_cast<int32_t>((k + GEMM_BK - 1) / GEMM_BK);
 }
 
+// The few-rows kernel for one product (groupRows null) or for groups of rows.  `tn` rows per tile, a power of two from 16 to 128.
+int LaunchSkinny(const void *a, const void *b, const int64_t *groupRows, void *c, int64_t m, int64_t n, int64_t k, int64_t groups, int tn, bool bf16,
+                 int epilogue, int32_t *status, int sms, TileXRStream stream)
+{
+    SkinnyArgs g;
+    std::memset(&g, 0, sizeof(g));
+    int ret = MakeMap(&g.tmapW, b, groups * n, k, 128, bf16);
+    if (ret != TILEXR_SUCCESS) return ret;
+    ret = MakeMap(&g.tmapX, a, m, k, tn, bf16);
+    if (ret != TILEXR_SUCCESS) return ret;
+    g.c = static_cast<uint8_t *>(c);
+    g.status = status;
+    g.groupRows = groupRows;
+    g.M = static_cast<int32_t>(m);
+    g.N = static_cast<int32_t>(n);
+    g.K = static_cast<int32_t>(k);
+    g.kBlocks = static_cast<int32_t>((k + GEMM_BK - 1) / GEMM_BK);
+    g.nTiles = static_cast<int32_t>((n + 127) / 128);
+    g.tn = tn;
+    g.stages = std::min<int>(GEMM_SKINNY_MAX_STAGES, GEMM_SKINNY_RING_BYTES / (GEMM_SKINNY_W_BYTES + tn * 128));
+    g.isBf16 = bf16 ? 1u : 0u;
+    g.epilogue = epilogue;
+    g.split = 1;
+    const int64_t places = 2 * static_cast<int64_t>(sms);
+    const int64_t rowTiles = groupRows != nullptr ? (m + tn - 1) / tn + std::min<int64_t>(groups, GEMM_SKINNY_MAX_GROUPS) : (m + tn - 1) / tn;
+    const int64_t items = rowTiles * g.nTiles;
+    if (groupRows == nullptr) {
+        // K is split while the parts still find a place at once and each keeps four steps of K; no part may be empty
+        while (g.split < GEMM_SKINNY_MAX_SPLIT && items * g.split * 2 <= places && g.kBlocks >= g.split * 2 * 4) g.split *= 2;
+        while (g.split > 1 && (g.kBlocks + g.split - 1) / g.split * (g.split - 1) >= g.kBlocks) g.split /= 2;
+    }
+    const unsigned grid = static_cast<unsigned>(g.split > 1 ? items * g.split : std::max<int64_t>(1, std::min(items, places)));
+    static std::once_flag once;
+    std::call_once(once, [] {
+        cudaFuncSetAttribute(GemmSkinnyKernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(GEMM_SKINNY_SMEM_BYTES));
+    });
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = static_cast<unsigned>(g.split);
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(GEMM_SKINNY_THREADS);
+    cfg.dynamicSmemBytes = GEMM_SKINNY_SMEM_BYTES;
+    cfg.stream = static_cast<cudaStream_t>(stream);
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    for (int64_t base = 0; base < groups; base += GEMM_SKINNY_MAX_GROUPS) {
+        g.groupBase = static_cast<int32_t>(base);
+        g.groups = static_cast<int32_t>(std::min<int64_t>(GEMM_SKINNY_MAX_GROUPS, groups - base));
+        void *params[] = {&g};
+        const cudaError_t e = cudaLaunchKernelExC(&cfg, GemmSkinnyKernel(), params);
+        if (e != cudaSuccess) {
+            TILEXR_LOG(ERROR) << "matmul (few rows) launch failed: " << cudaGetErrorString(e);
+            cudaGetLastError();
+            return TILEXR_ERROR_RUNTIME;
+        }
+        NoteLaunch();
+    }
+    return TILEXR_SUCCESS;
+}
+
+// Rows per tile of the few-rows kernel for `rows` rows: the smallest size that holds them, 128 at most.
+int SkinnyRows(int64_t rows) { return rows <= 16 ? 16 : rows <= 32 ? 32 : rows <= 64 ? 64 : 128; }
+
 } // namespace
 
 extern "C" {
@@ -137,6 +203,15 @@ int TileXRMatmul(const void *a, const void *b, void *c, int64_t m, int64_t n, in
     int ret = CheckShape(a, b, c, m, n, k, dtype);
     if (ret != TILEXR_SUCCESS) return ret;
     const bool bf16 = dtype == TILEXR_DATA_TYPE_BFP16;
+    int sms = 0;
+    ret = SmCount(&sms);
+    if (ret != TILEXR_SUCCESS) return ret;
+    // Few rows, or so few 256 x 256 tiles that more than half of the CTA pairs would have none: the kernel whose tiles are
+    // 128 columns by up to 128 rows and which splits K.
+    const int64_t squareTiles = ((m + 2 * GEMM_BM - 1) / (2 * GEMM_BM)) * ((n + GEMM_BN - 1) / GEMM_BN);
+    if ((m <= GEMM_BM || squareTiles * 4 <= sms) && EnvLong("TILEXR_GEMM_SKINNY", 1) != 0) {
+        return LaunchSkinny(a, b, nullptr, c, m, n, k, 1, SkinnyRows(m), bf16, GEMM_EPI_STORE, status, sms, stream);
+    }
     GemmArgs g;
     std::memset(&g, 0, sizeof(g));
     ret = MakeMap(&g.tmapA, a, m, k, GEMM_BM, bf16);
@@ -149,9 +224,6 @@ int TileXRMatmul(const void *a, const void *b, void *c, int64_t m, int64_t n, in
     g.mode = GEMM_PLAIN;
     g.isBf16 = bf16 ? 1u : 0u;
     FillTiling(&g, m, n, k);
-    int sms = 0;
-    ret = SmCount(&sms);
-    if (ret != TILEXR_SUCCESS) return ret;
     if (m > GEMM_BM && EnvLong("TILEXR_GEMM_PAIR", 1) != 0) {
         // CTA pairs on 256x256 tiles: each CTA loads half of the B tile (its own tensor map box of 128 rows)
         ret = MakeMap(&g.tmapB, b, n, k, GEMM_BN / 2, bf16);
@@ -207,6 +279,14 @@ int TileXRGroupedMatmul(const void *a, const void *b, const int64_t *groupRows, 
         return TILEXR_ERROR_PARA_CHECK_FAIL;
     }
     const bool bf16 = dtype == TILEXR_DATA_TYPE_BFP16;
+    int sms = 0;
+    ret = SmCount(&sms);
+    if (ret != TILEXR_SUCCESS) return ret;
+    // Few rows per group on average (the counts themselves are on the device): tiles of twice the average hold most groups
+    const int64_t perGroup = (maxRows + groups - 1) / groups;
+    if (perGroup <= EnvLong("TILEXR_GEMM_SKINNY_ROWS", 32)) {
+        return LaunchSkinny(a, b, groupRows, c, maxRows, n, k, groups, SkinnyRows(2 * perGroup), bf16, epilogue, status, sms, stream);
+    }
     GemmArgs g;
     std::memset(&g, 0, sizeof(g));
     ret = MakeMap(&g.tmapA, a, maxRows, k, GEMM_BM, bf16);
@@ -223,9 +303,6 @@ int TileXRGroupedMatmul(const void *a, const void *b, const int64_t *groupRows, 
     g.epilogue = epilogue;
     FillTiling(&g, maxRows, n, k);
     g.rasterGroup = static_cast<int32_t>(std::max<long>(1, EnvLong("TILEXR_GEMM_GROUP", 8)));
-    int sms = 0;
-    ret = SmCount(&sms);
-    if (ret != TILEXR_SUCCESS) return ret;
     static std::once_flag pairOnce;
     std::call_once(pairOnce, [] {
         cudaFuncSetAttribute(GemmPairKernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(GEMM_PAIR_SMEM_BYTES));

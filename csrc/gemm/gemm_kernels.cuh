@@ -114,6 +114,78 @@ struct GemmBlockArgs {
     int32_t shardRows, blocksPerShard, flagStride;
 };
 
+// GEMM for few rows (gemm_tcgen05_skinny.cu): 128 rows of the weight x tn rows of A per tile, two CTAs per SM.
+constexpr unsigned GEMM_SKINNY_THREADS = 192;
+constexpr int GEMM_SKINNY_MAX_STAGES = 6;
+constexpr int GEMM_SKINNY_MAX_GROUPS = 256;        // groups of one launch
+constexpr int GEMM_SKINNY_MAX_SPLIT = 8;           // CTAs of a cluster that share a tile's K
+constexpr uint32_t GEMM_SKINNY_W_BYTES = 128 * 128;
+constexpr uint32_t GEMM_SKINNY_STATE_BYTES = 256;
+constexpr uint32_t GEMM_SKINNY_RING_BYTES = 110592;      // stages x (16 KB + 128 tn): six of 18 KB down to three of 32 KB
+constexpr size_t GEMM_SKINNY_SMEM_BYTES = 1024 /* alignment slack */ + GEMM_SKINNY_RING_BYTES + GEMM_SKINNY_STATE_BYTES +
+                                          2 * (GEMM_SKINNY_MAX_GROUPS + 1) * 4;
+static_assert(2 * (GEMM_SKINNY_SMEM_BYTES + 1024) <= 228 * 1024, "two CTAs share an SM");
+
+struct SkinnyArgs {
+    CUtensorMap tmapW;        // B [groupsTotal * N, K], box 128 rows x 64 columns
+    CUtensorMap tmapX;        // A [M, K], box tn rows x 64 columns
+    uint8_t *c;               // [M, N], or [M, N / 2] with the SwiGLU epilogue
+    int32_t *status;
+    const int64_t *groupRows; // grouped: rows per group on the device; null: one product
+    int32_t M, N, K;
+    int32_t kBlocks, nTiles;  // 64-wide steps of K, 128-column tiles of N
+    int32_t tn, stages, split;
+    int32_t groups, groupBase;
+    uint32_t isBf16;
+    int32_t epilogue;
+};
+const void *GemmSkinnyKernel();
+
+#if defined(__CUDACC__)
+// Where the rows and the row blocks (of `blockRows`) of groups groupBase .. groupBase + groups - 1 start, with the total behind
+// the last group; a whole warp.  Counts below zero count as zero and rows past M do not exist.  The counts are fetched by 32
+// lanes at a time: one lane after the other it was a chain of loads in front of every tile of the launch.
+__device__ __forceinline__ void BuildGroupTable(const int64_t *groupRows, int groupBase, int groups, int M, int blockRows, int lane, int *rowStart,
+                                                int *blockStart)
+{
+    long long before = 0;
+    for (int g = lane; g < groupBase; g += 32) before += max(0ll, static_cast<long long>(groupRows[g]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+    int blocks = 0;                                            // row blocks of the groups before this step's
+    for (int base = 0; base < groups; base += 32) {
+        const int g = base + lane;
+        long long end = g < groups ? max(0ll, static_cast<long long>(groupRows[groupBase + g])) : 0ll;
+        const long long own = end;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const long long up = __shfl_up_sync(0xffffffffu, end, o);
+            if (lane >= o) end += up;
+        }
+        end += before;
+        const int last = static_cast<int>(min(end, static_cast<long long>(M)));
+        const int start = static_cast<int>(min(end - own, static_cast<long long>(M)));
+        const int mine = (last - start + blockRows - 1) / blockRows;
+        int incl = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int up = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += up;
+        }
+        if (g < groups) {
+            rowStart[g] = start;
+            blockStart[g] = blocks + incl - mine;
+            if (g == groups - 1) {
+                rowStart[groups] = last;
+                blockStart[groups] = blocks + incl;
+            }
+        }
+        before = __shfl_sync(0xffffffffu, end, 31);
+        blocks += __shfl_sync(0xffffffffu, incl, 31);
+    }
+}
+#endif
+
 const void *GemmFp8BlockKernel(int mode);            // a kernel per GemmMode (plain, all-gather, reduce-scatter)
 const void *GemmFp8BlockKernelEmulated(int mode);    // all-gather, reduce-scatter
 const void *GemmKernelSingle();

@@ -397,25 +397,7 @@ __device__ void PairBody(const GemmArgs &a)
         if (a.mode == GEMM_ALL_GATHER) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&a.tmapALocal)) : "memory");
     }
     if (a.mode == GEMM_GROUPED && warp == 2) {
-        // rows before this launch's first group, then the running row and block offsets of its groups
-        long long before = 0;
-        for (int g = lane; g < a.groupBase; g += 32) before += max(0ll, static_cast<long long>(a.groupRows[g]));
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
-        if (lane == 0) {
-            int row = static_cast<int>(min(before, static_cast<long long>(a.M)));
-            int block = 0;
-            for (int g = 0; g < a.groups; ++g) {
-                gt->rowStart[g] = row;
-                gt->blockStart[g] = block;
-                const long long want = max(0ll, static_cast<long long>(a.groupRows[a.groupBase + g]));
-                const int rows = static_cast<int>(min(want, static_cast<long long>(a.M - row)));      // never past the buffers
-                row += rows;
-                block += (rows + 2 * GEMM_BM - 1) / (2 * GEMM_BM);
-            }
-            gt->rowStart[a.groups] = row;
-            gt->blockStart[a.groups] = block;
-        }
+        BuildGroupTable(a.groupRows, a.groupBase, a.groups, a.M, 2 * GEMM_BM, lane, gt->rowStart, gt->blockStart);
     }
     __syncthreads();
     if (warp == 1) {

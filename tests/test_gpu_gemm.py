@@ -220,3 +220,39 @@ def test_matmul_reduce_scatter_fp8_block(txr, ranks, shard_rows, n, k):
         assert torch.allclose(got, ref, rtol=2e-2, atol=2e-2 * ref.abs().max().item()), (got - ref).abs().max()
         assert (got - ref).abs().mean() < 6e-3 * ref.abs().mean() + 1e-4
     world.destroy()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("m,n,k", [(1, 8, 8), (1, 128, 64), (16, 120, 72), (17, 7168, 2048), (33, 136, 2056), (65, 4096, 320), (128, 264, 4104),
+                                   (129, 512, 1000), (300, 1024, 640), (1000, 512, 4096), (5, 40960, 136)])
+def test_matmul_few_rows(txr, m, n, k, dtype):
+    """Tiles of 128 columns by 16 to 128 rows: remainders of both, K split over one to eight CTAs with a ragged last part,
+    more tiles than places."""
+    g = torch.Generator().manual_seed(m + n + k)
+    a = torch.randn(m, k, generator=g).to(dtype).cuda()
+    b = (torch.randn(n, k, generator=g) * k ** -0.5).to(dtype).cuda()
+    want = a.double() @ b.double().t()
+    for _ in range(2):
+        got = txr.gemm.matmul(a, b).double()
+        # fp32 sums of k products (k eps of the sum of magnitudes at the very most), rounded once to the output type
+        bound = want.abs() * torch.finfo(dtype).eps / 2 + (a.double().abs() @ b.double().abs().t()) * k * 2.0 ** -24 + 2.0 ** -24
+        assert ((got - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("epilogue", [0, 1])
+@pytest.mark.parametrize("groups,n,k,counts", [(3, 144, 72, [0, 5, 0]), (5, 256, 128, [1, 0, 40, 2, 17]), (70, 272, 64, None), (300, 128, 64, None)])
+def test_grouped_matmul_few_rows_per_group(txr, groups, n, k, counts, epilogue):
+    """Empty groups, a group of several row chunks, more groups than one launch takes, rows behind the last group."""
+    g = torch.Generator().manual_seed(groups)
+    if counts is None:
+        counts = torch.randint(0, 6, (groups,), generator=g).tolist()
+        counts[groups // 2] = 50
+    total = sum(counts)
+    rows = torch.randn(total + 7, k, generator=g).to(torch.bfloat16).cuda()
+    w = (torch.randn(groups, n, k, generator=g) * k ** -0.5).to(torch.bfloat16).cuda()
+    out = torch.full((total + 7, n // 2 if epilogue else n), 3.0, dtype=torch.bfloat16, device="cuda")
+    got = txr.gemm.grouped_matmul(rows, w, torch.tensor(counts, dtype=torch.int64, device="cuda"), epilogue=epilogue, out=out)
+    want = txr.gemm.grouped_matmul_ref(rows, w, torch.tensor(counts), epilogue)
+    # one rounding to bf16 of a value of order one
+    assert torch.allclose(got[:total].float(), want[:total], rtol=2.0 ** -7, atol=2.0 ** -7)
+    assert (got[total:] == 3.0).all()
