@@ -411,6 +411,7 @@ int TileXRMoeEpDispatchFused(const TileXREpDispatchParams *p, TileXRCommPtr comm
     a.elemSize = static_cast<uint32_t>(elemSize);
     a.isBf16 = p->dtype == TILEXR_DATA_TYPE_BFP16 ? 1u : 0u;
     a.zeroCopy = zeroCopy ? 1u : 0u;
+    a.directOwn = (reinterpret_cast<uintptr_t>(p->expandXOut) & 15u) == 0 ? 1u : 0u;
     a.outHandle = handle;
     a.outOffset = regionOffset;
     a.routeRowsOut = p->routeRowsOut;

@@ -81,7 +81,7 @@ __device__ __forceinline__ uint32_t Fp8x4E5m2(float a, float b, float c, float d
 // lower expert id; the gate weight is the unbiased score, optionally renormalised over the
 // selected experts and multiplied by `routedScale`.
 template <int PER_LANE>
-__device__ __forceinline__ void RouteTokenN(const float *logits, const float *bias, int numExperts, int topK, int scoreFunc,
+__device__ __forceinline__ int RouteTokenN(const float *logits, const float *bias, int numExperts, int topK, int scoreFunc,
                                             int renormalize, float routedScale, int lane, int32_t *idsOut, float *weightsOut)
 {
     float score[PER_LANE];
@@ -162,21 +162,21 @@ __device__ __forceinline__ void RouteTokenN(const float *logits, const float *bi
         idsOut[lane] = myId;
         weightsOut[lane] = w;
     }
+    return myId;
 }
 
 // The per-lane score table is sized for the expert count, so that 256 experts keep 8 scores per lane in
-// registers instead of the 32 that the largest supported count needs.
-__device__ __forceinline__ void RouteToken(const float *logits, const float *bias, int numExperts, int topK, int scoreFunc,
+// registers instead of the 32 that the largest supported count needs.  Returns the expert that lane k picked k-th.
+__device__ __forceinline__ int RouteToken(const float *logits, const float *bias, int numExperts, int topK, int scoreFunc,
                                            int renormalize, float routedScale, int lane, int32_t *idsOut, float *weightsOut)
 {
     if (numExperts <= 256) {
-        RouteTokenN<8>(logits, bias, numExperts, topK, scoreFunc, renormalize, routedScale, lane, idsOut, weightsOut);
-    } else if (numExperts <= 512) {
-        RouteTokenN<16>(logits, bias, numExperts, topK, scoreFunc, renormalize, routedScale, lane, idsOut, weightsOut);
-    } else {
-        RouteTokenN<EP_MAX_EXPERTS / 32>(logits, bias, numExperts, topK, scoreFunc, renormalize, routedScale, lane, idsOut,
-                                         weightsOut);
+        return RouteTokenN<8>(logits, bias, numExperts, topK, scoreFunc, renormalize, routedScale, lane, idsOut, weightsOut);
     }
+    if (numExperts <= 512) {
+        return RouteTokenN<16>(logits, bias, numExperts, topK, scoreFunc, renormalize, routedScale, lane, idsOut, weightsOut);
+    }
+    return RouteTokenN<EP_MAX_EXPERTS / 32>(logits, bias, numExperts, topK, scoreFunc, renormalize, routedScale, lane, idsOut, weightsOut);
 }
 
 __global__ void __launch_bounds__(256) RoutingTopKKernel(const RoutingArgs a)
@@ -293,26 +293,34 @@ __device__ void EpDispatchBody(const EpDispatchArgs &a)
     __shared__ int sIsLast;
     // A world of one rank: every row's final place is this rank's own output, so rows, scales and tuples are stored there
     // at once; nothing passes through the window and nobody has to be waited for.
-    const bool solo = R == 1;
+    const bool solo = R == 1 && a.directOwn != 0;
 
     const int t0 = min(a.bs, static_cast<int>(blockIdx.x * a.tokensPerBlock));
     const int t1 = min(a.bs, t0 + static_cast<int>(a.tokensPerBlock));
     const int nTok = t1 - t0;
     const int nRoutes = nTok * KR;
 
+    // The block's tokens start on their way to L2 now: memory is idle while the routes are counted.
+    {
+        const uint8_t *rows = a.x + static_cast<int64_t>(t0) * a.h * a.elemSize;
+        const int64_t bytes = static_cast<int64_t>(nTok) * a.h * a.elemSize;
+        for (int64_t off = static_cast<int64_t>(tid) * 128; off < bytes; off += static_cast<int64_t>(EP_BLOCK_THREADS) * 128) {
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(rows + off));
+        }
+    }
+
     // ---- 1. route, rank, count (routeExpert holds the COLUMN of a route, -1 when inactive) ---------------
     for (int e = tid; e < C; e += blockDim.x) sm.hist[e] = 0;
     for (int i = warp; i < nTok; i += EP_WARPS) {
         const int t = t0 + i;
+        int picked = -1;
         if (a.gateLogits != nullptr) {
-            RouteToken(a.gateLogits + static_cast<int64_t>(t) * E, a.selectionBias, E, K, a.scoreFunc, a.renormalize,
+            picked = RouteToken(a.gateLogits + static_cast<int64_t>(t) * E, a.selectionBias, E, K, a.scoreFunc, a.renormalize,
                        a.routedScale, lane, a.topkIdsOut + static_cast<int64_t>(t) * K,
                        a.topkWeightsOut + static_cast<int64_t>(t) * K);
-            __syncwarp();
         }
         if (lane < K) {
-            const int32_t *ids = a.gateLogits != nullptr ? a.topkIdsOut : a.expertIds;
-            int e = ids[static_cast<int64_t>(t) * K + lane];
+            int e = a.gateLogits != nullptr ? picked : a.expertIds[static_cast<int64_t>(t) * K + lane];
             if (e < 0 || e >= E) e = -1;
             if (a.maskType == TileXREp::TILEXR_EP_ACTIVE_MASK_TOKEN && a.activeMask[t] == 0) e = -1;
             if (a.maskType == TileXREp::TILEXR_EP_ACTIVE_MASK_EXPERT && a.activeMask[static_cast<int64_t>(t) * K + lane] == 0) e = -1;
@@ -428,20 +436,33 @@ __device__ void EpDispatchBody(const EpDispatchArgs &a)
         ok = BlockBroadcastOk(got) && ok;
     }
     if (ok) {
-        if (warp == 0) {
-            int carry = 0;
-            for (int base = 0; base < C; base += 32) {
-                int v = base + lane < C ? sm.total[base + lane] : 0;
+        // prefix sums of the totals: warps scan 32 columns each, then every warp scans the (at most 32) sums of those
+        const int groups32 = (C + 31) / 32;
+        int32_t *groupSum = reinterpret_cast<int32_t *>(sm.scaleStage) + EP_WARPS * 32;
+        for (int c = warp; c < groups32; c += EP_WARPS) {
+            int v = c * 32 + lane < C ? sm.total[c * 32 + lane] : 0;
 #pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int u = __shfl_up_sync(0xffffffffu, v, o);
-                    if (lane >= o) v += u;
-                }
-                v += carry;
-                if (base + lane < C) sm.colPrefix[base + lane + 1] = v;
-                carry = __shfl_sync(0xffffffffu, v, 31);
+            for (int o = 1; o < 32; o <<= 1) {
+                const int u = __shfl_up_sync(0xffffffffu, v, o);
+                if (lane >= o) v += u;
             }
-            if (lane == 0) sm.colPrefix[0] = 0;
+            if (c * 32 + lane < C) sm.colPrefix[c * 32 + lane + 1] = v;
+            if (lane == 31) groupSum[c] = v;
+        }
+        __syncthreads();
+        {
+            const int own = lane < groups32 ? groupSum[lane] : 0;
+            int v = own;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int u = __shfl_up_sync(0xffffffffu, v, o);
+                if (lane >= o) v += u;
+            }
+            for (int c = warp; c < groups32; c += EP_WARPS) {
+                const int before = __shfl_sync(0xffffffffu, v - own, c);
+                if (c * 32 + lane < C) sm.colPrefix[c * 32 + lane + 1] += before;
+            }
+            if (tid == 0) sm.colPrefix[0] = 0;
         }
         __syncthreads();
         for (int e = tid; e < C; e += blockDim.x) {
@@ -494,7 +515,7 @@ __device__ void EpDispatchBody(const EpDispatchArgs &a)
                     myRow = static_cast<uint32_t>(sm.dstRow[e] + sm.blockBase[e] + sm.routeRank[i * KR + lane]);
                     uint8_t *half = DataHalf(comm, dst, epoch);
                     // rows for this rank's own experts go to the output directly (the receive step skips their payload)
-                    uint8_t *payload = dst == rank
+                    uint8_t *payload = dst == rank && a.directOwn != 0
                                            ? a.expandXOut + static_cast<uint64_t>(myRow) * a.win.rowBytes
                                        : a.zeroCopy
                                            ? comm->registryPtr->regions[a.outHandle].peerBase[dst] + a.outOffset +
@@ -672,12 +693,36 @@ __device__ void EpDispatchBody(const EpDispatchArgs &a)
                 const uint64_t perPart = ((a.win.rowBytes + parts - 1) / parts + 511) & ~511ull;
                 const uint64_t b0 = min(static_cast<uint64_t>(a.win.rowBytes), perPart * part);
                 const uint64_t nBytes = min(static_cast<uint64_t>(a.win.rowBytes) - b0, perPart);
-                uint32_t m = payloadRoutes;
-                while (m != 0) {
-                    const int k = __ffs(m) - 1;
-                    m &= m - 1;
-                    uint8_t *p = reinterpret_cast<uint8_t *>(__shfl_sync(0xffffffffu, myPayload, k));
-                    if (nBytes > 0) CopyLanes(p + b0, row + b0, nBytes, lane, 32);
+                const bool odd = __any_sync(0xffffffffu, ((myPayload | reinterpret_cast<unsigned long long>(row)) & 15ull) != 0) || (nBytes & 15ull) != 0;
+                if (!odd) {
+                    // the part is fetched once and stored to every destination (one copy per destination fetched it again each
+                    // time, a round trip per 2 KB: 1009 x 4096, top-6, 10 us of the launch)
+                    const int vecs = static_cast<int>(nBytes / 16);
+                    for (int v0 = lane; v0 - lane < vecs; v0 += 4 * 32) {
+                        Vec16 q[4];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            if (v0 + u * 32 < vecs) q[u] = ld_vec16_stream(row + b0 + static_cast<int64_t>(v0 + u * 32) * 16);
+                        }
+                        uint32_t m = payloadRoutes;
+                        while (m != 0) {
+                            const int k = __ffs(m) - 1;
+                            m &= m - 1;
+                            uint8_t *p = reinterpret_cast<uint8_t *>(__shfl_sync(0xffffffffu, myPayload, k)) + b0;
+#pragma unroll
+                            for (int u = 0; u < 4; ++u) {
+                                if (v0 + u * 32 < vecs) st_vec16(p + static_cast<int64_t>(v0 + u * 32) * 16, q[u]);
+                            }
+                        }
+                    }
+                } else {
+                    uint32_t m = payloadRoutes;
+                    while (m != 0) {
+                        const int k = __ffs(m) - 1;
+                        m &= m - 1;
+                        uint8_t *p = reinterpret_cast<uint8_t *>(__shfl_sync(0xffffffffu, myPayload, k));
+                        if (nBytes > 0) CopyLanes(p + b0, row + b0, nBytes, lane, 32);
+                    }
                 }
             }
             if (myExpert >= 0 && part == 0) {
@@ -775,7 +820,7 @@ __device__ void EpDispatchBody(const EpDispatchArgs &a)
                 for (int i = warp; i < chunkRows; i += EP_WARPS) {
                     const int64_t r = base + i;
                     if ((reinterpret_cast<const uint2 *>(winExt + r * 8)->x & EP_LINK_FOLLOWER) != 0) continue;
-                    if (*reinterpret_cast<const int32_t *>(myHalf + a.win.assistOff + r * 16) == rank) continue;     // own token: already there
+                    if (a.directOwn != 0 && *reinterpret_cast<const int32_t *>(myHalf + a.win.assistOff + r * 16) == rank) continue;   // already there
                     CopyLanes(a.expandXOut + r * a.win.rowBytes, winPayload + r * a.win.rowBytes, a.win.rowBytes, lane, 32);
                 }
             }
@@ -1114,8 +1159,11 @@ __device__ void EpCombineBody(const EpCombineArgs &a)
         // ---- reduce this rank's tokens ------------------------------------------------------------------------
         const uint8_t *half = DataHalf(comm, rank, epoch);
         const uint32_t nReduce = static_cast<uint32_t>(a.bs) * P;
-        while (w.ok()) {
-            const uint32_t it = TakeItem(&cursors[1], lane);
+        // With no row to wait for the items are dealt out beforehand: a step of the cursor is a round trip to memory in front
+        // of every item.
+        const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+        for (uint32_t dealt = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w.ok(); dealt += warps) {
+            const uint32_t it = a.noSend != 0 ? dealt : TakeItem(&cursors[1], lane);
             if (it >= nReduce) break;
             const int64_t t = it / P;
             const uint32_t part = it - static_cast<uint32_t>(t) * P;
@@ -1124,6 +1172,7 @@ __device__ void EpCombineBody(const EpCombineArgs &a)
             int e = -1;
             float wk = 0.f;
             unsigned long long myRowPtr = 0;
+            const int64_t directRow = direct && lane < KR ? a.routeRows[t * KR + lane] : -1;     // beside the other loads, not behind them
             // `e` is the COLUMN of the route (shared ranks first, then routed experts), -1 when inactive
             if (lane < K) {
                 e = a.expertIds != nullptr ? a.expertIds[t * K + lane] : 0;
@@ -1154,7 +1203,7 @@ __device__ void EpCombineBody(const EpCombineArgs &a)
             }
             if (lane < KR && e >= 0) {
                 const int64_t slot = t * KR + lane;
-                const int64_t localRow = direct && myDst == rank ? a.routeRows[slot] : -1;
+                const int64_t localRow = myDst == rank ? directRow : -1;
                 if (localRow >= 0 && localRow < rows) {
                     myRowPtr = reinterpret_cast<unsigned long long>(a.expertOut + localRow * a.rowBytes);
                 } else {

@@ -103,6 +103,7 @@ struct EpDispatchArgs {
     float *expandScalesOut;          // [maxRecvRows] or null
     int32_t *assistExtOut;           // [maxRecvRows, 2] or null
     uint32_t dedup;
+    uint32_t directOwn;              // rows for this rank's own experts may be stored to expandXOut by the sender (16-byte aligned)
 };
 
 struct EpCombineArgs {

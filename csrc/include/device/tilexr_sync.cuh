@@ -286,8 +286,11 @@ __device__ __forceinline__ void KernelEpilogue(Waiter &w, bool ok, int scratchWo
     __shared__ int sLastToLeave;
     __syncthreads();
     CommArgs *a = w.args;
+    // Without peers the order among the rank's own blocks is all there is to keep (the counter's acquire and release, and
+    // the end of the launch): the system-wide fence of every block cost about 3 us in a launch of 32 small blocks.
+    const bool alone = a->rankSize == 1;
     if (threadIdx.x == 0) {
-        fence_acq_rel_sys();
+        if (!alone) fence_acq_rel_sys();
         uint32_t *exitCounter =
             reinterpret_cast<uint32_t *>(CtrlWord(a, a->rank, TILEXR_CTRL_GRIDBAR_WORD + TILEXR_CTRL_GRIDBAR_COUNT));
         sLastToLeave = atom_add_acq_rel_gpu_u32(exitCounter, 1) == gridDim.x - 1 ? 1 : 0;
@@ -305,7 +308,8 @@ __device__ __forceinline__ void KernelEpilogue(Waiter &w, bool ok, int scratchWo
             uint32_t *exitCounter =
                 reinterpret_cast<uint32_t *>(CtrlWord(a, a->rank, TILEXR_CTRL_GRIDBAR_WORD + TILEXR_CTRL_GRIDBAR_COUNT));
             st_release_gpu_u32(exitCounter, 0);
-            PublishDone(w);
+            if (alone) st_relaxed_sys_u64(CtrlWord(a, a->rank, TILEXR_CTRL_DONE_WORD + a->rank), MakeFlag(w.epoch, 0));
+            else PublishDone(w);
             *CtrlWord(a, a->rank, TILEXR_CTRL_EPOCH_WORD) = w.epoch;
             if (a->dfx[TileXR::TILEXR_DFX_FAIL_CODE] == 0 && ok) {
                 a->dfx[TileXR::TILEXR_DFX_RUN_STATUS] = TILEXR_RUN_FINISHED;

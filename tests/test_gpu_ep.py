@@ -514,3 +514,26 @@ def test_dispatch_of_a_single_rank_stores_rows_at_their_place(txr, tokens, exper
             assert torch.equal(d.expand_x[:n].view(torch.uint8), want.view(torch.uint8)) and torch.equal(d.dynamic_scales[:n], scales)
     finally:
         comm.destroy()
+
+
+@pytest.mark.parametrize("ranks", [1, 2])
+def test_dispatch_into_an_output_off_the_16_byte_grid(txr, ranks):
+    """A caller's output that starts between 16-byte boundaries takes the way through the window."""
+    ep = txr.ep
+    h, tokens, experts, top_k = 64, 37, 8, 3
+    g = torch.Generator().manual_seed(7)
+    xs = [torch.randn(tokens, h, generator=g).to(torch.bfloat16).cuda() for _ in range(ranks)]
+    ids = [torch.stack([torch.randperm(experts, generator=g)[:top_k] for _ in range(tokens)]).to(torch.int32).cuda() for _ in range(ranks)]
+    cap = tokens * ranks * top_k
+    outs = [torch.zeros(cap * h + 8, dtype=torch.bfloat16, device="cuda")[3:3 + cap * h].view(cap, h) for _ in range(ranks)]
+    world = txr.init_emulated_world(ranks, device=0, buffer_mb=64)
+    try:
+        ds = world.run(lambda c, r: ep.dispatch(c, xs[r], expert_ids=ids[r], num_experts=experts, top_k=top_k, max_recv_rows=cap, expand_x_out=outs[r]))
+        world.check()
+        for r, d in enumerate(ds):
+            assert d.expand_x.data_ptr() % 16 != 0
+            n = int(d.recv_total)
+            tuples = d.assist[:n].cpu().tolist()
+            assert n > 0 and torch.equal(d.expand_x[:n], torch.stack([xs[s][t] for s, t, _, _ in tuples]))
+    finally:
+        world.destroy()
