@@ -352,7 +352,7 @@ int TileXRMoeEpDispatchFused(const TileXREpDispatchParams *p, TileXRCommPtr comm
         }
         smem = EpDispatchSmemBytes(static_cast<int>(smemCols), static_cast<int>(tokensPerBlock * routesPerToken));
         unsigned maxGrid = 0;
-        ret = MaxCooperativeGrid(comm, EpDispatchKernelEntry(), EP_BLOCK_THREADS, smem, ranksPerDevice, &maxGrid);
+        ret = MaxCooperativeGrid(comm, EpDispatchKernelEntry(p->quantMode), EP_BLOCK_THREADS, smem, ranksPerDevice, &maxGrid);
         if (ret != TILEXR_SUCCESS) return ret;
         if (maxGrid == 0) return TILEXR_ERROR_NOT_SUPPORT;
         gridCap = maxGrid;
@@ -432,7 +432,7 @@ int TileXRMoeEpDispatchFused(const TileXREpDispatchParams *p, TileXRCommPtr comm
         a.perfTrace = PerfTracePrepareLaunch(info, stream);
     }
     LaunchConfig cfg{grid, EP_BLOCK_THREADS, smem, true};
-    return LaunchKernel(comm, EpDispatchKernelEntry(), &a, cfg, stream);
+    return LaunchKernel(comm, EpDispatchKernelEntry(p->quantMode), &a, cfg, stream);
 }
 
 int TileXRMoeEpCombineFused(const TileXREpCombineParams *p, TileXRCommPtr comm, TileXRStream stream)
@@ -823,6 +823,17 @@ int TileXRMxfp8Dequant(const void *y, const uint8_t *scales, int64_t rows, int64
     }
     return LaunchMxfp8Dequant(y, scales, rows, h, fp8Type == TILEXR_DATA_TYPE_FP8E5M2, dtype == TILEXR_DATA_TYPE_BFP16, xOut,
                               stream);
+}
+
+int TileXRMoeRouterLogits(const void *x, const float *gate, int64_t bs, int64_t h, int64_t moeExpertNum, TileXRDataType dtype, float *logitsOut,
+                          TileXRStream stream)
+{
+    if (x == nullptr || gate == nullptr || logitsOut == nullptr || bs <= 0 || h <= 0 || h % 8 != 0 || moeExpertNum <= 0 || !HalfType(dtype) ||
+        bs > INT32_MAX / 8 || h > INT32_MAX / 2 || moeExpertNum > 65535 * 32 ||
+        ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gate)) & 15u) != 0) {
+        return TILEXR_ERROR_PARA_CHECK_FAIL;
+    }
+    return LaunchRouterLogits(x, gate, bs, h, moeExpertNum, dtype == TILEXR_DATA_TYPE_BFP16, logitsOut, stream);
 }
 
 int TileXRMoeEpCombineBackward(const void *g, const float *weights, const void *rows, const int32_t *assist, const int32_t *rowCount,

@@ -256,6 +256,11 @@ __device__ void SumBlockCounts(const int32_t *counts, int E, int nb, int32_t *ou
 // nothing (combine); chunk_barrier = wait for the earlier blocks' counts; post_sync = count exchange and row placement;
 // local_input_to_ipc = rows pushed to their destinations; flag_poll_wait = waiting for arrivals;
 // peer_ipc_to_output = window to output (dispatch) or the weighted reduction (combine).
+// One kernel per kind of transport: with all of them in one the registers of a 512-thread block (64, two blocks per SM) ran
+// out (628 bytes of spill loads against 340; 4096 x 7168 fp8 96 -> 92 us).
+enum EpTransport : int { EP_PLAIN = 0, EP_FP8 = 1, EP_MXFP8 = 2, EP_INT8 = 3 };
+
+template <int TRANSPORT>
 __device__ void EpDispatchBody(const EpDispatchArgs &a)
 {
     extern __shared__ __align__(16) uint8_t smemRaw[];
@@ -485,11 +490,11 @@ __device__ void EpDispatchBody(const EpDispatchArgs &a)
     PerfStageBegin(perf, TILEXR_PERF_LOCAL_INPUT_TO_IPC);
     if (ok) {
         const bool bf16 = a.isBf16 != 0;
-        const bool mx = a.quantMode == TileXREp::TILEXR_EP_QUANT_MXFP8_E4M3 || a.quantMode == TileXREp::TILEXR_EP_QUANT_MXFP8_E5M2;
+        constexpr bool mx = TRANSPORT == EP_MXFP8;
         const bool mxE5m2 = a.quantMode == TileXREp::TILEXR_EP_QUANT_MXFP8_E5M2;
-        const bool quant = mx || a.quantMode == TileXREp::TILEXR_EP_QUANT_FP8_1X128;
+        constexpr bool quant = mx || TRANSPORT == EP_FP8;
         const bool int8Dynamic = a.quantMode == TileXREp::TILEXR_EP_QUANT_DYNAMIC_INT8;
-        const bool int8Mode = int8Dynamic || a.quantMode == TileXREp::TILEXR_EP_QUANT_STATIC_INT8;
+        constexpr bool int8Mode = TRANSPORT == EP_INT8;
         const int chunks = a.h / 16;             // 16 elements per lane and iteration (fp8 paths)
         const int iters = (chunks + 31) / 32;
         // A block with few tokens (small batches) cuts every token into column ranges for several warps.
@@ -1270,7 +1275,10 @@ __device__ void EpCombineBody(const EpCombineArgs &a)
     KernelEpilogue(w, ok, EP_SCRATCH_TOTALS_WORD);      // the cursors and the bucket counts
 }
 
-TILEXR_DEFINE_KERNEL_OCC(TileXREpDispatchKernel, EpDispatchArgs, EpDispatchBody, EP_BLOCK_THREADS, 2)
+TILEXR_DEFINE_KERNEL_OCC(TileXREpDispatchKernel, EpDispatchArgs, EpDispatchBody<EP_PLAIN>, EP_BLOCK_THREADS, 2)
+TILEXR_DEFINE_KERNEL_OCC(TileXREpDispatchKernelFp8, EpDispatchArgs, EpDispatchBody<EP_FP8>, EP_BLOCK_THREADS, 2)
+TILEXR_DEFINE_KERNEL_OCC(TileXREpDispatchKernelMxfp8, EpDispatchArgs, EpDispatchBody<EP_MXFP8>, EP_BLOCK_THREADS, 2)
+TILEXR_DEFINE_KERNEL_OCC(TileXREpDispatchKernelInt8, EpDispatchArgs, EpDispatchBody<EP_INT8>, EP_BLOCK_THREADS, 2)
 TILEXR_DEFINE_KERNEL_OCC(TileXREpCombineKernel, EpCombineArgs, EpCombineBody, EP_BLOCK_THREADS, 2)
 
 // ---- stand-alone quantisation and norm kernels ---------------------------------------------------------------
@@ -1599,7 +1607,17 @@ int CheckLaunch(const char *what)
 
 } // namespace
 
-const KernelEntry &EpDispatchKernelEntry() { return TileXREpDispatchKernelEntry; }
+const KernelEntry &EpDispatchKernelEntry(int64_t quantMode)
+{
+    switch (quantMode) {
+        case TileXREp::TILEXR_EP_QUANT_FP8_1X128: return TileXREpDispatchKernelFp8Entry;
+        case TileXREp::TILEXR_EP_QUANT_MXFP8_E4M3:
+        case TileXREp::TILEXR_EP_QUANT_MXFP8_E5M2: return TileXREpDispatchKernelMxfp8Entry;
+        case TileXREp::TILEXR_EP_QUANT_STATIC_INT8:
+        case TileXREp::TILEXR_EP_QUANT_DYNAMIC_INT8: return TileXREpDispatchKernelInt8Entry;
+        default: return TileXREpDispatchKernelEntry;
+    }
+}
 const KernelEntry &EpCombineKernelEntry() { return TileXREpCombineKernelEntry; }
 
 size_t EpDispatchSmemBytes(int numExperts, int routesPerBlock)

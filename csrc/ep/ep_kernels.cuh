@@ -153,13 +153,15 @@ struct RoutingArgs {
     float routedScale;
 };
 
-const KernelEntry &EpDispatchKernelEntry();
+const KernelEntry &EpDispatchKernelEntry(int64_t quantMode);      // a kernel per kind of transport
 const KernelEntry &EpCombineKernelEntry();
 
 // Plain (non communicating) kernels, launched directly.
 int LaunchRoutingTopK(const RoutingArgs &args, void *stream);
 // rows [gate | up] -> silu(gate) * up; with `scales` quantised to e4m3 per 128 elements (f % 128 == 0), else f % 8 == 0
 int LaunchSwiglu(const void *gateUp, int64_t rows, int64_t f, bool bf16, void *y, float *scales, void *stream);
+// logits [tokens, experts] = x [tokens, h] (16-bit) x gate [experts, h]^T (fp32) in fp32; h % 8 == 0, 16-byte aligned operands (router_logits.cu)
+int LaunchRouterLogits(const void *x, const float *gate, int64_t tokens, int64_t h, int64_t experts, bool bf16, float *out, void *stream);
 int LaunchCombineBackward(const void *g, const float *weights, const void *rows, const int32_t *assist, const int32_t *rowCount, int64_t capacity,
                           int64_t h, bool bf16, int slots, int wideCols, void *gradRows, void *wide, void *stream);
 int LaunchFp8Quant1x128(const void *x, int64_t rows, int64_t h, bool bf16, void *y, float *scales, void *stream);

@@ -203,6 +203,10 @@ int TileXRMxfp8Quant(const void *x, int64_t rows, int64_t h, TXR_DT dtype, TXR_D
                      TileXRStream stream);
 int TileXRMxfp8Dequant(const void *y, const uint8_t *scales, int64_t rows, int64_t h, TXR_DT fp8Type, TXR_DT dtype,
                        void *xOut, TileXRStream stream);
+// Router logits in fp32: logitsOut [bs, moeExpertNum] = x [bs, h] (fp16 / bf16) * gate [moeExpertNum, h]^T (fp32); h a multiple of 8,
+// x and gate 16-byte aligned.
+int TileXRMoeRouterLogits(const void *x, const float *gate, int64_t bs, int64_t h, int64_t moeExpertNum, TXR_DT dtype, float *logitsOut,
+                          TileXRStream stream);
 // Backward of a weighted combine, over the rows a dispatch of the output gradient delivered (`g` [capacity, h], its row weights,
 // assist tuples and *rowCount): gradRows[r] = weights[r] * g[r]; with `rows` (the expert rows the combine summed) also
 // <g[r], rows[r]> as a (high, low) bf16 pair in columns 2 s and 2 s + 1 of wide[r] ([capacity, wideCols] bf16, the other columns zero),

@@ -534,6 +534,18 @@ at::Tensor EpCombine(const CommPtr &c, const at::Tensor &expertOut, const at::Te
     return y;
 }
 
+at::Tensor RouterLogits(const at::Tensor &x, const at::Tensor &gate)
+{
+    TORCH_CHECK(x.is_cuda() && x.dim() == 2 && x.is_contiguous() && gate.is_cuda() && gate.dim() == 2 && gate.is_contiguous() &&
+                    gate.scalar_type() == at::kFloat && gate.size(1) == x.size(1),
+                "x [tokens, h] 16-bit and gate [experts, h] fp32, contiguous CUDA tensors");
+    at::Tensor out = at::empty({x.size(0), gate.size(0)}, gate.options());
+    Check(TileXRMoeRouterLogits(x.data_ptr(), gate.data_ptr<float>(), x.size(0), x.size(1), gate.size(0), ToDtype(x.scalar_type()),
+                                out.data_ptr<float>(), StreamOf(x)),
+          "TileXRMoeRouterLogits");
+    return out;
+}
+
 // (grad_rows, wide | None), see TileXRMoeEpCombineBackward
 py::tuple EpCombineBackward(const at::Tensor &g, const at::Tensor &weights, const c10::optional<at::Tensor> &rows, const at::Tensor &assist,
                             const at::Tensor &rowCount, int64_t slots, int64_t wideCols)
@@ -760,6 +772,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m)
     m.def("routing_topk", &RoutingTopK, py::arg("gate_logits"), py::arg("selection_bias") = py::none(), py::arg("top_k") = 1,
           py::arg("score_func") = 0, py::arg("renormalize") = true, py::arg("routed_scale") = 1.0);
     m.def("ep_combine_backward", &EpCombineBackward);
+    m.def("router_logits", &RouterLogits);
     m.def("fp8_quant_1x128", &Fp8Quant);
     m.def("swiglu", &Swiglu);
     m.def("swiglu_fp8_quant_1x128", &SwigluFp8Quant);

@@ -78,3 +78,18 @@ def test_mxfp8_dequant_rows_of_any_length(txr, rows, h, e5m2):
     got = txr.quant.mxfp8_dequant(q, s)
     scale = torch.exp2(s.float() - 127).repeat_interleave(32, dim=1)[:, :h]
     assert torch.equal(got, (q.float() * scale).to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("tokens,h,experts", [(1, 8, 1), (32, 2048, 64), (63, 264, 33), (65, 2048, 32), (130, 1032, 60), (1000, 7168, 256)])
+def test_router_logits_in_fp32(txr, tokens, h, experts, dtype):
+    """K shorter than a chunk, parts of K that are empty or ragged, tokens and experts off the tile."""
+    g = torch.Generator().manual_seed(h)
+    x = torch.randn(tokens, h, generator=g).to(dtype).cuda()
+    gate = (torch.randn(experts, h, generator=g) * h ** -0.5).cuda()
+    got = txr.quant.router_logits(x, gate)
+    want = x.double() @ gate.double().t()
+    # a chain of at most 32 * ceil(h / 256) multiply-adds per warp and 15 additions behind it, each half an fp32 unit of a partial sum
+    steps = 32 * ((h + 255) // 256) + 16
+    bound = (x.double().abs() @ gate.double().abs().t()) * steps * 2.0 ** -24
+    assert got.dtype == torch.float32 and ((got.double() - want).abs() <= bound).all()

@@ -54,6 +54,16 @@ class ExpertParallelMoE(torch.nn.Module):
             self.w2 = None
 
     def route_logits(self, x: torch.Tensor) -> torch.Tensor:
+        gate = self.gate
+        graph = torch.is_grad_enabled() and (x.requires_grad or gate.requires_grad)
+        # The kernel's multiply-adds run at about two thirds of the library's rate, but it reads 16-bit tokens where the library
+        # needs an fp32 copy: 66 against 221 us for 4096 x 7168 by 32 experts, 136 against 139 for 3000 x 4096 by 128, 457 against
+        # 371 for 4096 x 7168 by 256; with few tokens it wins at any expert count (43 against 73 us for 128 x 7168 by 256).
+        favourable = gate.shape[0] <= 128 or x.shape[0] * gate.shape[0] <= 131072
+        if (favourable and not graph and x.is_cuda and x.device == gate.device and x.dtype in (torch.float16, torch.bfloat16) and gate.dtype == torch.float32
+                and x.dim() == 2 and x.shape[0] > 0 and x.shape[1] == gate.shape[1] and x.shape[1] % 8 == 0 and x.is_contiguous()
+                and gate.is_contiguous() and x.data_ptr() % 16 == 0 and gate.data_ptr() % 16 == 0 and not torch.is_autocast_enabled()):
+            return quant.router_logits(x, gate)
         return torch.matmul(x.float(), self.gate.t()).contiguous()
 
     def experts(self, rows: torch.Tensor, token_nums: torch.Tensor) -> torch.Tensor:

@@ -39,6 +39,12 @@ def mxfp8_dequant(y: torch.Tensor, scales: torch.Tensor, dtype=torch.bfloat16) -
     return _C.mxfp8_dequant(y, scales, dtype)
 
 
+def router_logits(x: torch.Tensor, gate: torch.Tensor) -> torch.Tensor:
+    """``x.float() @ gate.T`` for 16-bit ``x`` [tokens, h] and an fp32 ``gate`` [experts, h] (h a multiple of 8) with fp32
+    multiply-adds and without the fp32 copy of ``x``."""
+    return _C.router_logits(x, gate)
+
+
 def routing_topk(gate_logits: torch.Tensor, top_k: int, score_func: int = SCORE_SOFTMAX, renormalize: bool = True,
                  routed_scale: float = 1.0, selection_bias: Optional[torch.Tensor] = None):
     return _C.routing_topk(gate_logits.contiguous(), selection_bias, top_k, score_func, renormalize, routed_scale)
