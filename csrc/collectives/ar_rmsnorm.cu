@@ -73,12 +73,11 @@ __device__ __forceinline__ uint64_t *FlagB(const ArNormArgs &a, int owner, int s
     return FlagSlot(a.comm, owner, TILEXR_FLAG_ACK_BASE + static_cast<int64_t>(src) * TILEXR_FLAGS_PER_PAIR + row);
 }
 
-// Sums row `row` over all ranks in rank order (`srcOf(s)` gives rank s's copy), adds the
-// residual, normalises.  Leaves y and the new residual in `yDst` / `resDst` (local) and,
-// when `stage` is not null, also in stage[0] (y) and stage[1] (residual) for the fan-out.
-template <typename SrcFn>
-__device__ __forceinline__ void ReduceNormRow(const ArNormArgs &a, SrcFn srcOf, int R, const uint8_t *resSrc, uint8_t *resDst,
-                                              uint8_t *yDst, float *sPartial)
+// Sums a row over all ranks in rank order (`srcOf(s)` gives rank s's copy), adds the residual, normalises.  Every 16-byte
+// column of the new residual goes to `putRes(v, column)` and of the result to `putY(v, column)`, straight from registers:
+// two-shot stores them to the own tensors and to every peer at once.
+template <typename SrcFn, typename ResFn, typename YFn>
+__device__ __forceinline__ void ReduceNormRow(const ArNormArgs &a, SrcFn srcOf, int R, const uint8_t *resSrc, ResFn putRes, YFn putY, float *sPartial)
 {
     const bool bf16 = a.isBf16 != 0;
     const int vecs = a.rowBytes / 16;
@@ -115,7 +114,7 @@ __device__ __forceinline__ void ReduceNormRow(const ArNormArgs &a, SrcFn srcOf, 
             }
             // the sum rounded to the storage type is the new residual AND the norm input
             const Vec16 packed = Pack8(acc, bf16);
-            if (resDst != nullptr) st_vec16(resDst + v * 16, packed);
+            if (resSrc != nullptr) putRes(v, packed);
             Unpack8(packed, bf16, vals[i]);
 #pragma unroll
             for (int j = 0; j < 8; ++j) ss += vals[i][j] * vals[i][j];
@@ -138,7 +137,33 @@ __device__ __forceinline__ void ReduceNormRow(const ArNormArgs &a, SrcFn srcOf, 
             Unpack8(ld_vec16(a.gamma + v * 16), bf16, g);
 #pragma unroll
             for (int j = 0; j < 8; ++j) o[j] = vals[i][j] * rstd * g[j];
-            st_vec16(yDst + v * 16, Pack8(o, bf16));
+            putY(v, Pack8(o, bf16));
+        }
+    }
+}
+
+// Rows a block copies, or reduces, before it raises their flags, or waits for them: one thread per flag behind one block barrier.
+// A system-wide release takes about 5 us while every SM stores; one per row and phase made up most of the launch
+// (256 x 7168 on four emulated ranks: 62 us with one row at a time, 40 us so).
+constexpr int ARN_GROUP = 8;
+constexpr int ARN_OWN_GROUP = 4;
+
+// Copies `rows` rows (at most ARN_GROUP) of `vecs` 16-byte columns; `srcRow(g)` and `dstRow(g)` give row g's ends.
+template <typename SrcFn, typename DstFn>
+__device__ __forceinline__ void CopyRows(int rows, int vecs, SrcFn srcRow, DstFn dstRow)
+{
+    const int total = rows * vecs;
+    for (int i0 = static_cast<int>(threadIdx.x); i0 < total; i0 += 4 * static_cast<int>(ARN_THREADS)) {
+        Vec16 q[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int i = i0 + u * static_cast<int>(ARN_THREADS);
+            if (i < total) q[u] = ld_vec16_stream(srcRow(i / vecs) + static_cast<int64_t>(i % vecs) * 16);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int i = i0 + u * static_cast<int>(ARN_THREADS);
+            if (i < total) st_vec16(dstRow(i / vecs) + static_cast<int64_t>(i % vecs) * 16, q[u]);
         }
     }
 }
@@ -155,25 +180,37 @@ __device__ void ArNormBody(const ArNormArgs &a)
     const int tid = threadIdx.x;
     const uint64_t rb = a.rowBytes;
 
+    const int vecs = static_cast<int>(rb / 16);
+    const int step = static_cast<int>(gridDim.x);
+
     if (ok && !a.twoShot) {
         // push every row of mine to every peer, then reduce every row
-        for (int row = blockIdx.x; row < a.rows; row += gridDim.x) {
+        for (int row = blockIdx.x; row < a.rows; row += step) {
             const uint8_t *src = a.x + row * rb;
-            for (int i = 1; i < R; ++i) {
-                const int peer = (rank + i) % R;
-                CopyLanes(PlaneA(a, peer, rank, row, epoch), src, rb, tid, blockDim.x);
+            for (int v0 = tid; v0 < vecs; v0 += 2 * static_cast<int>(ARN_THREADS)) {
+                const int v1 = v0 + static_cast<int>(ARN_THREADS);
+                const Vec16 q0 = ld_vec16_stream(src + v0 * 16);
+                Vec16 q1 = q0;
+                if (v1 < vecs) q1 = ld_vec16_stream(src + v1 * 16);
+                for (int i = 1; i < R; ++i) {
+                    uint8_t *dst = PlaneA(a, rank + i < R ? rank + i : rank + i - R, rank, row, epoch);
+                    st_vec16(dst + v0 * 16, q0);
+                    if (v1 < vecs) st_vec16(dst + v1 * 16, q1);
+                }
             }
             __syncthreads();
             if (tid < R && tid != rank) SetFlag(FlagA(a, tid, rank, row), epoch, 1);
         }
-        for (int row = blockIdx.x; row < a.rows && ok; row += gridDim.x) {
+        for (int row = blockIdx.x; row < a.rows && ok; row += step) {
             bool got = true;
             if (tid < R && tid != rank) got = WaitFlagGE(w, FlagA(a, rank, tid, row), 1, tid, row);
             ok = BlockBroadcastOk(got);
             if (!ok) break;
             auto srcOf = [&](int s) -> const uint8_t * { return s == rank ? a.x + row * rb : PlaneA(a, rank, s, row, epoch); };
             uint8_t *res = a.residual != nullptr ? a.residual + row * rb : nullptr;
-            ReduceNormRow(a, srcOf, R, res, res, a.y + row * rb, sPartial);
+            uint8_t *yRow = a.y + row * rb;
+            ReduceNormRow(a, srcOf, R, res, [&](int v, const Vec16 &q) { st_vec16(res + v * 16, q); },
+                          [&](int v, const Vec16 &q) { st_vec16(yRow + v * 16, q); }, sPartial);
         }
     } else if (ok) {
         const int per = a.rowsPerRank;
@@ -181,56 +218,72 @@ __device__ void ArNormBody(const ArNormArgs &a)
         const int myRows = max(0, min(per, a.rows - myFirst));
         // 1. rows of other owners go to their owner
         const int foreign = a.rows - myRows;
-        for (int it = blockIdx.x; it < foreign; it += gridDim.x) {
-            // enumerate foreign rows starting after my own range so that ranks start on different owners
-            const int row = (min(myFirst, a.rows) + myRows + it) % a.rows;   // with fewer rows than ranks myFirst lies past the end
-            const int owner = row / per;
-            const int local = row - owner * per;
-            CopyLanes(PlaneA(a, owner, rank, local, epoch), a.x + row * rb, rb, tid, blockDim.x);
+        // foreign rows are enumerated starting after my own range so that ranks start on different owners
+        auto foreignRow = [&](int it) { return (min(myFirst, a.rows) + myRows + it) % a.rows; };   // with fewer rows than ranks myFirst lies past the end
+        for (int it0 = blockIdx.x; it0 < foreign; it0 += ARN_GROUP * step) {
+            const int n = min(ARN_GROUP, (foreign - it0 + step - 1) / step);
+            CopyRows(n, vecs, [&](int g) { return a.x + foreignRow(it0 + g * step) * rb; },
+                     [&](int g) {
+                         const int row = foreignRow(it0 + g * step);
+                         return PlaneA(a, row / per, rank, row % per, epoch);
+                     });
             __syncthreads();
-            if (tid == 0) SetFlag(FlagA(a, owner, rank, local), epoch, 1);
+            if (tid < n) {
+                const int row = foreignRow(it0 + tid * step);
+                SetFlag(FlagA(a, row / per, rank, row % per), epoch, 1);
+            }
         }
         // 2. my rows: reduce, normalise, fan out
-        for (int local = blockIdx.x; local < myRows && ok; local += gridDim.x) {
-            const int row = myFirst + local;
-            bool got = true;
-            if (tid < R && tid != rank) got = WaitFlagGE(w, FlagA(a, rank, tid, local), 1, tid, local);
-            ok = BlockBroadcastOk(got);
-            if (!ok) break;
-            auto srcOf = [&](int s) -> const uint8_t * { return s == rank ? a.x + row * rb : PlaneA(a, rank, s, local, epoch); };
-            uint8_t *yRow = a.y + row * rb;
-            uint8_t *resRow = a.residual != nullptr ? a.residual + row * rb : nullptr;
-            ReduceNormRow(a, srcOf, R, resRow, resRow, yRow, sPartial);
-            __syncthreads();   // the finished row is read back below by other threads
-            for (int i = 1; i < R; ++i) {
-                const int peer = (rank + i) % R;
-                uint8_t *yDst, *rDst;
-                if (a.zeroCopy) {
-                    yDst = comm->registryPtr->regions[a.yHandle].peerBase[peer] + a.yOffset + row * rb;
-                    rDst = resRow != nullptr ? comm->registryPtr->regions[a.resHandle].peerBase[peer] + a.resOffset + row * rb : nullptr;
-                } else {
-                    yDst = PlaneB(a, peer, rank, local, 0, epoch, per);
-                    rDst = resRow != nullptr ? PlaneB(a, peer, rank, local, 1, epoch, per) : nullptr;
-                }
-                CopyLanes(yDst, yRow, rb, tid, blockDim.x);
-                if (rDst != nullptr) CopyLanes(rDst, resRow, rb, tid, blockDim.x);
+        for (int local0 = blockIdx.x; local0 < myRows && ok; local0 += ARN_OWN_GROUP * step) {
+            const int n = min(ARN_OWN_GROUP, (myRows - local0 + step - 1) / step);
+            for (int g = 0; g < n; ++g) {
+                const int local = local0 + g * step;
+                const int row = myFirst + local;
+                bool got = true;
+                if (tid < R && tid != rank) got = WaitFlagGE(w, FlagA(a, rank, tid, local), 1, tid, local);
+                ok = BlockBroadcastOk(got);
+                if (!ok) break;
+                auto srcOf = [&](int s) -> const uint8_t * { return s == rank ? a.x + row * rb : PlaneA(a, rank, s, local, epoch); };
+                uint8_t *yRow = a.y + row * rb;
+                uint8_t *resRow = a.residual != nullptr ? a.residual + row * rb : nullptr;
+                auto putAll = [&](int v, const Vec16 &q, uint8_t *mine, int which, uint32_t handle, uint64_t offset) {
+                    st_vec16(mine + v * 16, q);
+                    for (int i = 1; i < R; ++i) {
+                        const int peer = rank + i < R ? rank + i : rank + i - R;
+                        uint8_t *dst = a.zeroCopy ? comm->registryPtr->regions[handle].peerBase[peer] + offset + row * rb
+                                                  : PlaneB(a, peer, rank, local, which, epoch, per);
+                        st_vec16(dst + v * 16, q);
+                    }
+                };
+                ReduceNormRow(a, srcOf, R, resRow, [&](int v, const Vec16 &q) { putAll(v, q, resRow, 1, a.resHandle, a.resOffset); },
+                              [&](int v, const Vec16 &q) { putAll(v, q, yRow, 0, a.yHandle, a.yOffset); }, sPartial);
             }
+            if (!ok) break;
             __syncthreads();
-            if (tid < R && tid != rank) SetFlag(FlagB(a, tid, rank, local), epoch, 1);
+            for (int f = tid; f < n * R; f += static_cast<int>(ARN_THREADS)) {
+                if (f % R != rank) SetFlag(FlagB(a, f % R, rank, local0 + f / R * step), epoch, 1);
+            }
         }
         // 3. rows of other owners come back normalised
-        for (int it = blockIdx.x; it < foreign && ok; it += gridDim.x) {
-            const int row = (min(myFirst, a.rows) + myRows + it) % a.rows;   // with fewer rows than ranks myFirst lies past the end
-            const int owner = row / per;
-            const int local = row - owner * per;
+        for (int it0 = blockIdx.x; it0 < foreign && ok; it0 += ARN_GROUP * step) {
+            const int n = min(ARN_GROUP, (foreign - it0 + step - 1) / step);
             bool got = true;
-            if (tid == 0) got = WaitFlagGE(w, FlagB(a, rank, owner, local), 1, owner, local);
+            if (tid < n) {
+                const int row = foreignRow(it0 + tid * step);
+                got = WaitFlagGE(w, FlagB(a, rank, row / per, row % per), 1, row / per, row % per);
+            }
             ok = BlockBroadcastOk(got);
             if (ok && !a.zeroCopy) {
-                CopyLanes(a.y + row * rb, PlaneB(a, rank, owner, local, 0, epoch, per), rb, tid, blockDim.x);
-                if (a.residual != nullptr) {
-                    CopyLanes(a.residual + row * rb, PlaneB(a, rank, owner, local, 1, epoch, per), rb, tid, blockDim.x);
-                }
+                auto back = [&](uint8_t *base, int which) {
+                    CopyRows(n, vecs,
+                             [&](int g) {
+                                 const int row = foreignRow(it0 + g * step);
+                                 return static_cast<const uint8_t *>(PlaneB(a, rank, row / per, row % per, which, epoch, per));
+                             },
+                             [&](int g) { return base + foreignRow(it0 + g * step) * rb; });
+                };
+                back(a.y, 0);
+                if (a.residual != nullptr) back(a.residual, 1);
             }
         }
     }

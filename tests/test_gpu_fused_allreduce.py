@@ -71,3 +71,12 @@ def test_choice_by_size(txr):
     assert txr._C.all_reduce_rmsnorm_choose(16 * 1024, 8) == 1
     assert txr._C.all_reduce_rmsnorm_choose(4 << 20, 8) == 2
     assert txr._C.all_reduce_rmsnorm_choose(4 << 20, 2) == 1
+
+
+@pytest.mark.parametrize("ranks,rows,h,algo,with_res,symmetric", [
+    (4, 2000, 264, 2, True, False),       # several groups of rows per block in every phase, the last one ragged
+    (3, 1501, 1032, 2, True, True),
+    (2, 700, 9000, 1, False, False),      # rows longer than two 16-byte columns per thread
+])
+def test_all_reduce_rmsnorm_groups_of_rows(txr, ranks, rows, h, algo, with_res, symmetric):
+    test_all_reduce_rmsnorm(txr, ranks, rows, h, algo, with_res, symmetric)
