@@ -80,8 +80,9 @@ enum GemmEpilogue : int32_t { GEMM_EPI_STORE = 0, GEMM_EPI_SWIGLU = 1 };
 // Block-scaled fp8 GEMM (gemm_tcgen05_fp8_block.cu): warp 0 TMA, warp 1 MMA, warps 4-11 fold the scratch accumulators.
 constexpr unsigned GEMM_FP8_BLOCK_THREADS = 384;
 constexpr int GEMM_FP8_BLOCK_STAGES = 5;     // one stage less than the bf16 kernel: the weight scales of a tile live in shared memory too
+constexpr int GEMM_FP8_BLOCK_SCALE_SEG = 64; // blocks of K whose activation scales a CTA holds
 constexpr size_t GEMM_FP8_BLOCK_SMEM_BYTES = 1024 /* alignment slack */ + GEMM_FP8_BLOCK_STAGES * GEMM_PAIR_STAGE_BYTES + 1024 /* barriers */ +
-                                             GEMM_BM * 256 /* epilogue staging tile */;
+                                             GEMM_BM * (GEMM_FP8_BLOCK_SCALE_SEG + 1) * 4 /* activation scales, or the 256-byte rows of the staging tile */;
 
 struct GemmBlockArgs {
     CUtensorMap tmapA;        // A [M, K] 8-bit, box 128 rows x 128 bytes

@@ -65,6 +65,8 @@ constexpr int FB_SCRATCH = 2;               // scratch accumulators of 256 colum
 constexpr uint32_t FB_PEER_BIT_MASK = 0xFEFFFFFFu;
 constexpr int FB_HALF_N = GEMM_BN / 2;       // columns of one promoter group = one 128-wide block of the weight's scales
 constexpr int FB_MAX_KB = 256;               // blocks of K whose weight scales fit the shared-memory copy (K up to 32768)
+constexpr int FB_SEG = GEMM_FP8_BLOCK_SCALE_SEG;          // blocks of K whose activation scales are in shared memory at a time
+constexpr int FB_SEG_PITCH = FB_SEG + 1;                  // floats per row: an odd number keeps the rows on different banks
 constexpr int FB_FLAG_PLANE_A = TILEXR_FLAG_DATA_BASE;    // all-gather: piece (source rank, 128-row block) has landed
 constexpr int FB_FLAG_PLANE_B = TILEXR_FLAG_ACK_BASE;     // reduce-scatter: partial tile (source rank, tile) has landed
 
@@ -512,6 +514,7 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
         const int pt = static_cast<int>(threadIdx.x) - 128;       // 0..255 among the promoter threads
         __shared__ int sExit;
         __shared__ float sScaleB[2 * FB_MAX_KB];
+        float *sScaleA = reinterpret_cast<float *>(stageC);      // the reduce-scatter's staging tile is used when no scale is
         uint32_t kbAll = 0;                        // as the issuer counts it: scratch kbAll & 1, its (kbAll >> 1)-th use
         const int KB = a.kBlocks;
         const bool gathered = MODE == GEMM_ALL_GATHER;
@@ -522,12 +525,28 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
             const int64_t row0 = static_cast<int64_t>(mTile) * 2 * GEMM_BM + static_cast<int64_t>(ctaRank) * GEMM_BM;
             const int64_t gRow = row0 + myRow;
             const bool rowValid = gRow < a.M;
-            const float *saRow = a.scaleA + (rowValid ? gRow : 0) * KB;
+            const float *sa = a.scaleA + row0 * KB;
             bool wait = gathered;                  // the scales of these rows come from a peer during this launch
             if (gathered && row0 / a.shardRows == a.comm->rank) {
-                saRow = a.scaleALocal + (gRow - static_cast<int64_t>(a.comm->rank) * a.shardRows) * KB;
+                sa = a.scaleALocal + (row0 - static_cast<int64_t>(a.comm->rank) * a.shardRows) * KB;
                 wait = false;
             }
+            const int saRows = static_cast<int>(min(static_cast<int64_t>(GEMM_BM), a.M - row0));
+            auto loadScaleA = [&](int kb0) {
+#pragma unroll 8
+                for (int i = pt; i < saRows * FB_SEG; i += 256) {
+                    const int r = i / FB_SEG, c = i % FB_SEG;
+                    if (kb0 + c >= KB) continue;
+                    const float *src = sa + static_cast<int64_t>(r) * KB + kb0 + c;
+                    float *dst = sScaleA + r * FB_SEG_PITCH + c;
+                    if (wait) {
+                        *dst = __ldcg(src);        // written during this launch: through L2, never through the read-only path
+                    } else {
+                        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(SmemAddr(dst)), "l"(src) : "memory");
+                    }
+                }
+                asm volatile("cp.async.wait_all;" ::: "memory");
+            };
             // scale blocks of B for the two column halves
             const int nb0 = min(nBlock * 2, a.scaleBRows - 1);
             const int nb1 = min(nBlock * 2 + 1, a.scaleBRows - 1);
@@ -536,10 +555,10 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
             float acc[FB_HALF_N];
 #pragma unroll
             for (int j = 0; j < FB_HALF_N; ++j) acc[j] = 0.f;
-            // The weight's scales of this tile (two rows of the table) go to shared memory once per tile; the activation
-            // scale of the thread's row is fetched two blocks of K ahead of its use, so that its latency (an L2 round
-            // trip where it is not in L1, about one block's work) does not show.
-            asm volatile("bar.sync 1, 256;" ::: "memory");          // the previous tile's readers are done with sScaleB
+            // The scales go to shared memory, the weight's two rows of the table once per tile and the activations' 128 rows
+            // FB_SEG blocks of K at a time: a lane reading its own row's scale from memory for every block touches 32 lines
+            // per warp and block.
+            asm volatile("bar.sync 1, 256;" ::: "memory");          // the previous tile's readers are done with both
             for (int i = pt; i < 2 * KB && i < 2 * FB_MAX_KB; i += 256) {
                 sScaleB[i] = __ldg((i < KB ? sb0 + i : sb1 + (i - KB)));
             }
@@ -553,39 +572,43 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
                 }
                 __syncwarp();
             }
-            asm volatile("bar.sync 1, 256;" ::: "memory");
             const bool bInSmem = KB <= FB_MAX_KB;
-            // written during this launch in the all-gather mode: through L2, never through the read-only path
-            auto loadA = [&](int kb) { return !rowValid ? 0.f : gathered ? __ldcg(saRow + min(kb, KB - 1)) : __ldg(saRow + min(kb, KB - 1)); };
-            float sa0 = loadA(0), sa1 = loadA(1);
             const float *sbHalf = h == 0 ? sb0 : sb1;
             const float *sbShared = sScaleB + h * KB;
-            for (int kb = 0; kb < KB; ++kb) {
-                const float f = sa0 * (bInSmem ? sbShared[kb] : __ldg(sbHalf + kb));
-                sa0 = sa1;
-                sa1 = loadA(kb + 2);
-                const uint32_t p = kbAll & 1u;
-                if (!FbWaitBarWarp(&st->scratchFull[p], (kbAll >> 1) & 1u, st, peerAbortAddr, budgetNs)) break;
-                ++kbAll;
-                FbFenceAfter();
-                const uint32_t taddr = tmemBase + (static_cast<uint32_t>(quad * 32) << 16) + p * GEMM_BN + static_cast<uint32_t>(h * FB_HALF_N);
-                // Sixteen columns at a time, the next ones on their way while these are folded (8192^3: 8 columns 538 us,
-                // 16 columns 523 us, 32 columns 565 us, before the modes had kernels of their own).
-                uint32_t r[2][16];
-                FbTmemLoad16(taddr, r[0]);
+            const float *saShared = sScaleA + myRow * FB_SEG_PITCH;
+            for (int kb0 = 0; kb0 < KB; kb0 += FB_SEG) {
+                if (kb0 != 0) asm volatile("bar.sync 1, 256;" ::: "memory");      // everybody has read the segment before
+                loadScaleA(kb0);
+                asm volatile("bar.sync 1, 256;" ::: "memory");
+                const int n = min(FB_SEG, KB - kb0);
+                // One way in and one way out: with an exit for a wait that gave up, the 128 accumulators were moved to other
+                // registers and back in every block.  Such a wait has raised the abort flag; what is folded after it is
+                // never stored.
+                for (int kb = 0; kb < n; ++kb) {
+                    const float f = saShared[kb] * (bInSmem ? sbShared[kb0 + kb] : __ldg(sbHalf + kb0 + kb));
+                    const uint32_t p = kbAll & 1u;
+                    FbWaitBarWarp(&st->scratchFull[p], (kbAll >> 1) & 1u, st, peerAbortAddr, budgetNs);
+                    ++kbAll;
+                    FbFenceAfter();
+                    const uint32_t taddr = tmemBase + (static_cast<uint32_t>(quad * 32) << 16) + p * GEMM_BN + static_cast<uint32_t>(h * FB_HALF_N);
+                    // Sixteen columns at a time, the next ones on their way while these are folded (8192^3: 8 columns 538 us,
+                    // 16 columns 523 us, 32 columns 565 us, before the modes had kernels of their own).
+                    uint32_t r[2][16];
+                    FbTmemLoad16(taddr, r[0]);
 #pragma unroll
-                for (int cc = 0; cc < 8; ++cc) {
-                    FbTmemLoadWait16(r[cc & 1]);
-                    if (cc < 7) {
-                        FbTmemLoad16(taddr + (cc + 1) * 16, r[(cc + 1) & 1]);
-                    } else {
-                        // the half is in registers: the issuer may overwrite it two blocks of K from now
-                        FbFenceBefore();
-                        __syncwarp();
-                        if (lane == 0) FbArriveCluster(SmemAddr(&st->scratchEmpty[p]) & FB_PEER_BIT_MASK);
+                    for (int cc = 0; cc < 8; ++cc) {
+                        FbTmemLoadWait16(r[cc & 1]);
+                        if (cc < 7) {
+                            FbTmemLoad16(taddr + (cc + 1) * 16, r[(cc + 1) & 1]);
+                        } else {
+                            // the half is in registers: the issuer may overwrite it two blocks of K from now
+                            FbFenceBefore();
+                            __syncwarp();
+                            if (lane == 0) FbArriveCluster(SmemAddr(&st->scratchEmpty[p]) & FB_PEER_BIT_MASK);
+                        }
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) acc[cc * 16 + j] = fmaf(__uint_as_float(r[cc & 1][j]), f, acc[cc * 16 + j]);
                     }
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) acc[cc * 16 + j] = fmaf(__uint_as_float(r[cc & 1][j]), f, acc[cc * 16 + j]);
                 }
             }
             // All eight promoter warps of the CTA arrive here whether or not their waits succeeded, and leave the tile
