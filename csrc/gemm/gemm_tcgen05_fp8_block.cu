@@ -519,34 +519,31 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
         const int KB = a.kBlocks;
         const bool gathered = MODE == GEMM_ALL_GATHER;
         const uint64_t budgetNs = fused ? a.comm->waitTimeoutNs : 4000000000ull;
+        // Brings the scales of 128 rows from `tileRow` on, blocks kb0 .. kb0 + FB_SEG - 1 of K, to shared memory; a warp takes a row
+        // at a time.  Scales that a peer writes during this launch are read through L2, never through the read-only path.
+        auto loadScaleA = [&](int64_t tileRow, bool fromPeer, int kb0) {
+            const float *sa = a.scaleA + tileRow * KB;
+            if (gathered && !fromPeer) sa = a.scaleALocal + (tileRow - static_cast<int64_t>(a.comm->rank) * a.shardRows) * KB;
+            const int rows = static_cast<int>(min(static_cast<int64_t>(GEMM_BM), a.M - tileRow));
+            const int n = min(FB_SEG, KB - kb0);
+#pragma unroll 4
+            for (int r = pt >> 5; r < rows; r += 8) {
+                for (int c = lane; c < n; c += 32) {
+                    const float *src = sa + static_cast<int64_t>(r) * KB + kb0 + c;
+                    float *dst = sScaleA + r * FB_SEG_PITCH + c;
+                    if (fromPeer) *dst = __ldcg(src);
+                    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(SmemAddr(dst)), "l"(src) : "memory");
+                }
+            }
+        };
+        auto ofPeer = [&](int64_t tileRow) { return gathered && tileRow / a.shardRows != a.comm->rank; };
+        bool ahead = false;                        // the tile's first segment of scales is already on its way
         for (int t = pair; t < totalTiles; t += nPairs) {
             int mTile, nBlock;
             FbTileOf(a, t, mTiles, fused ? a.comm->rank : 0, &mTile, &nBlock);
             const int64_t row0 = static_cast<int64_t>(mTile) * 2 * GEMM_BM + static_cast<int64_t>(ctaRank) * GEMM_BM;
             const int64_t gRow = row0 + myRow;
             const bool rowValid = gRow < a.M;
-            const float *sa = a.scaleA + row0 * KB;
-            bool wait = gathered;                  // the scales of these rows come from a peer during this launch
-            if (gathered && row0 / a.shardRows == a.comm->rank) {
-                sa = a.scaleALocal + (row0 - static_cast<int64_t>(a.comm->rank) * a.shardRows) * KB;
-                wait = false;
-            }
-            const int saRows = static_cast<int>(min(static_cast<int64_t>(GEMM_BM), a.M - row0));
-            auto loadScaleA = [&](int kb0) {
-#pragma unroll 8
-                for (int i = pt; i < saRows * FB_SEG; i += 256) {
-                    const int r = i / FB_SEG, c = i % FB_SEG;
-                    if (kb0 + c >= KB) continue;
-                    const float *src = sa + static_cast<int64_t>(r) * KB + kb0 + c;
-                    float *dst = sScaleA + r * FB_SEG_PITCH + c;
-                    if (wait) {
-                        *dst = __ldcg(src);        // written during this launch: through L2, never through the read-only path
-                    } else {
-                        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(SmemAddr(dst)), "l"(src) : "memory");
-                    }
-                }
-                asm volatile("cp.async.wait_all;" ::: "memory");
-            };
             // scale blocks of B for the two column halves
             const int nb0 = min(nBlock * 2, a.scaleBRows - 1);
             const int nb1 = min(nBlock * 2 + 1, a.scaleBRows - 1);
@@ -562,7 +559,8 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
             for (int i = pt; i < 2 * KB && i < 2 * FB_MAX_KB; i += 256) {
                 sScaleB[i] = __ldg((i < KB ? sb0 + i : sb1 + (i - KB)));
             }
-            if (wait) {
+            const bool fromPeer = ofPeer(row0);
+            if (fromPeer) {
                 // the scales of these 128 rows were written by their owner during this launch: acquire the rows' flag first
                 if (lane == 0) {
                     const int block = static_cast<int>(row0 / GEMM_BM);
@@ -578,7 +576,8 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
             const float *saShared = sScaleA + myRow * FB_SEG_PITCH;
             for (int kb0 = 0; kb0 < KB; kb0 += FB_SEG) {
                 if (kb0 != 0) asm volatile("bar.sync 1, 256;" ::: "memory");      // everybody has read the segment before
-                loadScaleA(kb0);
+                if (kb0 != 0 || !ahead) loadScaleA(row0, fromPeer, kb0);
+                asm volatile("cp.async.wait_all;" ::: "memory");
                 asm volatile("bar.sync 1, 256;" ::: "memory");
                 const int n = min(FB_SEG, KB - kb0);
                 // One way in and one way out: with an exit for a wait that gave up, the 128 accumulators were moved to other
@@ -618,7 +617,16 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
             asm volatile("bar.sync 1, 256;" ::: "memory");
             if (sExit != 0) break;
             const int col0 = nBlock * GEMM_BN;
+            ahead = false;
             if (MODE != GEMM_REDUCE_SCATTER) {
+                // the next tile's scales come while this one is stored (everybody has left the loop that reads them)
+                if (t + nPairs < totalTiles) {
+                    int mNext, nNext;
+                    FbTileOf(a, t + nPairs, mTiles, fused ? a.comm->rank : 0, &mNext, &nNext);
+                    const int64_t rowNext = static_cast<int64_t>(mNext) * 2 * GEMM_BM + static_cast<int64_t>(ctaRank) * GEMM_BM;
+                    ahead = !ofPeer(rowNext);
+                    if (ahead) loadScaleA(rowNext, false, 0);
+                }
                 // Local memory: every thread stores its 256 bytes of a row straight from registers, without the two trips
                 // of the tile through shared memory and their barriers (the issuer has only two blocks of K of work ahead).
                 if (rowValid) {

@@ -256,3 +256,23 @@ def test_grouped_matmul_few_rows_per_group(txr, groups, n, k, counts, epilogue):
     # one rounding to bf16 of a value of order one
     assert torch.allclose(got[:total].float(), want[:total], rtol=2.0 ** -7, atol=2.0 ** -7)
     assert (got[total:] == 3.0).all()
+
+
+@pytest.mark.parametrize("m,n,k", [(260, 264, 128 * 65), (130, 256, 128 * 130), (4100, 5128, 128), (1300, 7176, 128 * 3), (100, 256, 128 * 260)])
+def test_matmul_fp8_block_scales_in_segments(txr, m, n, k):
+    """More blocks of K than a CTA holds scales for, one block only, several tiles per CTA (the next tile's scales are fetched while
+    one is stored), more blocks than the weight's shared-memory table has places."""
+    g = torch.Generator().manual_seed(k)
+    a = torch.randn(m, k, generator=g).cuda() * (0.25 + 4.0 * torch.rand(m, 1, generator=g).cuda())
+    a *= (0.5 + torch.rand(1, k // 128, generator=g).cuda()).repeat_interleave(128, dim=1)
+    w = torch.randn(n, k, generator=g).cuda() * (0.2 + torch.rand((n + 127) // 128, k // 128, generator=g).cuda()).repeat_interleave(
+        128, dim=0)[:n].repeat_interleave(128, dim=1)
+    qa, sa = txr.quant.fp8_quant_1x128(a.to(torch.bfloat16))
+    qw, sw = txr.gemm.quantize_weight_128x128(w)
+    da = (qa.double().view(m, -1, 128) * sa.double()[:, :, None]).view(m, k)
+    dw = qw.double() * sw.double().repeat_interleave(128, dim=0)[:n].repeat_interleave(128, dim=1)
+    want = da @ dw.t()
+    got = txr.gemm.matmul_fp8_block(qa, sa, qw, sw).double()
+    # fp32 sums of k products of fp8 values, one rounding to bf16
+    bound = want.abs() * 2.0 ** -8 + (da.abs() @ dw.abs().t()) * k * 2.0 ** -24
+    assert ((got - want).abs() <= bound).all()
