@@ -206,10 +206,15 @@ int TileXRMatmul(const void *a, const void *b, void *c, int64_t m, int64_t n, in
     int sms = 0;
     ret = SmCount(&sms);
     if (ret != TILEXR_SUCCESS) return ret;
-    // Few rows, or so few 256 x 256 tiles that more than half of the CTA pairs would have none: the kernel whose tiles are
-    // 128 columns by up to 128 rows and which splits K.
+    // Few rows, or few 256 x 256 tiles: the kernel whose tiles are 128 columns by up to 128 rows and which splits K.
+    // A wide tile takes about 0.005 us per element of K, however few rows it has; the few-rows kernel takes 8 us (16 rows) to 16 us
+    // (128 rows) before K and N count.  us, wide and few-rows: 1 x 4096 x 1024 (m, n, k) 10.5 and 8.4; 17 x 7168 x 2048 18.4 and 12.3;
+    // 64 x 4096 x 1024 10.5 and 12.4, x 4096 24.8 and 16.2; 64 x 7168 x 2048 16.6 both, 64 x 16384 x 2048 16.6 and 20.7;
+    // 128 x 2048 x 2048 16.6 and 17.5, 128 x 7168 x 4096 26.9 and 25.0, 128 x 8192 x 8192 57.6 and 40.2; 512 x 2048 x 4096
+    // (16 tiles) 29.1 and 27.3, 384 x 4096 x 4096 (32 tiles) 29.0 and 35.0, 512 x 2048 x 2048 18.7 and 22.8.
     const int64_t squareTiles = ((m + 2 * GEMM_BM - 1) / (2 * GEMM_BM)) * ((n + GEMM_BN - 1) / GEMM_BN);
-    if ((m <= GEMM_BM || squareTiles * 4 <= sms) && EnvLong("TILEXR_GEMM_SKINNY", 1) != 0) {
+    const bool fewRows = m <= 32 || (m <= 64 && k >= 2048 && n <= 8192) || (k >= 4096 && (m <= GEMM_BM || squareTiles <= 16));
+    if (fewRows && EnvLong("TILEXR_GEMM_SKINNY", 1) != 0) {
         return LaunchSkinny(a, b, nullptr, c, m, n, k, 1, SkinnyRows(m), bf16, GEMM_EPI_STORE, status, sms, stream);
     }
     GemmArgs g;
@@ -282,9 +287,11 @@ int TileXRGroupedMatmul(const void *a, const void *b, const int64_t *groupRows, 
     int sms = 0;
     ret = SmCount(&sms);
     if (ret != TILEXR_SUCCESS) return ret;
-    // Few rows per group on average (the counts themselves are on the device): tiles of twice the average hold most groups
+    // Few rows per group on average (the counts themselves are on the device): tiles of twice the average hold most groups.
+    // 64 groups of 4096 x 2048: 4 rows each 204 us with CTA pairs, 164 with this kernel; 32 rows 222 and 172; 64 rows 223 and 186;
+    // from 128 rows on a group needs several tiles and reads its weight again (192 rows 229 and 297).
     const int64_t perGroup = (maxRows + groups - 1) / groups;
-    if (perGroup <= EnvLong("TILEXR_GEMM_SKINNY_ROWS", 32)) {
+    if (perGroup <= EnvLong("TILEXR_GEMM_SKINNY_ROWS", 64)) {
         return LaunchSkinny(a, b, groupRows, c, maxRows, n, k, groups, SkinnyRows(2 * perGroup), bf16, epilogue, status, sms, stream);
     }
     GemmArgs g;

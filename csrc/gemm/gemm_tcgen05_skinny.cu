@@ -305,7 +305,8 @@ __global__ void __launch_bounds__(GEMM_SKINNY_THREADS, 2) TileXRGemmSkinny(const
         __syncthreads();
         SkClusterSync();
         const bool work = first < items && st->abortFlag == 0;
-        const int slice = a.tn / split;
+        const int slice = a.tn / split;                        // powers of two, both
+        const int sliceBits = 31 - __clz(slice);
         const int quad = warp & 3;
         if (warp >= 2 && work) {
             const uint32_t mine = SmemAddr(smem) + static_cast<uint32_t>((part * slice) * 128 + quad * 32 + lane) * 4u;
@@ -314,9 +315,9 @@ __global__ void __launch_bounds__(GEMM_SKINNY_THREADS, 2) TileXRGemmSkinny(const
                 SkTmemLoad16(tmemBase + (static_cast<uint32_t>(quad * 32) << 16) + static_cast<uint32_t>(c0), r);
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
-                    const int dst = (c0 + j) / slice;
+                    const int dst = (c0 + j) >> sliceBits;
                     uint32_t remote;
-                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(mine + static_cast<uint32_t>((c0 + j - dst * slice) * 512)), "r"(dst));
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(mine + static_cast<uint32_t>(((c0 + j) & (slice - 1)) * 512)), "r"(dst));
                     asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(remote), "r"(r[j]) : "memory");
                 }
             }

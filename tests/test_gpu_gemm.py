@@ -223,8 +223,8 @@ def test_matmul_reduce_scatter_fp8_block(txr, ranks, shard_rows, n, k):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("m,n,k", [(1, 8, 8), (1, 128, 64), (16, 120, 72), (17, 7168, 2048), (33, 136, 2056), (65, 4096, 320), (128, 264, 4104),
-                                   (129, 512, 1000), (300, 1024, 640), (1000, 512, 4096), (5, 40960, 136)])
+@pytest.mark.parametrize("m,n,k", [(1, 8, 8), (1, 128, 64), (16, 120, 72), (17, 7168, 2048), (33, 136, 2056), (64, 8200, 2048), (65, 4096, 320),
+                                   (65, 264, 4096), (128, 264, 4104), (129, 512, 4100 // 8 * 8), (300, 1024, 4096), (1000, 512, 4096), (5, 40960, 136)])
 def test_matmul_few_rows(txr, m, n, k, dtype):
     """Tiles of 128 columns by 16 to 128 rows: remainders of both, K split over one to eight CTAs with a ragged last part,
     more tiles than places."""
