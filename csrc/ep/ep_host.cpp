@@ -778,7 +778,8 @@ int TileXRFp8Quant1x128(const void *x, int64_t rows, int64_t h, TileXRDataType d
 
 int TileXRSwiglu(const void *gateUp, int64_t rows, int64_t f, TileXRDataType dtype, void *yOut, TileXRStream stream)
 {
-    if (gateUp == nullptr || yOut == nullptr || rows <= 0 || f <= 0 || f % 8 != 0 || f > INT32_MAX || !HalfType(dtype)) {
+    if (gateUp == nullptr || yOut == nullptr || rows <= 0 || f <= 0 || f % 8 != 0 || f > INT32_MAX || !HalfType(dtype) ||
+        ((reinterpret_cast<uintptr_t>(gateUp) | reinterpret_cast<uintptr_t>(yOut)) & 15u) != 0) {
         return TILEXR_ERROR_PARA_CHECK_FAIL;
     }
     return LaunchSwiglu(gateUp, rows, f, dtype == TILEXR_DATA_TYPE_BFP16, yOut, nullptr, stream);
@@ -788,7 +789,8 @@ int TileXRSwigluFp8Quant1x128(const void *gateUp, int64_t rows, int64_t f, TileX
                               TileXRStream stream)
 {
     if (gateUp == nullptr || yOut == nullptr || scalesOut == nullptr || rows <= 0 || f <= 0 || f % 128 != 0 || f > INT32_MAX ||
-        !HalfType(dtype)) {
+        !HalfType(dtype) ||
+        ((reinterpret_cast<uintptr_t>(gateUp) | reinterpret_cast<uintptr_t>(yOut)) & 15u) != 0) {
         return TILEXR_ERROR_PARA_CHECK_FAIL;
     }
     return LaunchSwiglu(gateUp, rows, f, dtype == TILEXR_DATA_TYPE_BFP16, yOut, scalesOut, stream);

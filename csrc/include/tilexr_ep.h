@@ -192,6 +192,7 @@ int TileXRFp8Quant1x128(const void *x, int64_t rows, int64_t h, TXR_DT dtype, vo
                         TileXRStream stream);
 // gateUp [rows, 2 * f] with the gate columns first: y[rows, f] = silu(gate) * up, computed in fp32 and rounded to `dtype`
 // (f a multiple of 8), or that result quantised as TileXRFp8Quant1x128 does (f a multiple of 128) without its trip through memory.
+// gateUp and yOut 16-byte aligned.
 int TileXRSwiglu(const void *gateUp, int64_t rows, int64_t f, TXR_DT dtype, void *yOut, TileXRStream stream);
 int TileXRSwigluFp8Quant1x128(const void *gateUp, int64_t rows, int64_t f, TXR_DT dtype, void *yOut, float *scalesOut,
                               TileXRStream stream);

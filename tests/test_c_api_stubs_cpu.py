@@ -109,3 +109,16 @@ def test_symmetric_allocator_plumbing_without_a_gpu(lib, tmp_path):
         assert lib.TileXRVmmDescriptorSelfTest(tag, 3, fd, 5, 1, None) == PARA_CHECK_FAIL
     finally:
         os.close(fd)
+
+
+@pytest.mark.parametrize("entry", ["TileXRSwiglu", "TileXRSwigluFp8Quant1x128"])
+def test_swiglu_refuses_memory_off_the_16_byte_grid(lib, entry):
+    """The kernels move 16 bytes at a time: an address between the grid points is an argument error, found before any launch."""
+    store = (ctypes.c_uint8 * 4096)()
+    base = (ctypes.addressof(store) + 15) & ~15
+    scales = (ctypes.c_float * 8)()
+    f, bf16 = 128, 11
+    n, none = ctypes.c_int64, _p(None)
+    for x, y in ((base + 2, base + 2048), (base, base + 2048 + 8), (base + 4, base + 2048 + 4)):
+        args = [_p(x), n(2), n(f), bf16, _p(y)] + ([_p(ctypes.addressof(scales))] if entry == "TileXRSwigluFp8Quant1x128" else []) + [none]
+        assert getattr(lib, entry)(*args) == PARA_CHECK_FAIL

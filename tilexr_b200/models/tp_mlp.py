@@ -82,8 +82,10 @@ class SequenceParallelMLP(torch.nn.Module):
             gu = self.ops.all_gather_matmul_fp8_block(self.comm, qx, sx, self.stage_rows, self.stage_scales, self.w13, self.s13, cfg.dtype)
         else:
             gu = self.ops.all_gather_matmul(self.comm, x_shard, self.w13, self.stage_rows)
-        # one pass over the product where the kernels apply; other devices, types and injected quantisers take the plain form
-        native = gu.is_cuda and gu.dtype == cfg.dtype and cfg.dtype in (torch.float16, torch.bfloat16) and self.f_loc % 8 == 0
+        # one pass over the product where the kernels apply; other devices, types, a product off the 16-byte grid and injected
+        # quantisers take the plain form
+        native = (gu.is_cuda and gu.dtype == cfg.dtype and cfg.dtype in (torch.float16, torch.bfloat16) and self.f_loc % 8 == 0
+                  and gu.is_contiguous() and gu.data_ptr() % 16 == 0)
         fused_quant = getattr(self.quant, "swiglu_fp8_quant_1x128", None) if native and cfg.fp8_block else None
         if fused_quant is not None:
             qa, sa = fused_quant(gu)

@@ -17,7 +17,8 @@ def fp8_quant_1x128(x: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
 
 
 def swiglu(gate_up: torch.Tensor) -> torch.Tensor:
-    """``silu(gate) * up`` of ``gate_up`` [rows, 2 * f] (gate columns first; f a multiple of 8), computed in fp32."""
+    """``silu(gate) * up`` of ``gate_up`` [rows, 2 * f] (gate columns first; f a multiple of 8, the data 16-byte aligned), computed
+    in fp32."""
     return _C.swiglu(gate_up.contiguous())
 
 
