@@ -330,15 +330,17 @@ int TileXRMoeEpDispatchFused(const TileXREpDispatchParams *p, TileXRCommPtr comm
         return TILEXR_ERROR_PARA_CHECK_FAIL;
     }
 
-    // grid: one block per ~8 tokens per warp-set, capped by what can be co-resident
+    // grid: capped by what can be co-resident
     const int ranksPerDevice = (c.hostArgs->extraFlag & TILEXR_FLAG_EMULATED) ? c.rankSize : 1;
     // At least minBlocks blocks even for a handful of tokens: the receive side of the kernel (rows from all
     // ranks) and the column split of the send side both want the parallelism; blocks may own no token.
     const int64_t capBlocks = std::min<int64_t>(EP_COUNT_FLAG_SLOT - 1, std::max<int64_t>(1, EnvLong("TILEXR_EP_BLOCKS", 296)));
     const int64_t minBlocks = std::min<int64_t>(capBlocks, std::max<int64_t>(1, EnvLong("TILEXR_EP_MIN_BLOCKS", 32)));
-    // Four tokens to a block until the cap: a warp per quarter of a row.  With sixteen to a block 1009 tokens sat on 64 of the
-    // 148 SMs, and 4096 tokens left 40 of the 296 places empty.
-    const int64_t wantBlocks = std::max<int64_t>(minBlocks, std::min<int64_t>((p->bs + 3) / 4, capBlocks));
+    // Alone, four tokens to a block until the cap, a warp per quarter of a row: with sixteen to a block 1009 tokens sat on 64 of the
+    // 148 SMs, and 4096 tokens left 40 of the 296 places empty.  With peers sixteen: every block raises a flag on every rank and every
+    // block polls them all, and ranks whose batches differ a little launch grids of one size, as an emulated world requires.
+    const int64_t perBlock = c.rankSize == 1 ? 4 : 16;
+    const int64_t wantBlocks = std::max<int64_t>(minBlocks, std::min<int64_t>((p->bs + perBlock - 1) / perBlock, capBlocks));
     unsigned grid = static_cast<unsigned>(wantBlocks);
     unsigned gridCap = 0;
     uint32_t tokensPerBlock = 0;

@@ -537,3 +537,24 @@ def test_dispatch_into_an_output_off_the_16_byte_grid(txr, ranks):
             assert n > 0 and torch.equal(d.expand_x[:n], torch.stack([xs[s][t] for s, t, _, _ in tuples]))
     finally:
         world.destroy()
+
+
+def test_dispatch_of_ranks_with_slightly_different_batches(txr):
+    """The ranks of an emulated world share one launch: batches that differ a little must come out at one grid."""
+    ep = txr.ep
+    h, experts, top_k, sizes = 64, 8, 2, (290, 300)
+    g = torch.Generator().manual_seed(11)
+    xs = [torch.randn(n, h, generator=g).to(torch.bfloat16).cuda() for n in sizes]
+    ids = [torch.stack([torch.randperm(experts, generator=g)[:top_k] for _ in range(n)]).to(torch.int32).cuda() for n in sizes]
+    cap = sum(sizes) * top_k
+    world = txr.init_emulated_world(2, device=0, buffer_mb=64)
+    try:
+        ds = world.run(lambda c, r: ep.dispatch(c, xs[r], expert_ids=ids[r], num_experts=experts, top_k=top_k, max_recv_rows=cap))
+        world.check()
+        assert sum(int(d.recv_total) for d in ds) == cap
+        for d in ds:
+            n = int(d.recv_total)
+            tuples = d.assist[:n].cpu().tolist()
+            assert torch.equal(d.expand_x[:n], torch.stack([xs[s][t] for s, t, _, _ in tuples]))
+    finally:
+        world.destroy()
