@@ -336,33 +336,6 @@ int TileXRMoeEpDispatchFused(const TileXREpDispatchParams *p, TileXRCommPtr comm
     // ranks) and the column split of the send side both want the parallelism; blocks may own no token.
     const int64_t capBlocks = std::min<int64_t>(EP_COUNT_FLAG_SLOT - 1, std::max<int64_t>(1, EnvLong("TILEXR_EP_BLOCKS", 296)));
     const int64_t minBlocks = std::min<int64_t>(capBlocks, std::max<int64_t>(1, EnvLong("TILEXR_EP_MIN_BLOCKS", 32)));
-    // Alone, four tokens to a block until the cap, a warp per quarter of a row: with sixteen to a block 1009 tokens sat on 64 of the
-    // 148 SMs, and 4096 tokens left 40 of the 296 places empty.  With peers sixteen: every block raises a flag on every rank and every
-    // block polls them all, and ranks whose batches differ a little launch grids of one size, as an emulated world requires.
-    const int64_t perBlock = c.rankSize == 1 ? 4 : 16;
-    const int64_t wantBlocks = std::max<int64_t>(minBlocks, std::min<int64_t>((p->bs + perBlock - 1) / perBlock, capBlocks));
-    unsigned grid = static_cast<unsigned>(wantBlocks);
-    unsigned gridCap = 0;
-    uint32_t tokensPerBlock = 0;
-    size_t smem = 0;
-    for (;;) {
-        tokensPerBlock = static_cast<uint32_t>((p->bs + grid - 1) / grid);
-        if (static_cast<int64_t>(tokensPerBlock) * routesPerToken > EP_MAX_ROUTES_PER_BLOCK) {
-            TILEXR_LOG(ERROR) << "EP dispatch: " << tokensPerBlock << " tokens per block exceed the per-block route table; "
-                              << "raise TILEXR_EP_BLOCKS";
-            return TILEXR_ERROR_NOT_SUPPORT;
-        }
-        smem = EpDispatchSmemBytes(static_cast<int>(smemCols), static_cast<int>(tokensPerBlock * routesPerToken));
-        unsigned maxGrid = 0;
-        ret = MaxCooperativeGrid(comm, EpDispatchKernelEntry(p->quantMode), EP_BLOCK_THREADS, smem, ranksPerDevice, &maxGrid);
-        if (ret != TILEXR_SUCCESS) return ret;
-        if (maxGrid == 0) return TILEXR_ERROR_NOT_SUPPORT;
-        gridCap = maxGrid;
-        if (grid <= maxGrid) break;
-        grid = maxGrid;
-    }
-    grid = static_cast<unsigned>(std::max<int64_t>((p->bs + tokensPerBlock - 1) / tokensPerBlock, std::min<int64_t>(minBlocks, gridCap)));
-
     const size_t elemSize = TileXRDataTypeSize(p->dtype);
     const bool quant = fp8Mode || int8Mode;
     const uint64_t outBytes = static_cast<uint64_t>(p->maxRecvRows) * (quant ? p->h : p->h * elemSize);
@@ -373,13 +346,42 @@ int TileXRMoeEpDispatchFused(const TileXREpDispatchParams *p, TileXRCommPtr comm
 
     EpDispatchArgs a;
     std::memset(&a, 0, sizeof(a));
-    if (!DispatchLayout(p->h, numCols, c.rankSize, p->maxRecvRows, p->quantMode, elemSize, grid, zeroCopy, &a.win)) {
-        return TILEXR_ERROR_PARA_CHECK_FAIL;
-    }
-    if (a.win.totalBytes > c.hostArgs->dataHalfBytes) {
-        TILEXR_LOG(ERROR) << "EP dispatch needs " << a.win.totalBytes << " bytes of window per half, the communicator has "
-                          << c.hostArgs->dataHalfBytes << "; create it with a larger buffer or register expandXOut";
-        return TILEXR_ERROR_PARA_CHECK_FAIL;
+    unsigned grid = 0;
+    uint32_t tokensPerBlock = 0;
+    size_t smem = 0;
+    // Alone, four tokens to a block until the cap, a warp per quarter of a row: with sixteen to a block 1009 tokens sat on 64 of the
+    // 148 SMs, and 4096 tokens left 40 of the 296 places empty.  With peers sixteen: every block raises a flag on every rank and every
+    // block polls them all, and ranks whose batches differ a little launch grids of one size, as an emulated world requires.
+    // Every block also takes a row of counts in the window: sixteen where the window is too small for the counts of more blocks.
+    for (int64_t perBlock = c.rankSize == 1 ? 4 : 16;; perBlock = 16) {
+        grid = static_cast<unsigned>(std::max<int64_t>(minBlocks, std::min<int64_t>((p->bs + perBlock - 1) / perBlock, capBlocks)));
+        unsigned gridCap = 0;
+        for (;;) {
+            tokensPerBlock = static_cast<uint32_t>((p->bs + grid - 1) / grid);
+            if (static_cast<int64_t>(tokensPerBlock) * routesPerToken > EP_MAX_ROUTES_PER_BLOCK) {
+                TILEXR_LOG(ERROR) << "EP dispatch: " << tokensPerBlock << " tokens per block exceed the per-block route table; "
+                                  << "raise TILEXR_EP_BLOCKS";
+                return TILEXR_ERROR_NOT_SUPPORT;
+            }
+            smem = EpDispatchSmemBytes(static_cast<int>(smemCols), static_cast<int>(tokensPerBlock * routesPerToken));
+            unsigned maxGrid = 0;
+            ret = MaxCooperativeGrid(comm, EpDispatchKernelEntry(p->quantMode), EP_BLOCK_THREADS, smem, ranksPerDevice, &maxGrid);
+            if (ret != TILEXR_SUCCESS) return ret;
+            if (maxGrid == 0) return TILEXR_ERROR_NOT_SUPPORT;
+            gridCap = maxGrid;
+            if (grid <= maxGrid) break;
+            grid = maxGrid;
+        }
+        grid = static_cast<unsigned>(std::max<int64_t>((p->bs + tokensPerBlock - 1) / tokensPerBlock, std::min<int64_t>(minBlocks, gridCap)));
+        if (!DispatchLayout(p->h, numCols, c.rankSize, p->maxRecvRows, p->quantMode, elemSize, grid, zeroCopy, &a.win)) {
+            return TILEXR_ERROR_PARA_CHECK_FAIL;
+        }
+        if (a.win.totalBytes <= c.hostArgs->dataHalfBytes) break;
+        if (perBlock == 16) {
+            TILEXR_LOG(ERROR) << "EP dispatch needs " << a.win.totalBytes << " bytes of window per half, the communicator has "
+                              << c.hostArgs->dataHalfBytes << "; create it with a larger buffer or register expandXOut";
+            return TILEXR_ERROR_PARA_CHECK_FAIL;
+        }
     }
     a.x = static_cast<const uint8_t *>(p->x);
     a.expertIds = p->expertIds;

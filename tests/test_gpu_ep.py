@@ -558,3 +558,25 @@ def test_dispatch_of_ranks_with_slightly_different_batches(txr):
             assert torch.equal(d.expand_x[:n], torch.stack([xs[s][t] for s, t, _, _ in tuples]))
     finally:
         world.destroy()
+
+
+def test_dispatch_in_a_window_with_room_for_few_blocks(txr, port):
+    """Every block of a dispatch keeps a row of counts in the window: a window that the rows nearly fill still takes the batch."""
+    ep = txr.ep
+    h, experts, top_k, tokens = 256, 1024, 2, 1024
+    comm = txr.init_process(0, 1, comm_id=f"127.0.0.1:{port}", buffer_mb=16, device=0)
+    try:
+        # what sixteen tokens to a block need fits (64 blocks of 1024 counts), what four to a block need does not
+        rows = (comm.data_half_bytes - 64 * experts * 4 - 2048) // (h * 2 + 16 + 8)
+        g = torch.Generator().manual_seed(12)
+        x = torch.randn(tokens, h, generator=g).to(torch.bfloat16).cuda()
+        ids = torch.stack([torch.randperm(experts, generator=g)[:top_k] for _ in range(tokens)]).to(torch.int32).cuda()
+        d = ep.dispatch(comm, x, num_experts=experts, top_k=top_k, expert_ids=ids, max_recv_rows=rows)
+        torch.cuda.synchronize()
+        n = tokens * top_k
+        assert comm.device_status() == 0 and int(d.recv_total) == n
+        assert torch.equal(d.expand_x[:n], x[d.assist[:n, 1].long()])
+        with pytest.raises(RuntimeError):
+            ep.dispatch(comm, x, num_experts=experts, top_k=top_k, expert_ids=ids, max_recv_rows=rows + 128)
+    finally:
+        comm.destroy()
