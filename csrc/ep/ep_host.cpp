@@ -269,6 +269,13 @@ uint64_t TileXREpAbiStamp(void) { return TILEXR_EP_ABI_STAMP; }
 
 int TileXRMoeEpDispatchFused(const TileXREpDispatchParams *p, TileXRCommPtr comm, TileXRStream stream)
 {
+    return TileXR::EpDispatch(p, nullptr, comm, stream);
+}
+
+} // extern "C"
+
+int TileXR::EpDispatch(const TileXREpDispatchParams *p, int32_t *laneCountOut, TileXRCommPtr comm, TileXRStream stream)
+{
     Ctx c;
     int ret = Prepare(comm, &c);
     if (ret != TILEXR_SUCCESS) return ret;
@@ -396,7 +403,7 @@ int TileXRMoeEpDispatchFused(const TileXREpDispatchParams *p, TileXRCommPtr comm
     a.expertTokenNumsOut = p->expertTokenNumsOut;
     a.sendCountsOut = p->sendCountsOut;
     a.recvTotalOut = p->recvTotalOut;
-    a.laneCountOut = p->tpRecvCountsOut;
+    a.laneCountOut = laneCountOut;
     a.comm = reinterpret_cast<CommArgs *>(c.devArgs);
     a.bs = static_cast<int32_t>(p->bs);
     a.h = static_cast<int32_t>(p->h);
@@ -438,6 +445,8 @@ int TileXRMoeEpDispatchFused(const TileXREpDispatchParams *p, TileXRCommPtr comm
     LaunchConfig cfg{grid, EP_BLOCK_THREADS, smem, true};
     return LaunchKernel(comm, EpDispatchKernelEntry(p->quantMode), &a, cfg, stream);
 }
+
+extern "C" {
 
 int TileXRMoeEpCombineFused(const TileXREpCombineParams *p, TileXRCommPtr comm, TileXRStream stream)
 {
@@ -627,7 +636,7 @@ int TileXRMoeEpDispatchMemoryV2(void *x, int32_t *expertIds, void *scales, bool 
     p.maxRecvRows = bs * c.rankSize * std::min<int64_t>(topK, moeExpertNum / std::max<int64_t>(1, c.rankSize / T - sharedExpertRankNum));
     p.tpWorldSize = T;
     p.tpRankId = tpRankId;
-    p.tpRecvCountsOut = T > 1 ? tpRecvCountsOut : nullptr;
+    p.tpRecvCountsOut = tpRecvCountsOut;
     p.expertScales = static_cast<const float *>(expertScales);
     p.expandScalesOut = static_cast<float *>(expandScalesOut);
     p.expandXOut = expandXOut;

@@ -299,6 +299,8 @@ __device__ void EpDispatchBody(const EpDispatchArgs &a)
     // A world of one rank: every row's final place is this rank's own output, so rows, scales and tuples are stored there
     // at once; nothing passes through the window and nobody has to be waited for.
     const bool solo = R == 1 && a.directOwn != 0;
+    // whatever becomes of the launch, like the caller's other zeros would have been
+    if (blockIdx.x == 0 && tid == 0 && a.laneCountOut != nullptr) *a.laneCountOut = 0;
 
     const int t0 = min(a.bs, static_cast<int>(blockIdx.x * a.tokensPerBlock));
     const int t1 = min(a.bs, t0 + static_cast<int>(a.tokensPerBlock));
@@ -912,7 +914,6 @@ __device__ void EpDispatchBody(const EpDispatchArgs &a)
                                                ? static_cast<int64_t>(sm.total[firstLocal + le])
                                                : static_cast<int64_t>(sm.hist[le * R + R - 1]);
             }
-            if (tid == 0 && a.laneCountOut != nullptr) *a.laneCountOut = 0;
             if (tid == 0 && a.recvTotalOut != nullptr) *a.recvTotalOut = n > 0 ? sm.hist[n - 1] : 0;
         }
     }

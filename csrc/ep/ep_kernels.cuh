@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include "tilexr_comm_args.h"
+#include "tilexr_ep.h"
 #include "tilexr_launch.h"
 
 namespace TileXR {
@@ -81,7 +82,7 @@ struct EpDispatchArgs {
     int64_t *expertTokenNumsOut;
     int32_t *sendCountsOut;
     int32_t *recvTotalOut;
-    int32_t *laneCountOut;           // the caller's count per tensor-parallel lane where there is one lane: set to zero; or null
+    int32_t *laneCountOut;           // [1] set to zero, or null (EpDispatch)
     CommArgs *comm;
     int64_t magic;
     EpDispatchWindow win;
@@ -155,6 +156,10 @@ struct RoutingArgs {
 
 const KernelEntry &EpDispatchKernelEntry(int64_t quantMode);      // a kernel per kind of transport
 const KernelEntry &EpCombineKernelEntry();
+
+// TileXRMoeEpDispatchFused that also sets *laneCountOut (null: nothing) to zero, in the dispatch launch: what the Python results
+// report for a world without tensor-parallel lanes, whose C callers get no such count.
+int EpDispatch(const TileXREpDispatchParams *p, int32_t *laneCountOut, TileXRCommPtr comm, TileXRStream stream);
 
 // Plain (non communicating) kernels, launched directly.
 int LaunchRoutingTopK(const RoutingArgs &args, void *stream);

@@ -96,7 +96,7 @@ typedef struct TileXREpDispatchParams {
     // field of the assist tuples use these slots, and the expert field holds the lane expert
     // ((group * T + l) * expertsPerGroup + local expert).  expertTokenNumsOut has one entry per expert of the group,
     // sendCountsOut expertsPerGroup * R.  tpRecvCountsOut [T] (required) receives the rows that came from the ranks
-    // of each lane (one lane: set to 0 where given).  T > 1 needs explicit expertIds, no shared-expert ranks, and topK * T <= 32.
+    // of each lane.  Needs explicit expertIds, no shared-expert ranks, and topK * T <= 32.
     int64_t tpWorldSize;
     int64_t tpRankId;
     int32_t *tpRecvCountsOut;

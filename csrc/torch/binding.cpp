@@ -14,6 +14,7 @@
 #include <string>
 #include <vector>
 
+#include "ep_kernels.cuh"
 #include "tilexr_api.h"
 #include "tilexr_collectives.h"
 #include "tilexr_collectives_perf.h"
@@ -415,7 +416,7 @@ py::tuple EpDispatch(const CommPtr &c, const at::Tensor &x, const c10::optional<
     std::memset(&p, 0, sizeof(p));
     p.tpWorldSize = T;
     p.tpRankId = c->rank() % T;
-    p.tpRecvCountsOut = tpRecvCounts.data_ptr<int32_t>();
+    p.tpRecvCountsOut = T > 1 ? tpRecvCounts.data_ptr<int32_t>() : nullptr;
     p.x = x.data_ptr();
     if (expertIds.has_value() && expertIds->defined()) {
         TORCH_CHECK(expertIds->scalar_type() == at::kInt && expertIds->is_contiguous(), "expert_ids must be contiguous int32");
@@ -470,7 +471,7 @@ py::tuple EpDispatch(const CommPtr &c, const at::Tensor &x, const c10::optional<
                                 assistExt, expandScales, tpRecvCounts}) {
         Keep(t);
     }
-    Check(TileXRMoeEpDispatchFused(&p, c->ptr(), StreamOf(x)), "TileXRMoeEpDispatchFused");
+    Check(TileXR::EpDispatch(&p, T > 1 ? nullptr : tpRecvCounts.data_ptr<int32_t>(), c->ptr(), StreamOf(x)), "TileXRMoeEpDispatchFused");
     return py::make_tuple(expandX, hasScales ? py::cast(scales) : py::none(), assist, tokenNums, sendCounts, recvTotal, topkIds,
                           topkWeights, routeRows, assistExt, expandScales, tpRecvCounts);
 }

@@ -580,3 +580,49 @@ def test_dispatch_in_a_window_with_room_for_few_blocks(txr, port):
             ep.dispatch(comm, x, num_experts=experts, top_k=top_k, expert_ids=ids, max_recv_rows=rows + 128)
     finally:
         comm.destroy()
+
+
+def test_lane_counts_are_zero_whatever_becomes_of_a_dispatch(txr, port):
+    """One tensor-parallel lane: its count is zero after a launch that gave up on too many rows, too, and the C entry leaves the
+    caller's buffer alone."""
+    import ctypes
+
+    ep = txr.ep
+    comm = txr.init_process(0, 1, comm_id=f"127.0.0.1:{port}", buffer_mb=16, device=0)
+    try:
+        x = torch.randn(16, 256).to(torch.bfloat16).cuda()
+        ids = torch.zeros(16, 2, dtype=torch.int32).cuda()
+        ids[:, 1] = 1
+        for cap, status in ((64, 0), (8, 4)):            # 4: TILEXR_DEV_BAD_ARGUMENT, 32 rows do not fit 8
+            used = [torch.full((1,), 7, dtype=torch.int32, device="cuda") for _ in range(64)]
+            del used                                     # the dispatch's small outputs come from this memory
+            d = ep.dispatch(comm, x, expert_ids=ids, num_experts=4, top_k=2, max_recv_rows=cap)
+            torch.cuda.synchronize()
+            assert comm.device_status() == status and d.tp_recv_counts.tolist() == [0]
+        comm.reset_status()
+
+        pointer, i64 = ctypes.c_void_p, ctypes.c_int64
+
+        class Params(ctypes.Structure):                  # TileXREpDispatchParams
+            _fields_ = ([(n, pointer) for n in ("x", "expertIds", "gateLogits", "selectionBias", "xActiveMask")] +
+                        [(n, i64) for n in ("activeMaskType", "bs", "h", "topK", "moeExpertNum", "quantMode", "scoreFunc", "renormalize")] +
+                        [("routedScalingFactor", ctypes.c_float), ("expertTokenNumsType", i64), ("maxRecvRows", i64)] +
+                        [(n, pointer) for n in ("topkIdsOut", "topkWeightsOut", "expandXOut", "dynamicScalesOut", "assistInfoForCombineOut",
+                                                "expertTokenNumsOut", "sendCountsOut", "recvTotalOut")] +
+                        [("dtype", ctypes.c_int), ("routeRowsOut", pointer), ("expertScales", pointer), ("expandScalesOut", pointer), ("dedup", i64),
+                         ("assistExtOut", pointer), ("scales", pointer), ("sharedExpertNum", i64), ("sharedExpertRankNum", i64), ("tpWorldSize", i64),
+                         ("tpRankId", i64), ("tpRecvCountsOut", pointer)])
+
+        out = {n: torch.zeros(size, dtype=t, device="cuda") for n, size, t in (
+            ("expandXOut", (64, 256), torch.bfloat16), ("assistInfoForCombineOut", (64, 4), torch.int32),
+            ("expertTokenNumsOut", (4,), torch.int64), ("sendCountsOut", (4,), torch.int32), ("recvTotalOut", (1,), torch.int32))}
+        mine = torch.full((1,), 7, dtype=torch.int32, device="cuda")
+        p = Params(x=x.data_ptr(), expertIds=ids.data_ptr(), bs=16, h=256, topK=2, moeExpertNum=4, maxRecvRows=64, dtype=11, tpWorldSize=1,
+                   tpRecvCountsOut=mine.data_ptr(), **{n: t.data_ptr() for n, t in out.items()})
+        from pathlib import Path
+        lib = ctypes.CDLL(str(Path(txr.__file__).parent / "lib" / "libtilexr.so"))
+        assert lib.TileXRMoeEpDispatchFused(ctypes.byref(p), pointer(comm.handle), pointer(torch.cuda.current_stream().cuda_stream)) == 0
+        torch.cuda.synchronize()
+        assert comm.device_status() == 0 and int(out["recvTotalOut"]) == 32 and out["expertTokenNumsOut"].sum() > 0 and int(mine) == 7
+    finally:
+        comm.destroy()
