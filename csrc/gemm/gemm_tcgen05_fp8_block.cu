@@ -210,6 +210,15 @@ __device__ __forceinline__ void FbTmemLoadWait16(uint32_t *r)
                  : "memory");
 }
 
+// A wait of this CTA has given up: neither CTA of the pair stores another tile.  A promoter that gave up goes on releasing scratch
+// accumulators, which the issuer may then overwrite while the partner CTA still folds them: the partner has to know before such a
+// release can be seen, hence the fence behind the store to its flag.
+__device__ __forceinline__ void FbRaiseAbort(BlockState *st, uint32_t peerAbortAddr)
+{
+    st->abortFlag = 1;
+    asm volatile("st.volatile.shared::cluster.s32 [%0], %1;\nfence.acq_rel.cluster;" ::"r"(peerAbortAddr), "r"(1) : "memory");
+}
+
 __device__ __forceinline__ bool FbWaitBar(uint64_t *bar, uint32_t parity, BlockState *st, uint32_t peerAbortAddr, uint64_t budgetNs)
 {
     if (MbarTryWait(bar, parity)) return true;
@@ -219,14 +228,14 @@ __device__ __forceinline__ bool FbWaitBar(uint64_t *bar, uint32_t parity, BlockS
         if (MbarTryWait(bar, parity)) return true;
         if ((++polls & 127u) == 0) {
             if (st->abortFlag != 0 || FbLoadRemoteInt(peerAbortAddr) != 0) {
-                st->abortFlag = 1;
+                FbRaiseAbort(st, peerAbortAddr);
                 return false;
             }
             const uint64_t t = now_ns();
             if (deadline == 0) {
                 deadline = t + budgetNs;
             } else if (t > deadline) {
-                st->abortFlag = 1;
+                FbRaiseAbort(st, peerAbortAddr);
                 return false;
             }
         }
@@ -581,8 +590,8 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
                 asm volatile("bar.sync 1, 256;" ::: "memory");
                 const int n = min(FB_SEG, KB - kb0);
                 // One way in and one way out: with an exit for a wait that gave up, the 128 accumulators were moved to other
-                // registers and back in every block.  Such a wait has raised the abort flag; what is folded after it is
-                // never stored.
+                // registers and back in every block.  Such a wait has raised the abort flag of both CTAs; what either folds after
+                // it is never stored (a test of the verdict in front of the release cost 2 %).
                 for (int kb = 0; kb < n; ++kb) {
                     const float f = saShared[kb] * (bInSmem ? sbShared[kb0 + kb] : __ldg(sbHalf + kb0 + kb));
                     const uint32_t p = kbAll & 1u;
