@@ -13,7 +13,8 @@
 // tiles with persistent CTAs; chunks of one group are neighbours, so a second chunk finds the weight in L2.
 //
 // Roles per CTA (192 threads): warp 0 TMA, warp 1 tensor memory and MMA, warps 2-5 epilogue.  Every mbarrier wait is bounded;
-// on a give-up all roles fall through to the cluster barriers and the tear-down, and `status` tells the host.
+// on a give-up all roles fall through to the cluster barriers and the tear-down, no CTA of the cluster stores a sum that the part is
+// missing from, and `status`, where the caller gives one, tells the host.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -304,11 +305,17 @@ __global__ void __launch_bounds__(GEMM_SKINNY_THREADS, 2) TileXRGemmSkinny(const
         // it receives its slice of columns from each part, [split][tn / split][128] fp32.
         __syncthreads();
         SkClusterSync();
-        const bool work = first < items && st->abortFlag == 0;
+        const bool whole = first < items && st->abortFlag == 0;
+        if (st->abortFlag != 0 && static_cast<int>(threadIdx.x) < split) {
+            // this part is missing: everybody who would add it up learns so with the second barrier
+            uint32_t remote;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(SmemAddr(const_cast<int *>(&st->abortFlag))), "r"(threadIdx.x));
+            asm volatile("st.volatile.shared::cluster.s32 [%0], %1;" ::"r"(remote), "r"(1) : "memory");
+        }
         const int slice = a.tn / split;                        // powers of two, both
         const int sliceBits = 31 - __clz(slice);
         const int quad = warp & 3;
-        if (warp >= 2 && work) {
+        if (warp >= 2 && whole) {
             const uint32_t mine = SmemAddr(smem) + static_cast<uint32_t>((part * slice) * 128 + quad * 32 + lane) * 4u;
             for (int c0 = 0; c0 < a.tn; c0 += 16) {
                 uint32_t r[16];
@@ -324,7 +331,7 @@ __global__ void __launch_bounds__(GEMM_SKINNY_THREADS, 2) TileXRGemmSkinny(const
         }
         __syncthreads();
         SkClusterSync();
-        if (warp >= 2 && work) {
+        if (warp >= 2 && first < items && st->abortFlag == 0) {
             const SkinnyTile t = SkTileOf(a, first, rowStart, chunkStart, mTiles);
             const float *got = reinterpret_cast<const float *>(smem) + quad * 32 + lane;
             const int n = t.n0 + quad * 32 + lane;
