@@ -93,3 +93,42 @@ def test_router_logits_in_fp32(txr, tokens, h, experts, dtype):
     steps = 32 * ((h + 255) // 256) + 16
     bound = (x.double().abs() @ gate.double().abs().t()) * steps * 2.0 ** -24
     assert got.dtype == torch.float32 and ((got.double() - want).abs() <= bound).all()
+
+
+def _router(experts=8, h=64):
+    from types import SimpleNamespace
+
+    from tilexr_b200.models import ExpertParallelMoE, MoEConfig
+
+    return ExpertParallelMoE(SimpleNamespace(world_size=1, rank=0), MoEConfig(hidden=h, num_experts=experts), with_experts=False).requires_grad_(False)
+
+
+@pytest.mark.parametrize("how", ["forward_mode", "vmap", "jvp", "jit_trace", "make_fx"])
+def test_route_logits_under_transforms_and_tracing(txr, how):
+    """The router's kernel is not an operator of torch: transforms and tracers must see the matmul it stands for."""
+    layer = _router()
+    g = torch.Generator().manual_seed(4)
+    x = torch.randn(5, 64, generator=g).to(torch.bfloat16).cuda()
+    t = torch.randn(5, 64, generator=g).to(torch.bfloat16).cuda()
+    plain = lambda v: v.float() @ layer.gate.t()      # noqa: E731
+    close = dict(rtol=1e-5, atol=1e-5)                # fp32 sums of 64 products of order 1/50
+    with torch.no_grad():
+        if how == "forward_mode":
+            with torch.autograd.forward_ad.dual_level():
+                out = layer.route_logits(torch.autograd.forward_ad.make_dual(x, t))
+                tangent = torch.autograd.forward_ad.unpack_dual(out).tangent
+            assert tangent is not None and torch.allclose(tangent, plain(t), **close)
+        elif how == "jvp":
+            out, tangent = torch.func.jvp(layer.route_logits, (x,), (t,))
+            assert torch.allclose(out, plain(x), **close) and torch.allclose(tangent, plain(t), **close)
+        elif how == "vmap":
+            out = torch.func.vmap(layer.route_logits)(torch.stack((x, t)))
+            assert torch.allclose(out, torch.stack((plain(x), plain(t))), **close)
+        elif how == "jit_trace":
+            traced = torch.jit.trace(lambda v: layer.route_logits(v), x, check_trace=False)
+            assert torch.allclose(traced(t), plain(t), **close)
+        else:
+            from torch.fx.experimental.proxy_tensor import make_fx
+
+            traced = make_fx(lambda v: layer.route_logits(v))(x)
+            assert torch.allclose(traced(t), plain(t), **close)

@@ -32,6 +32,14 @@ class MoEConfig:
     dtype: torch.dtype = torch.bfloat16
 
 
+def _eager(*tensors: torch.Tensor) -> bool:
+    """Whether a kernel may stand in for torch operators on these tensors: nobody transforms, traces or intercepts the call
+    (forward-mode tangents, vmap and the other function transforms, tracing, tensor subclasses)."""
+    return (not torch.jit.is_tracing() and not torch.compiler.is_compiling() and torch._C._len_torch_dispatch_stack() == 0
+            and all(type(t) in (torch.Tensor, torch.nn.Parameter) and not torch._C._functorch.is_functorch_wrapped_tensor(t)
+                    and torch.autograd.forward_ad.unpack_dual(t).tangent is None for t in tensors))
+
+
 class ExpertParallelMoE(torch.nn.Module):
     """One MoE block whose experts are sharded over the ranks of ``comm``."""
 
@@ -60,7 +68,7 @@ class ExpertParallelMoE(torch.nn.Module):
         # needs an fp32 copy: 66 against 221 us for 4096 x 7168 by 32 experts, 136 against 139 for 3000 x 4096 by 128, 457 against
         # 371 for 4096 x 7168 by 256; with few tokens it wins at any expert count (43 against 73 us for 128 x 7168 by 256).
         favourable = gate.shape[0] <= 128 or x.shape[0] * gate.shape[0] <= 131072
-        if (favourable and not graph and x.is_cuda and x.device == gate.device and x.dtype in (torch.float16, torch.bfloat16) and gate.dtype == torch.float32
+        if (favourable and not graph and _eager(x, gate) and x.is_cuda and x.device == gate.device and x.dtype in (torch.float16, torch.bfloat16) and gate.dtype == torch.float32
                 and x.dim() == 2 and x.shape[0] > 0 and x.shape[1] == gate.shape[1] and x.shape[1] % 8 == 0 and x.is_contiguous()
                 and gate.is_contiguous() and x.data_ptr() % 16 == 0 and gate.data_ptr() % 16 == 0 and not torch.is_autocast_enabled()):
             return quant.router_logits(x, gate)
