@@ -14,7 +14,6 @@
 
 #include <algorithm>
 #include <cstdio>
-#include <mutex>
 
 #include <cuda_runtime_api.h>
 
@@ -190,12 +189,7 @@ __global__ void __launch_bounds__(RL_THREADS, 1) RouterLogitsKernel(const Router
 } // namespace
 
 template <bool BF16, int I>
-static const void *RouterKernel()
-{
-    static std::once_flag once;
-    std::call_once(once, [] { cudaFuncSetAttribute(RouterLogitsKernel<BF16, I>, cudaFuncAttributeMaxDynamicSharedMemorySize, RlSmemBytes(8 * I)); });
-    return reinterpret_cast<const void *>(&RouterLogitsKernel<BF16, I>);
-}
+static const void *RouterKernel() { return reinterpret_cast<const void *>(&RouterLogitsKernel<BF16, I>); }
 
 int LaunchRouterLogits(const void *x, const float *gate, int64_t tokens, int64_t h, int64_t experts, bool bf16, float *out, void *stream)
 {
@@ -224,7 +218,9 @@ int LaunchRouterLogits(const void *x, const float *gate, int64_t tokens, int64_t
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
     void *params[] = {&a};
-    const cudaError_t e = cudaLaunchKernelExC(&cfg, kernel, params);
+    // the limit belongs to the kernel on the current device: raised on every call, so that a second device of the process has it, too
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, RlSmemBytes(perBlock));
+    if (e == cudaSuccess) e = cudaLaunchKernelExC(&cfg, kernel, params);
     if (e != cudaSuccess) {
         fprintf(stderr, "[TileXR] router logits launch failed: %s\n", cudaGetErrorString(e));
         cudaGetLastError();

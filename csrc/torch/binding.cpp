@@ -540,6 +540,7 @@ at::Tensor RouterLogits(const at::Tensor &x, const at::Tensor &gate)
     TORCH_CHECK(x.is_cuda() && x.dim() == 2 && x.is_contiguous() && gate.is_cuda() && gate.dim() == 2 && gate.is_contiguous() &&
                     gate.scalar_type() == at::kFloat && gate.size(1) == x.size(1),
                 "x [tokens, h] 16-bit and gate [experts, h] fp32, contiguous CUDA tensors");
+    const c10::DeviceGuard guard(x.device());        // as the torch operators that this stands for
     at::Tensor out = at::empty({x.size(0), gate.size(0)}, gate.options());
     Check(TileXRMoeRouterLogits(x.data_ptr(), gate.data_ptr<float>(), x.size(0), x.size(1), gate.size(0), ToDtype(x.scalar_type()),
                                 out.data_ptr<float>(), StreamOf(x)),
@@ -603,6 +604,7 @@ at::Tensor Swiglu(const at::Tensor &gateUp)
 {
     TORCH_CHECK(gateUp.is_cuda() && gateUp.dim() == 2 && gateUp.is_contiguous() && gateUp.size(1) % 2 == 0,
                 "gate_up must be a contiguous [rows, 2 * f] CUDA tensor");
+    const c10::DeviceGuard guard(gateUp.device());
     const int64_t f = gateUp.size(1) / 2;
     at::Tensor y = at::empty({gateUp.size(0), f}, gateUp.options());
     Check(TileXRSwiglu(gateUp.data_ptr(), gateUp.size(0), f, ToDtype(gateUp.scalar_type()), y.data_ptr(), StreamOf(gateUp)), "TileXRSwiglu");
@@ -613,6 +615,7 @@ py::tuple SwigluFp8Quant(const at::Tensor &gateUp)
 {
     TORCH_CHECK(gateUp.is_cuda() && gateUp.dim() == 2 && gateUp.is_contiguous() && gateUp.size(1) % 256 == 0,
                 "gate_up must be a contiguous [rows, 2 * f] CUDA tensor with f a multiple of 128");
+    const c10::DeviceGuard guard(gateUp.device());
     const int64_t f = gateUp.size(1) / 2;
     at::Tensor y = at::empty({gateUp.size(0), f}, gateUp.options().dtype(at::kFloat8_e4m3fn));
     at::Tensor s = at::empty({gateUp.size(0), f / 128}, gateUp.options().dtype(at::kFloat));

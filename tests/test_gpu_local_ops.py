@@ -132,3 +132,14 @@ def test_route_logits_under_transforms_and_tracing(txr, how):
 
             traced = make_fx(lambda v: layer.route_logits(v))(x)
             assert torch.allclose(traced(t), plain(t), **close)
+
+
+def test_router_logits_and_swiglu_on_another_device(txr):
+    """Both stand for torch operators, which follow their tensors' device: the current one does not matter, nor which came first."""
+    if torch.cuda.device_count() < 2:
+        pytest.skip("needs two devices in one process")
+    g = torch.Generator().manual_seed(6)
+    x, gate = torch.randn(40, 2048, generator=g).to(torch.bfloat16), torch.randn(64, 2048, generator=g) / 64
+    with torch.cuda.device(0):
+        got = [(txr.quant.router_logits(x.to(d), gate.to(d)).cpu(), txr.quant.swiglu(x.to(d)).cpu()) for d in ("cuda:0", "cuda:1")]
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
