@@ -149,16 +149,8 @@ int LaunchSkinny(const void *a, const void *b, const int64_t *groupRows, void *c
     g.stages = std::min<int>(GEMM_SKINNY_MAX_STAGES, GEMM_SKINNY_RING_BYTES / (GEMM_SKINNY_W_BYTES + tn * 128));
     g.isBf16 = bf16 ? 1u : 0u;
     g.epilogue = epilogue;
-    g.split = 1;
-    const int64_t places = 2 * static_cast<int64_t>(sms);
-    const int64_t rowTiles = groupRows != nullptr ? (m + tn - 1) / tn + std::min<int64_t>(groups, GEMM_SKINNY_MAX_GROUPS) : (m + tn - 1) / tn;
-    const int64_t items = rowTiles * g.nTiles;
-    if (groupRows == nullptr) {
-        // K is split while the parts still find a place at once and each keeps four steps of K; no part may be empty
-        while (g.split < GEMM_SKINNY_MAX_SPLIT && items * g.split * 2 <= places && g.kBlocks >= g.split * 2 * 4) g.split *= 2;
-        while (g.split > 1 && (g.kBlocks + g.split - 1) / g.split * (g.split - 1) >= g.kBlocks) g.split /= 2;
-    }
-    const unsigned grid = static_cast<unsigned>(g.split > 1 ? items * g.split : std::max<int64_t>(1, std::min(items, places)));
+    const FewRowsLaunch plan = PlanFewRows(m, n, k, groupRows != nullptr ? groups : 0, tn, sms, EnvLong("TILEXR_GEMM_CTAS", 0));
+    g.split = plan.split;
     static std::once_flag once;
     std::call_once(once, [] {
         cudaFuncSetAttribute(GemmSkinnyKernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(GEMM_SKINNY_SMEM_BYTES));
@@ -169,7 +161,7 @@ int LaunchSkinny(const void *a, const void *b, const int64_t *groupRows, void *c
     attr.val.clusterDim.y = 1;
     attr.val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
+    cfg.gridDim = dim3(plan.grid);
     cfg.blockDim = dim3(GEMM_SKINNY_THREADS);
     cfg.dynamicSmemBytes = GEMM_SKINNY_SMEM_BYTES;
     cfg.stream = static_cast<cudaStream_t>(stream);
@@ -190,9 +182,6 @@ int LaunchSkinny(const void *a, const void *b, const int64_t *groupRows, void *c
     return TILEXR_SUCCESS;
 }
 
-// Rows per tile of the few-rows kernel for `rows` rows: the smallest size that holds them, 128 at most.
-int SkinnyRows(int64_t rows) { return rows <= 16 ? 16 : rows <= 32 ? 32 : rows <= 64 ? 64 : 128; }
-
 } // namespace
 
 extern "C" {
@@ -206,16 +195,9 @@ int TileXRMatmul(const void *a, const void *b, void *c, int64_t m, int64_t n, in
     int sms = 0;
     ret = SmCount(&sms);
     if (ret != TILEXR_SUCCESS) return ret;
-    // Few rows, or few 256 x 256 tiles: the kernel whose tiles are 128 columns by up to 128 rows and which splits K.
-    // A wide tile takes about 0.005 us per element of K, however few rows it has; the few-rows kernel takes 8 us (16 rows) to 16 us
-    // (128 rows) before K and N count.  us, wide and few-rows: 1 x 4096 x 1024 (m, n, k) 10.5 and 8.4; 17 x 7168 x 2048 18.4 and 12.3;
-    // 64 x 4096 x 1024 10.5 and 12.4, x 4096 24.8 and 16.2; 64 x 7168 x 2048 16.6 both, 64 x 16384 x 2048 16.6 and 20.7;
-    // 128 x 2048 x 2048 16.6 and 17.5, 128 x 7168 x 4096 26.9 and 25.0, 128 x 8192 x 8192 57.6 and 40.2; 512 x 2048 x 4096
-    // (16 tiles) 29.1 and 27.3, 384 x 4096 x 4096 (32 tiles) 29.0 and 35.0, 512 x 2048 x 2048 18.7 and 22.8.
-    const int64_t squareTiles = ((m + 2 * GEMM_BM - 1) / (2 * GEMM_BM)) * ((n + GEMM_BN - 1) / GEMM_BN);
-    const bool fewRows = m <= 32 || (m <= 64 && k >= 2048 && n <= 8192) || (k >= 4096 && (m <= GEMM_BM || squareTiles <= 16));
-    if (fewRows && EnvLong("TILEXR_GEMM_SKINNY", 1) != 0) {
-        return LaunchSkinny(a, b, nullptr, c, m, n, k, 1, SkinnyRows(m), bf16, GEMM_EPI_STORE, status, sms, stream);
+    // TILEXR_GEMM_PAIR=0 asks for the one-CTA kernel at every size.
+    if (FewRows(m, n, k) && EnvLong("TILEXR_GEMM_SKINNY", 1) != 0 && EnvLong("TILEXR_GEMM_PAIR", 1) != 0) {
+        return LaunchSkinny(a, b, nullptr, c, m, n, k, 1, FewRowsTile(m), bf16, GEMM_EPI_STORE, status, sms, stream);
     }
     GemmArgs g;
     std::memset(&g, 0, sizeof(g));
@@ -292,7 +274,7 @@ int TileXRGroupedMatmul(const void *a, const void *b, const int64_t *groupRows, 
     // from 128 rows on a group needs several tiles and reads its weight again (192 rows 229 and 297).
     const int64_t perGroup = (maxRows + groups - 1) / groups;
     if (perGroup <= EnvLong("TILEXR_GEMM_SKINNY_ROWS", 64)) {
-        return LaunchSkinny(a, b, groupRows, c, maxRows, n, k, groups, SkinnyRows(2 * perGroup), bf16, epilogue, status, sms, stream);
+        return LaunchSkinny(a, b, groupRows, c, maxRows, n, k, groups, FewRowsTile(2 * perGroup), bf16, epilogue, status, sms, stream);
     }
     GemmArgs g;
     std::memset(&g, 0, sizeof(g));

@@ -5,6 +5,7 @@
 #include <cuda.h>
 #include <stdint.h>
 
+#include "gemm_few_rows.h"
 #include "tilexr_comm_args.h"
 #include "tilexr_launch.h"
 
@@ -118,8 +119,6 @@ struct GemmBlockArgs {
 // GEMM for few rows (gemm_tcgen05_skinny.cu): 128 rows of the weight x tn rows of A per tile, two CTAs per SM.
 constexpr unsigned GEMM_SKINNY_THREADS = 192;
 constexpr int GEMM_SKINNY_MAX_STAGES = 6;
-constexpr int GEMM_SKINNY_MAX_GROUPS = 256;        // groups of one launch
-constexpr int GEMM_SKINNY_MAX_SPLIT = 8;           // CTAs of a cluster that share a tile's K
 constexpr uint32_t GEMM_SKINNY_W_BYTES = 128 * 128;
 constexpr uint32_t GEMM_SKINNY_STATE_BYTES = 256;
 constexpr uint32_t GEMM_SKINNY_RING_BYTES = 110592;      // stages x (16 KB + 128 tn): six of 18 KB down to three of 32 KB

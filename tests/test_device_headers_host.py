@@ -144,3 +144,45 @@ def test_reference_named_verbs_on_the_host(tmp_path):
     assert proc.returncode == 0, proc.stderr[-3000:]
     run = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
     assert run.returncode == 0 and run.stdout.strip() == "ok", (run.returncode, run.stdout, run.stderr)
+
+
+FEW_ROWS_PROGRAM = r'''
+#include <cstdio>
+#include "gemm_few_rows.h"
+using namespace TileXR;
+int main()
+{
+    const int sms = 148;
+    const int64_t sizes[] = {1, 16, 17, 33, 64, 128, 200, 1000};
+    const int64_t ns[] = {8, 128, 136, 2048, 7168, 131072}, ks[] = {8, 64, 520, 2048, 4104, 16384};
+    const int64_t groupCounts[] = {0, 1, 64, 300}, caps[] = {0, 1, 2, 7, 32, 148, 1000};
+    for (int64_t m : sizes) for (int64_t n : ns) for (int64_t k : ks) for (int64_t groups : groupCounts) for (int64_t cap : caps) {
+        const int tn = FewRowsTile(m);
+        const FewRowsLaunch p = PlanFewRows(m, n, k, groups, tn, sms, cap);
+        if (p.grid < 1 || p.grid > 2u * sms || (cap > 0 && p.grid > static_cast<unsigned>(cap))) return 1;      // within the cap
+        if (p.split < 1 || p.split > GEMM_SKINNY_MAX_SPLIT || (p.split & (p.split - 1)) != 0 || tn % p.split != 0) return 2;
+        if (groups > 0 && p.split != 1) return 3;
+        const int64_t kBlocks = (k + 63) / 64, per = (kBlocks + p.split - 1) / p.split;
+        if (p.split > 1 && per * (p.split - 1) >= kBlocks) return 4;                                            // no empty part
+        if (p.split > 1 && p.grid != ((m + tn - 1) / tn) * ((n + 127) / 128) * p.split) return 5;               // one tile per cluster
+    }
+    std::puts("ok");
+    return 0;
+}
+'''
+
+
+def _run_host_program(tmp_path, text, include):
+    if shutil.which("g++") is None:
+        pytest.skip("no C++ compiler")
+    src, exe = tmp_path / "program.cpp", tmp_path / "program"
+    src.write_text(text)
+    proc = subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", "-Werror", f"-I{include}", str(src), "-o", str(exe)], capture_output=True, text=True)
+    assert proc.returncode == 0, proc.stderr[-3000:]
+    run = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
+    assert run.returncode == 0 and run.stdout.strip() == "ok", (run.returncode, run.stdout, run.stderr)
+
+
+def test_few_rows_gemm_keeps_to_the_callers_ctas(tmp_path):
+    """The launch of the few-rows GEMM: never more CTAs than a caller allows, and a split of K that leaves no part empty."""
+    _run_host_program(tmp_path, FEW_ROWS_PROGRAM, ROOT / "csrc" / "gemm")

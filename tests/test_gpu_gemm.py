@@ -276,3 +276,24 @@ def test_matmul_fp8_block_scales_in_segments(txr, m, n, k):
     # fp32 sums of k products of fp8 values, one rounding to bf16
     bound = want.abs() * 2.0 ** -8 + (da.abs() @ dw.abs().t()) * k * 2.0 ** -24
     assert ((got - want).abs() <= bound).all()
+
+
+def test_matmul_few_rows_under_the_switches_of_the_other_kernels(txr, monkeypatch):
+    """TILEXR_GEMM_PAIR=0 asks for the one-CTA kernel, whose sums run over K in one piece; a cap on the CTAs leaves the result as it is."""
+    g = torch.Generator().manual_seed(2)
+    a = torch.randn(17, 2048, generator=g).to(torch.bfloat16).cuda()
+    b = (torch.randn(7168, 2048, generator=g) / 45).to(torch.bfloat16).cuda()
+    w = (torch.randn(6, 512, 2048, generator=g) / 45).to(torch.bfloat16).cuda()
+    counts = torch.tensor([3, 0, 9, 1, 0, 4], dtype=torch.int64, device="cuda")
+    with monkeypatch.context() as env:
+        env.setenv("TILEXR_GEMM_SKINNY", "0")
+        one_piece = txr.gemm.matmul(a, b)
+        env.delenv("TILEXR_GEMM_SKINNY")
+        env.setenv("TILEXR_GEMM_PAIR", "0")
+        assert torch.equal(txr.gemm.matmul(a, b), one_piece)
+    want, grouped = a.double() @ b.double().t(), txr.gemm.grouped_matmul(a, w, counts)
+    bound = want.abs() * 2.0 ** -8 + (a.double().abs() @ b.double().abs().t()) * 2048 * 2.0 ** -24
+    for ctas in ("1", "7", "64"):
+        monkeypatch.setenv("TILEXR_GEMM_CTAS", ctas)
+        assert ((txr.gemm.matmul(a, b).double() - want).abs() <= bound).all()
+        assert torch.equal(txr.gemm.grouped_matmul(a, w, counts), grouped)        # never split: the cap changes no order of sums
