@@ -12,14 +12,20 @@ constexpr int GEMM_SKINNY_MAX_GROUPS = 256;        // groups of one launch
 
 // Few rows, or few 256 x 256 tiles: the kernel whose tiles are 128 columns by up to 128 rows and which splits K.
 // A wide tile takes about 0.005 us per element of K, however few rows it has; the few-rows kernel takes 8 us (16 rows) to 16 us
-// (128 rows) before K and N count.  us, wide and few-rows: 1 x 4096 x 1024 (m, n, k) 10.5 and 8.4; 17 x 7168 x 2048 18.4 and 12.3;
-// 64 x 4096 x 1024 10.5 and 12.4, x 4096 24.8 and 16.2; 64 x 7168 x 2048 16.6 both, 64 x 16384 x 2048 16.6 and 20.7;
-// 128 x 2048 x 2048 16.6 and 17.5, 128 x 7168 x 4096 26.9 and 25.0, 128 x 8192 x 8192 57.6 and 40.2; 512 x 2048 x 4096
-// (16 tiles) 29.1 and 27.3, 384 x 4096 x 4096 (32 tiles) 29.0 and 35.0, 512 x 2048 x 2048 18.7 and 22.8.
+// (128 rows) before K and N count, and where the columns fill the chip a step of K of a tile of many rows costs it more.
+// us, wide and few-rows, weights from memory (n x k):
+//    16 rows     8192 x 256    7.1   7.6     16384 x 256    8.4   8.4     16384 x 1024  14.5  13.5     65536 x 4096  94.3  91.1
+//    32 rows    16384 x 256    8.3  10.4      8192 x 512    9.1  12.3     16384 x 1024  14.7  15.3     32768 x 4096  51.7  51.5
+//    64 rows     8192 x 2048  18.6  16.9     16384 x 2048  20.5  24.6     16384 x 4096  35.3  35.3     24576 x 4096  41.3  45.0
+//   128 rows     8192 x 2048  19.9  23.9      8192 x 4096  32.8  28.9     16384 x 4096  37.2  43.5     32768 x 4096  54.4  63.9
+//   tiles, k = 4096: 1024 x 1024 (16 tiles) 29.0 25.1, 256 x 4096 (16) 31.1 28.4; 384 x 4096 (32) 29.0 35.0
 inline bool FewRows(int64_t m, int64_t n, int64_t k)
 {
     const int64_t squareTiles = ((m + 255) / 256) * ((n + 255) / 256);
-    return m <= 32 || (m <= 64 && k >= 2048 && n <= 8192) || (k >= 4096 && (m <= 128 || squareTiles <= 16));
+    if (m <= 16) return true;
+    if (m <= 32) return k >= 1024;
+    if (m <= 64) return (k >= 2048 && n <= 8192) || (k >= 4096 && n <= 16384);
+    return k >= 4096 && (squareTiles <= 16 || (m <= 128 && n <= 8192));
 }
 
 // Rows per tile for `rows` rows: the smallest size that holds them, 128 at most.

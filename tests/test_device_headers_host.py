@@ -186,3 +186,35 @@ def _run_host_program(tmp_path, text, include):
 def test_few_rows_gemm_keeps_to_the_callers_ctas(tmp_path):
     """The launch of the few-rows GEMM: never more CTAs than a caller allows, and a split of K that leaves no part empty."""
     _run_host_program(tmp_path, FEW_ROWS_PROGRAM, ROOT / "csrc" / "gemm")
+
+
+FEW_ROWS_LINE_PROGRAM = r'''
+#include <cstdio>
+#include "gemm_few_rows.h"
+int main()
+{
+    // m, n, k, microseconds of the wide and of the few-rows kernel on a B200
+    const struct { int64_t m, n, k; double wide, few; } measured[] = {
+        {1, 1024, 4096, 28.2, 9.2},     {16, 8192, 256, 7.1, 7.6},      {16, 16384, 1024, 14.5, 13.5},  {16, 65536, 4096, 94.3, 91.1},
+        {24, 1024, 256, 6.7, 8.5},      {32, 16384, 256, 8.3, 10.4},    {24, 256, 512, 8.4, 10.5},      {32, 8192, 512, 9.1, 12.3},
+        {17, 7168, 2048, 18.5, 14.0},   {32, 16384, 1024, 14.7, 15.3},  {32, 32768, 4096, 51.7, 51.5},  {64, 4096, 1024, 12.0, 11.8},
+        {64, 8192, 2048, 18.6, 16.9},   {64, 16384, 2048, 20.5, 24.6},  {64, 16384, 4096, 35.3, 35.3},  {64, 24576, 4096, 41.3, 45.0},
+        {96, 12288, 4096, 35.1, 39.3},  {128, 8192, 2048, 19.9, 23.9},  {128, 8192, 4096, 32.8, 28.9},  {128, 16384, 4096, 37.2, 43.5},
+        {128, 32768, 4096, 54.4, 63.9}, {1024, 1024, 4096, 29.0, 25.1}, {256, 4096, 8192, 47.2, 33.6},  {384, 4096, 4096, 29.0, 35.0},
+    };
+    for (const auto &p : measured) {
+        const double taken = TileXR::FewRows(p.m, p.n, p.k) ? p.few : p.wide, other = TileXR::FewRows(p.m, p.n, p.k) ? p.wide : p.few;
+        if (taken > other * 1.08) {
+            std::printf("%d x %d x %d\n", static_cast<int>(p.m), static_cast<int>(p.n), static_cast<int>(p.k));
+            return 1;
+        }
+    }
+    std::puts("ok");
+    return 0;
+}
+'''
+
+
+def test_few_rows_line_lies_where_it_was_measured(tmp_path):
+    """The choice between the wide and the few-rows GEMM takes the slower one nowhere by more than the measurements' spread."""
+    _run_host_program(tmp_path, FEW_ROWS_LINE_PROGRAM, ROOT / "csrc" / "gemm")
