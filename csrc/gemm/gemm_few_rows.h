@@ -31,6 +31,19 @@ inline bool FewRows(int64_t m, int64_t n, int64_t k)
 // Rows per tile for `rows` rows: the smallest size that holds them, 128 at most.
 inline int FewRowsTile(int64_t rows) { return rows <= 16 ? 16 : rows <= 32 ? 32 : rows <= 64 ? 64 : 128; }
 
+// Rows per tile for `rows` rows in `groups` groups whose sizes are on the device.  Tiles of twice the average hold most groups, but a
+// group of many rows then takes many tiles: 64 groups of 4096 x 2048, 512 rows, all in one group, 49 us with tiles of 16 rows, 29 with 64
+// (38 before there was this kernel); with eight rows each 171 and 167, so larger tiles cost the even case nothing from some 100 rows on.
+// Below that the rows themselves weigh: one row in each of 8 groups of 4096 x 4096 48 us with 16, 58 with 64.  128 rows where a group
+// holds 64 on average: 64 each 179 us with 64 and 183 with 128, sizes falling as 1 / g 214 and 200; up to 48 on average 64 rows are the safer ones
+// (2048 x 1024, 48 on average, all in a quarter of the groups: 37 and 43 us, 36 before).
+inline int FewRowsGroupTile(int64_t rows, int64_t groups)
+{
+    if (rows < 128) return 16;
+    if (rows <= 256) return 32;
+    return rows < 1024 || rows <= 48 * groups ? 64 : 128;
+}
+
 struct FewRowsLaunch {
     int split;          // CTAs of a cluster that share a tile's K
     unsigned grid;      // CTAs

@@ -269,12 +269,13 @@ int TileXRGroupedMatmul(const void *a, const void *b, const int64_t *groupRows, 
     int sms = 0;
     ret = SmCount(&sms);
     if (ret != TILEXR_SUCCESS) return ret;
-    // Few rows per group on average (the counts themselves are on the device): tiles of twice the average hold most groups.
-    // 64 groups of 4096 x 2048: 4 rows each 204 us with CTA pairs, 164 with this kernel; 32 rows 222 and 172; 64 rows 223 and 186;
-    // from 128 rows on a group needs several tiles and reads its weight again (192 rows 229 and 297).
+    // Few rows per group on average (the counts themselves are on the device).
+    // 64 groups of 4096 x 2048: 4 rows each 195 us with CTA pairs, 166 with this kernel; 32 rows 236 and 171; 64 rows 223 and 184;
+    // from 128 rows on a group needs several tiles and reads its weight again (192 rows 229 and 297).  At 64 rows on average sizes that fall
+    // as 1 / g keep the gain (235 and 205; of 2048 x 1024 68 and 63); all rows in a quarter of the groups lose: 83 and 89, of 2048 x 1024 27 and 45.
     const int64_t perGroup = (maxRows + groups - 1) / groups;
     if (perGroup <= EnvLong("TILEXR_GEMM_SKINNY_ROWS", 64)) {
-        return LaunchSkinny(a, b, groupRows, c, maxRows, n, k, groups, FewRowsTile(2 * perGroup), bf16, epilogue, status, sms, stream);
+        return LaunchSkinny(a, b, groupRows, c, maxRows, n, k, groups, FewRowsGroupTile(maxRows, groups), bf16, epilogue, status, sms, stream);
     }
     GemmArgs g;
     std::memset(&g, 0, sizeof(g));

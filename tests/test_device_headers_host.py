@@ -209,6 +209,20 @@ int main()
             return 1;
         }
     }
+    // groups of uneven sizes: rows, groups, microseconds before there was the kernel and with tiles of 16, 32, 64 and 128 rows
+    const struct { int64_t rows, groups; double before, t16, t32, t64, t128; } uneven[] = {
+        {8, 8, 80.1, 48.4, 49.1, 58.3, 80.5},         {64, 64, 32.0, 15.2, 17.0, 19.3, 20.1},    {512, 64, 37.6, 49.2, 34.1, 29.0, 35.3},
+        {1024, 64, 40.8, 69.5, 47.7, 37.4, 35.6},     {512, 8, 45.0, 68.0, 45.8, 39.6, 46.8},    {3072, 64, 35.7, 51.7, 36.5, 35.4, 42.5},
+        {16384, 256, 123.2, 282.3, 165.4, 115.6, 101.9},
+    };
+    for (const auto &p : uneven) {
+        const int tn = TileXR::FewRowsGroupTile(p.rows, p.groups);
+        const double taken = tn == 16 ? p.t16 : tn == 32 ? p.t32 : tn == 64 ? p.t64 : p.t128;
+        if (taken > p.before) {
+            std::printf("%d rows, %d groups\n", static_cast<int>(p.rows), static_cast<int>(p.groups));
+            return 2;
+        }
+    }
     std::puts("ok");
     return 0;
 }
