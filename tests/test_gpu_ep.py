@@ -626,3 +626,57 @@ def test_lane_counts_are_zero_whatever_becomes_of_a_dispatch(txr, port):
         assert comm.device_status() == 0 and int(out["recvTotalOut"]) == 32 and out["expertTokenNumsOut"].sum() > 0 and int(mine) == 7
     finally:
         comm.destroy()
+
+
+@pytest.mark.parametrize("score_func", [0, 1])
+@pytest.mark.parametrize("experts,top_k", [(5, 5), (33, 8), (256, 8), (500, 6), (1000, 32)])
+def test_routing_topk_of_equal_and_invalid_scores(txr, experts, top_k, score_func):
+    """Equal scores go to the lower expert; an expert whose score is NaN or minus infinity is never picked, and slots without a candidate
+    have weight zero and an id that no expert has."""
+    g = torch.Generator().manual_seed(experts)
+    logits = torch.randint(-2, 3, (64, experts), generator=g).float()          # five values: ties in every row
+    bias = torch.zeros(experts)
+    logits[1] = 0.5                                                            # all equal
+    if score_func == 1:
+        bias = torch.randint(0, 2, (experts,), generator=g) * 0.25 - 0.5       # sums below, at and above zero
+        bias[::7] = float("-inf")
+        logits[2, 1::2] = float("nan")
+        logits[3, 1:] = float("nan")                                           # at most one valid expert
+        logits[4] = float("nan")
+        logits[5, 0], logits[5, 1] = float("inf"), float("-inf")
+    ids, w = txr.quant.routing_topk(logits.cuda(), top_k, score_func, True, 2.0, bias.cuda() if score_func == 1 else None)
+    ids, w = ids.cpu(), w.cpu()
+    scores = torch.softmax(logits, -1) if score_func == 0 else torch.sigmoid(logits)
+    sel = scores + bias
+    for t in range(64):
+        valid = [e for e in range(experts) if sel[t, e] > float("-inf")]
+        want = sorted(valid, key=lambda e: (-float(sel[t, e]), e))[:top_k]
+        assert ids[t, :len(want)].tolist() == want, t
+        assert all(i == 0x7fffffff for i in ids[t, len(want):].tolist())
+        if want:
+            picked = scores[t, want]
+            assert torch.allclose(w[t, :len(want)], picked / picked.sum() * 2.0, rtol=1e-5, atol=0)
+            assert not w[t, len(want):].any()
+
+
+def test_dispatch_of_tokens_with_few_valid_experts(txr, port):
+    """Routing fused into the dispatch: a slot without a candidate is an inactive route."""
+    ep = txr.ep
+    g = torch.Generator().manual_seed(9)
+    tokens, experts, top_k = 40, 16, 4
+    logits = torch.randn(tokens, experts, generator=g)
+    for t in range(tokens):
+        logits[t, torch.randperm(experts, generator=g)[:experts - t % 6]] = float("nan")      # t % 6 valid experts
+    x = torch.randn(tokens, 64, generator=g).to(torch.bfloat16).cuda()
+    comm = txr.init_process(0, 1, comm_id=f"127.0.0.1:{port}", buffer_mb=16, device=0)
+    try:
+        d = ep.dispatch(comm, x, gate_logits=logits.cuda(), num_experts=experts, top_k=top_k, score_func=1)
+        torch.cuda.synchronize()
+        assert comm.device_status() == 0
+        want = [(e, t) for t in range(tokens) for e in torch.argsort(logits[t].nan_to_num(-100.0), descending=True)[:min(top_k, t % 6)].tolist()]
+        n = len(want)
+        assert int(d.recv_total) == n and [(e, t) for _, t, _, e in d.assist[:n].tolist()] == sorted(want)
+        assert torch.equal(d.expand_x[:n], x[[t for _, t in sorted(want)]])
+        assert ((d.route_rows >= 0).sum(dim=1).cpu() == torch.tensor([min(top_k, t % 6) for t in range(tokens)])).all()
+    finally:
+        comm.destroy()

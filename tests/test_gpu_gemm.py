@@ -278,6 +278,73 @@ def test_matmul_fp8_block_scales_in_segments(txr, m, n, k):
     assert ((got - want).abs() <= bound).all()
 
 
+def _exact_block_operands(rows, n, k, seed):
+    """Small whole numbers with scales that are powers of two from 2^-2 to 2^2, so that every sum is exact: products are multiples of
+    2^-4, and sums of them that stay below 2^20 (_exact_block_product asserts it) fit 24 bits.  Neighbouring blocks have different scales."""
+    g = torch.Generator().manual_seed(seed)
+    kb, nb = k // 128, (n + 127) // 128
+    qa = torch.randint(-2, 3, (rows, k), generator=g).float().to(torch.float8_e4m3fn).cuda()
+    qw = torch.randint(-1, 2, (n, k), generator=g).float().to(torch.float8_e4m3fn).cuda()
+    exponent = lambda r: (torch.randint(0, 5, (r, 1), generator=g) + torch.cumsum(torch.randint(1, 5, (r, kb), generator=g), 1)) % 5 - 2      # noqa: E731
+    return qa, torch.exp2(exponent(rows).float()).cuda(), qw, torch.exp2(exponent(nb).float()).cuda()
+
+
+def _exact_block_product(qa, sa, qw, sw):
+    """The product in 64 bits, checked to be one that 32-bit sums give exactly in any order."""
+    rows, k = qa.shape
+    da = (qa.double().view(rows, -1, 128) * sa.double()[:, :, None]).view(rows, k)
+    dw = qw.double() * sw.double().repeat_interleave(128, dim=0)[:qw.shape[0]].repeat_interleave(128, dim=1)
+    want = da @ dw.t()
+    assert (da.abs() @ dw.abs().t()).max() < 2.0 ** 20 and torch.equal(want * 16, (want * 16).round())
+    return want
+
+
+@pytest.mark.parametrize("m,n,k", [(260, 264, 128 * 65), (130, 256, 128 * 130), (4100, 5128, 128), (1300, 7176, 128 * 3), (100, 256, 128 * 260)])
+def test_matmul_fp8_block_scales_exactly(txr, m, n, k):
+    """The sizes of the test above with operands whose product is exact: one wrong scale of one block of K shows."""
+    ops = _exact_block_operands(m, n, k, k + m)
+    assert torch.equal(txr.gemm.matmul_fp8_block(*ops), _exact_block_product(*ops).to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("ranks,shard_rows,n,k", [(4, 256, 2568, 128 * 68), (2, 512, 2824, 512), (2, 256, 136, 128 * 132)])
+def test_all_gather_matmul_fp8_block_exactly(txr, ranks, shard_rows, n, k):
+    """Several tiles per CTA pair, own and peers' in turn (the next tile's scales are fetched ahead for own rows only), and more blocks of K than
+    a CTA holds scales for, with operands whose product is exact."""
+    world = txr.init_emulated_world(ranks, device=0, buffer_mb=16)
+    try:
+        ops = [_exact_block_operands(shard_rows, n, k, 90 + r) for r in range(ranks)]
+        a_staging = world.symm_empty((ranks * shard_rows, k), torch.float8_e4m3fn)
+        s_staging = world.symm_empty((ranks * shard_rows, k // 128), torch.float32)
+        qa, sa = torch.cat([o[0] for o in ops]), torch.cat([o[1] for o in ops])
+        for _ in range(2):
+            outs = world.run(lambda c, r: txr.gemm.all_gather_matmul_fp8_block(c, ops[r][0], ops[r][1], a_staging[r], s_staging[r], ops[r][2], ops[r][3]))
+            world.check()
+            for r in range(ranks):
+                assert torch.equal(outs[r], _exact_block_product(qa, sa, ops[r][2], ops[r][3]).to(torch.bfloat16))
+                assert torch.equal(a_staging[r].view(torch.uint8), qa.view(torch.uint8)) and torch.equal(s_staging[r], sa)
+    finally:
+        world.destroy()
+
+
+@pytest.mark.parametrize("ranks,shard_rows,n,k", [(4, 256, 2568, 128 * 65), (2, 512, 2824, 128), (2, 256, 136, 128 * 129)])
+def test_matmul_reduce_scatter_fp8_block_exactly(txr, ranks, shard_rows, n, k):
+    """Several tiles per CTA pair (a tile's staging shares its memory with the next tile's scales) and more blocks of K than a CTA holds
+    scales for, with operands whose partial products are exact."""
+    world = txr.init_emulated_world(ranks, device=0, buffer_mb=16)
+    try:
+        m = ranks * shard_rows
+        ops = [_exact_block_operands(m, n, k, 110 + r) for r in range(ranks)]
+        staging = world.symm_empty((m, n), torch.bfloat16)
+        want = sum(_exact_block_product(*o).to(torch.bfloat16).float() for o in ops)        # in rank order, as the owner adds them
+        for _ in range(2):
+            outs = world.run(lambda c, r: txr.gemm.matmul_reduce_scatter_fp8_block(c, ops[r][0], ops[r][1], ops[r][2], ops[r][3], staging[r]))
+            world.check()
+            for r in range(ranks):
+                assert torch.equal(outs[r], want[r * shard_rows:(r + 1) * shard_rows].to(torch.bfloat16))
+    finally:
+        world.destroy()
+
+
 def test_matmul_few_rows_under_the_switches_of_the_other_kernels(txr, monkeypatch):
     """TILEXR_GEMM_PAIR=0 asks for the one-CTA kernel, whose sums run over K in one piece; a cap on the CTAs leaves the result as it is."""
     g = torch.Generator().manual_seed(2)
