@@ -11,7 +11,7 @@
 //   warps 2-5   epilogue: tcgen05.ld the accumulator (each warp owns 32 TMEM lanes = 32 rows),
 //               convert, store.
 // Every mbarrier wait is bounded: if one gives up, the CTA raises a shared abort flag, every
-// role leaves its loop, tensor memory is released and `status` tells the host.
+// role leaves its loop, tensor memory is released and `status`, where the caller gives one, tells the host.
 //
 // All-gather -> GEMM: the leading `commBlocks` CTAs do no math; they push this rank's A shard
 // into every peer's staging buffer in (128 rows x K/4) pieces and raise one flag per piece.

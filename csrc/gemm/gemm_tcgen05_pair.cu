@@ -13,7 +13,7 @@
 // multicast: both CTAs signal the LEADER's "full" barrier); warp 1 owns tensor memory and, in the leader, issues
 // the MMAs and commits them to both CTAs' barriers; warps 2-5 read the accumulator with tcgen05.ld and store C.
 // Every mbarrier wait is bounded and checks the pair's abort flags; on a give-up all roles fall through to the
-// tear-down, both CTAs meet at the cluster barrier, tensor memory is released and `status` tells the host.
+// tear-down, both CTAs meet at the cluster barrier, tensor memory is released and `status`, where the caller gives one, tells the host.
 //
 // Fused modes: all-gather -> GEMM: warps 6-7 of EVERY CTA write this rank's A shard into the peers' staging buffers
 // piece by piece (128 rows x a chunk of K) and raise each piece's flag -- through the NVLink multicast alias of the
