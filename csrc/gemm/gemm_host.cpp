@@ -215,6 +215,8 @@ int TileXRMatmul(const void *a, const void *b, void *c, int64_t m, int64_t n, in
         // CTA pairs on 256x256 tiles: each CTA loads half of the B tile (its own tensor map box of 128 rows)
         ret = MakeMap(&g.tmapB, b, n, k, GEMM_BN / 2, bf16);
         if (ret != TILEXR_SUCCESS) return ret;
+        ret = MakeMap(&g.tmapTail, a, m, k, GEMM_TAIL_BOX, bf16);
+        if (ret != TILEXR_SUCCESS) return ret;
         g.rasterGroup = static_cast<int32_t>(std::max<long>(1, EnvLong("TILEXR_GEMM_GROUP", 8)));
         const int pairTiles = static_cast<int>((m + 2 * GEMM_BM - 1) / (2 * GEMM_BM)) * g.nBlocks;
         const int pairs = std::max(1, std::min<int>(pairTiles, static_cast<int>(EnvLong("TILEXR_GEMM_CTAS", sms)) / 2));
@@ -283,6 +285,8 @@ int TileXRGroupedMatmul(const void *a, const void *b, const int64_t *groupRows, 
     if (ret != TILEXR_SUCCESS) return ret;
     ret = MakeMap(&g.tmapB, b, groups * n, k, GEMM_BN / 2, bf16);
     if (ret != TILEXR_SUCCESS) return ret;
+    ret = MakeMap(&g.tmapTail, a, maxRows, k, GEMM_TAIL_BOX, bf16);
+    if (ret != TILEXR_SUCCESS) return ret;
     g.tmapALocal = g.tmapA;
     g.c = static_cast<uint8_t *>(c);
     g.status = status;
@@ -336,6 +340,8 @@ int TileXRMatmulFp8(const void *a, const void *b, void *c, int64_t m, int64_t n,
     int ret = MakeMap8(&g.tmapA, a, m, k, GEMM_BM);
     if (ret != TILEXR_SUCCESS) return ret;
     ret = MakeMap8(&g.tmapB, b, n, k, GEMM_BN / 2);
+    if (ret != TILEXR_SUCCESS) return ret;
+    ret = MakeMap8(&g.tmapTail, a, m, k, GEMM_TAIL_BOX);
     if (ret != TILEXR_SUCCESS) return ret;
     g.tmapALocal = g.tmapA;
     g.c = static_cast<uint8_t *>(c);

@@ -26,6 +26,8 @@ constexpr int GEMM_MAX_K_CHUNKS = 4;     // all-gather flags per 128-row block
 // CTA-pair kernel (cta_group::2): per CTA and stage 128 rows of A and half of the 256-row B tile.
 constexpr uint32_t GEMM_PAIR_STAGE_BYTES = GEMM_STAGE_A_BYTES + GEMM_STAGE_B_BYTES / 2;
 constexpr int GEMM_PAIR_STAGES = 6;
+constexpr int GEMM_TAIL_BOX = 32;        // rows of A per load of a tile that is computed as C^T (a row block that is not full)
+constexpr uint32_t GEMM_TAIL_BOX_BYTES = GEMM_TAIL_BOX * GEMM_BK * 2;
 constexpr size_t GEMM_PAIR_SMEM_BYTES = 1024 /* alignment slack */ + GEMM_PAIR_STAGES * GEMM_PAIR_STAGE_BYTES + 1024 /* barriers */ +
                                         GEMM_BM * 256 /* epilogue staging tile */;
 
@@ -41,6 +43,7 @@ struct GemmArgs {
     CUtensorMap tmapA;        // A [M, K] row-major (all-gather: the staging buffer [R * shardRows, K])
     CUtensorMap tmapALocal;   // all-gather: this rank's shard [shardRows, K]
     CUtensorMap tmapB;        // B [N, K] row-major (the weight; C = A x B^T)
+    CUtensorMap tmapTail;     // CTA-pair kernel, plain and grouped modes: A again, boxes of GEMM_TAIL_BOX rows
     uint8_t *c;               // plain / all-gather: C [M, N]; reduce-scatter: out [shardRows, N]
     const uint8_t *aLocal;    // all-gather: shard to push to the peers
     CommArgs *comm;

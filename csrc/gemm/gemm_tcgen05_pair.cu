@@ -111,13 +111,13 @@ __device__ __forceinline__ uint64_t MakeSmemDesc(uint32_t smemAddr)
     return d;
 }
 
-// kind::f16, D fp32, A/B K-major; M = 256 rows over the pair, N = 256.
+// kind::f16, D fp32, A/B K-major; M = 256 rows over the pair; N comes with the tile (InstrWidth).
 __device__ __forceinline__ uint32_t MakeInstrDesc(bool bf16)
 {
     const uint32_t fmt = bf16 ? 1u : 0u;
-    return (1u << 4) | (fmt << 7) | (fmt << 10) | (static_cast<uint32_t>(GEMM_BN >> 3) << 17) |
-           (static_cast<uint32_t>((2 * GEMM_BM) >> 4) << 24);
+    return (1u << 4) | (fmt << 7) | (fmt << 10) | (static_cast<uint32_t>((2 * GEMM_BM) >> 4) << 24);
 }
+__device__ __forceinline__ uint32_t InstrWidth(int n) { return static_cast<uint32_t>(n >> 3) << 17; }
 
 __device__ __forceinline__ void UmmaPairF16(uint32_t tmemD, uint64_t descA, uint64_t descB, uint32_t idesc, uint32_t accumulate)
 {
@@ -136,8 +136,7 @@ __device__ __forceinline__ void UmmaPairF16(uint32_t tmemD, uint64_t descA, uint
 __device__ __forceinline__ uint32_t MakeInstrDescFp8(int fp8Format)
 {
     const uint32_t fmt = fp8Format == 2 ? 1u : 0u;
-    return (1u << 4) | (fmt << 7) | (fmt << 10) | (static_cast<uint32_t>(GEMM_BN >> 3) << 17) |
-           (static_cast<uint32_t>((2 * GEMM_BM) >> 4) << 24);
+    return (1u << 4) | (fmt << 7) | (fmt << 10) | (static_cast<uint32_t>((2 * GEMM_BM) >> 4) << 24);
 }
 
 __device__ __forceinline__ void UmmaPairF8(uint32_t tmemD, uint64_t descA, uint64_t descB, uint32_t idesc, uint32_t accumulate)
@@ -249,7 +248,26 @@ struct PairTile {
     int row0;       // grouped mode: first row of the pair's 256-row block in A and C
     int rowEnd;     // grouped mode: end of the group's rows
     int rowB0;      // grouped mode: first row of the group's weight in B
+    int width;      // columns of the instruction: 256, or what is left in the plain and grouped modes, in steps of 32
+    bool flipped;   // the tile is computed as C^T: 256 rows of B by `width` rows of A
 };
+
+// The last row block of a product, or of a group, seldom has 256 rows, and the last column block seldom 256 columns.  The
+// instruction's M is 256 whatever exists, its N is not: the operand with less left in the tile becomes N.  With 32 groups of
+// some 1024 rows every group's last block was an eighth of the work, nearly all of it rows that do not exist (4096 tokens, top-8,
+// 7168 x 2048 SwiGLU experts: the two launches 2739 -> 2437 us).
+// The epilogue of a tile of C^T takes some 10 ns per row longer, which a launch of a few waves waits for and a longer one
+// hides behind the next tile: `flipRows` is the most rows that are taken this way (FlipRows).
+__device__ __forceinline__ void SetWidth(PairTile *c, int rowsLeft, int colsLeft, int flipRows)
+{
+    const int rows = min(2 * GEMM_BM, (rowsLeft + 31) & ~31);
+    const int cols = min(GEMM_BN, (colsLeft + 31) & ~31);
+    c->flipped = rows < cols && rows <= flipRows;
+    c->width = c->flipped ? rows : cols;
+}
+// 200 x 8192 x 4096 (one wave) 28.9 us as 200 rows by 256 columns, 33.1 flipped; 700 x 8192 x 1024 (96 tiles on 74 pairs) 20.6 and 24.7;
+// 1200 x 8192 x 8192 (160 tiles, the last row block of 176 rows) 139 and 140; up to 128 rows neither form is ahead in one wave.
+__device__ __forceinline__ int FlipRows(int tiles, int pairs) { return tiles >= 4 * pairs ? 2 * GEMM_BM : GEMM_BM; }
 
 // Grouped mode: where the rows and the 256-row blocks of each group of this launch start (shared memory, behind the barriers).
 struct GroupTable {
@@ -257,7 +275,7 @@ struct GroupTable {
     int blockStart[GEMM_MAX_GROUPS + 1];
 };
 
-__device__ __forceinline__ PairTile TileOf(const GemmArgs &a, int t, int mTiles, int rank, int ranks, const GroupTable *gt)
+__device__ __forceinline__ PairTile TileOf(const GemmArgs &a, int t, int mTiles, int rank, int ranks, const GroupTable *gt, int flipRows)
 {
     PairTile c;
     if (a.mode == GEMM_GROUPED) {
@@ -273,13 +291,19 @@ __device__ __forceinline__ PairTile TileOf(const GemmArgs &a, int t, int mTiles,
         c.row0 = gt->rowStart[lo] + c.mLocalPair * 2 * GEMM_BM;
         c.rowEnd = gt->rowStart[lo + 1];
         c.rowB0 = (a.groupBase + lo) * a.N;
+        SetWidth(&c, c.rowEnd - c.row0, a.N - c.nBlock * GEMM_BN, flipRows);
         return c;
     }
-    c.row0 = c.rowEnd = c.rowB0 = 0;
+    c.rowEnd = a.M;
+    c.rowB0 = 0;
+    c.width = GEMM_BN;
+    c.flipped = false;
     if (a.mode == GEMM_PLAIN) {
         PairTileAt(t, mTiles, a.nBlocks, a.rasterGroup, &c.mTile, &c.nBlock);
         c.shard = 0;
         c.mLocalPair = c.mTile;
+        c.row0 = c.mTile * 2 * GEMM_BM;
+        SetWidth(&c, a.M - c.row0, a.N - c.nBlock * GEMM_BN, flipRows);
     } else {
         const int pairsPerShard = a.blocksPerShard / 2;
         const int perShard = pairsPerShard * a.nBlocks;
@@ -290,6 +314,7 @@ __device__ __forceinline__ PairTile TileOf(const GemmArgs &a, int t, int mTiles,
         // of pairs would otherwise span all of the shard's A rows and little of B, and A would stream from DRAM
         PairTileAt(u, pairsPerShard, a.nBlocks, max(1, a.rasterGroup), &c.mLocalPair, &c.nBlock);
         c.mTile = c.shard * pairsPerShard + c.mLocalPair;
+        c.row0 = c.mTile * 2 * GEMM_BM;
     }
     return c;
 }
@@ -417,6 +442,7 @@ __device__ void PairBody(const GemmArgs &a)
     const int commPairs = firstCta >> 1;
     const int mTiles = a.mode == GEMM_GROUPED ? gt->blockStart[a.groups] : (a.M + 2 * GEMM_BM - 1) / (2 * GEMM_BM);
     const int allTiles = mTiles * a.nBlocks;
+    const int flipRows = FlipRows(allTiles, static_cast<int>(gridDim.x) >> 1);
     const int commTiles = min(allTiles, commPairs * static_cast<int>(a.commTilesPerPair));
     int pair, nPairs, totalTiles, tileBase, tileSign;
     if (commCta) {
@@ -437,19 +463,22 @@ __device__ void PairBody(const GemmArgs &a)
     const int kPerStage = fp8 ? 2 * GEMM_BK : GEMM_BK;      // elements of K in one 128-byte swizzle row
 
     if (warp == 0) {
-        // ---- TMA producer: this CTA's 128 rows of A and its half of the B tile ---------------------------------
+        // ---- TMA producer: this CTA's 128 rows of A and its half of the B tile (the other way round in a tile of C^T) ----
         uint32_t stage = 0, phase = 0;
         for (int t = pair; t < totalTiles && __all_sync(0xffffffffu, st->abortFlag == 0); t += nPairs) {
-            const PairTile tc = TileOf(a, tileBase + tileSign * t, mTiles, rank, ranks, gt);
+            const PairTile tc = TileOf(a, tileBase + tileSign * t, mTiles, rank, ranks, gt, flipRows);
             const int mLocal = tc.mLocalPair * 2 + static_cast<int>(ctaRank);        // this CTA's 128-row block in the shard
             const bool remoteA = a.mode == GEMM_ALL_GATHER && tc.shard != rank;
             const CUtensorMap *mapA = (a.mode == GEMM_ALL_GATHER && !remoteA) ? &a.tmapALocal : &a.tmapA;
             // grouped: a block starts wherever its group's rows start; rows past the group's end belong to the
             // next group (or are filled with zeros past the end of A) and are computed but never stored
-            const int rowA = a.mode == GEMM_GROUPED ? tc.row0 + static_cast<int>(ctaRank) * GEMM_BM
-                             : (a.mode == GEMM_ALL_GATHER && !remoteA) ? mLocal * GEMM_BM
-                                                                       : tc.mTile * 2 * GEMM_BM + static_cast<int>(ctaRank) * GEMM_BM;
-            const int rowB = tc.rowB0 + tc.nBlock * GEMM_BN + static_cast<int>(ctaRank) * (GEMM_BN / 2);
+            const int rowA = (a.mode == GEMM_ALL_GATHER && !remoteA) ? mLocal * GEMM_BM : tc.row0 + static_cast<int>(ctaRank) * GEMM_BM;
+            // each CTA of the pair supplies half of the instruction's N: rows of B, or of A in a tile of C^T
+            const int half = tc.width / 2;
+            const int rowB = tc.rowB0 + tc.nBlock * GEMM_BN + static_cast<int>(ctaRank) * (tc.flipped ? GEMM_BM : half);
+            const int rowTail = tc.row0 + static_cast<int>(ctaRank) * half;
+            const int tailBoxes = (half + GEMM_TAIL_BOX - 1) / GEMM_TAIL_BOX;
+            const uint32_t stageBytes = tc.flipped ? GEMM_STAGE_A_BYTES + static_cast<uint32_t>(tailBoxes) * GEMM_TAIL_BOX_BYTES : GEMM_PAIR_STAGE_BYTES;
             bool broke = false;
             for (int kb = 0; kb < a.kBlocks; ++kb) {
                 if (!WaitBarWarp(&st->empty[stage], phase ^ 1u, st, peerAbortAddr, budgetNs)) {
@@ -472,9 +501,16 @@ __device__ void PairBody(const GemmArgs &a)
                 if (ElectOne()) {
                     uint8_t *sa = stageBase + stage * GEMM_PAIR_STAGE_BYTES;
                     uint8_t *sb = sa + GEMM_STAGE_A_BYTES;
-                    if (leader) MbarExpectTx(&st->full[stage], 2 * GEMM_PAIR_STAGE_BYTES);
-                    TmaLoadPair2D(sa, mapA, kb * kPerStage, rowA, &st->full[stage]);
-                    TmaLoadPair2D(sb, &a.tmapB, kb * kPerStage, rowB, &st->full[stage]);
+                    if (leader) MbarExpectTx(&st->full[stage], 2 * stageBytes);
+                    if (tc.flipped) {
+                        TmaLoadPair2D(sa, &a.tmapB, kb * kPerStage, rowB, &st->full[stage]);
+                        for (int i = 0; i < tailBoxes; ++i) {
+                            TmaLoadPair2D(sb + i * GEMM_TAIL_BOX_BYTES, &a.tmapTail, kb * kPerStage, rowTail + i * GEMM_TAIL_BOX, &st->full[stage]);
+                        }
+                    } else {
+                        TmaLoadPair2D(sa, mapA, kb * kPerStage, rowA, &st->full[stage]);
+                        TmaLoadPair2D(sb, &a.tmapB, kb * kPerStage, rowB, &st->full[stage]);
+                    }
                 }
                 if (++stage == GEMM_PAIR_STAGES) {
                     stage = 0;
@@ -486,7 +522,7 @@ __device__ void PairBody(const GemmArgs &a)
     } else if (warp == 1) {
         // ---- MMA issuer: one elected lane of the leader drives the tensor cores of both SMs -----------------------
         if (leader) {
-            const uint32_t idesc = fp8 ? MakeInstrDescFp8(a.fp8Format) : MakeInstrDesc(bf16);
+            const uint32_t idesc0 = fp8 ? MakeInstrDescFp8(a.fp8Format) : MakeInstrDesc(bf16);
             const uint64_t descA0 = MakeSmemDesc(SmemAddr(stageBase));
             const uint64_t descB0 = MakeSmemDesc(SmemAddr(stageBase) + GEMM_STAGE_A_BYTES);
             uint32_t stage = 0, phase = 0;
@@ -494,6 +530,7 @@ __device__ void PairBody(const GemmArgs &a)
             for (int t = pair; t < totalTiles && __all_sync(0xffffffffu, st->abortFlag == 0); t += nPairs, ++iter) {
                 const int acc = iter & 1;
                 const uint32_t accPhase = (iter >> 1) & 1;
+                const uint32_t idesc = idesc0 | InstrWidth(TileOf(a, tileBase + tileSign * t, mTiles, rank, ranks, gt, flipRows).width);
                 if (!WaitBarWarp(&st->tmemEmpty[acc], accPhase ^ 1u, st, peerAbortAddr, budgetNs)) break;
                 TcFenceAfter();
                 const uint32_t tmemD = tmemBase + static_cast<uint32_t>(acc) * GEMM_BN;
@@ -597,7 +634,7 @@ __device__ void PairBody(const GemmArgs &a)
         const float outScale = fp8 ? a.alpha : 1.0f;
         int iter = 0;
         for (int t = pair; t < totalTiles; t += nPairs, ++iter) {
-            const PairTile tc = TileOf(a, tileBase + tileSign * t, mTiles, rank, ranks, gt);
+            const PairTile tc = TileOf(a, tileBase + tileSign * t, mTiles, rank, ranks, gt, flipRows);
             const int nBlock = tc.nBlock;
             const int acc = iter & 1;
             const uint32_t accPhase = (iter >> 1) & 1;
@@ -620,26 +657,44 @@ __device__ void PairBody(const GemmArgs &a)
                 rowsValid = static_cast<int>(max(static_cast<int64_t>(0), min(static_cast<int64_t>(GEMM_BM), a.shardRows - localRow0)));
                 rowBase = reg->regions[a.stageHandle].peerBase[tc.shard] + a.stageOffset +
                           (static_cast<uint64_t>(rank) * a.shardRows + static_cast<uint64_t>(localRow0)) * a.N * 2;
-            } else if (a.mode == GEMM_GROUPED) {
-                const int row0 = tc.row0 + static_cast<int>(ctaRank) * GEMM_BM;
-                rowsValid = max(0, min(GEMM_BM, tc.rowEnd - row0));
-                rowBase = a.c + static_cast<uint64_t>(row0) * outRowBytes;
             } else {
-                const int64_t row0 = static_cast<int64_t>(tc.mTile) * 2 * GEMM_BM + static_cast<int64_t>(ctaRank) * GEMM_BM;
-                rowsValid = static_cast<int>(max(static_cast<int64_t>(0), min(static_cast<int64_t>(GEMM_BM), a.M - row0)));
+                // both CTAs store all rows of a tile of C^T, each 128 of its columns
+                const int row0 = tc.row0 + (tc.flipped ? 0 : static_cast<int>(ctaRank) * GEMM_BM);
+                rowsValid = max(0, min(tc.flipped ? tc.width : GEMM_BM, tc.rowEnd - row0));
                 rowBase = a.c + static_cast<uint64_t>(row0) * outRowBytes;
             }
-            const int col0 = nBlock * GEMM_BN;
+            const int col0 = nBlock * GEMM_BN + (tc.flipped ? static_cast<int>(ctaRank) * GEMM_BM : 0);
+            const int passes = (tc.width + 127) / 128;
 #pragma unroll 1
-            for (int pass = 0; pass < 2; ++pass) {                   // 128 columns of the product at a time
+            for (int pass = 0; pass < passes; ++pass) {              // 128 columns of the accumulator at a time
+                const int chunks = min(4, (tc.width - pass * 128) / 32);
 #pragma unroll 1
-                for (int cc = 0; cc < 4; ++cc) {
+                for (int cc = 0; cc < chunks; ++cc) {
                     uint32_t r[32];
                     const uint32_t taddr = tmemBase + (static_cast<uint32_t>(quad * 32) << 16) +
                                            static_cast<uint32_t>(acc * GEMM_BN + pass * 128 + cc * 32);
                     TmemLoad32(taddr, r);
                     TmemLoadWait();
-                    if (swiglu) {
+                    if (tc.flipped) {
+                        // lane = column of C, register = row of C: neighbouring lanes trade values of neighbouring rows, so that each
+                        // holds two columns (or gate and up) of one row, and the staging tile is as in the other form
+                        const int odd = lane & 1;
+                        uint8_t *to = stageC + (cc * 32 + odd) * 256;       // row j of the 32 is row j of `to`: its chunks are swizzled by its number
+                        const uint32_t at = (swiglu ? static_cast<uint32_t>(quad * 16 + (lane >> 1)) * 2u : static_cast<uint32_t>(quad * 32 + (lane & ~1)) * 2u) ^
+                                            static_cast<uint32_t>(odd << 4);
+#pragma unroll
+                        for (int j = 0; j < 32; j += 2) {
+                            const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? r[j] : r[j + 1], 1);
+                            const float lo = __uint_as_float(odd ? got : r[j]) * outScale;
+                            const float hi = __uint_as_float(odd ? r[j + 1] : got) * outScale;
+                            if (swiglu) {
+                                const uint32_t o = PackPair(lo / (1.0f + __expf(-lo)) * hi, 0.f, bf16);
+                                *reinterpret_cast<uint16_t *>(to + j * 256 + (at ^ ((j & 7) << 4))) = static_cast<uint16_t>(o);
+                            } else {
+                                *reinterpret_cast<uint32_t *>(to + j * 256 + (at ^ ((j & 15) << 4))) = PackPair(lo, hi, bf16);
+                            }
+                        }
+                    } else if (swiglu) {
                         // 32 columns = 16 (gate, up) pairs -> 16 outputs = two 16-byte chunks of a 128-byte row piece
                         uint32_t packed[8];
 #pragma unroll
@@ -673,23 +728,27 @@ __device__ void PairBody(const GemmArgs &a)
                         }
                     }
                 }
-                if (pass == 1) {
+                if (pass == passes - 1) {
                     // the accumulator buffer is read out: the MMA lane may overwrite it with the tile after next
                     TcFenceBefore();
                     __syncwarp();
                     if (lane == 0) ArriveCluster(SmemAddr(&st->tmemEmpty[acc]) & PEER_BIT_MASK);
                 }
                 asm volatile("bar.sync 1, 128;" ::: "memory");
+                // the 128 rows (or fewer) by 128 columns of the product in the staging tile and where they go
+                const int col1 = tc.flipped ? col0 : col0 + pass * 128;
+                const int rowsHere = tc.flipped ? rowsValid - pass * 128 : rowsValid;
+                uint8_t *rowsTo = rowBase + (tc.flipped ? static_cast<uint64_t>(pass) * 128 * outRowBytes : 0);
                 if (swiglu) {
 #pragma unroll 4
                     for (int k = 0; k < 8; ++k) {
                         const int idx = et + k * 128;
                         const int rr = idx >> 3;
                         const int ch = idx & 7;
-                        const int col = (col0 + pass * 128) / 2 + ch * 8;
-                        if (rr < rowsValid && col < outN) {
+                        const int col = col1 / 2 + ch * 8;
+                        if (rr < rowsHere && col < outN) {
                             const uint4 v = *reinterpret_cast<const uint4 *>(stageC + rr * 256 + ((ch ^ (rr & 7)) * 16));
-                            st_vec16(rowBase + static_cast<uint64_t>(rr) * outRowBytes + static_cast<uint64_t>(col) * 2, Vec16{v.x, v.y, v.z, v.w});
+                            st_vec16(rowsTo + static_cast<uint64_t>(rr) * outRowBytes + static_cast<uint64_t>(col) * 2, Vec16{v.x, v.y, v.z, v.w});
                         }
                     }
                 } else {
@@ -698,10 +757,10 @@ __device__ void PairBody(const GemmArgs &a)
                         const int idx = et + k * 128;
                         const int rr = idx >> 4;
                         const int ch = idx & 15;
-                        const int col = col0 + pass * 128 + ch * 8;
-                        if (rr < rowsValid && col < a.N) {
+                        const int col = col1 + ch * 8;
+                        if (rr < rowsHere && col < a.N) {
                             const uint4 v = *reinterpret_cast<const uint4 *>(stageC + rr * 256 + ((ch ^ (rr & 15)) * 16));
-                            st_vec16(rowBase + static_cast<uint64_t>(rr) * a.N * 2 + static_cast<uint64_t>(col) * 2, Vec16{v.x, v.y, v.z, v.w});
+                            st_vec16(rowsTo + static_cast<uint64_t>(rr) * a.N * 2 + static_cast<uint64_t>(col) * 2, Vec16{v.x, v.y, v.z, v.w});
                         }
                     }
                 }

@@ -364,3 +364,51 @@ def test_matmul_few_rows_under_the_switches_of_the_other_kernels(txr, monkeypatc
         monkeypatch.setenv("TILEXR_GEMM_CTAS", ctas)
         assert ((txr.gemm.matmul(a, b).double() - want).abs() <= bound).all()
         assert torch.equal(txr.gemm.grouped_matmul(a, w, counts), grouped)        # never split: the cap changes no order of sums
+
+
+def _small_ints(g, *shape, dtype=torch.bfloat16):
+    return torch.randint(-2, 3, shape, generator=g, device="cuda").to(dtype)
+
+
+@pytest.mark.parametrize("m", [129, 160, 161, 255, 256, 257, 288, 289, 384, 385, 479, 481, 511, 513])
+@pytest.mark.parametrize("n,k", [(8, 64), (264, 200), (512, 328), (4104, 136)])
+def test_matmul_of_partial_tiles_exactly(txr, m, n, k):
+    """Row and column blocks that are not full: the operand with less left becomes the instruction's N, in steps of 32.  Small whole
+    numbers (|sum| <= 4 k, exact in fp32), so the only rounding is the one of the output."""
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    a, b = _small_ints(g, m, k), _small_ints(g, n, k)
+    want = (a.double() @ b.double().t()).to(torch.bfloat16)
+    assert torch.equal(txr.gemm.matmul(a, b), want)
+    assert torch.equal(txr.gemm.matmul(a.half(), b.half()), (a.double() @ b.double().t()).half())
+    if k % 16 == 0:
+        f8 = torch.float8_e4m3fn
+        assert torch.equal(txr.gemm.matmul_fp8(a.to(f8), b.to(f8), 1.0), want)
+
+
+@pytest.mark.parametrize("m,n", [(1160, 19208), (1249, 9480)])
+def test_matmul_of_partial_tiles_in_many_waves(txr, m, n):
+    """More than four tiles per CTA pair: row blocks of more than 128 rows are computed as C^T, too."""
+    g = torch.Generator(device="cuda").manual_seed(m)
+    a, b = _small_ints(g, m, 72), _small_ints(g, n, 72)
+    assert torch.equal(txr.gemm.matmul(a, b), (a.double() @ b.double().t()).to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("epilogue", [0, 1])
+@pytest.mark.parametrize("n,k,counts", [(272, 136, [257, 0, 33, 512, 200, 1, 480]), (512, 64, [300, 31, 32, 225, 224]), (16, 72, [129, 600]),
+                                        (9488, 64, [700, 0, 161, 400, 224, 225, 96])])
+def test_grouped_matmul_of_partial_tiles(txr, n, k, counts, epilogue):
+    """Groups that end inside a row block, computed as C^T where fewer rows than columns are left; rows behind the last group stay."""
+    g = torch.Generator(device="cuda").manual_seed(n + k)
+    total = sum(counts)
+    rows, w = _small_ints(g, total + 3, k), _small_ints(g, len(counts), n, k)
+    nums = torch.tensor(counts, dtype=torch.int64, device="cuda")
+    out = torch.full((total + 3, n // 2 if epilogue else n), 7.0, dtype=torch.bfloat16, device="cuda")
+    got = txr.gemm.grouped_matmul(rows, w, nums, epilogue, out)
+    prod = torch.cat([r.double() @ w[i].double().t() for i, r in enumerate(rows[:total].split(counts))])
+    if epilogue == 0:
+        assert torch.equal(got[:total], prod.to(torch.bfloat16))
+    else:
+        want = torch.nn.functional.silu(prod[:, 0::2]) * prod[:, 1::2]
+        # one rounding to bf16 (2^-9) of an fp32 value whose exponential and division are a few ulp of fp32 off
+        assert torch.allclose(got[:total].double(), want, rtol=2 ** -8, atol=1e-6)
+    assert torch.equal(got[total:], torch.full_like(got[total:], 7.0))
