@@ -65,6 +65,36 @@ inline FewRowsLaunch PlanFewRows(int64_t m, int64_t n, int64_t k, int64_t groups
     return {split, static_cast<unsigned>(split > 1 ? items * split : std::max<int64_t>(1, std::min(items, places)))};
 }
 
+// How the 256 x 256 tiles of a block-scaled fp8 product are dealt out to CTA pairs: the first `wide` whole, the others in slices of
+// `width` columns, so that a last wave of a few tiles, or a product of a few tiles, does not leave most pairs without work.  Every slice
+// reads its tile's rows of A again and waits for the same round trips per block of K, so the narrow ones are not cheap.
+// us, whole tiles and the choice: 2048 x 7168 x 4096 (224 tiles on 74 pairs, the last two in slices of 32) 86.7 78.4; 4096 x 7168 x 4096
+// (448, the last four so) 149 139; 16 x 7168 x 2048 (28, slices of 128) 14.6 12.6; 100 x 4096 x 4096 (16, slices of 64) 21.7 17.6.
+struct Fp8Slices {
+    int wide, width, items;
+};
+inline Fp8Slices PlanFp8Slices(int64_t tiles, int64_t pairs)
+{
+    constexpr int WIDTHS[] = {128, 64, 32};
+    constexpr int COST[] = {56, 36, 30};             // of a slice, a whole tile 100
+    Fp8Slices best = {static_cast<int>(tiles), 256, static_cast<int>(tiles)};
+    int64_t bestCost = (tiles + pairs - 1) / pairs * 100;
+    const int64_t rounds = tiles / pairs;
+    for (int64_t keep = rounds; keep >= std::max<int64_t>(0, rounds - 1); --keep) {
+        const int64_t rest = tiles - keep * pairs;
+        if (rest == 0) continue;
+        for (int i = 0; i < 3; ++i) {
+            const int64_t slices = rest * (256 / WIDTHS[i]);
+            const int64_t cost = keep * 100 + (slices + pairs - 1) / pairs * COST[i];
+            if (cost < bestCost) {
+                bestCost = cost;
+                best = {static_cast<int>(keep * pairs), WIDTHS[i], static_cast<int>(keep * pairs + slices)};
+            }
+        }
+    }
+    return best;
+}
+
 } // namespace TileXR
 
 #endif // TILEXR_GEMM_FEW_ROWS_H

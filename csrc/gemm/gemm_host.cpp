@@ -182,6 +182,17 @@ int LaunchSkinny(const void *a, const void *b, const int64_t *groupRows, void *c
     return TILEXR_SUCCESS;
 }
 
+// Whole tiles and slices of a block-scaled fp8 product for `pairs` CTA pairs, and the tensor map that slices of B are loaded with.
+int Fp8Slicing(GemmBlockArgs *g, const void *b, int64_t pairs)
+{
+    const int64_t tiles = (static_cast<int64_t>(g->M) + 2 * GEMM_BM - 1) / (2 * GEMM_BM) * g->nBlocks;
+    const Fp8Slices s = PlanFp8Slices(tiles, std::max<int64_t>(1, pairs));
+    g->wideTiles = s.wide;
+    g->sliceWidth = s.width;
+    g->items = s.items;
+    return MakeMap8(&g->tmapBSlice, b, g->N, g->K, GEMM_FP8_SLICE_BOX);
+}
+
 } // namespace
 
 extern "C" {
@@ -412,8 +423,9 @@ int TileXRMatmulFp8BlockScaled(const void *a, const float *scaleA, const void *b
     int sms = 0;
     ret = SmCount(&sms);
     if (ret != TILEXR_SUCCESS) return ret;
-    const int pairTiles = static_cast<int>((m + 2 * GEMM_BM - 1) / (2 * GEMM_BM)) * g.nBlocks;
-    const int pairs = std::max(1, std::min<int>(pairTiles, static_cast<int>(EnvLong("TILEXR_GEMM_CTAS", sms)) / 2));
+    ret = Fp8Slicing(&g, b, EnvLong("TILEXR_GEMM_CTAS", sms) / 2);
+    if (ret != TILEXR_SUCCESS) return ret;
+    const int pairs = std::max(1, std::min<int>(g.items, static_cast<int>(EnvLong("TILEXR_GEMM_CTAS", sms)) / 2));
     static std::once_flag once;
     std::call_once(once, [] {
         cudaFuncSetAttribute(GemmFp8BlockKernel(GEMM_PLAIN), cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(GEMM_FP8_BLOCK_SMEM_BYTES));
@@ -667,6 +679,9 @@ static int Fp8BlockCommon(GemmBlockArgs *g, const void *b, const float *scaleB, 
     g->shardRows = static_cast<int32_t>(shardRows);
     g->blocksPerShard = static_cast<int32_t>(shardRows / GEMM_BM);
     g->flagStride = TILEXR_MAX_RANK_SIZE * TILEXR_FLAGS_PER_PAIR / R;
+    g->items = static_cast<int32_t>((m + 2 * GEMM_BM - 1) / (2 * GEMM_BM)) * g->nBlocks;
+    g->wideTiles = g->items;
+    g->sliceWidth = GEMM_BN;
     return TILEXR_SUCCESS;
 }
 
@@ -721,6 +736,8 @@ int TileXRAllGatherMatmulFp8Block(const void *aShard, const float *scaleAShard, 
     g.sOffset = sOffset;
     unsigned grid = 0;
     ret = Fp8BlockFusedGrid(comm, hostArgs, g.mode, &grid);
+    if (ret != TILEXR_SUCCESS) return ret;
+    ret = Fp8Slicing(&g, b, grid / 2);
     if (ret != TILEXR_SUCCESS) return ret;
     int64_t magic = 0;
     ret = TileXRCommNextMagic(comm, &magic);

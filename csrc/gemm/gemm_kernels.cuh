@@ -84,6 +84,7 @@ enum GemmEpilogue : int32_t { GEMM_EPI_STORE = 0, GEMM_EPI_SWIGLU = 1 };
 // Block-scaled fp8 GEMM (gemm_tcgen05_fp8_block.cu): warp 0 TMA, warp 1 MMA, warps 4-11 fold the scratch accumulators.
 constexpr unsigned GEMM_FP8_BLOCK_THREADS = 384;
 constexpr int GEMM_FP8_BLOCK_STAGES = 5;     // one stage less than the bf16 kernel: the weight scales of a tile live in shared memory too
+constexpr int GEMM_FP8_SLICE_BOX = 16;       // rows of B per load of a slice
 constexpr int GEMM_FP8_BLOCK_SCALE_SEG = 64; // blocks of K whose activation scales a CTA holds
 constexpr size_t GEMM_FP8_BLOCK_SMEM_BYTES = 1024 /* alignment slack */ + GEMM_FP8_BLOCK_STAGES * GEMM_PAIR_STAGE_BYTES + 1024 /* barriers */ +
                                              GEMM_BM * (GEMM_FP8_BLOCK_SCALE_SEG + 1) * 4 /* activation scales, or the 256-byte rows of the staging tile */;
@@ -92,6 +93,7 @@ struct GemmBlockArgs {
     CUtensorMap tmapA;        // A [M, K] 8-bit, box 128 rows x 128 bytes
     CUtensorMap tmapALocal;   // all-gather: this rank's shard [shardRows, K]
     CUtensorMap tmapB;        // B [N, K] 8-bit, box 128 rows x 128 bytes
+    CUtensorMap tmapBSlice;   // B again, box GEMM_FP8_SLICE_BOX rows x 128 bytes
     const float *scaleA;      // [M, K / 128]
     const float *scaleB;      // [scaleBRows, K / 128], one row per 128 rows of B
     uint8_t *c;               // [M, N] bf16 or fp16
@@ -101,6 +103,9 @@ struct GemmBlockArgs {
     int32_t kBlocks;          // K / 128
     int32_t scaleBRows;       // ceil(N / 128)
     int32_t rasterGroup;
+    // The first wideTiles tiles of the walk are computed whole (256 columns), the others in slices of sliceWidth columns (128, 64 or 32;
+    // 256 where there are none): `items` pieces of work altogether.  PlanFp8Slices (gemm_few_rows.h)
+    int32_t wideTiles, sliceWidth, items;
     uint32_t isBf16;
     int32_t fp8Format;        // 1 = e4m3, 2 = e5m2
     // Fused modes (GemmMode).  ALL_GATHER: tmapA and scaleA describe THIS rank's staging buffers ([R * shardRows, K] rows,

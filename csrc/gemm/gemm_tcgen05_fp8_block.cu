@@ -163,12 +163,11 @@ __device__ __forceinline__ uint64_t FbSmemDesc(uint32_t smemAddr)
     return d;
 }
 
-// kind::f8f6f4, D fp32, A and B K-major, M = 256 rows over the pair, N = 256.
-__device__ __forceinline__ uint32_t FbInstrDesc(int fp8Format)
+// kind::f8f6f4, D fp32, A and B K-major, M = 256 rows over the pair, N = `width`.
+__device__ __forceinline__ uint32_t FbInstrDesc(int fp8Format, int width)
 {
     const uint32_t fmt = fp8Format == 2 ? 1u : 0u;
-    return (1u << 4) | (fmt << 7) | (fmt << 10) | (static_cast<uint32_t>(GEMM_BN >> 3) << 17) |
-           (static_cast<uint32_t>((2 * GEMM_BM) >> 4) << 24);
+    return (1u << 4) | (fmt << 7) | (fmt << 10) | (static_cast<uint32_t>(width >> 3) << 17) | (static_cast<uint32_t>((2 * GEMM_BM) >> 4) << 24);
 }
 
 __device__ __forceinline__ void FbUmma(uint32_t tmemD, uint64_t descA, uint64_t descB, uint32_t idesc, uint32_t accumulate)
@@ -305,6 +304,32 @@ __device__ __forceinline__ void FbTileOf(const GemmBlockArgs &a, int t, int mTil
     }
 }
 
+template <int N> struct FbCols { static constexpr int value = N; };
+
+struct FbItem {
+    int mTile, nBlock;
+    int col0, width;     // columns of C
+};
+
+// Item `i` of the launch: a whole tile or a slice of one.  A slice may lie past the last column (col0 >= N): nobody works on it.
+template <int MODE>
+__device__ __forceinline__ FbItem FbItemOf(const GemmBlockArgs &a, int i, int mTiles, int rank)
+{
+    FbItem it;
+    int t = i, slice = 0;
+    it.width = GEMM_BN;
+    if (MODE != GEMM_REDUCE_SCATTER && i >= a.wideTiles) {
+        const int per = GEMM_BN / a.sliceWidth;
+        const int u = i - a.wideTiles;
+        t = a.wideTiles + u / per;
+        slice = u % per;
+        it.width = a.sliceWidth;
+    }
+    FbTileOf(a, t, mTiles, rank, &it.mTile, &it.nBlock);
+    it.col0 = it.nBlock * GEMM_BN + slice * it.width;
+    return it;
+}
+
 // Twelve warps start with 168 registers each (the most a block of this size can have); the first warpgroup then
 // shrinks to 80 and the two promoter warpgroups grow to 208 (128 x 80 + 256 x 208 of the 384 x 168 registers of the launch),
 // so that 128 accumulators and two 16-register tensor-memory reads fit.
@@ -373,7 +398,7 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
     const uint32_t tmemBase = st->tmemBase;
 
     const int mTiles = (a.M + 2 * GEMM_BM - 1) / (2 * GEMM_BM);
-    const int totalTiles = mTiles * a.nBlocks;
+    const int items = a.items;
     const int pair = static_cast<int>(blockIdx.x) >> 1;
     const int nPairs = static_cast<int>(gridDim.x) >> 1;
     const bool bf16 = a.isBf16 != 0;
@@ -387,11 +412,12 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
         const int rank = fused ? a.comm->rank : 0;
         Waiter w{fused ? a.comm : nullptr, st->epoch, static_cast<int32_t>(blockIdx.x), TILEXR_DEV_OK, 0};
         uint32_t stage = 0, phase = 0;
-        for (int t = pair; t < totalTiles && __all_sync(0xffffffffu, st->abortFlag == 0); t += nPairs) {
-            int mTile, nBlock;
-            FbTileOf(a, t, mTiles, rank, &mTile, &nBlock);
-            const int rowA = mTile * 2 * GEMM_BM + static_cast<int>(ctaRank) * GEMM_BM;
-            const int rowB = nBlock * GEMM_BN + static_cast<int>(ctaRank) * (GEMM_BN / 2);
+        for (int t = pair; t < items && __all_sync(0xffffffffu, st->abortFlag == 0); t += nPairs) {
+            const FbItem it = FbItemOf<MODE>(a, t, mTiles, rank);
+            if (it.col0 >= a.N) continue;
+            const int rowA = it.mTile * 2 * GEMM_BM + static_cast<int>(ctaRank) * GEMM_BM;
+            const int rowB = it.col0 + static_cast<int>(ctaRank) * (it.width / 2);       // each CTA supplies half of the item's rows of B
+            const uint32_t stageBytes = GEMM_STAGE_A_BYTES + static_cast<uint32_t>(it.width / 2) * 128u;
             bool own = false;              // the rows are this rank's shard
             if (MODE == GEMM_ALL_GATHER) {
                 // this CTA's 128 rows of the gathered A: wait until their owner has written them here
@@ -419,9 +445,13 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
                 if (ElectOne()) {
                     uint8_t *sa = stageBase + stage * GEMM_PAIR_STAGE_BYTES;
                     uint8_t *sb = sa + GEMM_STAGE_A_BYTES;
-                    if (leader) MbarExpectTx(&st->full[stage], 2 * GEMM_PAIR_STAGE_BYTES);
+                    if (leader) MbarExpectTx(&st->full[stage], 2 * stageBytes);
                     FbTmaLoad(sa, mapA, kb * 128, yA, &st->full[stage]);       // x in bytes = elements: a multiple of 128
-                    FbTmaLoad(sb, &a.tmapB, kb * 128, rowB, &st->full[stage]);
+                    if (MODE == GEMM_REDUCE_SCATTER || it.width == GEMM_BN) {
+                        FbTmaLoad(sb, &a.tmapB, kb * 128, rowB, &st->full[stage]);
+                    } else {
+                        for (int r = 0; r < it.width / 2; r += GEMM_FP8_SLICE_BOX) FbTmaLoad(sb + r * 128, &a.tmapBSlice, kb * 128, rowB + r, &st->full[stage]);
+                    }
                 }
                 if (++stage == GEMM_FP8_BLOCK_STAGES) {
                     stage = 0;
@@ -434,12 +464,14 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
         // ---- MMA issuer: per block of K, four N = 256 instructions into the scratch of its parity --------------------
         if (leader) {
             const uint64_t budgetNs = fused ? a.comm->waitTimeoutNs : 4000000000ull;
-            const uint32_t idesc = FbInstrDesc(a.fp8Format);
             const uint64_t descA0 = FbSmemDesc(SmemAddr(stageBase));
             const uint64_t descB0 = FbSmemDesc(SmemAddr(stageBase) + GEMM_STAGE_A_BYTES);
             uint32_t stage = 0, phase = 0;
             uint32_t kbAll = 0;                    // blocks of K issued so far, over all tiles: the scratch buffers alternate with it
-            for (int t = pair; t < totalTiles && __all_sync(0xffffffffu, st->abortFlag == 0); t += nPairs) {
+            for (int t = pair; t < items && __all_sync(0xffffffffu, st->abortFlag == 0); t += nPairs) {
+                const FbItem it = FbItemOf<MODE>(a, t, mTiles, 0);       // its width and whether it exists, the same for every rank
+                if (it.col0 >= a.N) continue;
+                const uint32_t idesc = FbInstrDesc(a.fp8Format, it.width);
                 bool broke = false;
                 for (int kb = 0; kb < a.kBlocks; ++kb, ++kbAll) {
                     const uint32_t p = kbAll & 1u;
@@ -548,21 +580,20 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
             }
         };
         auto ofPeer = [&](int64_t tileRow) { return gathered && tileRow / a.shardRows != a.comm->rank; };
-        bool ahead = false;                        // the tile's first segment of scales is already on its way
-        for (int t = pair; t < totalTiles; t += nPairs) {
-            int mTile, nBlock;
-            FbTileOf(a, t, mTiles, fused ? a.comm->rank : 0, &mTile, &nBlock);
-            const int64_t row0 = static_cast<int64_t>(mTile) * 2 * GEMM_BM + static_cast<int64_t>(ctaRank) * GEMM_BM;
+        bool ahead = false;                        // the item's first segment of scales is already on its way
+        // One item, of which this thread folds COLS columns of its row.  False: a wait has given up, nobody goes on.
+        auto foldItem = [&](auto tag, const FbItem &it, int t) -> bool {
+            constexpr int COLS = decltype(tag)::value;
+            const int64_t row0 = static_cast<int64_t>(it.mTile) * 2 * GEMM_BM + static_cast<int64_t>(ctaRank) * GEMM_BM;
             const int64_t gRow = row0 + myRow;
             const bool rowValid = gRow < a.M;
+            const int myCol = it.col0 + h * COLS;
             // scale blocks of B for the two column halves
-            const int nb0 = min(nBlock * 2, a.scaleBRows - 1);
-            const int nb1 = min(nBlock * 2 + 1, a.scaleBRows - 1);
-            const float *sb0 = a.scaleB + static_cast<int64_t>(nb0) * KB;
-            const float *sb1 = a.scaleB + static_cast<int64_t>(nb1) * KB;
-            float acc[FB_HALF_N];
+            const float *sb0 = a.scaleB + static_cast<int64_t>(min(it.col0 / 128, a.scaleBRows - 1)) * KB;
+            const float *sb1 = a.scaleB + static_cast<int64_t>(min((it.col0 + COLS) / 128, a.scaleBRows - 1)) * KB;
+            float acc[COLS];
 #pragma unroll
-            for (int j = 0; j < FB_HALF_N; ++j) acc[j] = 0.f;
+            for (int j = 0; j < COLS; ++j) acc[j] = 0.f;
             // The scales go to shared memory, the weight's two rows of the table once per tile and the activations' 128 rows
             // FB_SEG blocks of K at a time: a lane reading its own row's scale from memory for every block touches 32 lines
             // per warp and block.
@@ -600,18 +631,18 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
                     FbWaitBarWarp(&st->scratchFull[p], (kbAll >> 1) & 1u, st, peerAbortAddr, budgetNs);
                     ++kbAll;
                     FbFenceAfter();
-                    const uint32_t taddr = tmemBase + (static_cast<uint32_t>(quad * 32) << 16) + p * GEMM_BN + static_cast<uint32_t>(h * FB_HALF_N);
+                    const uint32_t taddr = tmemBase + (static_cast<uint32_t>(quad * 32) << 16) + p * GEMM_BN + static_cast<uint32_t>(h * COLS);
                     // Sixteen columns at a time, the next ones on their way while these are folded (8192^3: 8 columns 538 us,
                     // 16 columns 523 us, 32 columns 565 us, before the modes had kernels of their own).
                     uint32_t r[2][16];
                     FbTmemLoad16(taddr, r[0]);
 #pragma unroll
-                    for (int cc = 0; cc < 8; ++cc) {
+                    for (int cc = 0; cc < COLS / 16; ++cc) {
                         FbTmemLoadWait16(r[cc & 1]);
-                        if (cc < 7) {
+                        if (cc < COLS / 16 - 1) {
                             FbTmemLoad16(taddr + (cc + 1) * 16, r[(cc + 1) & 1]);
                         } else {
-                            // the half is in registers: the issuer may overwrite it two blocks of K from now
+                            // the columns are in registers: the issuer may overwrite them two blocks of K from now
                             FbFenceBefore();
                             __syncwarp();
                             if (lane == 0) FbArriveCluster(SmemAddr(&st->scratchEmpty[p]) & FB_PEER_BIT_MASK);
@@ -626,32 +657,33 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
             asm volatile("bar.sync 1, 256;" ::: "memory");
             if (pt == 0) sExit = (st->abortFlag != 0) ? 1 : 0;
             asm volatile("bar.sync 1, 256;" ::: "memory");
-            if (sExit != 0) break;
-            const int col0 = nBlock * GEMM_BN;
+            if (sExit != 0) return false;
             ahead = false;
             if (MODE != GEMM_REDUCE_SCATTER) {
-                // the next tile's scales come while this one is stored (everybody has left the loop that reads them)
-                if (t + nPairs < totalTiles) {
-                    int mNext, nNext;
-                    FbTileOf(a, t + nPairs, mTiles, fused ? a.comm->rank : 0, &mNext, &nNext);
-                    const int64_t rowNext = static_cast<int64_t>(mNext) * 2 * GEMM_BM + static_cast<int64_t>(ctaRank) * GEMM_BM;
-                    ahead = !ofPeer(rowNext);
+                // the next item's scales come while this one is stored (everybody has left the loop that reads them)
+                if (t + nPairs < items) {
+                    const FbItem next = FbItemOf<MODE>(a, t + nPairs, mTiles, fused ? a.comm->rank : 0);
+                    const int64_t rowNext = static_cast<int64_t>(next.mTile) * 2 * GEMM_BM + static_cast<int64_t>(ctaRank) * GEMM_BM;
+                    ahead = next.col0 < a.N && !ofPeer(rowNext);
                     if (ahead) loadScaleA(rowNext, false, 0);
                 }
-                // Local memory: every thread stores its 256 bytes of a row straight from registers, without the two trips
+                // Local memory: every thread stores its piece of a row straight from registers, without the two trips
                 // of the tile through shared memory and their barriers (the issuer has only two blocks of K of work ahead).
                 if (rowValid) {
-                    uint8_t *rowPtr = a.c + (static_cast<uint64_t>(gRow) * a.N + col0 + h * FB_HALF_N) * 2;
+                    uint8_t *rowPtr = a.c + (static_cast<uint64_t>(gRow) * a.N + myCol) * 2;
 #pragma unroll
-                    for (int v = 0; v < 16; ++v) {
-                        if (col0 + h * FB_HALF_N + v * 8 < a.N) {
+                    for (int v = 0; v < COLS / 8; ++v) {
+                        if (myCol + v * 8 < a.N) {
                             st_vec16(rowPtr + v * 16, Vec16{FbPackPair(acc[8 * v], acc[8 * v + 1], bf16), FbPackPair(acc[8 * v + 2], acc[8 * v + 3], bf16),
                                                             FbPackPair(acc[8 * v + 4], acc[8 * v + 5], bf16), FbPackPair(acc[8 * v + 6], acc[8 * v + 7], bf16)});
                         }
                     }
                 }
-                continue;
+                return true;
             }
+            if constexpr (COLS == FB_HALF_N) {
+            const int nBlock = it.nBlock;
+            const int col0 = it.col0;
             // ---- the partial tile goes into the row owner's staging slot for this rank, behind NVLink: through a swizzled
             // staging tile, so that every warp store covers whole row pieces; the two groups take turns with it ----------
             const int block = static_cast<int>(row0 / GEMM_BM);
@@ -691,6 +723,18 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
                 st_relaxed_sys_u64(FlagSlot(a.comm, owner, FB_FLAG_PLANE_B + static_cast<int64_t>(a.comm->rank) * a.flagStride + tileLocal),
                                    MakeFlag(st->epoch, 1));
             }
+            }
+            return true;
+        };
+        for (int t = pair; t < items; t += nPairs) {
+            const FbItem it = FbItemOf<MODE>(a, t, mTiles, fused ? a.comm->rank : 0);
+            if (it.col0 >= a.N) continue;
+            bool go = true;
+            if (MODE == GEMM_REDUCE_SCATTER || it.width == GEMM_BN) go = foldItem(FbCols<FB_HALF_N>{}, it, t);
+            else if (it.width == 128) go = foldItem(FbCols<64>{}, it, t);
+            else if (it.width == 64) go = foldItem(FbCols<32>{}, it, t);
+            else go = foldItem(FbCols<16>{}, it, t);
+            if (!go) break;
         }
         // ---- reduce-scatter: add the partial tiles of the output tiles this CTA owns, in rank order ---------------------
         if (MODE == GEMM_REDUCE_SCATTER) {

@@ -412,3 +412,11 @@ def test_grouped_matmul_of_partial_tiles(txr, n, k, counts, epilogue):
         # one rounding to bf16 (2^-9) of an fp32 value whose exponential and division are a few ulp of fp32 off
         assert torch.allclose(got[:total].double(), want, rtol=2 ** -8, atol=1e-6)
     assert torch.equal(got[total:], torch.full_like(got[total:], 7.0))
+
+
+@pytest.mark.parametrize("m,n,k", [(300, 9480, 256), (6401, 776, 128 * 29), (100, 7176, 384), (257, 2184, 128 * 57)])
+def test_matmul_fp8_block_slices_exactly(txr, m, n, k):
+    """One tile or two behind a wave of whole ones (slices of 32 columns, the last of them past N), and few tiles altogether (slices of
+    128 and of 64 columns)."""
+    ops = _exact_block_operands(m, n, k, k + m)
+    assert torch.equal(txr.gemm.matmul_fp8_block(*ops), _exact_block_product(*ops).to(torch.bfloat16))
