@@ -83,11 +83,13 @@ enum GemmEpilogue : int32_t { GEMM_EPI_STORE = 0, GEMM_EPI_SWIGLU = 1 };
 
 // Block-scaled fp8 GEMM (gemm_tcgen05_fp8_block.cu): warp 0 TMA, warp 1 MMA, warps 4-11 fold the scratch accumulators.
 constexpr unsigned GEMM_FP8_BLOCK_THREADS = 384;
-constexpr int GEMM_FP8_BLOCK_STAGES = 5;     // one stage less than the bf16 kernel: the weight scales of a tile live in shared memory too
+constexpr int GEMM_FP8_BLOCK_STAGES = 5;     // one stage less than the bf16 kernel: scales and staging tiles live in shared memory too
 constexpr int GEMM_FP8_SLICE_BOX = 16;       // rows of B per load of a slice
-constexpr int GEMM_FP8_BLOCK_SCALE_SEG = 64; // blocks of K whose activation scales a CTA holds
-constexpr size_t GEMM_FP8_BLOCK_SMEM_BYTES = 1024 /* alignment slack */ + GEMM_FP8_BLOCK_STAGES * GEMM_PAIR_STAGE_BYTES + 1024 /* barriers */ +
-                                             GEMM_BM * (GEMM_FP8_BLOCK_SCALE_SEG + 1) * 4 /* activation scales, or the 256-byte rows of the staging tile */;
+constexpr int GEMM_FP8_BLOCK_SCALE_SEG = 28; // most blocks of K whose scales are brought to shared memory at a time, twice: one in use, one on its way
+constexpr uint32_t GEMM_FP8_BLOCK_SCALES_BYTES = GEMM_BM * (GEMM_FP8_BLOCK_SCALE_SEG + 1) * 4;
+constexpr uint32_t GEMM_FP8_BLOCK_STAGE_C_BYTES = 8 * 32 * 128;      // eight promoter warps, 32 rows of 128 bytes each
+constexpr size_t GEMM_FP8_BLOCK_SMEM_BYTES = 1024 /* alignment slack */ + GEMM_FP8_BLOCK_STAGES * GEMM_PAIR_STAGE_BYTES + 1024 /* barriers, weight scales */ +
+                                             2 * GEMM_FP8_BLOCK_SCALES_BYTES + GEMM_FP8_BLOCK_STAGE_C_BYTES;
 
 struct GemmBlockArgs {
     CUtensorMap tmapA;        // A [M, K] 8-bit, box 128 rows x 128 bytes

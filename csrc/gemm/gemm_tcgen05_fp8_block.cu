@@ -66,8 +66,7 @@ constexpr uint32_t FB_TMEM_COLS = 512;
 constexpr int FB_SCRATCH = 2;               // scratch accumulators of 256 columns: two blocks of K in flight
 constexpr uint32_t FB_PEER_BIT_MASK = 0xFEFFFFFFu;
 constexpr int FB_HALF_N = GEMM_BN / 2;       // columns of one promoter group = one 128-wide block of the weight's scales
-constexpr int FB_MAX_KB = 256;               // blocks of K whose weight scales fit the shared-memory copy (K up to 32768)
-constexpr int FB_SEG = GEMM_FP8_BLOCK_SCALE_SEG;          // blocks of K whose activation scales are in shared memory at a time
+constexpr int FB_SEG = GEMM_FP8_BLOCK_SCALE_SEG;
 constexpr int FB_SEG_PITCH = FB_SEG + 1;                  // floats per row: an odd number keeps the rows on different banks
 constexpr int FB_FLAG_PLANE_A = TILEXR_FLAG_DATA_BASE;    // all-gather: piece (source rank, 128-row block) has landed
 constexpr int FB_FLAG_PLANE_B = TILEXR_FLAG_ACK_BASE;     // reduce-scatter: partial tile (source rank, tile) has landed
@@ -108,8 +107,11 @@ struct BlockState {
     uint64_t scratchEmpty[FB_SCRATCH];     // leader: the sixteen promoter warps of the pair have read scratch s
     uint32_t tmemBase;
     volatile int abortFlag;
+    volatile int leave[2];                 // promoters: the abort flag as they all see it at the start of a segment of scales
     uint32_t epoch;                        // fused modes: the epoch of this launch (kept here, not in every thread's registers)
+    float scaleB[2][2][FB_SEG];            // weight scales of the two column halves, segment by segment like the activations'
 };
+static_assert(sizeof(BlockState) <= 1024, "barriers and weight scales share a KB");
 
 __device__ __forceinline__ uint32_t FbCtaRank()
 {
@@ -279,6 +281,20 @@ __device__ __forceinline__ uint32_t FbPackPair(float lo, float hi, bool bf16)
     return *reinterpret_cast<const uint32_t *>(&v);
 }
 
+// Two fp32 values as the operand of a packed instruction, and two multiply-adds, each rounded like fmaf.
+__device__ __forceinline__ uint64_t FbPair(uint32_t lo, uint32_t hi)
+{
+    uint64_t v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(lo), "r"(hi));
+    return v;
+}
+__device__ __forceinline__ uint64_t FbFma2(uint64_t x, uint64_t y, uint64_t z)
+{
+    uint64_t v;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(x), "l"(y), "l"(z));
+    return v;
+}
+
 // The grouped tile walk of the bf16 CTA-pair kernel: 256-row blocks advance fastest inside a group.
 __device__ __forceinline__ void FbTileAt(int t, int mTiles, int nBlocks, int GROUP, int *mTile, int *nBlock)
 {
@@ -341,7 +357,8 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~static_cast<uintptr_t>(1023));
     uint8_t *stageBase = smem;
     BlockState *st = reinterpret_cast<BlockState *>(smem + GEMM_FP8_BLOCK_STAGES * GEMM_PAIR_STAGE_BYTES);
-    uint8_t *stageC = smem + GEMM_FP8_BLOCK_STAGES * GEMM_PAIR_STAGE_BYTES + 1024;      // 128 rows x 256 bytes
+    uint8_t *scales = smem + GEMM_FP8_BLOCK_STAGES * GEMM_PAIR_STAGE_BYTES + 1024;      // two buffers of 128 rows' scales
+    uint8_t *stageC = scales + 2 * GEMM_FP8_BLOCK_SCALES_BYTES;                         // the promoter warps' staging tiles
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -555,85 +572,103 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
         const int h = (warp - 4) >> 2;
         const int myRow = quad * 32 + lane;                       // row of this CTA's 128-row sub-tile
         const int pt = static_cast<int>(threadIdx.x) - 128;       // 0..255 among the promoter threads
-        __shared__ int sExit;
-        __shared__ float sScaleB[2 * FB_MAX_KB];
-        float *sScaleA = reinterpret_cast<float *>(stageC);      // the reduce-scatter's staging tile is used when no scale is
+        uint8_t *myStage = stageC + (warp - 4) * (32 * 128);
         uint32_t kbAll = 0;                        // as the issuer counts it: scratch kbAll & 1, its (kbAll >> 1)-th use
         const int KB = a.kBlocks;
+        const int segments = (KB + FB_SEG - 1) / FB_SEG;
+        const int segBlocks = (KB + segments - 1) / segments;
         const bool gathered = MODE == GEMM_ALL_GATHER;
         const uint64_t budgetNs = fused ? a.comm->waitTimeoutNs : 4000000000ull;
-        // Brings the scales of 128 rows from `tileRow` on, blocks kb0 .. kb0 + FB_SEG - 1 of K, to shared memory; a warp takes a row
-        // at a time.  Scales that a peer writes during this launch are read through L2, never through the read-only path.
-        auto loadScaleA = [&](int64_t tileRow, bool fromPeer, int kb0) {
+        auto ofPeer = [&](int mTile) {
+            const int64_t row = static_cast<int64_t>(mTile) * 2 * GEMM_BM + static_cast<int64_t>(ctaRank) * GEMM_BM;
+            return gathered && row / a.shardRows != a.comm->rank;
+        };
+        // Brings the scales of an item, blocks kb0 .. kb0 + segBlocks - 1 of K, to buffer `buf`: of this CTA's 128 rows, a warp takes a row
+        // at a time, and of the two column halves.  Scales that a peer writes during this launch are read through L2, never through the
+        // read-only path.
+        auto loadScales = [&](const FbItem &it, bool fromPeer, int kb0, uint32_t buf) {
+            const int64_t tileRow = static_cast<int64_t>(it.mTile) * 2 * GEMM_BM + static_cast<int64_t>(ctaRank) * GEMM_BM;
             const float *sa = a.scaleA + tileRow * KB;
             if (gathered && !fromPeer) sa = a.scaleALocal + (tileRow - static_cast<int64_t>(a.comm->rank) * a.shardRows) * KB;
             const int rows = static_cast<int>(min(static_cast<int64_t>(GEMM_BM), a.M - tileRow));
-            const int n = min(FB_SEG, KB - kb0);
+            const int n = min(segBlocks, KB - kb0);
+            float *to = reinterpret_cast<float *>(scales + buf * GEMM_FP8_BLOCK_SCALES_BYTES);
+            if (lane < n) {
 #pragma unroll 4
-            for (int r = pt >> 5; r < rows; r += 8) {
-                for (int c = lane; c < n; c += 32) {
-                    const float *src = sa + static_cast<int64_t>(r) * KB + kb0 + c;
-                    float *dst = sScaleA + r * FB_SEG_PITCH + c;
+                for (int r = pt >> 5; r < rows; r += 8) {
+                    const float *src = sa + static_cast<int64_t>(r) * KB + kb0 + lane;
+                    float *dst = to + r * FB_SEG_PITCH + lane;
                     if (fromPeer) *dst = __ldcg(src);
                     else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(SmemAddr(dst)), "l"(src) : "memory");
                 }
+                if (pt < 64) {
+                    const int block = min((it.col0 + (pt >> 5) * (it.width / 2)) / FB_HALF_N, a.scaleBRows - 1);
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(SmemAddr(&st->scaleB[buf][pt >> 5][lane])),
+                                 "l"(a.scaleB + static_cast<int64_t>(block) * KB + kb0 + lane) : "memory");
+                }
             }
         };
-        auto ofPeer = [&](int64_t tileRow) { return gathered && tileRow / a.shardRows != a.comm->rank; };
-        bool ahead = false;                        // the item's first segment of scales is already on its way
-        // One item, of which this thread folds COLS columns of its row.  False: a wait has given up, nobody goes on.
-        auto foldItem = [&](auto tag, const FbItem &it, int t) -> bool {
-            constexpr int COLS = decltype(tag)::value;
-            const int64_t row0 = static_cast<int64_t>(it.mTile) * 2 * GEMM_BM + static_cast<int64_t>(ctaRank) * GEMM_BM;
-            const int64_t gRow = row0 + myRow;
-            const bool rowValid = gRow < a.M;
-            const int myCol = it.col0 + h * COLS;
-            // scale blocks of B for the two column halves
-            const float *sb0 = a.scaleB + static_cast<int64_t>(min(it.col0 / 128, a.scaleBRows - 1)) * KB;
-            const float *sb1 = a.scaleB + static_cast<int64_t>(min((it.col0 + COLS) / 128, a.scaleBRows - 1)) * KB;
-            float acc[COLS];
-#pragma unroll
-            for (int j = 0; j < COLS; ++j) acc[j] = 0.f;
-            // The scales go to shared memory, the weight's two rows of the table once per tile and the activations' 128 rows
-            // FB_SEG blocks of K at a time: a lane reading its own row's scale from memory for every block touches 32 lines
-            // per warp and block.
-            asm volatile("bar.sync 1, 256;" ::: "memory");          // the previous tile's readers are done with both
-            for (int i = pt; i < 2 * KB && i < 2 * FB_MAX_KB; i += 256) {
-                sScaleB[i] = __ldg((i < KB ? sb0 + i : sb1 + (i - KB)));
+        uint32_t seg = 0;                          // segments so far: the scales' buffers alternate with it
+        bool ahead = false;                        // the segment's scales are already on their way
+        FbItem nextItem;
+        int nextT = pair;
+        auto findItem = [&] {                      // the next item that exists
+            for (; nextT < items; nextT += nPairs) {
+                nextItem = FbItemOf<MODE>(a, nextT, mTiles, fused ? a.comm->rank : 0);
+                if (nextItem.col0 < a.N) return;
             }
-            const bool fromPeer = ofPeer(row0);
+        };
+        // One item, of which this thread folds COLS columns of its row.  False: a wait has given up, nobody goes on.
+        auto foldItem = [&](auto tag, const FbItem &it) -> bool {
+            constexpr int COLS = decltype(tag)::value;
+            const bool fromPeer = ofPeer(it.mTile);
             if (fromPeer) {
                 // the scales of these 128 rows were written by their owner during this launch: acquire the rows' flag first
                 if (lane == 0) {
-                    const int block = static_cast<int>(row0 / GEMM_BM);
+                    const int block = it.mTile * 2 + static_cast<int>(ctaRank);
                     const int shard = block / a.blocksPerShard;
                     const int64_t slot = FB_FLAG_PLANE_A + static_cast<int64_t>(shard) * a.flagStride + (block - shard * a.blocksPerShard);
                     FbAcquireFlag(FlagSlot(a.comm, a.comm->rank, slot), MakeFlag(st->epoch, 1), st, budgetNs);
                 }
                 __syncwarp();
             }
-            const bool bInSmem = KB <= FB_MAX_KB;
-            const float *sbHalf = h == 0 ? sb0 : sb1;
-            const float *sbShared = sScaleB + h * KB;
-            const float *saShared = sScaleA + myRow * FB_SEG_PITCH;
-            for (int kb0 = 0; kb0 < KB; kb0 += FB_SEG) {
-                if (kb0 != 0) asm volatile("bar.sync 1, 256;" ::: "memory");      // everybody has read the segment before
-                if (kb0 != 0 || !ahead) loadScaleA(row0, fromPeer, kb0);
+            uint64_t acc[COLS / 2];                // pairs of columns
+#pragma unroll
+            for (int j = 0; j < COLS / 2; ++j) acc[j] = 0;
+            for (int kb0 = 0; kb0 < KB; kb0 += segBlocks, ++seg) {
+                // The scales go through shared memory: a lane reading its own row's scale from memory for every block touches 32 lines per warp
+                // and block.  Those of the next segment, of this item or the next one, come while this one is folded: fetched between
+                // two items they, and the stores of a row per lane, took 7.8 us of every tile (2.4 now).
+                const uint32_t buf = seg & 1u;
+                if (!ahead) loadScales(it, fromPeer, kb0, buf);
                 asm volatile("cp.async.wait_all;" ::: "memory");
-                asm volatile("bar.sync 1, 256;" ::: "memory");
-                const int n = min(FB_SEG, KB - kb0);
+                if (pt == 0) st->leave[buf] = st->abortFlag;
+                asm volatile("bar.sync 1, 256;" ::: "memory");      // this segment's scales are there, the one before has been read
+                if (st->leave[buf] != 0) return false;              // all eight warps together: none may miss a barrier
+                if (kb0 + segBlocks < KB) {
+                    ahead = !fromPeer;
+                    if (ahead) loadScales(it, false, kb0 + segBlocks, buf ^ 1u);
+                } else {
+                    nextT += nPairs;
+                    findItem();
+                    ahead = nextT < items && !ofPeer(nextItem.mTile);
+                    if (ahead) loadScales(nextItem, false, 0, buf ^ 1u);
+                }
+                const float *sa = reinterpret_cast<const float *>(scales + buf * GEMM_FP8_BLOCK_SCALES_BYTES) + myRow * FB_SEG_PITCH;
+                const float *sb = st->scaleB[buf][h];
+                const int n = min(segBlocks, KB - kb0);
                 // One way in and one way out: with an exit for a wait that gave up, the 128 accumulators were moved to other
                 // registers and back in every block.  Such a wait has raised the abort flag of both CTAs; what either folds after
                 // it is never stored (a test of the verdict in front of the release cost 2 %).
                 for (int kb = 0; kb < n; ++kb) {
-                    const float f = saShared[kb] * (bInSmem ? sbShared[kb0 + kb] : __ldg(sbHalf + kb0 + kb));
+                    const float f = sa[kb] * sb[kb];
+                    const uint64_t ff = FbPair(__float_as_uint(f), __float_as_uint(f));
                     const uint32_t p = kbAll & 1u;
                     FbWaitBarWarp(&st->scratchFull[p], (kbAll >> 1) & 1u, st, peerAbortAddr, budgetNs);
                     ++kbAll;
                     FbFenceAfter();
                     const uint32_t taddr = tmemBase + (static_cast<uint32_t>(quad * 32) << 16) + p * GEMM_BN + static_cast<uint32_t>(h * COLS);
-                    // Sixteen columns at a time, the next ones on their way while these are folded (8192^3: 8 columns 538 us,
-                    // 16 columns 523 us, 32 columns 565 us, before the modes had kernels of their own).
+                    // Sixteen columns at a time, the next ones on their way while these are folded, two columns per multiply-add.
                     uint32_t r[2][16];
                     FbTmemLoad16(taddr, r[0]);
 #pragma unroll
@@ -648,93 +683,79 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
                             if (lane == 0) FbArriveCluster(SmemAddr(&st->scratchEmpty[p]) & FB_PEER_BIT_MASK);
                         }
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) acc[cc * 16 + j] = fmaf(__uint_as_float(r[cc & 1][j]), f, acc[cc * 16 + j]);
-                    }
-                }
-            }
-            // All eight promoter warps of the CTA arrive here whether or not their waits succeeded, and leave the tile
-            // loop together: the store below uses block-wide barriers, which a lone warp must never reach.
-            asm volatile("bar.sync 1, 256;" ::: "memory");
-            if (pt == 0) sExit = (st->abortFlag != 0) ? 1 : 0;
-            asm volatile("bar.sync 1, 256;" ::: "memory");
-            if (sExit != 0) return false;
-            ahead = false;
-            if (MODE != GEMM_REDUCE_SCATTER) {
-                // the next item's scales come while this one is stored (everybody has left the loop that reads them)
-                if (t + nPairs < items) {
-                    const FbItem next = FbItemOf<MODE>(a, t + nPairs, mTiles, fused ? a.comm->rank : 0);
-                    const int64_t rowNext = static_cast<int64_t>(next.mTile) * 2 * GEMM_BM + static_cast<int64_t>(ctaRank) * GEMM_BM;
-                    ahead = next.col0 < a.N && !ofPeer(rowNext);
-                    if (ahead) loadScaleA(rowNext, false, 0);
-                }
-                // Local memory: every thread stores its piece of a row straight from registers, without the two trips
-                // of the tile through shared memory and their barriers (the issuer has only two blocks of K of work ahead).
-                if (rowValid) {
-                    uint8_t *rowPtr = a.c + (static_cast<uint64_t>(gRow) * a.N + myCol) * 2;
-#pragma unroll
-                    for (int v = 0; v < COLS / 8; ++v) {
-                        if (myCol + v * 8 < a.N) {
-                            st_vec16(rowPtr + v * 16, Vec16{FbPackPair(acc[8 * v], acc[8 * v + 1], bf16), FbPackPair(acc[8 * v + 2], acc[8 * v + 3], bf16),
-                                                            FbPackPair(acc[8 * v + 4], acc[8 * v + 5], bf16), FbPackPair(acc[8 * v + 6], acc[8 * v + 7], bf16)});
+                        for (int j = 0; j < 8; ++j) {
+                            acc[cc * 8 + j] = FbFma2(FbPair(r[cc & 1][2 * j], r[cc & 1][2 * j + 1]), ff, acc[cc * 8 + j]);
                         }
                     }
                 }
-                return true;
             }
-            if constexpr (COLS == FB_HALF_N) {
-            const int nBlock = it.nBlock;
-            const int col0 = it.col0;
-            // ---- the partial tile goes into the row owner's staging slot for this rank, behind NVLink: through a swizzled
-            // staging tile, so that every warp store covers whole row pieces; the two groups take turns with it ----------
-            const int block = static_cast<int>(row0 / GEMM_BM);
-            const int owner = block / a.blocksPerShard;
-            const int localBlock = block - owner * a.blocksPerShard;
-            const int tileLocal = localBlock * a.nBlocks + nBlock;
-            uint8_t *rowBase = a.comm->registryPtr->regions[a.outHandle].peerBase[owner] + a.outOffset +
-                               (static_cast<uint64_t>(a.comm->rank) * a.shardRows + static_cast<uint64_t>(localBlock) * GEMM_BM) * a.N * 2;
-#pragma unroll 1
-            for (int pass = 0; pass < 2; ++pass) {
-                if (h == pass) {
+            // What a wait that gave up has spoilt is not stored: its warp raised the flag before it released the scratch, so every warp that
+            // folded what came after sees it here.
+            const bool whole = __all_sync(0xffffffffu, st->abortFlag == 0) != 0;
+            const int64_t row0 = static_cast<int64_t>(it.mTile) * 2 * GEMM_BM + static_cast<int64_t>(ctaRank) * GEMM_BM;
+            uint8_t *base;                         // row `row0` of C, or of its owner's staging slot for this rank
+            int rows = GEMM_BM;
+            int owner = 0, tileLocal = 0;
+            if (MODE == GEMM_REDUCE_SCATTER) {
+                const int block = static_cast<int>(row0 / GEMM_BM);
+                owner = block / a.blocksPerShard;
+                const int localBlock = block - owner * a.blocksPerShard;
+                tileLocal = localBlock * a.nBlocks + it.nBlock;
+                base = a.comm->registryPtr->regions[a.outHandle].peerBase[owner] + a.outOffset +
+                       (static_cast<uint64_t>(a.comm->rank) * a.shardRows + static_cast<uint64_t>(localBlock) * GEMM_BM) * a.N * 2;
+            } else {
+                base = a.c + static_cast<uint64_t>(row0) * a.N * 2;
+                rows = static_cast<int>(min(static_cast<int64_t>(GEMM_BM), a.M - row0));
+            }
+            // Through a staging tile of the warp's own, 32 rows by 64 columns, so that a warp stores whole lines: a row per lane is 32 lines per
+            // instruction.
+            if (whole) {
+                constexpr int CHUNKS = (COLS < 64 ? COLS : 64) / 8;      // 16-byte chunks of a row per round
 #pragma unroll
-                    for (int v = 0; v < 16; ++v) {
-                        const int chunk = v ^ (myRow & 15);           // 16-byte chunks of a 256-byte row, XOR-swizzled
-                        *reinterpret_cast<uint4 *>(stageC + myRow * 256 + chunk * 16) =
-                            make_uint4(FbPackPair(acc[8 * v], acc[8 * v + 1], bf16), FbPackPair(acc[8 * v + 2], acc[8 * v + 3], bf16),
-                                       FbPackPair(acc[8 * v + 4], acc[8 * v + 5], bf16), FbPackPair(acc[8 * v + 6], acc[8 * v + 7], bf16));
+                for (int round = 0; round < COLS / (CHUNKS * 8); ++round) {
+                    __syncwarp();
+#pragma unroll
+                    for (int v = 0; v < CHUNKS; ++v) {
+                        uint32_t w[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const uint64_t two = acc[(round * CHUNKS + v) * 4 + j];
+                            w[j] = FbPackPair(__uint_as_float(static_cast<uint32_t>(two)), __uint_as_float(static_cast<uint32_t>(two >> 32)), bf16);
+                        }
+                        *reinterpret_cast<uint4 *>(myStage + lane * 128 + ((v ^ (lane & 7)) * 16)) = make_uint4(w[0], w[1], w[2], w[3]);
+                    }
+                    __syncwarp();
+                    const int colRound = it.col0 + h * COLS + round * CHUNKS * 8;
+#pragma unroll
+                    for (int k = 0; k < CHUNKS; ++k) {
+                        const int idx = k * 32 + lane;
+                        const int rr = idx / CHUNKS, ch = idx % CHUNKS;
+                        const int col = colRound + ch * 8;
+                        if (quad * 32 + rr < rows && col < a.N) {
+                            const uint4 v = *reinterpret_cast<const uint4 *>(myStage + rr * 128 + ((ch ^ (rr & 7)) * 16));
+                            st_vec16(base + static_cast<uint64_t>(quad * 32 + rr) * a.N * 2 + static_cast<uint64_t>(col) * 2, Vec16{v.x, v.y, v.z, v.w});
+                        }
                     }
                 }
+            }
+            if (MODE == GEMM_REDUCE_SCATTER) {
                 asm volatile("bar.sync 1, 256;" ::: "memory");
-#pragma unroll 2
-                for (int k = 0; k < 8; ++k) {
-                    const int idx = pt + k * 256;
-                    const int rr = idx >> 4;
-                    const int ch = idx & 15;
-                    const int col = col0 + pass * FB_HALF_N + ch * 8;
-                    if (col < a.N) {
-                        const uint4 v = *reinterpret_cast<const uint4 *>(stageC + rr * 256 + ((ch ^ (rr & 15)) * 16));
-                        st_vec16(rowBase + static_cast<uint64_t>(rr) * a.N * 2 + static_cast<uint64_t>(col) * 2, Vec16{v.x, v.y, v.z, v.w});
-                    }
+                if (pt == 0 && st->abortFlag == 0) {
+                    // all 256 promoter threads have stored (the barrier above): order their stores, then tell the owner
+                    fence_acq_rel_sys();
+                    st_relaxed_sys_u64(FlagSlot(a.comm, owner, FB_FLAG_PLANE_B + static_cast<int64_t>(a.comm->rank) * a.flagStride + tileLocal),
+                                       MakeFlag(st->epoch, 1));
                 }
-                asm volatile("bar.sync 1, 256;" ::: "memory");
-            }
-            if (pt == 0) {
-                // all 256 promoter threads have stored (the barrier above): order their stores, then tell the owner
-                fence_acq_rel_sys();
-                st_relaxed_sys_u64(FlagSlot(a.comm, owner, FB_FLAG_PLANE_B + static_cast<int64_t>(a.comm->rank) * a.flagStride + tileLocal),
-                                   MakeFlag(st->epoch, 1));
-            }
             }
             return true;
         };
-        for (int t = pair; t < items; t += nPairs) {
-            const FbItem it = FbItemOf<MODE>(a, t, mTiles, fused ? a.comm->rank : 0);
-            if (it.col0 >= a.N) continue;
-            bool go = true;
-            if (MODE == GEMM_REDUCE_SCATTER || it.width == GEMM_BN) go = foldItem(FbCols<FB_HALF_N>{}, it, t);
-            else if (it.width == 128) go = foldItem(FbCols<64>{}, it, t);
-            else if (it.width == 64) go = foldItem(FbCols<32>{}, it, t);
-            else go = foldItem(FbCols<16>{}, it, t);
-            if (!go) break;
+        findItem();
+        for (bool go = true; go && nextT < items;) {
+            const FbItem it = nextItem;
+            if (MODE == GEMM_REDUCE_SCATTER || it.width == GEMM_BN) go = foldItem(FbCols<FB_HALF_N>{}, it);
+            else if (it.width == 128) go = foldItem(FbCols<64>{}, it);
+            else if (it.width == 64) go = foldItem(FbCols<32>{}, it);
+            else go = foldItem(FbCols<16>{}, it);
         }
         // ---- reduce-scatter: add the partial tiles of the output tiles this CTA owns, in rank order ---------------------
         if (MODE == GEMM_REDUCE_SCATTER) {
@@ -744,10 +765,10 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
             const uint8_t *stage = a.comm->registryPtr->regions[a.outHandle].peerBase[rank] + a.outOffset;
             const uint64_t rowBytes = static_cast<uint64_t>(a.N) * 2;
             for (int tl = static_cast<int>(blockIdx.x); tl < owned; tl += static_cast<int>(gridDim.x)) {
-                asm volatile("bar.sync 1, 256;" ::: "memory");          // sExit of the previous round has been read
-                if (pt == 0) sExit = (st->abortFlag != 0) ? 1 : 0;
+                asm volatile("bar.sync 1, 256;" ::: "memory");          // the word of the previous round has been read
+                if (pt == 0) st->leave[0] = st->abortFlag;
                 asm volatile("bar.sync 1, 256;" ::: "memory");
-                if (sExit != 0) break;
+                if (st->leave[0] != 0) break;
                 if (pt < ranks) {
                     const int64_t slot = FB_FLAG_PLANE_B + static_cast<int64_t>(pt) * a.flagStride + tl;
                     FbAcquireFlag(FlagSlot(a.comm, rank, slot), MakeFlag(epoch, 1), st, budgetNs);
