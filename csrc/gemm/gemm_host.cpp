@@ -776,6 +776,12 @@ int TileXRMatmulReduceScatterFp8Block(const void *a, const float *scaleA, const 
         TILEXR_LOG(ERROR) << "block-scaled matmul reduce-scatter: the staging buffer must be registered on every rank (TileXRSymmAlloc)";
         return TILEXR_ERROR_PARA_CHECK_FAIL;
     }
+    if (R == 1 && (hostArgs->extraFlag & TILEXR_FLAG_EMULATED) == 0) {
+        // The sum over one rank is its own partial product: no staging, no flags, no second pass over it.  A wait that gives up is told
+        // where the fused kernel tells it.
+        int32_t *failed = reinterpret_cast<int32_t *>(devArgs + offsetof(TileXRCommArgs, dfx) + TILEXR_DFX_FAIL_CODE * sizeof(int64_t));
+        return TileXRMatmulFp8BlockScaled(a, scaleA, b, scaleB, out, m, n, k, inDtype, outDtype, failed, stream);
+    }
     ret = MakeMap8(&g.tmapA, a, m, k, GEMM_BM);
     if (ret != TILEXR_SUCCESS) return ret;
     g.scaleA = scaleA;
