@@ -1,5 +1,6 @@
 #include "tilexr_launch.h"
 
+#include <algorithm>
 #include <atomic>
 #include <cstring>
 #include <functional>
@@ -59,23 +60,28 @@ int IssueWorldLaunch(EmulatedWorld *world, std::vector<PendingLaunch *> &perRank
     }
     if (cudaSetDevice(world->device) != cudaSuccess) return TILEXR_ERROR_RUNTIME;
     const size_t argBytes = first.kernel->argBytes;
-    std::vector<uint8_t> packed(argBytes * ranks);
-    for (int r = 0; r < ranks; ++r) std::memcpy(packed.data() + r * argBytes, perRank[r]->args.data(), argBytes);
+    const int inlineRanks = first.kernel->inlineRanks;
+    // EmulatedArgs<ARGS>: a pointer in a header, then `inlineRanks` argument structs; without room for any, the pointer alone
+    std::vector<uint8_t> packed(EMULATED_HEADER_BYTES + argBytes * std::max(ranks, inlineRanks));
+    for (int r = 0; r < ranks; ++r) std::memcpy(packed.data() + EMULATED_HEADER_BYTES + r * argBytes, perRank[r]->args.data(), argBytes);
     void *devArgs = nullptr;
-    // stream-ordered scratch: freed after the kernel on the same stream
-    if (cudaMallocAsync(&devArgs, packed.size(), first.stream) != cudaSuccess) return TILEXR_ERROR_RUNTIME;
-    if (cudaMemcpyAsync(devArgs, packed.data(), packed.size(), cudaMemcpyHostToDevice, first.stream) != cudaSuccess) {
-        return TILEXR_ERROR_RUNTIME;
+    if (ranks > inlineRanks) {
+        // stream-ordered scratch: freed after the kernel on the same stream
+        if (cudaMallocAsync(&devArgs, argBytes * ranks, first.stream) != cudaSuccess) return TILEXR_ERROR_RUNTIME;
+        if (cudaMemcpyAsync(devArgs, packed.data() + EMULATED_HEADER_BYTES, argBytes * ranks, cudaMemcpyHostToDevice, first.stream) != cudaSuccess) {
+            return TILEXR_ERROR_RUNTIME;
+        }
+        // pageable source: the copy is staged before the call returns, `packed` may go away
     }
-    // pageable source: the copy is staged before the call returns, `packed` may go away
+    std::memcpy(packed.data(), &devArgs, sizeof(devArgs));
     int ret = SetSmemLimit(first.kernel->emulated, first.cfg.smemBytes);
     if (ret != TILEXR_SUCCESS) return ret;
-    void *params[] = {&devArgs};
+    void *params[] = {packed.data()};
     const dim3 grid(first.cfg.grid, ranks, 1);
     const dim3 block(first.cfg.block, 1, 1);
     cudaError_t e = cudaLaunchCooperativeKernel(first.kernel->emulated, grid, block, params, first.cfg.smemBytes,
                                                 first.stream);
-    cudaFreeAsync(devArgs, first.stream);
+    if (devArgs != nullptr) cudaFreeAsync(devArgs, first.stream);
     if (e != cudaSuccess) {
         TILEXR_LOG(ERROR) << "cooperative launch of " << first.kernel->name << " for " << ranks << " emulated ranks x "
                           << first.cfg.grid << " blocks failed: " << cudaGetErrorString(e);

@@ -22,11 +22,17 @@
 
 namespace TileXR {
 
+constexpr int EMULATED_INLINE_RANKS = 8;
+constexpr size_t EMULATED_HEADER_BYTES = 16;
+
 struct KernelEntry {
     const void *single;
     const void *emulated;
     size_t argBytes;
     const char *name;
+    // How `emulated` takes its argument structs: up to this many ranks inside the launch's parameters (EmulatedArgs), zero: always a
+    // device array, which every launch allocates, uploads and frees.
+    int inlineRanks = 0;
 };
 
 struct LaunchConfig {
@@ -58,20 +64,35 @@ int MaxCooperativeGrid(TileXRCommPtr comm, const KernelEntry &kernel, unsigned b
 } // namespace TileXR
 
 #if defined(__CUDACC__)
+namespace TileXR {
+// The parameter of an emulated kernel.  The argument structs of up to EMULATED_INLINE_RANKS ranks travel with the launch: an
+// allocation, a copy and a release per launch cost 15 us of host time, and where the stream-ordered pool had returned its memory
+// to the driver, several hundred.  More ranks than that come as a device array.
+template <typename ARGS> struct EmulatedArgs {
+    static_assert(alignof(ARGS) <= EMULATED_HEADER_BYTES, "the structs start behind the header");
+    union {
+        const ARGS *array;            // null: `rank` holds them
+        char header[EMULATED_HEADER_BYTES];
+    };
+    ARGS rank[EMULATED_INLINE_RANKS];
+};
+} // namespace TileXR
+
 // Defines NAME_single / NAME_emulated around a device body `BODY(const ARGS &)` and a
 // KernelEntry named NAME##Entry.
 #define TILEXR_DEFINE_KERNEL(NAME, ARGS, BODY, MAX_THREADS) TILEXR_DEFINE_KERNEL_OCC(NAME, ARGS, BODY, MAX_THREADS, 1)
 // Same, asking the compiler to keep MIN_BLOCKS blocks of MAX_THREADS threads resident per SM.
 #define TILEXR_DEFINE_KERNEL_OCC(NAME, ARGS, BODY, MAX_THREADS, MIN_BLOCKS)                            \
     __global__ void __launch_bounds__(MAX_THREADS, MIN_BLOCKS) NAME##_single(const ARGS a) { BODY(a); } \
-    __global__ void __launch_bounds__(MAX_THREADS, MIN_BLOCKS) NAME##_emulated(const ARGS *perRank)    \
+    __global__ void __launch_bounds__(MAX_THREADS, MIN_BLOCKS)                                         \
+    NAME##_emulated(const __grid_constant__ TileXR::EmulatedArgs<ARGS> perRank)                        \
     {                                                                                                  \
-        const ARGS a = perRank[blockIdx.y];                                                            \
+        const ARGS a = perRank.array != nullptr ? perRank.array[blockIdx.y] : perRank.rank[blockIdx.y]; \
         BODY(a);                                                                                       \
     }                                                                                                  \
     static const TileXR::KernelEntry NAME##Entry = {reinterpret_cast<const void *>(&NAME##_single),    \
                                                     reinterpret_cast<const void *>(&NAME##_emulated),  \
-                                                    sizeof(ARGS), #NAME};
+                                                    sizeof(ARGS), #NAME, TileXR::EMULATED_INLINE_RANKS};
 #endif
 
 #endif // TILEXR_LAUNCH_H

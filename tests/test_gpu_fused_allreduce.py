@@ -80,3 +80,27 @@ def test_choice_by_size(txr):
 ])
 def test_all_reduce_rmsnorm_groups_of_rows(txr, ranks, rows, h, algo, with_res, symmetric):
     test_all_reduce_rmsnorm(txr, ranks, rows, h, algo, with_res, symmetric)
+
+
+def test_emulated_world_of_more_ranks_than_travel_with_a_launch():
+    """Argument blocks of more ranks than fit the launch's parameters come as a device array."""
+    require_cuda()
+    import tilexr_b200 as txr
+    from tilexr_b200.ops import collectives
+
+    ranks, rows, h = 9, 5, 64
+    world = txr.init_emulated_world(ranks, device=0, buffer_mb=16)
+    try:
+        g = torch.Generator().manual_seed(3)
+        xs = [torch.randn(rows, h, generator=g).to(torch.bfloat16).cuda() for _ in range(ranks)]
+        gamma = torch.ones(h, dtype=torch.bfloat16, device="cuda")
+        for _ in range(3):
+            ys = world.run(lambda c, r: collectives.all_reduce_rmsnorm(c, xs[r], gamma))
+            world.check()
+        total = sum(x.float() for x in xs).to(torch.bfloat16).float()
+        want = total * torch.rsqrt(total.square().mean(dim=1, keepdim=True) + 1e-6)
+        for y in ys:
+            # one rounding to bf16 of an fp32 product whose reciprocal root is a few ulp of fp32 off
+            assert torch.allclose(y.float(), want, rtol=2 ** -7, atol=2 ** -7) and torch.equal(y, ys[0])
+    finally:
+        world.destroy()
