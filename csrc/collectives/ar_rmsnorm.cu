@@ -143,7 +143,7 @@ __device__ __forceinline__ void ReduceNormRow(const ArNormArgs &a, SrcFn srcOf, 
 }
 
 // Rows a block copies, or reduces, before it raises their flags, or waits for them: one thread per flag behind one block barrier.
-// A system-wide release takes about 5 us while every SM stores; one per row and phase made up most of the launch
+// A system-wide release takes about 5 us while every SM stores (one among the threads of a GPU less, SetFlagScoped); one per row and phase made up most of the launch
 // (256 x 7168 on four emulated ranks, device time from cold caches: 74 us with one row at a time, 48 us so; 1024 x 4096: 173 and 81).
 constexpr int ARN_GROUP = 8;
 constexpr int ARN_OWN_GROUP = 4;
@@ -182,6 +182,7 @@ __device__ void ArNormBody(const ArNormArgs &a)
 
     const int vecs = static_cast<int>(rb / 16);
     const int step = static_cast<int>(gridDim.x);
+    const bool oneGpu = OneGpu(comm);
 
     if (ok && !a.twoShot) {
         // push every row of mine to every peer, then reduce every row
@@ -199,7 +200,7 @@ __device__ void ArNormBody(const ArNormArgs &a)
                 }
             }
             __syncthreads();
-            if (tid < R && tid != rank) SetFlag(FlagA(a, tid, rank, row), epoch, 1);
+            if (tid < R && tid != rank) SetFlagScoped(FlagA(a, tid, rank, row), epoch, 1, oneGpu);
         }
         for (int row = blockIdx.x; row < a.rows && ok; row += step) {
             bool got = true;
@@ -230,7 +231,7 @@ __device__ void ArNormBody(const ArNormArgs &a)
             __syncthreads();
             if (tid < n) {
                 const int row = foreignRow(it0 + tid * step);
-                SetFlag(FlagA(a, row / per, rank, row % per), epoch, 1);
+                SetFlagScoped(FlagA(a, row / per, rank, row % per), epoch, 1, oneGpu);
             }
         }
         // 2. my rows: reduce, normalise, fan out
@@ -261,7 +262,7 @@ __device__ void ArNormBody(const ArNormArgs &a)
             if (!ok) break;
             __syncthreads();
             for (int f = tid; f < n * R; f += static_cast<int>(ARN_THREADS)) {
-                if (f % R != rank) SetFlag(FlagB(a, f % R, rank, local0 + f / R * step), epoch, 1);
+                if (f % R != rank) SetFlagScoped(FlagB(a, f % R, rank, local0 + f / R * step), epoch, 1, oneGpu);
             }
         }
         // 3. rows of other owners come back normalised

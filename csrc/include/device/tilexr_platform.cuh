@@ -73,6 +73,16 @@ TXR_D void st_relaxed_sys_u64(uint64_t *p, uint64_t v)
 #endif
 }
 
+TXR_D void st_release_gpu_u64(uint64_t *p, uint64_t v)
+{
+#if TXR_ON_DEVICE
+    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+#else
+    if (HostTraceHooks *h = HostTraceSlot()) h->onFlagStore(h->ctx, p, v);
+    __atomic_store_n(p, v, __ATOMIC_RELEASE);
+#endif
+}
+
 TXR_D uint64_t ld_acquire_sys_u64(const uint64_t *p)
 {
 #if TXR_ON_DEVICE

@@ -162,6 +162,17 @@ TXR_D void SetFlag(uint64_t *flag, uint32_t epoch, uint32_t value)
     st_release_sys_u64(flag, MakeFlag(epoch, value));
 }
 
+// Whether every reader of this rank's flags is on this rank's own GPU: alone, or in an emulated world.  The order among the GPU's own
+// threads is then all there is to keep, and a release of that scope is much the cheaper one while every SM stores (the two-shot
+// all-reduce + norm of 256 x 7168 on four emulated ranks: 40 us with system-wide releases, 33 so).
+TXR_D bool OneGpu(const CommArgs *a) { return a->rankSize == 1 || (a->extraFlag & TileXR::TILEXR_FLAG_EMULATED) != 0; }
+
+TXR_D void SetFlagScoped(uint64_t *flag, uint32_t epoch, uint32_t value, bool oneGpu)
+{
+    if (oneGpu) st_release_gpu_u64(flag, MakeFlag(epoch, value));
+    else st_release_sys_u64(flag, MakeFlag(epoch, value));
+}
+
 // Non-blocking probe (reference: CheckRankInnerFlag).
 TXR_D bool CheckFlagGE(const uint64_t *flag, uint32_t epoch, uint32_t value)
 {
@@ -242,7 +253,7 @@ TXR_D void PublishDone(const Waiter &w)
     CommArgs *a = w.args;
     // One fence orders everything this rank did before all of the stores below; a release store per peer would
     // wait for the previous peer's store to be acknowledged over NVLink, rankSize - 1 round trips in a row.
-    fence_acq_rel_sys();
+    if (!OneGpu(a)) fence_acq_rel_sys();      // else the exit counter has ordered it
     for (int i = 0; i < a->rankSize; ++i) {
         const int r = (a->rank + i) % a->rankSize;
         st_relaxed_sys_u64(CtrlWord(a, r, TILEXR_CTRL_DONE_WORD + a->rank), MakeFlag(w.epoch, 0));
@@ -286,11 +297,11 @@ __device__ __forceinline__ void KernelEpilogue(Waiter &w, bool ok, int scratchWo
     __shared__ int sLastToLeave;
     __syncthreads();
     CommArgs *a = w.args;
-    // Without peers the order among the rank's own blocks is all there is to keep (the counter's acquire and release, and
-    // the end of the launch): the system-wide fence of every block cost about 3 us in a launch of 32 small blocks.
-    const bool alone = a->rankSize == 1;
+    // Without a reader on another GPU the counter's acquire and release order all there is to keep: the system-wide fence of every
+    // block cost about 3 us in a launch of 32 small blocks.
+    const bool oneGpu = OneGpu(a);
     if (threadIdx.x == 0) {
-        if (!alone) fence_acq_rel_sys();
+        if (!oneGpu) fence_acq_rel_sys();
         uint32_t *exitCounter =
             reinterpret_cast<uint32_t *>(CtrlWord(a, a->rank, TILEXR_CTRL_GRIDBAR_WORD + TILEXR_CTRL_GRIDBAR_COUNT));
         sLastToLeave = atom_add_acq_rel_gpu_u32(exitCounter, 1) == gridDim.x - 1 ? 1 : 0;
@@ -308,8 +319,7 @@ __device__ __forceinline__ void KernelEpilogue(Waiter &w, bool ok, int scratchWo
             uint32_t *exitCounter =
                 reinterpret_cast<uint32_t *>(CtrlWord(a, a->rank, TILEXR_CTRL_GRIDBAR_WORD + TILEXR_CTRL_GRIDBAR_COUNT));
             st_release_gpu_u32(exitCounter, 0);
-            if (alone) st_relaxed_sys_u64(CtrlWord(a, a->rank, TILEXR_CTRL_DONE_WORD + a->rank), MakeFlag(w.epoch, 0));
-            else PublishDone(w);
+            PublishDone(w);
             *CtrlWord(a, a->rank, TILEXR_CTRL_EPOCH_WORD) = w.epoch;
             if (a->dfx[TileXR::TILEXR_DFX_FAIL_CODE] == 0 && ok) {
                 a->dfx[TileXR::TILEXR_DFX_RUN_STATUS] = TILEXR_RUN_FINISHED;
