@@ -1,0 +1,235 @@
+// Device code that the expert-parallel kernels share: routing of a token, block quantisation.
+#ifndef TILEXR_EP_DEVICE_CUH
+#define TILEXR_EP_DEVICE_CUH
+
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+#include <cuda_fp8.h>
+
+#include "device/tilexr_convert.cuh"
+#include "device/tilexr_rma.cuh"
+#include "device/tilexr_sync.cuh"
+#include "ep_kernels.cuh"
+#include "tilexr_ep.h"
+
+namespace TileXR {
+
+using namespace tilexr;
+
+namespace {
+
+// One kernel per kind of transport: with all of them in one the registers of a 512-thread block (64, two blocks per SM) ran
+// out (628 bytes of spill loads against 340; 4096 x 7168 fp8 96 -> 92 us).
+enum EpTransport : int { EP_PLAIN = 0, EP_FP8 = 1, EP_MXFP8 = 2, EP_INT8 = 3 };
+
+constexpr float FP8_E4M3_MAX = 448.0f;
+constexpr float FP8_AMAX_FLOOR = 1e-4f;
+
+__device__ __forceinline__ float WarpMax(float v)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+__device__ __forceinline__ float WarpSum(float v)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+__device__ __forceinline__ uint32_t Fp8x4(float a, float b, float c, float d)
+{
+    const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(a, b), __NV_SATFINITE, __NV_E4M3);
+    const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(c, d), __NV_SATFINITE, __NV_E4M3);
+    return lo | (hi << 16);
+}
+
+__device__ __forceinline__ uint32_t Fp8x4E5m2(float a, float b, float c, float d)
+{
+    const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(a, b), __NV_SATFINITE, __NV_E5M2);
+    const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(c, d), __NV_SATFINITE, __NV_E5M2);
+    return lo | (hi << 16);
+}
+
+// ---- routing: one warp scores one token and picks its top-k -------------------------------------------
+// Lane l owns experts l, l+32, ...  Selection is by score (+ optional bias), ties go to the
+// lower expert id; the gate weight is the unbiased score, optionally renormalised over the
+// selected experts and multiplied by `routedScale`.
+template <int PER_LANE>
+__device__ __forceinline__ int RouteTokenN(const float *logits, const float *bias, int numExperts, int topK, int scoreFunc,
+                                            int renormalize, float routedScale, int lane, int32_t *idsOut, float *weightsOut, float *picked)
+{
+    float score[PER_LANE];
+    float sel[PER_LANE];
+    float mx = -INFINITY;
+#pragma unroll
+    for (int j = 0; j < PER_LANE; ++j) {
+        const int e = j * 32 + lane;
+        score[j] = e < numExperts ? logits[e] : -INFINITY;
+        mx = fmaxf(mx, score[j]);
+    }
+    if (scoreFunc == TileXREp::TILEXR_EP_SCORE_SOFTMAX) {
+        mx = WarpMax(mx);
+        float sum = 0.f;
+#pragma unroll
+        for (int j = 0; j < PER_LANE; ++j) {
+            const int e = j * 32 + lane;
+            score[j] = e < numExperts ? expf(score[j] - mx) : 0.f;
+            sum += score[j];
+        }
+        sum = WarpSum(sum);
+        const float inv = 1.0f / sum;
+#pragma unroll
+        for (int j = 0; j < PER_LANE; ++j) score[j] *= inv;
+    } else {
+#pragma unroll
+        for (int j = 0; j < PER_LANE; ++j) {
+            const int e = j * 32 + lane;
+            score[j] = e < numExperts ? 1.0f / (1.0f + expf(-score[j])) : 0.f;
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < PER_LANE; ++j) {
+        const int e = j * 32 + lane;
+        sel[j] = e < numExperts ? score[j] + (bias != nullptr ? bias[e] : 0.f) : -INFINITY;
+    }
+    float myWeight = 0.f;   // lane k keeps the k-th pick
+    int myId = -1;
+    float total = 0.f;
+    for (int k = 0; k < topK; ++k) {
+        float best = -INFINITY;
+        int bestE = 0x7fffffff;
+        float bestScore = 0.f;
+#pragma unroll
+        for (int j = 0; j < PER_LANE; ++j) {
+            const int e = j * 32 + lane;
+            if (sel[j] > best) {   // ascending e within a lane: first maximum wins the tie
+                best = sel[j];
+                bestE = e;
+                bestScore = score[j];
+            }
+        }
+        // The lanes' maxima are compared as integers of the same order (a zero of either sign is one value; a lane without
+        // a candidate, whose scores are NaN, minus infinity or used up, has the smallest key): two warp reductions and a
+        // shuffle per pick instead of fifteen shuffles.
+        const uint32_t bits = __float_as_uint(best + 0.f);
+        const uint32_t key = bestE == 0x7fffffff ? 0u : (bits & 0x80000000u) != 0 ? ~bits : bits | 0x80000000u;
+        const uint32_t top = __reduce_max_sync(0xffffffffu, key);
+        bestE = static_cast<int>(__reduce_min_sync(0xffffffffu, key == top ? static_cast<uint32_t>(bestE) : 0x7fffffffu));
+        bestScore = __shfl_sync(0xffffffffu, bestScore, bestE & 31);
+        if (top == 0u) bestScore = 0.f;
+        if ((bestE & 31) == lane) {
+#pragma unroll
+            for (int j = 0; j < PER_LANE; ++j) {
+                if (j == (bestE >> 5)) sel[j] = -INFINITY;
+            }
+        }
+        if (lane == k) {
+            myWeight = bestScore;
+            myId = bestE;
+        }
+        total += bestScore;
+    }
+    if (lane < topK) {
+        float w = myWeight;
+        if (renormalize) w = w / total;
+        w *= routedScale;
+        idsOut[lane] = myId;
+        weightsOut[lane] = w;
+        *picked = w;
+    }
+    return myId;
+}
+
+// The per-lane score table is sized for the expert count, so that 256 experts keep 8 scores per lane in
+// registers instead of the 32 that the largest supported count needs.  Returns the expert that lane k picked k-th, and its gate
+// weight in *picked.
+__device__ __forceinline__ int RouteToken(const float *logits, const float *bias, int numExperts, int topK, int scoreFunc,
+                                           int renormalize, float routedScale, int lane, int32_t *idsOut, float *weightsOut, float *picked)
+{
+    if (numExperts <= 256) {
+        return RouteTokenN<8>(logits, bias, numExperts, topK, scoreFunc, renormalize, routedScale, lane, idsOut, weightsOut, picked);
+    }
+    if (numExperts <= 512) {
+        return RouteTokenN<16>(logits, bias, numExperts, topK, scoreFunc, renormalize, routedScale, lane, idsOut, weightsOut, picked);
+    }
+    return RouteTokenN<EP_MAX_EXPERTS / 32>(logits, bias, numExperts, topK, scoreFunc, renormalize, routedScale, lane, idsOut, weightsOut, picked);
+}
+
+// The end of a launch whose blocks read neither the epoch nor the counters of the control block: what KernelEpilogue keeps, by one thread.
+__device__ __forceinline__ void EndLocalLaunch(CommArgs *c, const Waiter &w)
+{
+    c->dfx[TILEXR_DFX_LAUNCHES] += 1;
+    if (c->dfx[TILEXR_DFX_FAIL_CODE] == 0) c->dfx[TILEXR_DFX_RUN_STATUS] = TILEXR_RUN_FINISHED;
+    st_relaxed_sys_u64(CtrlWord(c, c->rank, TILEXR_CTRL_DONE_WORD + c->rank), MakeFlag(w.epoch, 0));
+    *CtrlWord(c, c->rank, TILEXR_CTRL_EPOCH_WORD) = w.epoch;
+}
+
+// Sixteen elements per lane, eight neighbouring lanes share a block of 128: e4m3 values, and in *scales the four fp32 scales of the
+// warp's 512 elements (16 bytes of the row's scales), the same in all lanes.  Called by a whole warp.
+__device__ __forceinline__ Vec16 QuantFp8Block16(const float *f, Vec16 *scales)
+{
+    float amax = 0.f;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) amax = fmaxf(amax, fabsf(f[j]));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
+    amax = fmaxf(amax, FP8_AMAX_FLOOR);
+    const float inv = FP8_E4M3_MAX / amax;
+    const float scale = amax / FP8_E4M3_MAX;
+    scales->x = __float_as_uint(__shfl_sync(0xffffffffu, scale, 0));
+    scales->y = __float_as_uint(__shfl_sync(0xffffffffu, scale, 8));
+    scales->z = __float_as_uint(__shfl_sync(0xffffffffu, scale, 16));
+    scales->w = __float_as_uint(__shfl_sync(0xffffffffu, scale, 24));
+    Vec16 q;
+    q.x = Fp8x4(f[0] * inv, f[1] * inv, f[2] * inv, f[3] * inv);
+    q.y = Fp8x4(f[4] * inv, f[5] * inv, f[6] * inv, f[7] * inv);
+    q.z = Fp8x4(f[8] * inv, f[9] * inv, f[10] * inv, f[11] * inv);
+    q.w = Fp8x4(f[12] * inv, f[13] * inv, f[14] * inv, f[15] * inv);
+    return q;
+}
+
+// MXFP8: 32 elements = 2 lanes share the exponent 2^(floor(log2 amax) - emax); *scales are the warp's 16 exponent bytes.
+__device__ __forceinline__ Vec16 QuantMx16(const float *f, bool e5m2, int lane, Vec16 *scales)
+{
+    float amax = 0.f;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) amax = fmaxf(amax, fabsf(f[j]));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+    const int emax = e5m2 ? 15 : 8;
+    int ex = -127;
+    if (amax > 0.f) {
+        const uint32_t biased = (__float_as_uint(amax) >> 23) & 0xffu;
+        ex = (biased == 0 ? -126 : static_cast<int>(biased) - 127) - emax;
+    }
+    ex = max(-127, min(127, ex));
+    const float inv = exp2f(static_cast<float>(-ex));
+    uint32_t word = (lane & 1) == 0 ? static_cast<uint32_t>(ex + 127) << (8 * ((lane >> 1) & 3)) : 0u;
+    word |= __shfl_xor_sync(0xffffffffu, word, 2);
+    word |= __shfl_xor_sync(0xffffffffu, word, 4);
+    scales->x = __shfl_sync(0xffffffffu, word, 0);
+    scales->y = __shfl_sync(0xffffffffu, word, 8);
+    scales->z = __shfl_sync(0xffffffffu, word, 16);
+    scales->w = __shfl_sync(0xffffffffu, word, 24);
+    Vec16 q;
+    if (e5m2) {
+        q.x = Fp8x4E5m2(f[0] * inv, f[1] * inv, f[2] * inv, f[3] * inv);
+        q.y = Fp8x4E5m2(f[4] * inv, f[5] * inv, f[6] * inv, f[7] * inv);
+        q.z = Fp8x4E5m2(f[8] * inv, f[9] * inv, f[10] * inv, f[11] * inv);
+        q.w = Fp8x4E5m2(f[12] * inv, f[13] * inv, f[14] * inv, f[15] * inv);
+    } else {
+        q.x = Fp8x4(f[0] * inv, f[1] * inv, f[2] * inv, f[3] * inv);
+        q.y = Fp8x4(f[4] * inv, f[5] * inv, f[6] * inv, f[7] * inv);
+        q.z = Fp8x4(f[8] * inv, f[9] * inv, f[10] * inv, f[11] * inv);
+        q.w = Fp8x4(f[12] * inv, f[13] * inv, f[14] * inv, f[15] * inv);
+    }
+    return q;
+}
+
+} // namespace
+
+} // namespace TileXR
+
+#endif

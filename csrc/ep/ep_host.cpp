@@ -360,6 +360,9 @@ int TileXR::EpDispatch(const TileXREpDispatchParams *p, int32_t *laneCountOut, T
     // 148 SMs, and 4096 tokens left 40 of the 296 places empty.  With peers sixteen: every block raises a flag on every rank and every
     // block polls them all, and ranks whose batches differ a little launch grids of one size, as an emulated world requires.
     // Every block also takes a row of counts in the window: sixteen where the window is too small for the counts of more blocks.
+    const bool aligned = (reinterpret_cast<uintptr_t>(p->expandXOut) & 15u) == 0;
+    const bool local = c.rankSize == 1 && aligned;       // no peers: a kernel of its own
+    const KernelEntry &kernel = local ? EpDispatchLocalKernelEntry(p->quantMode) : EpDispatchKernelEntry(p->quantMode);
     for (int64_t perBlock = c.rankSize == 1 ? 4 : 16;; perBlock = 16) {
         grid = static_cast<unsigned>(std::max<int64_t>(minBlocks, std::min<int64_t>((p->bs + perBlock - 1) / perBlock, capBlocks)));
         unsigned gridCap = 0;
@@ -370,9 +373,10 @@ int TileXR::EpDispatch(const TileXREpDispatchParams *p, int32_t *laneCountOut, T
                                   << "raise TILEXR_EP_BLOCKS";
                 return TILEXR_ERROR_NOT_SUPPORT;
             }
-            smem = EpDispatchSmemBytes(static_cast<int>(smemCols), static_cast<int>(tokensPerBlock * routesPerToken));
+            smem = local ? EpDispatchLocalSmemBytes(static_cast<int>(numCols), static_cast<int>(tokensPerBlock * routesPerToken))
+                         : EpDispatchSmemBytes(static_cast<int>(smemCols), static_cast<int>(tokensPerBlock * routesPerToken));
             unsigned maxGrid = 0;
-            ret = MaxCooperativeGrid(comm, EpDispatchKernelEntry(p->quantMode), EP_BLOCK_THREADS, smem, ranksPerDevice, &maxGrid);
+            ret = MaxCooperativeGrid(comm, kernel, EP_BLOCK_THREADS, smem, ranksPerDevice, &maxGrid);
             if (ret != TILEXR_SUCCESS) return ret;
             if (maxGrid == 0) return TILEXR_ERROR_NOT_SUPPORT;
             gridCap = maxGrid;
@@ -380,7 +384,8 @@ int TileXR::EpDispatch(const TileXREpDispatchParams *p, int32_t *laneCountOut, T
             grid = maxGrid;
         }
         grid = static_cast<unsigned>(std::max<int64_t>((p->bs + tokensPerBlock - 1) / tokensPerBlock, std::min<int64_t>(minBlocks, gridCap)));
-        if (!DispatchLayout(p->h, numCols, c.rankSize, p->maxRecvRows, p->quantMode, elemSize, grid, zeroCopy, &a.win)) {
+        // (the table of the local kernel, one or two bytes per block in rows of 16 bytes, fits that of eight blocks' 32-bit counts)
+        if (!DispatchLayout(p->h, numCols, c.rankSize, p->maxRecvRows, p->quantMode, elemSize, local ? std::max<int64_t>(grid, 8) : grid, zeroCopy, &a.win)) {
             return TILEXR_ERROR_PARA_CHECK_FAIL;
         }
         if (a.win.totalBytes <= c.hostArgs->dataHalfBytes) break;
@@ -422,7 +427,7 @@ int TileXR::EpDispatch(const TileXREpDispatchParams *p, int32_t *laneCountOut, T
     a.elemSize = static_cast<uint32_t>(elemSize);
     a.isBf16 = p->dtype == TILEXR_DATA_TYPE_BFP16 ? 1u : 0u;
     a.zeroCopy = zeroCopy ? 1u : 0u;
-    a.directOwn = (reinterpret_cast<uintptr_t>(p->expandXOut) & 15u) == 0 ? 1u : 0u;
+    a.directOwn = aligned ? 1u : 0u;
     a.outHandle = handle;
     a.outOffset = regionOffset;
     a.routeRowsOut = p->routeRowsOut;
@@ -443,7 +448,7 @@ int TileXR::EpDispatch(const TileXREpDispatchParams *p, int32_t *laneCountOut, T
         a.perfTrace = PerfTracePrepareLaunch(info, stream);
     }
     LaunchConfig cfg{grid, EP_BLOCK_THREADS, smem, true};
-    return LaunchKernel(comm, EpDispatchKernelEntry(p->quantMode), &a, cfg, stream);
+    return LaunchKernel(comm, kernel, &a, cfg, stream);
 }
 
 extern "C" {

@@ -37,6 +37,7 @@
 #include "device/tilexr_rma.cuh"
 #include "device/tilexr_sync.cuh"
 #include "device/tilexr_convert.cuh"
+#include "ep_device.cuh"
 #include "ep_kernels.cuh"
 #include "tilexr_ep.h"
 
@@ -46,147 +47,15 @@ using namespace tilexr;
 
 namespace {
 
-constexpr float FP8_E4M3_MAX = 448.0f;
-constexpr float FP8_AMAX_FLOOR = 1e-4f;
-
-__device__ __forceinline__ float WarpMax(float v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-__device__ __forceinline__ float WarpSum(float v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
-__device__ __forceinline__ uint32_t Fp8x4(float a, float b, float c, float d)
-{
-    const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(a, b), __NV_SATFINITE, __NV_E4M3);
-    const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(c, d), __NV_SATFINITE, __NV_E4M3);
-    return lo | (hi << 16);
-}
-
-__device__ __forceinline__ uint32_t Fp8x4E5m2(float a, float b, float c, float d)
-{
-    const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(a, b), __NV_SATFINITE, __NV_E5M2);
-    const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(c, d), __NV_SATFINITE, __NV_E5M2);
-    return lo | (hi << 16);
-}
-
-// ---- routing: one warp scores one token and picks its top-k -------------------------------------------
-// Lane l owns experts l, l+32, ...  Selection is by score (+ optional bias), ties go to the
-// lower expert id; the gate weight is the unbiased score, optionally renormalised over the
-// selected experts and multiplied by `routedScale`.
-template <int PER_LANE>
-__device__ __forceinline__ int RouteTokenN(const float *logits, const float *bias, int numExperts, int topK, int scoreFunc,
-                                            int renormalize, float routedScale, int lane, int32_t *idsOut, float *weightsOut)
-{
-    float score[PER_LANE];
-    float sel[PER_LANE];
-    float mx = -INFINITY;
-#pragma unroll
-    for (int j = 0; j < PER_LANE; ++j) {
-        const int e = j * 32 + lane;
-        score[j] = e < numExperts ? logits[e] : -INFINITY;
-        mx = fmaxf(mx, score[j]);
-    }
-    if (scoreFunc == TileXREp::TILEXR_EP_SCORE_SOFTMAX) {
-        mx = WarpMax(mx);
-        float sum = 0.f;
-#pragma unroll
-        for (int j = 0; j < PER_LANE; ++j) {
-            const int e = j * 32 + lane;
-            score[j] = e < numExperts ? expf(score[j] - mx) : 0.f;
-            sum += score[j];
-        }
-        sum = WarpSum(sum);
-        const float inv = 1.0f / sum;
-#pragma unroll
-        for (int j = 0; j < PER_LANE; ++j) score[j] *= inv;
-    } else {
-#pragma unroll
-        for (int j = 0; j < PER_LANE; ++j) {
-            const int e = j * 32 + lane;
-            score[j] = e < numExperts ? 1.0f / (1.0f + expf(-score[j])) : 0.f;
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < PER_LANE; ++j) {
-        const int e = j * 32 + lane;
-        sel[j] = e < numExperts ? score[j] + (bias != nullptr ? bias[e] : 0.f) : -INFINITY;
-    }
-    float myWeight = 0.f;   // lane k keeps the k-th pick
-    int myId = -1;
-    float total = 0.f;
-    for (int k = 0; k < topK; ++k) {
-        float best = -INFINITY;
-        int bestE = 0x7fffffff;
-        float bestScore = 0.f;
-#pragma unroll
-        for (int j = 0; j < PER_LANE; ++j) {
-            const int e = j * 32 + lane;
-            if (sel[j] > best) {   // ascending e within a lane: first maximum wins the tie
-                best = sel[j];
-                bestE = e;
-                bestScore = score[j];
-            }
-        }
-        // The lanes' maxima are compared as integers of the same order (a zero of either sign is one value; a lane without
-        // a candidate, whose scores are NaN, minus infinity or used up, has the smallest key): two warp reductions and a
-        // shuffle per pick instead of fifteen shuffles.
-        const uint32_t bits = __float_as_uint(best + 0.f);
-        const uint32_t key = bestE == 0x7fffffff ? 0u : (bits & 0x80000000u) != 0 ? ~bits : bits | 0x80000000u;
-        const uint32_t top = __reduce_max_sync(0xffffffffu, key);
-        bestE = static_cast<int>(__reduce_min_sync(0xffffffffu, key == top ? static_cast<uint32_t>(bestE) : 0x7fffffffu));
-        bestScore = __shfl_sync(0xffffffffu, bestScore, bestE & 31);
-        if (top == 0u) bestScore = 0.f;
-        if ((bestE & 31) == lane) {
-#pragma unroll
-            for (int j = 0; j < PER_LANE; ++j) {
-                if (j == (bestE >> 5)) sel[j] = -INFINITY;
-            }
-        }
-        if (lane == k) {
-            myWeight = bestScore;
-            myId = bestE;
-        }
-        total += bestScore;
-    }
-    if (lane < topK) {
-        float w = myWeight;
-        if (renormalize) w = w / total;
-        w *= routedScale;
-        idsOut[lane] = myId;
-        weightsOut[lane] = w;
-    }
-    return myId;
-}
-
-// The per-lane score table is sized for the expert count, so that 256 experts keep 8 scores per lane in
-// registers instead of the 32 that the largest supported count needs.  Returns the expert that lane k picked k-th.
-__device__ __forceinline__ int RouteToken(const float *logits, const float *bias, int numExperts, int topK, int scoreFunc,
-                                           int renormalize, float routedScale, int lane, int32_t *idsOut, float *weightsOut)
-{
-    if (numExperts <= 256) {
-        return RouteTokenN<8>(logits, bias, numExperts, topK, scoreFunc, renormalize, routedScale, lane, idsOut, weightsOut);
-    }
-    if (numExperts <= 512) {
-        return RouteTokenN<16>(logits, bias, numExperts, topK, scoreFunc, renormalize, routedScale, lane, idsOut, weightsOut);
-    }
-    return RouteTokenN<EP_MAX_EXPERTS / 32>(logits, bias, numExperts, topK, scoreFunc, renormalize, routedScale, lane, idsOut, weightsOut);
-}
-
 __global__ void __launch_bounds__(256) RoutingTopKKernel(const RoutingArgs a)
 {
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) / 32;
     const int lane = threadIdx.x & 31;
     if (warp >= a.bs) return;
+    float picked;
     RouteToken(a.gateLogits + static_cast<int64_t>(warp) * a.numExperts, a.selectionBias, a.numExperts, a.topK, a.scoreFunc,
                a.renormalize, a.routedScale, lane, a.topkIdsOut + static_cast<int64_t>(warp) * a.topK,
-               a.topkWeightsOut + static_cast<int64_t>(warp) * a.topK);
+               a.topkWeightsOut + static_cast<int64_t>(warp) * a.topK, &picked);
 }
 
 // ---- dispatch ---------------------------------------------------------------------------------------------
@@ -256,9 +125,6 @@ __device__ void SumBlockCounts(const int32_t *counts, int E, int nb, int32_t *ou
 // nothing (combine); chunk_barrier = wait for the earlier blocks' counts; post_sync = count exchange and row placement;
 // local_input_to_ipc = rows pushed to their destinations; flag_poll_wait = waiting for arrivals;
 // peer_ipc_to_output = window to output (dispatch) or the weighted reduction (combine).
-// One kernel per kind of transport: with all of them in one the registers of a 512-thread block (64, two blocks per SM) ran
-// out (628 bytes of spill loads against 340; 4096 x 7168 fp8 96 -> 92 us).
-enum EpTransport : int { EP_PLAIN = 0, EP_FP8 = 1, EP_MXFP8 = 2, EP_INT8 = 3 };
 
 template <int TRANSPORT>
 __device__ void EpDispatchBody(const EpDispatchArgs &a)
@@ -296,9 +162,6 @@ __device__ void EpDispatchBody(const EpDispatchArgs &a)
     const int units = (C + 1 + 2) / 3;           // 16-byte units of one source's counts: C counts and its block count
     const uint8_t *llMine = LlHalf(comm, rank, epoch);
     __shared__ int sIsLast;
-    // A world of one rank: every row's final place is this rank's own output, so rows, scales and tuples are stored there
-    // at once; nothing passes through the window and nobody has to be waited for.
-    const bool solo = R == 1 && a.directOwn != 0;
     // whatever becomes of the launch, like the caller's other zeros would have been
     if (blockIdx.x == 0 && tid == 0 && a.laneCountOut != nullptr) *a.laneCountOut = 0;
 
@@ -322,9 +185,10 @@ __device__ void EpDispatchBody(const EpDispatchArgs &a)
         const int t = t0 + i;
         int picked = -1;
         if (a.gateLogits != nullptr) {
+            float weight;
             picked = RouteToken(a.gateLogits + static_cast<int64_t>(t) * E, a.selectionBias, E, K, a.scoreFunc, a.renormalize,
                        a.routedScale, lane, a.topkIdsOut + static_cast<int64_t>(t) * K,
-                       a.topkWeightsOut + static_cast<int64_t>(t) * K);
+                       a.topkWeightsOut + static_cast<int64_t>(t) * K, &weight);
         }
         if (lane < K) {
             int e = a.gateLogits != nullptr ? picked : a.expertIds[static_cast<int64_t>(t) * K + lane];
@@ -503,8 +367,7 @@ __device__ void EpDispatchBody(const EpDispatchArgs &a)
         const int parts = nTok > 0 ? max(1, min(min(8, iters), static_cast<int>(EP_WARPS) / nTok)) : 1;
         // where the scales of row `rr` go at the destination whose window half is `half`
         auto scaleRow = [&](unsigned long long half, uint32_t rr) {
-            return (solo ? reinterpret_cast<uint8_t *>(a.dynamicScalesOut) : reinterpret_cast<uint8_t *>(half) + a.win.scalesOff) +
-                   static_cast<uint64_t>(rr) * a.win.scaleRowBytes;
+            return reinterpret_cast<uint8_t *>(half) + a.win.scalesOff + static_cast<uint64_t>(rr) * a.win.scaleRowBytes;
         };
         for (int item = warp; item < nTok * parts; item += EP_WARPS) {
             const int i = item / parts;
@@ -586,8 +449,7 @@ __device__ void EpDispatchBody(const EpDispatchArgs &a)
                         if (amax > 0.f) inv = 127.0f / amax;
                         if (part == 0 && lane == 0) {
                             const float scale = amax > 0.f ? amax / 127.0f : 1.0f;
-                            if (solo) a.dynamicScalesOut[rr] = scale;              // a 16-byte cell in the window, one fp32 in the output
-                            else st_vec16(scaleRow(half, rr), Vec16{__float_as_uint(scale), 0u, 0u, 0u});
+                            st_vec16(scaleRow(half, rr), Vec16{__float_as_uint(scale), 0u, 0u, 0u});     // a 16-byte cell in the window
                         }
                     }
                     for (int it = part; it < iters; it += parts) {
@@ -620,74 +482,10 @@ __device__ void EpDispatchBody(const EpDispatchArgs &a)
 #pragma unroll
                         for (int j = 0; j < 16; ++j) f[j] = 0.f;
                     }
-                    float amax = 0.f;
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) amax = fmaxf(amax, fabsf(f[j]));
-                    if (mx) {
-                        // MXFP8: 32 elements = 2 lanes share the exponent 2^(floor(log2 amax) - emax); this
-                        // iteration's 16 exponent bytes are 16 bytes of the scale row
-                        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-                        const int emax = mxE5m2 ? 15 : 8;
-                        int ex = -127;
-                        if (amax > 0.f) {
-                            const uint32_t biased = (__float_as_uint(amax) >> 23) & 0xffu;
-                            ex = (biased == 0 ? -126 : static_cast<int>(biased) - 127) - emax;
-                        }
-                        ex = max(-127, min(127, ex));
-                        const float inv = exp2f(static_cast<float>(-ex));
-                        uint32_t word = (lane & 1) == 0 ? static_cast<uint32_t>(ex + 127) << (8 * ((lane >> 1) & 3)) : 0u;
-                        word |= __shfl_xor_sync(0xffffffffu, word, 2);
-                        word |= __shfl_xor_sync(0xffffffffu, word, 4);
-                        Vec16 sv;
-                        sv.x = __shfl_sync(0xffffffffu, word, 0);
-                        sv.y = __shfl_sync(0xffffffffu, word, 8);
-                        sv.z = __shfl_sync(0xffffffffu, word, 16);
-                        sv.w = __shfl_sync(0xffffffffu, word, 24);
-                        if ((payloadRoutes >> lane) & 1u) {
-                            st_vec16(scaleRow(myHalf, myRow) + it * 16, sv);
-                        }
-                        Vec16 q;
-                        if (mxE5m2) {
-                            q.x = Fp8x4E5m2(f[0] * inv, f[1] * inv, f[2] * inv, f[3] * inv);
-                            q.y = Fp8x4E5m2(f[4] * inv, f[5] * inv, f[6] * inv, f[7] * inv);
-                            q.z = Fp8x4E5m2(f[8] * inv, f[9] * inv, f[10] * inv, f[11] * inv);
-                            q.w = Fp8x4E5m2(f[12] * inv, f[13] * inv, f[14] * inv, f[15] * inv);
-                        } else {
-                            q.x = Fp8x4(f[0] * inv, f[1] * inv, f[2] * inv, f[3] * inv);
-                            q.y = Fp8x4(f[4] * inv, f[5] * inv, f[6] * inv, f[7] * inv);
-                            q.z = Fp8x4(f[8] * inv, f[9] * inv, f[10] * inv, f[11] * inv);
-                            q.w = Fp8x4(f[12] * inv, f[13] * inv, f[14] * inv, f[15] * inv);
-                        }
-                        uint32_t m = payloadRoutes;
-                        while (m != 0) {
-                            const int k = __ffs(m) - 1;
-                            m &= m - 1;
-                            uint8_t *p = reinterpret_cast<uint8_t *>(__shfl_sync(0xffffffffu, myPayload, k));
-                            if (c < chunks) st_vec16(p + static_cast<int64_t>(c) * 16, q);
-                        }
-                        continue;
-                    }
-                    // 128 elements = 8 consecutive lanes
-                    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-                    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-                    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
-                    amax = fmaxf(amax, FP8_AMAX_FLOOR);
-                    const float inv = FP8_E4M3_MAX / amax;
-                    // the four scales of this iteration are 16 bytes of the scale row: lane k stores them for route k
-                    const float scale = amax / FP8_E4M3_MAX;
+                    // this iteration's 16 bytes of the scale row: lane k stores them for route k
                     Vec16 sv;
-                    sv.x = __float_as_uint(__shfl_sync(0xffffffffu, scale, 0));
-                    sv.y = __float_as_uint(__shfl_sync(0xffffffffu, scale, 8));
-                    sv.z = __float_as_uint(__shfl_sync(0xffffffffu, scale, 16));
-                    sv.w = __float_as_uint(__shfl_sync(0xffffffffu, scale, 24));
-                    if ((payloadRoutes >> lane) & 1u) {
-                        st_vec16(scaleRow(myHalf, myRow) + it * 16, sv);
-                    }
-                    Vec16 q;
-                    q.x = Fp8x4(f[0] * inv, f[1] * inv, f[2] * inv, f[3] * inv);
-                    q.y = Fp8x4(f[4] * inv, f[5] * inv, f[6] * inv, f[7] * inv);
-                    q.z = Fp8x4(f[8] * inv, f[9] * inv, f[10] * inv, f[11] * inv);
-                    q.w = Fp8x4(f[12] * inv, f[13] * inv, f[14] * inv, f[15] * inv);
+                    const Vec16 q = mx ? QuantMx16(f, mxE5m2, lane, &sv) : QuantFp8Block16(f, &sv);
+                    if ((payloadRoutes >> lane) & 1u) st_vec16(scaleRow(myHalf, myRow) + it * 16, sv);
                     uint32_t m = payloadRoutes;
                     while (m != 0) {
                         const int k = __ffs(m) - 1;
@@ -733,29 +531,21 @@ __device__ void EpDispatchBody(const EpDispatchArgs &a)
                 }
             }
             if (myExpert >= 0 && part == 0) {
-                st_vec16((solo ? reinterpret_cast<uint8_t *>(a.assistOut) : reinterpret_cast<uint8_t *>(myHalf) + a.win.assistOff) +
-                             static_cast<uint64_t>(myRow) * 16,
+                st_vec16(reinterpret_cast<uint8_t *>(myHalf) + a.win.assistOff + static_cast<uint64_t>(myRow) * 16,
                          Vec16{static_cast<uint32_t>(rank), static_cast<uint32_t>(t), static_cast<uint32_t>(lane),
                                static_cast<uint32_t>(lane < K ? myExpert - a.topo.sharedRanks : lane - K)});   // routed expert id, or shared expert id
                 const int64_t route = static_cast<int64_t>(t) * K + lane;
                 const float wgt = lane >= K ? 1.0f
                                   : a.gateLogits != nullptr ? a.topkWeightsOut[route]
                                                             : (a.expertScales != nullptr ? a.expertScales[route] : 1.0f);
-                if (solo) {
-                    if (a.assistExtOut != nullptr) {
-                        *reinterpret_cast<uint2 *>(a.assistExtOut + static_cast<int64_t>(myRow) * 2) = make_uint2(myLink, __float_as_uint(wgt));
-                    }
-                    if (a.expandScalesOut != nullptr) a.expandScalesOut[myRow] = wgt;
-                } else {
-                    *reinterpret_cast<uint2 *>(reinterpret_cast<uint8_t *>(myHalf) + a.win.extOff + static_cast<uint64_t>(myRow) * 8) =
-                        make_uint2(myLink, __float_as_uint(wgt));
-                }
+                *reinterpret_cast<uint2 *>(reinterpret_cast<uint8_t *>(myHalf) + a.win.extOff + static_cast<uint64_t>(myRow) * 8) =
+                    make_uint2(myLink, __float_as_uint(wgt));
             }
             __syncwarp();
         }
     }
     __syncthreads();
-    if (ok && !solo && tid < R) {
+    if (ok && tid < R) {
         SetFlag(FlagSlot(comm, tid, TILEXR_FLAG_OP_BASE + static_cast<int64_t>(rank) * TILEXR_FLAGS_PER_PAIR + blockIdx.x), epoch, 1);
     }
     PerfStageEnd(perf, TILEXR_PERF_LOCAL_INPUT_TO_IPC, static_cast<uint64_t>(nRoutes) * a.win.rowBytes);
@@ -765,7 +555,7 @@ __device__ void EpDispatchBody(const EpDispatchArgs &a)
     {
         // every thread polls its share of the (source, block) flags; a source's block count came with its counts
         bool got = true;
-        if (ok && !solo) {
+        if (ok) {
             for (int s = 0; s < R && got; ++s) {
                 const int64_t base = TILEXR_FLAG_OP_BASE + static_cast<int64_t>(s) * TILEXR_FLAGS_PER_PAIR;
                 const int blocksOfS = min(srcBlocks[s], static_cast<int>(EP_COUNT_FLAG_SLOT));
@@ -781,7 +571,7 @@ __device__ void EpDispatchBody(const EpDispatchArgs &a)
     if (ok) {
         const int firstLocal = EpRankFirstCol(a.topo, rank);
         const int localCols = EpRankCols(a.topo, rank);
-        const int64_t rows = solo ? 0 : sm.colPrefix[firstLocal + localCols] - sm.colPrefix[firstLocal];      // rows to take out of the window
+        const int64_t rows = sm.colPrefix[firstLocal + localCols] - sm.colPrefix[firstLocal];
         // Rows are dealt out to blocks in chunks of one row per thread.  Per chunk: (a) a thread per row copies
         // the tuple, link and weight and notes the head rows that have followers; (b) a thread per 16 bytes
         // copies the scales of the rows that arrived with a payload; (c) without zero-copy a warp per row moves
@@ -882,7 +672,7 @@ __device__ void EpDispatchBody(const EpDispatchArgs &a)
             }
             __syncthreads();
         }
-        if (blockIdx.x == (solo ? G - 1 : 0)) {      // alone, the block with the fewest tokens
+        if (blockIdx.x == 0) {
             // cumulative counts in (local expert, source) order: an inclusive scan of E_local * R numbers
             const int n = localCols * R;
             __syncthreads();

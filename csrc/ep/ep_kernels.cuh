@@ -156,6 +156,7 @@ struct RoutingArgs {
 
 const KernelEntry &EpDispatchKernelEntry(int64_t quantMode);      // a kernel per kind of transport
 const KernelEntry &EpCombineKernelEntry();
+const KernelEntry &EpDispatchLocalKernelEntry(int64_t quantMode); // one rank, output on the 16-byte grid (ep_dispatch_local.cu)
 
 // TileXRMoeEpDispatchFused that also sets *laneCountOut (null: nothing) to zero, in the dispatch launch: what the Python results
 // report for a world without tensor-parallel lanes, whose C callers get no such count.
@@ -178,6 +179,7 @@ int LaunchRmsNorm(const void *x, void *residual, const void *gamma, float eps, i
                   void *stream);
 
 size_t EpDispatchSmemBytes(int numExperts, int routesPerBlock);
+size_t EpDispatchLocalSmemBytes(int numExperts, int routesPerBlock);
 
 } // namespace TileXR
 

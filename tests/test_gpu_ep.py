@@ -680,3 +680,33 @@ def test_dispatch_of_tokens_with_few_valid_experts(txr, port):
         assert ((d.route_rows >= 0).sum(dim=1).cpu() == torch.tensor([min(top_k, t % 6) for t in range(tokens)])).all()
     finally:
         comm.destroy()
+
+
+@pytest.mark.parametrize("blocks,tokens,experts,top_k", [(8, 600, 40, 8), (1, 37, 8, 8), (3, 1, 5, 2), (37, 1200, 1024, 8), (296, 4099, 257, 2)])
+def test_dispatch_of_a_single_rank_over_block_counts(txr, monkeypatch, blocks, tokens, experts, top_k):
+    """The counts of a block take one byte, or two where it has more than 255 routes; fewer blocks than a vector of counts, and more."""
+    from conftest import free_port
+
+    ep = txr.ep
+    monkeypatch.setenv("TILEXR_EP_BLOCKS", str(blocks))
+    g = torch.Generator().manual_seed(tokens)
+    x = torch.randn(tokens, 64, generator=g).to(torch.bfloat16).cuda()
+    ids = torch.randint(-1, experts, (tokens, top_k), generator=g).to(torch.int32)
+    ids[: tokens // 3] = 1                                  # one expert with far more routes than the others, several per token
+    weights = torch.rand(tokens, top_k, generator=g)
+    comm = txr.init_process(0, 1, comm_id=f"127.0.0.1:{free_port()}", buffer_mb=64, device=0)
+    try:
+        for _ in range(2):
+            d = ep.dispatch(comm, x, num_experts=experts, top_k=top_k, expert_ids=ids.cuda(), expert_scales=weights.cuda(), max_recv_rows=tokens * top_k)
+        torch.cuda.synchronize()
+        assert comm.device_status() == 0
+        flat = torch.where(ids >= 0, ids, torch.full_like(ids, experts)).reshape(-1).long()
+        order = torch.sort(flat, stable=True).indices[:int((ids >= 0).sum())]
+        n, counts = order.numel(), torch.bincount(flat[order], minlength=experts)
+        assert int(d.recv_total) == n and torch.equal(d.expert_token_nums.cpu(), counts)
+        assert torch.equal(d.send_counts.cpu().long(), counts.cumsum(0))
+        assert torch.equal(d.expand_x[:n], x[(order // top_k).cuda()])
+        assert torch.equal(d.assist[:n, 1:].cpu(), torch.stack((order // top_k, order % top_k, flat[order]), 1).int())
+        assert torch.equal(d.assist_ext[:n, 1].cpu().view(torch.float32), weights.reshape(-1)[order]) and not d.assist_ext[:n, 0].any()
+    finally:
+        comm.destroy()
