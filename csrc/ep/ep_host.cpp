@@ -245,6 +245,31 @@ int CombineWithTp(const TileXREpCombineParams *p, TileXRCommPtr comm, TileXRStre
     return TileXRMoeEpCombineFused(&q, comm, stream);
 }
 
+// Combine without peers (EpCombineLocalBody): (token, column part) items dealt out to the warps beforehand.
+int LaunchCombineLocal(EpCombineArgs *a, const TileXREpCombineParams &p, TileXRCommPtr comm, TileXRStream stream, const Ctx &c)
+{
+    unsigned places = 0;
+    int ret = MaxCooperativeGrid(comm, EpCombineLocalKernelEntry(), EP_LOCAL_THREADS, 0, 1, &places);
+    if (ret != TILEXR_SUCCESS) return ret;
+    if (places == 0) return TILEXR_ERROR_NOT_SUPPORT;
+    // A part is 32 vectors (a column of 16 bytes per lane, one round trip) until every warp has eight of them: then longer parts, for
+    // fewer looks at the routes, and still enough items that the last round of them is short.  (2 to 32 of them, or no longer parts: within
+    // 2 % at 1009 and 4096 tokens.)
+    constexpr int64_t perBlock = EP_LOCAL_THREADS / 32;
+    const int64_t rowChunks = (a->rowBytes / 16 + 31) / 32;
+    const int64_t warps = static_cast<int64_t>(places) * perBlock;
+    const int64_t chunks = std::min<int64_t>(rowChunks, std::max<int64_t>(1, p.bs * rowChunks / (8 * warps)));
+    a->partVecs = static_cast<uint32_t>(32 * chunks);
+    a->parts = static_cast<uint32_t>((rowChunks + chunks - 1) / chunks);
+    const int64_t items = p.bs * a->parts;
+    const unsigned grid = static_cast<unsigned>(std::min<int64_t>(places, (items + perBlock - 1) / perBlock));
+    PerfLaunchInfo info{static_cast<uint32_t>(TILEXR_OP_EP_COMBINE), static_cast<uint32_t>(p.dtype), static_cast<uint32_t>(c.rank),
+                        static_cast<uint32_t>(c.rankSize), grid, static_cast<uint64_t>(p.bs) * a->rowBytes};
+    a->perfTrace = PerfTracePrepareLaunch(info, stream);
+    LaunchConfig cfg{grid, EP_LOCAL_THREADS, 0, false};
+    return LaunchKernel(comm, EpCombineLocalKernelEntry(), a, cfg, stream);
+}
+
 } // namespace
 
 extern "C" {
@@ -510,6 +535,8 @@ int TileXRMoeEpCombineFused(const TileXREpCombineParams *p, TileXRCommPtr comm, 
     ret = TileXRCommNextMagic(comm, &magic);
     if (ret != TILEXR_SUCCESS) return ret;
     a.magic = magic;
+    // one rank that knows the row of each of its own routes: nothing travels, and a kernel of its own does the sum
+    if (c.rankSize == 1 && a.routeRows != nullptr && a.expertIds != nullptr) return LaunchCombineLocal(&a, *p, comm, stream, c);
     const int ranksPerDevice = (c.hostArgs->extraFlag & TILEXR_FLAG_EMULATED) ? c.rankSize : 1;
     unsigned maxGrid = 0;
     ret = MaxCooperativeGrid(comm, EpCombineKernelEntry(), EP_BLOCK_THREADS, 0, ranksPerDevice, &maxGrid);
@@ -531,17 +558,10 @@ int TileXRMoeEpCombineFused(const TileXREpCombineParams *p, TileXRCommPtr comm, 
             for (int64_t k = 0; k < slotsPerToken; ++k) miss *= 1.0 - 1.0 / c.rankSize;
             travel = static_cast<double>(p->bs) * (c.rankSize - 1) * (1.0 - miss);
         }
-        // one rank that knows the row of each of its own routes: nothing travels
-        a.noSend = (c.rankSize == 1 && a.routeRows != nullptr && a.expertIds != nullptr) ? 1u : 0u;
         // Column parts: a warp should get through about eight send items in a row, so that rows leave in the
         // order of the queue (the reducers follow that order) instead of all at once; small batches are cut up
         // so that every warp has something to do.
-        int64_t parts;
-        if (a.noSend != 0) {
-            parts = std::min<int64_t>(8, std::max<int64_t>(1, (4 * warps + routes - 1) / routes));
-        } else {
-            parts = static_cast<int64_t>(std::min(8.0, std::max(1.0, std::ceil(8.0 * warps / std::max(1.0, travel)))));
-        }
+        int64_t parts = static_cast<int64_t>(std::min(8.0, std::max(1.0, std::ceil(8.0 * warps / std::max(1.0, travel)))));
         parts = std::min<int64_t>(parts, std::max<int64_t>(1, rowVecs / 32));
         parts = std::min<int64_t>(parts, std::max<int64_t>(1, TILEXR_FLAG_SLOT_SLOTS / routes));
         const int64_t partVecs = ((rowVecs + parts - 1) / parts + 31) / 32 * 32;

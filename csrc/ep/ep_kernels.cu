@@ -846,7 +846,7 @@ __device__ void EpCombineBody(const EpCombineArgs &a)
         // Rows of this rank's own tokens stay where they are when the reducer knows their row (direct), and the
         // followers of a group are summed into their head's row.
         const bool direct = a.routeRows != nullptr && a.expertIds != nullptr;
-        const bool sender = a.noSend == 0 && blockIdx.x + a.reducerBlocks < gridDim.x;
+        const bool sender = blockIdx.x + a.reducerBlocks < gridDim.x;
         // What a lane learns about row r: does it travel, where to, which bucket of the source's tokens.
         auto classify = [&](int64_t r, int &src, int64_t &slot, uint2 &ext, uint32_t &bucket) -> bool {
             const Vec16 tuple = ld_vec16(a.assist + r * 4);
@@ -955,11 +955,8 @@ __device__ void EpCombineBody(const EpCombineArgs &a)
         // ---- reduce this rank's tokens ------------------------------------------------------------------------
         const uint8_t *half = DataHalf(comm, rank, epoch);
         const uint32_t nReduce = static_cast<uint32_t>(a.bs) * P;
-        // With no row to wait for the items are dealt out beforehand: a step of the cursor is a round trip to memory in front
-        // of every item.
-        const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-        for (uint32_t dealt = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w.ok(); dealt += warps) {
-            const uint32_t it = a.noSend != 0 ? dealt : TakeItem(&cursors[1], lane);
+        while (w.ok()) {
+            const uint32_t it = TakeItem(&cursors[1], lane);
             if (it >= nReduce) break;
             const int64_t t = it / P;
             const uint32_t part = it - static_cast<uint32_t>(t) * P;
@@ -1066,11 +1063,116 @@ __device__ void EpCombineBody(const EpCombineArgs &a)
     KernelEpilogue(w, ok, EP_SCRATCH_TOTALS_WORD);      // the cursors and the bucket counts
 }
 
+// Combine on one rank that knows the row of each of its routes: nothing is sent and nobody is waited for, so no block needs
+// the others and the launch is an ordinary one.  A warp takes (token, column part) items, dealt out beforehand, and keeps the
+// columns of up to eight routes' rows in flight; they are added in k order in fp32 and rounded once, as above.
+// Bound by memory where the batch is large and by four dependent round trips (arguments, routes, rows, store) where it is small.
+// EpCombineBody has its send part in the same registers and fetches two columns of one row at a time, a chain of sixteen round trips per
+// warp for 16 tokens: 16 x 7168, top-8 13.5 us, 5.0 so; 1009 x 4096, top-6 14.7 and 13.2; 4096 x 7168 101 and 95.  Two or four columns
+// of fewer rows at a time, or fewer warps with more, are slower (4096 x 7168 97 to 288 us, 1009 x 4096 15 to 57).
+struct LocalRoute {
+    float weight;
+    int32_t row;       // -1: inactive, -2: active without a row
+};
+
+__device__ __forceinline__ LocalRoute LoadLocalRoute(const EpCombineArgs &a, int64_t t, int64_t rows, int lane)
+{
+    LocalRoute route{0.f, -1};
+    if (lane < a.topK) {
+        const int64_t i = t * a.topK + lane;
+        const int e = a.expertIds[i];
+        const int64_t row = a.routeRows[i];
+        route.weight = a.expertScales != nullptr ? a.expertScales[i] : 1.0f;
+        bool active = e >= 0 && e < a.numExperts;
+        if (a.maskType == TileXREp::TILEXR_EP_ACTIVE_MASK_TOKEN && a.activeMask[t] == 0) active = false;
+        if (a.maskType == TileXREp::TILEXR_EP_ACTIVE_MASK_EXPERT && a.activeMask[i] == 0) active = false;
+        if (active) route.row = row >= 0 && row < rows ? static_cast<int32_t>(row) : -2;
+    }
+    return route;
+}
+
+__device__ void EpCombineLocalBody(const EpCombineArgs &a)
+{
+    constexpr int KU = 8;              // routes whose columns are in flight together
+    const int lane = threadIdx.x & 31;
+    Waiter w = MakeWaiter(a.comm, a.magic, blockIdx.x);
+    PerfScope perf = PerfInit(threadIdx.x == 0 ? a.perfTrace : nullptr, static_cast<uint32_t>(a.comm->rank), blockIdx.x);
+    PerfStageBegin(perf, TILEXR_PERF_KERNEL_TOTAL);
+    PerfStageBegin(perf, TILEXR_PERF_PEER_IPC_TO_OUTPUT);
+    const bool bf16 = a.isBf16 != 0;
+    const int rowVecs = a.rowBytes / 16;
+    const int64_t rows = a.sendCounts[a.sendCountEntries - 1];
+    const int64_t items = static_cast<int64_t>(a.bs) * a.parts;
+    const int64_t warps = static_cast<int64_t>(gridDim.x) * (EP_LOCAL_THREADS / 32);
+    int64_t it = static_cast<int64_t>(blockIdx.x) * (EP_LOCAL_THREADS / 32) + (threadIdx.x >> 5);
+    LocalRoute next = it < items ? LoadLocalRoute(a, it / a.parts, rows, lane) : LocalRoute{0.f, -1};
+    for (; it < items; it += warps) {
+        const LocalRoute route = next;
+        const int64_t t = it / a.parts;
+        const int vBegin = static_cast<int>(it - t * a.parts) * static_cast<int>(a.partVecs);
+        const int vEnd = min(rowVecs, vBegin + static_cast<int>(a.partVecs));
+        const uint32_t active = __ballot_sync(0xffffffffu, route.row >= 0);
+        if (__any_sync(0xffffffffu, route.row == -2)) {
+            // the caller's ids name a route that the dispatch did not place (a world with peers waits for it and gives up)
+            if (route.row == -2) RaiseFailure(w, TILEXR_DEV_WAIT_TIMEOUT, 0, t * a.topK + lane, static_cast<uint64_t>(rows), 0);
+            break;
+        }
+        if (it + warps < items) next = LoadLocalRoute(a, (it + warps) / a.parts, rows, lane);     // on its way beside this item's rows
+        uint8_t *y = a.yOut + t * a.rowBytes;
+        for (int v0 = vBegin; v0 < vEnd; v0 += 32) {
+            const int v = v0 + lane;
+            float acc[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc[j] = 0.f;
+            for (int k0 = 0; k0 < a.topK; k0 += KU) {
+                Vec16 q[KU];
+#pragma unroll
+                for (int u = 0; u < KU; ++u) {
+                    const int32_t row = __shfl_sync(0xffffffffu, route.row, (k0 + u) & 31);
+                    if (((active >> k0) >> u & 1u) != 0) {
+                        const uint8_t *src = a.expertOut + static_cast<int64_t>(row) * a.rowBytes + static_cast<int64_t>(v) * 16;
+                        if (v < vEnd) q[u] = ld_vec16_stream(src);
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < KU; ++u) {
+                    const float wgt = __shfl_sync(0xffffffffu, route.weight, (k0 + u) & 31);
+                    if (((active >> k0) >> u & 1u) != 0) {
+                        float f[8];
+                        Unpack8(q[u], bf16, f);
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) acc[j] = fmaf(wgt, f[j], acc[j]);
+                    }
+                }
+            }
+            if (v >= vEnd) continue;
+            if (a.sharedExpertX != nullptr) {
+                float f[8];
+                Unpack8(ld_vec16(a.sharedExpertX + t * a.rowBytes + static_cast<int64_t>(v) * 16), bf16, f);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) acc[j] += f[j];
+            }
+            st_vec16(y + static_cast<int64_t>(v) * 16, Pack8(acc, bf16));
+        }
+    }
+    PerfStageEnd(perf, TILEXR_PERF_PEER_IPC_TO_OUTPUT);
+    PerfStageEnd(perf, TILEXR_PERF_KERNEL_TOTAL);
+    // The launch counts like the others; no other block of it reads these words, so one thread keeps them without waiting for anybody.
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        CommArgs *c = a.comm;
+        c->dfx[TILEXR_DFX_MAGIC] = w.epoch;
+        c->dfx[TILEXR_DFX_OP] = TILEXR_OP_EP_COMBINE;
+        c->dfx[TILEXR_DFX_COUNT_ARG] = a.bs;
+        EndLocalLaunch(c, w);
+    }
+}
+
 TILEXR_DEFINE_KERNEL_OCC(TileXREpDispatchKernel, EpDispatchArgs, EpDispatchBody<EP_PLAIN>, EP_BLOCK_THREADS, 2)
 TILEXR_DEFINE_KERNEL_OCC(TileXREpDispatchKernelFp8, EpDispatchArgs, EpDispatchBody<EP_FP8>, EP_BLOCK_THREADS, 2)
 TILEXR_DEFINE_KERNEL_OCC(TileXREpDispatchKernelMxfp8, EpDispatchArgs, EpDispatchBody<EP_MXFP8>, EP_BLOCK_THREADS, 2)
 TILEXR_DEFINE_KERNEL_OCC(TileXREpDispatchKernelInt8, EpDispatchArgs, EpDispatchBody<EP_INT8>, EP_BLOCK_THREADS, 2)
 TILEXR_DEFINE_KERNEL_OCC(TileXREpCombineKernel, EpCombineArgs, EpCombineBody, EP_BLOCK_THREADS, 2)
+TILEXR_DEFINE_KERNEL_OCC(TileXREpCombineLocalKernel, EpCombineArgs, EpCombineLocalBody, EP_LOCAL_THREADS, EP_LOCAL_BLOCKS_PER_SM)
 
 // ---- stand-alone quantisation and norm kernels ---------------------------------------------------------------
 
@@ -1409,6 +1511,7 @@ const KernelEntry &EpDispatchKernelEntry(int64_t quantMode)
         default: return TileXREpDispatchKernelEntry;
     }
 }
+const KernelEntry &EpCombineLocalKernelEntry() { return TileXREpCombineLocalKernelEntry; }
 const KernelEntry &EpCombineKernelEntry() { return TileXREpCombineKernelEntry; }
 
 size_t EpDispatchSmemBytes(int numExperts, int routesPerBlock)

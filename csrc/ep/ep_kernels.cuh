@@ -12,6 +12,8 @@ namespace TileXR {
 
 constexpr unsigned EP_BLOCK_THREADS = 512;
 constexpr unsigned EP_WARPS = EP_BLOCK_THREADS / 32;
+constexpr unsigned EP_LOCAL_THREADS = 256;         // combine on one rank
+constexpr unsigned EP_LOCAL_BLOCKS_PER_SM = 4;
 constexpr int EP_MAX_EXPERTS = 1024;
 constexpr int EP_MAX_TOPK = 32;
 constexpr int EP_MAX_ROUTES_PER_BLOCK = 4096;
@@ -135,7 +137,6 @@ struct EpCombineArgs {
     uint32_t buckets;                // ranges of the source token index that the senders walk in order
     uint32_t bucketTokens;           // tokens per bucket
     uint32_t reducerBlocks;          // trailing blocks that only reduce
-    uint32_t noSend;                 // 1: no row leaves this rank, the send items are skipped
     uint64_t listOff;                // bucket lists of travelling rows inside this rank's data half: [buckets][listCap] int32
     uint32_t listCap;                // rows a list can hold; with more rows than that the senders walk the rows unsorted
 };
@@ -156,6 +157,7 @@ struct RoutingArgs {
 
 const KernelEntry &EpDispatchKernelEntry(int64_t quantMode);      // a kernel per kind of transport
 const KernelEntry &EpCombineKernelEntry();
+const KernelEntry &EpCombineLocalKernelEntry();                   // one rank that knows the row of each of its routes
 const KernelEntry &EpDispatchLocalKernelEntry(int64_t quantMode); // one rank, output on the 16-byte grid (ep_dispatch_local.cu)
 
 // TileXRMoeEpDispatchFused that also sets *laneCountOut (null: nothing) to zero, in the dispatch launch: what the Python results

@@ -710,3 +710,62 @@ def test_dispatch_of_a_single_rank_over_block_counts(txr, monkeypatch, blocks, t
         assert torch.equal(d.assist_ext[:n, 1].cpu().view(torch.float32), weights.reshape(-1)[order]) and not d.assist_ext[:n, 0].any()
     finally:
         comm.destroy()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("tokens,hidden,experts,top_k", [(1, 8, 3, 1), (5, 264, 7, 3), (130, 1032, 40, 8), (33, 512, 40, 11), (300, 7168, 64, 17)])
+def test_combine_on_one_rank(txr, tokens, hidden, experts, top_k, dtype):
+    """Inactive routes, masks, shared expert outputs, more than eight routes, rows of any length; against 64 bits."""
+    from conftest import free_port
+
+    ep = txr.ep
+    g = torch.Generator().manual_seed(tokens + hidden)
+    x = torch.randn(tokens, hidden, generator=g).to(dtype).cuda()
+    ids = torch.stack([torch.randperm(experts, generator=g)[:top_k] for _ in range(tokens)]).to(torch.int32)
+    ids[torch.rand(tokens, top_k, generator=g) < 0.1] = -1
+    weights = torch.rand(tokens, top_k, generator=g).cuda()
+    shared = torch.randn(tokens, hidden, generator=g).to(dtype).cuda()
+    mask = (torch.rand(tokens, generator=g) > 0.2).cuda()
+    comm = txr.init_process(0, 1, comm_id=f"127.0.0.1:{free_port()}", buffer_mb=256, device=0)
+    try:
+        d = ep.dispatch(comm, x, num_experts=experts, top_k=top_k, expert_ids=ids.cuda(), max_recv_rows=tokens * top_k)
+        out = torch.randn(d.expand_x.shape, generator=g).to(dtype).cuda()
+        rows = d.route_rows.long()
+        picked = torch.where((rows >= 0)[..., None], out.double()[rows.clamp_min(0)], torch.zeros((), dtype=torch.float64, device="cuda"))
+        for scales, sx, m in ((weights, None, None), (None, shared, None), (weights, shared, mask)):
+            y = ep.combine(comm, out, d, expert_scales=scales, shared_expert_x=sx, active_mask=m)
+            torch.cuda.synchronize()
+            assert comm.device_status() == 0
+            terms = picked * (scales.double()[..., None] if scales is not None else 1.0)
+            if m is not None:
+                terms = terms * m[:, None, None]
+            want = terms.sum(dim=1) + (sx.double() if sx is not None else 0.0)
+            # the fp32 sum of top_k + 1 terms, rounded once to the 16-bit type
+            size = terms.abs().sum(dim=1) + (sx.double().abs() if sx is not None else 0.0)
+            bound = want.abs() * (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11) + size * (top_k + 1) * 2.0 ** -23 + 2.0 ** -24
+            assert ((y.double() - want).abs() <= bound).all()
+    finally:
+        comm.destroy()
+
+
+def test_combine_of_a_route_that_the_dispatch_did_not_place(txr, port):
+    """Ids that name a route without a row: reported, as in a world with peers, and the communicator goes on after a reset."""
+    ep = txr.ep
+    comm = txr.init_process(0, 1, comm_id=f"127.0.0.1:{port}", buffer_mb=16, device=0)
+    try:
+        x = torch.randn(9, 64).to(torch.bfloat16).cuda()
+        ids = torch.arange(9, dtype=torch.int32).view(9, 1).cuda() % 4
+        ids[3] = -1
+        d = ep.dispatch(comm, x, num_experts=4, top_k=1, expert_ids=ids)
+        y = ep.combine(comm, d.expand_x, d)
+        torch.cuda.synchronize()
+        assert comm.device_status() == 0 and torch.equal(y, torch.where((ids >= 0), x, torch.zeros_like(x)))
+        d.topk_ids = ids.clone().fill_(1)
+        ep.combine(comm, d.expand_x, d)
+        torch.cuda.synchronize()
+        assert comm.device_status() != 0
+        comm.reset_status()
+        d.topk_ids = ids
+        assert torch.equal(ep.combine(comm, d.expand_x, d), y) and comm.device_status() == 0
+    finally:
+        comm.destroy()
