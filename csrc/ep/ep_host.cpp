@@ -893,6 +893,22 @@ int TileXRMoeEpCombineBackward(const void *g, const float *weights, const void *
                                  static_cast<int>(wideCols), gradRowsOut, wideOut, stream);
 }
 
+int TileXRMoeEpCombineBackwardLocal(const void *gradY, const float *weights, const void *rows, const int32_t *routeRows, const int32_t *rowCount,
+                                    int64_t bs, int64_t topK, int64_t capacity, int64_t h, TileXRDataType dtype, void *gradRowsOut,
+                                    float *gradWeightsOut, TileXRStream stream)
+{
+    if (gradY == nullptr || weights == nullptr || routeRows == nullptr || rowCount == nullptr || gradRowsOut == nullptr || bs <= 0 || topK <= 0 ||
+        topK > EP_MAX_TOPK || capacity <= 0 || h <= 0 || h % 8 != 0 || h > INT32_MAX || !HalfType(dtype) || (gradWeightsOut != nullptr && rows == nullptr)) {
+        return TILEXR_ERROR_PARA_CHECK_FAIL;
+    }
+    if (((reinterpret_cast<uintptr_t>(gradY) | reinterpret_cast<uintptr_t>(rows) | reinterpret_cast<uintptr_t>(gradRowsOut)) & 15u) != 0) {
+        return TILEXR_ERROR_PARA_CHECK_FAIL;
+    }
+    if (std::max(bs * topK, capacity) > 8ll * INT32_MAX) return TILEXR_ERROR_PARA_CHECK_FAIL;
+    return LaunchCombineBackwardLocal(gradY, weights, rows, routeRows, rowCount, bs, topK, capacity, h, dtype == TILEXR_DATA_TYPE_BFP16, gradRowsOut,
+                                      gradWeightsOut, stream);
+}
+
 int TileXRRmsNorm(const void *x, void *residualInOut, const void *gamma, float eps, int64_t rows, int64_t h,
                   TileXRDataType dtype, void *yOut, TileXRStream stream)
 {

@@ -172,6 +172,8 @@ int LaunchSwiglu(const void *gateUp, int64_t rows, int64_t f, bool bf16, void *y
 int LaunchRouterLogits(const void *x, const float *gate, int64_t tokens, int64_t h, int64_t experts, bool bf16, float *out, void *stream);
 int LaunchCombineBackward(const void *g, const float *weights, const void *rows, const int32_t *assist, const int32_t *rowCount, int64_t capacity,
                           int64_t h, bool bf16, int slots, int wideCols, void *gradRows, void *wide, void *stream);
+int LaunchCombineBackwardLocal(const void *gradY, const float *weights, const void *rows, const int32_t *routeRows, const int32_t *rowCount, int64_t bs,
+                               int64_t topK, int64_t capacity, int64_t h, bool bf16, void *gradRows, float *gradWeights, void *stream);
 int LaunchFp8Quant1x128(const void *x, int64_t rows, int64_t h, bool bf16, void *y, float *scales, void *stream);
 int LaunchFp8Dequant1x128(const void *y, const float *scales, int64_t rows, int64_t h, bool bf16, void *x, void *stream);
 int LaunchMxfp8Quant(const void *x, int64_t rows, int64_t h, bool bf16, bool e5m2, void *y, uint8_t *scales, void *stream);

@@ -215,6 +215,13 @@ int TileXRMoeRouterLogits(const void *x, const float *gate, int64_t bs, int64_t 
 int TileXRMoeEpCombineBackward(const void *g, const float *weights, const void *rows, const int32_t *assist, const int32_t *rowCount,
                                int64_t capacity, int64_t h, int64_t slots, int64_t wideCols, TXR_DT dtype, void *gradRowsOut, void *wideOut,
                                TileXRStream stream);
+// The same for a world of one rank, from the output gradient itself: routeRows [bs, topK] and *rowCount are those of the forward
+// dispatch, weights [bs, topK] its gate weights.  gradRows[routeRows[t, k]] = weights[t, k] * gradY[t]; with gradWeights [bs, topK]
+// also <gradY[t], rows[routeRows[t, k]]> in fp32 (`rows` may be null without it).  Inactive routes (row -1) get a zero weight gradient,
+// rows from *rowCount to `capacity` a zero gradient.
+int TileXRMoeEpCombineBackwardLocal(const void *gradY, const float *weights, const void *rows, const int32_t *routeRows, const int32_t *rowCount,
+                                    int64_t bs, int64_t topK, int64_t capacity, int64_t h, TXR_DT dtype, void *gradRowsOut, float *gradWeightsOut,
+                                    TileXRStream stream);
 // RMSNorm: y = x * rsqrt(mean(x^2) + eps) * gamma, optionally x += residual first (and the sum is written back).
 int TileXRRmsNorm(const void *x, void *residualInOut, const void *gamma, float eps, int64_t rows, int64_t h, TXR_DT dtype,
                   void *yOut, TileXRStream stream);

@@ -623,6 +623,27 @@ py::tuple EpCombineBackward(const at::Tensor &g, const at::Tensor &weights, cons
     return py::make_tuple(grad, dots ? py::cast(wide) : py::none());
 }
 
+// (grad_rows, grad_weights | None), see TileXRMoeEpCombineBackwardLocal
+py::tuple EpCombineBackwardLocal(const at::Tensor &gradY, const at::Tensor &weights, const at::Tensor &rows, const at::Tensor &routeRows,
+                                 const at::Tensor &rowCount, bool wantWeights)
+{
+    TORCH_CHECK(gradY.is_cuda() && gradY.dim() == 2 && gradY.is_contiguous() && rows.is_cuda() && rows.dim() == 2 && rows.is_contiguous() &&
+                    rows.size(1) == gradY.size(1) && rows.scalar_type() == gradY.scalar_type(),
+                "grad_y [tokens, h] and rows [capacity, h] must be contiguous CUDA tensors of one type");
+    TORCH_CHECK(routeRows.is_cuda() && routeRows.scalar_type() == at::kInt && routeRows.dim() == 2 && routeRows.is_contiguous() &&
+                    routeRows.size(0) == gradY.size(0) && weights.is_cuda() && weights.scalar_type() == at::kFloat && weights.is_contiguous() &&
+                    weights.numel() == routeRows.numel() && rowCount.is_cuda() && rowCount.scalar_type() == at::kInt && rowCount.numel() == 1,
+                "route_rows int32 [tokens, top_k] and the row count int32 [1] of the dispatch, weights fp32 [tokens, top_k]");
+    at::Tensor grad = at::empty_like(rows);
+    at::Tensor gradWeights = wantWeights ? at::empty(routeRows.sizes(), weights.options()) : at::Tensor();
+    Check(TileXRMoeEpCombineBackwardLocal(gradY.data_ptr(), weights.data_ptr<float>(), wantWeights ? rows.data_ptr() : nullptr,
+                                          routeRows.data_ptr<int32_t>(), rowCount.data_ptr<int32_t>(), gradY.size(0), routeRows.size(1), rows.size(0),
+                                          gradY.size(1), ToDtype(gradY.scalar_type()), grad.data_ptr(),
+                                          wantWeights ? gradWeights.data_ptr<float>() : nullptr, StreamOf(gradY)),
+          "TileXRMoeEpCombineBackwardLocal");
+    return py::make_tuple(grad, wantWeights ? py::cast(gradWeights) : py::none());
+}
+
 py::tuple RoutingTopK(const at::Tensor &logits, const c10::optional<at::Tensor> &bias, int64_t topK, int64_t scoreFunc,
                       bool renormalize, double routedScale)
 {
@@ -824,6 +845,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m)
     m.def("routing_topk", &RoutingTopK, py::arg("gate_logits"), py::arg("selection_bias") = py::none(), py::arg("top_k") = 1,
           py::arg("score_func") = 0, py::arg("renormalize") = true, py::arg("routed_scale") = 1.0);
     m.def("ep_combine_backward", &EpCombineBackward);
+    m.def("ep_combine_backward_local", &EpCombineBackwardLocal);
+    m.def("in_group", [] { return g_groupDepth > 0; });
     m.def("router_logits", &RouterLogits);
     m.def("fp8_quant_1x128", &Fp8Quant);
     m.def("swiglu", &Swiglu);

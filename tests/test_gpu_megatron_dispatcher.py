@@ -126,3 +126,42 @@ def test_combine_backward_rows_match_the_unfused_form(tokens, hidden, top_k, cap
     assert not rest.any()
     only_grad, none = ep.combine_backward_rows(d, None, top_k, width)
     assert none is None and torch.equal(only_grad, grad)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("tokens,hidden,top_k,extra", [(1, 8, 1, 0), (5, 264, 3, 19), (130, 1032, 8, 1)])
+def test_combine_backward_on_one_rank(tokens, hidden, top_k, extra, dtype):
+    """Row gradients and gate-weight gradients from the output gradient where it is; inactive routes, rows that no route fills."""
+    require_cuda()
+    import tilexr_b200 as txr
+    from tilexr_b200.ops import ep
+
+    comm = txr.init_process(0, 1, comm_id=f"127.0.0.1:{free_port()}", buffer_mb=64, device=0)
+    try:
+        gen = torch.Generator().manual_seed(tokens)
+        experts = 11
+        x = torch.randn(tokens, hidden, generator=gen).to(dtype).cuda()
+        ids = torch.stack([torch.randperm(experts, generator=gen)[:top_k] for _ in range(tokens)]).to(torch.int32)
+        if tokens > 1:
+            ids[torch.rand(tokens, top_k, generator=gen) < 0.2] = -1
+        w = torch.rand(tokens, top_k, generator=gen).cuda()
+        d = ep.dispatch(comm, x, num_experts=experts, top_k=top_k, expert_ids=ids.cuda(), max_recv_rows=tokens * top_k + extra)
+        out = torch.randn(d.expand_x.shape, generator=gen).to(dtype).cuda()
+        gy = torch.randn(tokens, hidden, generator=gen).to(dtype).cuda()
+        grad, gw = ep.combine_backward_local(comm, d, gy, out, w, True)
+        rows = d.route_rows.long()
+        want, filled = torch.zeros_like(out), torch.zeros(out.shape[0], dtype=torch.bool, device="cuda")
+        t, k = torch.nonzero(rows >= 0, as_tuple=True)
+        want[rows[t, k]] = (w[t, k, None] * gy[t].float()).to(dtype)
+        filled[rows[t, k]] = True
+        assert torch.equal(grad, want) and not grad[~filled].any() and int(filled.sum()) == int(d.recv_total)
+        terms = gy[t].double() * out[rows[t, k]].double()
+        dots = torch.zeros(tokens, top_k, dtype=torch.float64, device="cuda")
+        bound = torch.zeros_like(dots)
+        dots[t, k], bound[t, k] = terms.sum(dim=1), terms.abs().sum(dim=1) * hidden * 2.0 ** -24
+        assert ((gw.double() - dots).abs() <= bound).all()
+        only, none = ep.combine_backward_local(comm, d, gy, out, w, False)
+        assert none is None and torch.equal(only, grad)
+        assert ep.combine_backward_local(comm, d, gy.float(), out, w, True) is None        # not the kernel's types
+    finally:
+        comm.destroy()

@@ -24,6 +24,8 @@ the same two kernels in swapped roles:
                                                                        as a bf16 (high, low) pair
     d loss / d hidden[token]     = sum over k of grad_rows[row(token, k)]          a combine with unit weights
 
+On one rank the first two need no exchange: one kernel reads grad_y and the expert rows where they are (``ep.combine_backward_local``).
+
 The context of a step (what the reference's adapter keeps in its ``ctx`` dict) is the ``DispatchResult`` held between
 the two calls; ``ctx()`` exposes it.
 
@@ -87,6 +89,12 @@ class _Unpermute(torch.autograd.Function):
         owner, d = ctx.owner, ctx.d
         expert_out, probs = ctx.saved_tensors
         owner._barrier()
+        want_probs = ctx.needs_input_grad[1]
+        if owner.ops is _ep:
+            # one rank: the rows of a token's routes are known, grad_y need not travel to them
+            local = _ep.combine_backward_local(owner.comm, d, grad_y, expert_out, probs, want_probs)
+            if local is not None:
+                return local[0], None if local[1] is None else local[1].to(probs.dtype), None, None
         # grad_y goes where the tokens went; the gate weight of every row arrives beside it
         g = owner.ops.dispatch(owner.comm, grad_y.contiguous(), num_experts=owner.num_experts, top_k=owner.top_k,
                                expert_ids=owner._ids, expert_scales=probs, quant_mode=_ep.QUANT_NONE,
@@ -96,7 +104,6 @@ class _Unpermute(torch.autograd.Function):
         # the origin with unit weights: column k of the result is the dot product of route (token, k)
         K = owner.top_k * owner.tp_world_size
         width = max(256, (2 * K + 7) // 8 * 8)           # rows of at least 512 bytes, the width the kernels are tuned for
-        want_probs = ctx.needs_input_grad[1]
         fused = None
         if isinstance(g, _ep.DispatchResult) and g.expand_x.dtype == expert_out.dtype:
             fused = _ep.combine_backward_rows(g, expert_out if want_probs else None, K, width)

@@ -105,3 +105,20 @@ def combine_backward_rows(g: DispatchResult, expert_rows: Optional[torch.Tensor]
         if expert_rows.dtype != rows.dtype or expert_rows.shape != rows.shape or expert_rows.data_ptr() % 16 != 0:
             return None
     return _C.ep_combine_backward(rows, g.expand_scales, expert_rows, g.assist, g.recv_total, slots, wide_cols)
+
+
+def combine_backward_local(comm, d: DispatchResult, grad_y: torch.Tensor, expert_rows: torch.Tensor, weights: torch.Tensor, want_weights: bool):
+    """The backward of ``combine(comm, expert_rows, d, expert_scales=weights)`` in a world of one rank, in one pass and without a dispatch of
+    ``grad_y``: ``(grad_rows, grad_weights)`` with ``grad_rows[route_rows[t, k]] = weights[t, k] * grad_y[t]`` and, where wanted,
+    ``grad_weights[t, k] = <grad_y[t], expert_rows[route_rows[t, k]]>`` in fp32 (else None).  None where there are peers or the kernel does
+    not take the tensors."""
+    if (comm.world_size != 1 or not isinstance(d, DispatchResult) or d.tp_world_size != 1 or d.shared_expert_num != 0 or _C.in_group()
+            or not grad_y.is_cuda or grad_y.dim() != 2 or grad_y.dtype not in (torch.float16, torch.bfloat16) or grad_y.shape[0] != d.bs
+            or expert_rows.dtype != grad_y.dtype or expert_rows.dim() != 2 or expert_rows.shape[1] != grad_y.shape[1]
+            or expert_rows.device != grad_y.device or expert_rows.shape[0] != d.expand_x.shape[0]
+            or weights.dtype != torch.float32 or weights.shape != d.route_rows.shape):
+        return None
+    grad_y, expert_rows, weights = grad_y.contiguous(), expert_rows.contiguous(), weights.contiguous()
+    if grad_y.shape[0] == 0 or grad_y.shape[1] % 8 != 0 or grad_y.data_ptr() % 16 != 0 or expert_rows.data_ptr() % 16 != 0:
+        return None
+    return _C.ep_combine_backward_local(grad_y, weights, expert_rows, d.route_rows, d.recv_total, bool(want_weights))
