@@ -20,7 +20,7 @@ namespace {
 
 // One kernel per kind of transport: with all of them in one the registers of a 512-thread block (64, two blocks per SM) ran
 // out (628 bytes of spill loads against 340; 4096 x 7168 fp8 96 -> 92 us).
-enum EpTransport : int { EP_PLAIN = 0, EP_FP8 = 1, EP_MXFP8 = 2, EP_INT8 = 3 };
+enum EpTransport : int { EP_PLAIN = 0, EP_FP8 = 1, EP_MXFP8 = 2, EP_INT8 = 3, EP_FP8_ROUND = 4 };   // the last: fp8 and back, one rank only
 
 constexpr float FP8_E4M3_MAX = 448.0f;
 constexpr float FP8_AMAX_FLOOR = 1e-4f;
@@ -166,9 +166,24 @@ __device__ __forceinline__ void EndLocalLaunch(CommArgs *c, const Waiter &w)
     *CtrlWord(c, c->rank, TILEXR_CTRL_EPOCH_WORD) = w.epoch;
 }
 
+__device__ __forceinline__ void Fp8Unpack8(uint2 raw, __nv_fp8_interpretation_t kind, float s, float *f)
+{
+    const uint32_t w[2] = {raw.x, raw.y};
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const __half2_raw h2 = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>((w[i] >> (16 * j)) & 0xffffu), kind);
+            const float2 f2 = __half22float2(*reinterpret_cast<const __half2 *>(&h2));
+            f[i * 4 + j * 2] = f2.x * s;
+            f[i * 4 + j * 2 + 1] = f2.y * s;
+        }
+    }
+}
+
 // Sixteen elements per lane, eight neighbouring lanes share a block of 128: e4m3 values, and in *scales the four fp32 scales of the
-// warp's 512 elements (16 bytes of the row's scales), the same in all lanes.  Called by a whole warp.
-__device__ __forceinline__ Vec16 QuantFp8Block16(const float *f, Vec16 *scales)
+// warp's 512 elements (16 bytes of the row's scales), the same in all lanes; the lane's own in *own.  Called by a whole warp.
+__device__ __forceinline__ Vec16 QuantFp8Block16(const float *f, Vec16 *scales, float *own = nullptr)
 {
     float amax = 0.f;
 #pragma unroll
@@ -179,6 +194,7 @@ __device__ __forceinline__ Vec16 QuantFp8Block16(const float *f, Vec16 *scales)
     amax = fmaxf(amax, FP8_AMAX_FLOOR);
     const float inv = FP8_E4M3_MAX / amax;
     const float scale = amax / FP8_E4M3_MAX;
+    if (own != nullptr) *own = scale;
     scales->x = __float_as_uint(__shfl_sync(0xffffffffu, scale, 0));
     scales->y = __float_as_uint(__shfl_sync(0xffffffffu, scale, 8));
     scales->z = __float_as_uint(__shfl_sync(0xffffffffu, scale, 16));

@@ -53,6 +53,14 @@ __device__ __forceinline__ LocalSmem CarveLocalSmem(uint8_t *base, int E, int ro
     return s;
 }
 
+// 32 bytes to a 32-byte boundary (whole sectors; two 16-byte stores per lane would each touch every sector of the row's piece).
+__device__ __forceinline__ void StoreVec32(uint8_t *p, const Vec16 &lo, const Vec16 &hi)
+{
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(lo.x), "r"(lo.y), "r"(lo.z), "r"(lo.w), "r"(hi.x), "r"(hi.y),
+                 "r"(hi.z), "r"(hi.w)
+                 : "memory");
+}
+
 // Sum of the first `n` (0 to 16 / sizeof(COUNT)) counts of a 16-byte vector.
 template <typename COUNT>
 __device__ __forceinline__ uint32_t SumCounts(const uint4 &v, int n)
@@ -282,7 +290,8 @@ __device__ void DispatchLocalBody(const EpDispatchArgs &a)
     if (ok) {
         const bool bf16 = a.isBf16 != 0;
         constexpr bool mx = TRANSPORT == EP_MXFP8;
-        constexpr bool quant = mx || TRANSPORT == EP_FP8;
+        constexpr bool round = TRANSPORT == EP_FP8_ROUND;
+        constexpr bool quant = mx || round || TRANSPORT == EP_FP8;
         const bool mxE5m2 = a.quantMode == TileXREp::TILEXR_EP_QUANT_MXFP8_E5M2;
         const bool int8Dynamic = a.quantMode == TileXREp::TILEXR_EP_QUANT_DYNAMIC_INT8;
         const int chunks = a.h / 16;             // 16 elements per lane and iteration (8-bit transports)
@@ -360,6 +369,20 @@ __device__ void DispatchLocalBody(const EpDispatchArgs &a)
                         for (int j = 0; j < 16; ++j) f[j] = 0.f;
                     }
                     Vec16 sv;
+                    if (round) {
+                        // what the receiver of the 8-bit row would make of it, 32 bytes per lane
+                        float own;
+                        const Vec16 q = QuantFp8Block16(f, &sv, &own);
+                        Fp8Unpack8(make_uint2(q.x, q.y), __NV_E4M3, own, f);
+                        Fp8Unpack8(make_uint2(q.z, q.w), __NV_E4M3, own, f + 8);
+                        const Vec16 lo = Pack8(f, bf16), hi = Pack8(f + 8, bf16);
+                        uint8_t *dst = a.expandXOut + static_cast<int64_t>(c) * 32;
+                        for (uint32_t m = routes; m != 0; m &= m - 1) {
+                            const uint32_t rr = __shfl_sync(0xffffffffu, myRow, __ffs(m) - 1);
+                            if (c < chunks) StoreVec32(dst + rr * rowBytes, lo, hi);
+                        }
+                        continue;
+                    }
                     const Vec16 q = mx ? QuantMx16(f, mxE5m2, lane, &sv) : QuantFp8Block16(f, &sv);
                     // this iteration's 16 bytes of the scale row: lane k stores them for route k
                     if ((routes >> lane) & 1u) st_vec16(scalesOut + static_cast<uint64_t>(myRow) * a.win.scaleRowBytes + it * 16, sv);
@@ -423,13 +446,15 @@ __device__ void DispatchLocalBody(const EpDispatchArgs &a)
 
 TILEXR_DEFINE_KERNEL_OCC(TileXREpDispatchLocalKernel, EpDispatchArgs, DispatchLocalBody<EP_PLAIN>, EP_BLOCK_THREADS, 2)
 TILEXR_DEFINE_KERNEL_OCC(TileXREpDispatchLocalKernelFp8, EpDispatchArgs, DispatchLocalBody<EP_FP8>, EP_BLOCK_THREADS, 2)
+TILEXR_DEFINE_KERNEL_OCC(TileXREpDispatchLocalKernelFp8Round, EpDispatchArgs, DispatchLocalBody<EP_FP8_ROUND>, EP_BLOCK_THREADS, 2)
 TILEXR_DEFINE_KERNEL_OCC(TileXREpDispatchLocalKernelMxfp8, EpDispatchArgs, DispatchLocalBody<EP_MXFP8>, EP_BLOCK_THREADS, 2)
 TILEXR_DEFINE_KERNEL_OCC(TileXREpDispatchLocalKernelInt8, EpDispatchArgs, DispatchLocalBody<EP_INT8>, EP_BLOCK_THREADS, 2)
 
 } // namespace
 
-const KernelEntry &EpDispatchLocalKernelEntry(int64_t quantMode)
+const KernelEntry &EpDispatchLocalKernelEntry(int64_t quantMode, bool round)
 {
+    if (round) return TileXREpDispatchLocalKernelFp8RoundEntry;
     switch (quantMode) {
         case TileXREp::TILEXR_EP_QUANT_NONE: return TileXREpDispatchLocalKernelEntry;
         case TileXREp::TILEXR_EP_QUANT_FP8_1X128: return TileXREpDispatchLocalKernelFp8Entry;

@@ -294,12 +294,12 @@ uint64_t TileXREpAbiStamp(void) { return TILEXR_EP_ABI_STAMP; }
 
 int TileXRMoeEpDispatchFused(const TileXREpDispatchParams *p, TileXRCommPtr comm, TileXRStream stream)
 {
-    return TileXR::EpDispatch(p, nullptr, comm, stream);
+    return TileXR::EpDispatch(p, nullptr, false, comm, stream);
 }
 
 } // extern "C"
 
-int TileXR::EpDispatch(const TileXREpDispatchParams *p, int32_t *laneCountOut, TileXRCommPtr comm, TileXRStream stream)
+int TileXR::EpDispatch(const TileXREpDispatchParams *p, int32_t *laneCountOut, bool round, TileXRCommPtr comm, TileXRStream stream)
 {
     Ctx c;
     int ret = Prepare(comm, &c);
@@ -307,6 +307,9 @@ int TileXR::EpDispatch(const TileXREpDispatchParams *p, int32_t *laneCountOut, T
     if (p == nullptr || p->x == nullptr || p->expandXOut == nullptr || p->assistInfoForCombineOut == nullptr ||
         p->expertTokenNumsOut == nullptr || p->sendCountsOut == nullptr) {
         TILEXR_LOG(ERROR) << "EP dispatch: null tensor";
+        return TILEXR_ERROR_PARA_CHECK_FAIL;
+    }
+    if (round && (c.rankSize != 1 || p->quantMode != TILEXR_EP_QUANT_FP8_1X128 || p->tpWorldSize > 1 || (reinterpret_cast<uintptr_t>(p->expandXOut) & 31u) != 0)) {
         return TILEXR_ERROR_PARA_CHECK_FAIL;
     }
     if (p->tpWorldSize > 1) return DispatchWithTp(p, comm, stream, c);
@@ -349,7 +352,7 @@ int TileXR::EpDispatch(const TileXREpDispatchParams *p, int32_t *laneCountOut, T
         }
     }
     if (fp8Mode) {
-        if (p->dynamicScalesOut == nullptr || p->h % 512 != 0 || p->h > EP_FP8_MAX_H) {
+        if ((p->dynamicScalesOut == nullptr && !round) || p->h % 512 != 0 || p->h > EP_FP8_MAX_H) {
             TILEXR_LOG(ERROR) << "EP dispatch: fp8 mode needs dynamicScalesOut and h a multiple of 512 up to " << EP_FP8_MAX_H;
             return TILEXR_ERROR_PARA_CHECK_FAIL;
         }
@@ -387,7 +390,7 @@ int TileXR::EpDispatch(const TileXREpDispatchParams *p, int32_t *laneCountOut, T
     // Every block also takes a row of counts in the window: sixteen where the window is too small for the counts of more blocks.
     const bool aligned = (reinterpret_cast<uintptr_t>(p->expandXOut) & 15u) == 0;
     const bool local = c.rankSize == 1 && aligned;       // no peers: a kernel of its own
-    const KernelEntry &kernel = local ? EpDispatchLocalKernelEntry(p->quantMode) : EpDispatchKernelEntry(p->quantMode);
+    const KernelEntry &kernel = local ? EpDispatchLocalKernelEntry(p->quantMode, round) : EpDispatchKernelEntry(p->quantMode);
     for (int64_t perBlock = c.rankSize == 1 ? 4 : 16;; perBlock = 16) {
         grid = static_cast<unsigned>(std::max<int64_t>(minBlocks, std::min<int64_t>((p->bs + perBlock - 1) / perBlock, capBlocks)));
         unsigned gridCap = 0;
@@ -420,6 +423,7 @@ int TileXR::EpDispatch(const TileXREpDispatchParams *p, int32_t *laneCountOut, T
             return TILEXR_ERROR_PARA_CHECK_FAIL;
         }
     }
+    if (round) a.win.rowBytes = static_cast<uint32_t>(p->h * 2);
     a.x = static_cast<const uint8_t *>(p->x);
     a.expertIds = p->expertIds;
     a.gateLogits = p->gateLogits;

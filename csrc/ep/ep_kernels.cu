@@ -1250,21 +1250,6 @@ __global__ void __launch_bounds__(256) SwigluFp8Quant1x128Kernel(const uint8_t *
 }
 
 // Eight fp8 values times a scale.
-__device__ __forceinline__ void Fp8Unpack8(uint2 raw, __nv_fp8_interpretation_t kind, float s, float *f)
-{
-    const uint32_t w[2] = {raw.x, raw.y};
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const __half2_raw h2 = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>((w[i] >> (16 * j)) & 0xffffu), kind);
-            const float2 f2 = __half22float2(*reinterpret_cast<const __half2 *>(&h2));
-            f[i * 4 + j * 2] = f2.x * s;
-            f[i * 4 + j * 2 + 1] = f2.y * s;
-        }
-    }
-}
-
 constexpr int DEQUANT_STEPS = 4;
 
 // Bound by memory: 32768 x 7168 reads 242 MB and writes 470 MB, 142 us with one step, a 64-bit division and a row index per thread, 107 us so (6.7 TB/s).

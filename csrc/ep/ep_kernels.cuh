@@ -158,11 +158,14 @@ struct RoutingArgs {
 const KernelEntry &EpDispatchKernelEntry(int64_t quantMode);      // a kernel per kind of transport
 const KernelEntry &EpCombineKernelEntry();
 const KernelEntry &EpCombineLocalKernelEntry();                   // one rank that knows the row of each of its routes
-const KernelEntry &EpDispatchLocalKernelEntry(int64_t quantMode); // one rank, output on the 16-byte grid (ep_dispatch_local.cu)
+// One rank, output on the 16-byte grid (ep_dispatch_local.cu); `round`: fp8 and back on the way.
+const KernelEntry &EpDispatchLocalKernelEntry(int64_t quantMode, bool round);
 
 // TileXRMoeEpDispatchFused that also sets *laneCountOut (null: nothing) to zero, in the dispatch launch: what the Python results
 // report for a world without tensor-parallel lanes, whose C callers get no such count.
-int EpDispatch(const TileXREpDispatchParams *p, int32_t *laneCountOut, TileXRCommPtr comm, TileXRStream stream);
+// `round` (one rank, quantMode fp8 1 x 128, expandXOut 32-byte aligned): expandXOut gets 16-bit rows of x's type that have been through fp8,
+// what dequantising the 8-bit rows would give, and dynamicScalesOut nothing.
+int EpDispatch(const TileXREpDispatchParams *p, int32_t *laneCountOut, bool round, TileXRCommPtr comm, TileXRStream stream);
 
 // Plain (non communicating) kernels, launched directly.
 int LaunchRoutingTopK(const RoutingArgs &args, void *stream);

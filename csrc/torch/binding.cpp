@@ -412,7 +412,7 @@ py::tuple EpDispatch(const CommPtr &c, const at::Tensor &x, const c10::optional<
                      int64_t scoreFunc, bool renormalize, double routedScale, int64_t tokenNumsType, int64_t maxRecvRows,
                      const c10::optional<at::Tensor> &expandXOut, const c10::optional<at::Tensor> &expertScales, bool dedup,
                      const c10::optional<at::Tensor> &quantScales, int64_t sharedExpertNum, int64_t sharedExpertRankNum,
-                     int64_t tpWorldSize)
+                     int64_t tpWorldSize, bool roundTrip)
 {
     RequireContiguous(x, "x");
     const int64_t T = tpWorldSize > 1 ? tpWorldSize : 1;
@@ -436,10 +436,12 @@ py::tuple EpDispatch(const CommPtr &c, const at::Tensor &x, const c10::optional<
                                  : quantMode == TileXREp::TILEXR_EP_QUANT_MXFP8_E5M2 ? at::kFloat8_e5m2 : at::kFloat8_e4m3fn;
     at::Tensor expandX = expandXOut.has_value() && expandXOut->defined()
                              ? *expandXOut
-                             : at::empty({maxRecvRows, h}, x.options().dtype(quant ? qType : x.scalar_type()));
+                             : at::empty({maxRecvRows, h}, x.options().dtype(quant && !roundTrip ? qType : x.scalar_type()));
     TORCH_CHECK(expandX.is_contiguous() && expandX.size(0) >= maxRecvRows && expandX.size(1) == h, "bad expand_x_out");
-    const bool hasScales = quant && quantMode != TileXREp::TILEXR_EP_QUANT_STATIC_INT8;
-    at::Tensor scales = mx                                                      ? at::empty({maxRecvRows, h / 32}, x.options().dtype(at::kByte))
+    const bool hasScales = quant && quantMode != TileXREp::TILEXR_EP_QUANT_STATIC_INT8 && !roundTrip;
+    TORCH_CHECK(!roundTrip || expandX.scalar_type() == x.scalar_type(), "the round trip returns rows of x's type");
+    at::Tensor scales = roundTrip                                               ? at::Tensor()
+                        : mx                                                    ? at::empty({maxRecvRows, h / 32}, x.options().dtype(at::kByte))
                         : quantMode == TileXREp::TILEXR_EP_QUANT_DYNAMIC_INT8 ? at::empty({maxRecvRows}, x.options().dtype(at::kFloat))
                         : hasScales                                            ? at::empty({maxRecvRows, h / 128}, x.options().dtype(at::kFloat))
                                                                                : at::Tensor();
@@ -519,7 +521,7 @@ py::tuple EpDispatch(const CommPtr &c, const at::Tensor &x, const c10::optional<
                                 assistExt, expandScales, tpRecvCounts}) {
         Keep(t);
     }
-    Check(TileXR::EpDispatch(&p, T > 1 ? nullptr : tpRecvCounts.data_ptr<int32_t>(), c->ptr(), StreamOf(x)), "TileXRMoeEpDispatchFused");
+    Check(TileXR::EpDispatch(&p, T > 1 ? nullptr : tpRecvCounts.data_ptr<int32_t>(), roundTrip, c->ptr(), StreamOf(x)), "TileXRMoeEpDispatchFused");
     return py::make_tuple(expandX, hasScales ? py::cast(scales) : py::none(), assist, tokenNums, sendCounts, recvTotal, topkIds,
                           topkWeights, routeRows, assistExt, expandScales, tpRecvCounts);
 }
@@ -835,7 +837,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m)
           py::arg("renormalize") = true, py::arg("routed_scale") = 1.0, py::arg("token_nums_type") = 1,
           py::arg("max_recv_rows") = 0, py::arg("expand_x_out") = py::none(), py::arg("expert_scales") = py::none(),
           py::arg("dedup") = false, py::arg("scales") = py::none(), py::arg("shared_expert_num") = 0,
-          py::arg("shared_expert_rank_num") = 0, py::arg("tp_world_size") = 1);
+          py::arg("shared_expert_rank_num") = 0, py::arg("tp_world_size") = 1, py::arg("round_trip") = false);
     m.def("ep_combine", &EpCombine, py::arg("comm"), py::arg("expert_out"), py::arg("assist"), py::arg("send_counts"),
           py::arg("expert_ids") = py::none(), py::arg("expert_scales") = py::none(), py::arg("active_mask") = py::none(),
           py::arg("shared_expert_x") = py::none(), py::arg("bs") = 0, py::arg("top_k") = 1, py::arg("num_experts") = 1,

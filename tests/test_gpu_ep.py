@@ -769,3 +769,28 @@ def test_combine_of_a_route_that_the_dispatch_did_not_place(txr, port):
         assert torch.equal(ep.combine(comm, d.expand_x, d), y) and comm.device_status() == 0
     finally:
         comm.destroy()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("tokens,hidden,experts", [(1, 512, 8), (33, 1536, 40), (700, 7168, 256)])
+def test_dispatch_through_fp8_and_back(txr, port, tokens, hidden, experts, dtype):
+    """One pass gives what quantised rows and their dequantisation give, bit for bit."""
+    ep = txr.ep
+    g = torch.Generator().manual_seed(tokens)
+    x = (torch.randn(tokens, hidden, generator=g) * torch.logspace(-4, 2, hidden)).to(dtype).cuda()
+    x[0, :128] = 0
+    logits = torch.randn(tokens, experts, generator=g).cuda()
+    comm = txr.init_process(0, 1, comm_id=f"127.0.0.1:{port}", buffer_mb=128, device=0)
+    try:
+        args = dict(gate_logits=logits, num_experts=experts, top_k=4, quant_mode=ep.QUANT_FP8_1X128, max_recv_rows=tokens * 4)
+        d = ep.dispatch(comm, x, **args)
+        r = ep.dispatch(comm, x, round_trip=True, **args)
+        torch.cuda.synchronize()
+        assert comm.device_status() == 0 and r.dynamic_scales is None and r.expand_x.dtype == dtype
+        assert torch.equal(r.expand_x.view(torch.int16), txr.quant.fp8_dequant_1x128(d.expand_x, d.dynamic_scales, dtype).view(torch.int16))
+        for name in ("assist", "expert_token_nums", "send_counts", "recv_total", "topk_ids", "topk_weights", "route_rows", "expand_scales"):
+            assert torch.equal(getattr(d, name), getattr(r, name)), name
+        with pytest.raises(RuntimeError):
+            ep.dispatch(comm, x, round_trip=True, **dict(args, quant_mode=ep.QUANT_NONE))
+    finally:
+        comm.destroy()

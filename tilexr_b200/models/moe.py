@@ -88,10 +88,12 @@ class ExpertParallelMoE(torch.nn.Module):
         cfg = self.cfg
         if gate_logits is None:
             gate_logits = self.route_logits(x)
+        # one rank: the rows leave the dispatch as the experts want them, quantised and dequantised on the way
+        round_trip = cfg.fp8_dispatch and self.comm.world_size == 1 and expand_x_out is None and x.dtype == cfg.dtype
         d = ep.dispatch(self.comm, x, gate_logits=gate_logits, num_experts=cfg.num_experts, top_k=cfg.top_k,
                         quant_mode=ep.QUANT_FP8_1X128 if cfg.fp8_dispatch else ep.QUANT_NONE, score_func=cfg.score_func,
                         renormalize=cfg.renormalize, routed_scale=cfg.routed_scale, max_recv_rows=max_recv_rows,
-                        expand_x_out=expand_x_out)
-        rows = quant.fp8_dequant_1x128(d.expand_x, d.dynamic_scales, cfg.dtype) if cfg.fp8_dispatch else d.expand_x
+                        expand_x_out=expand_x_out, round_trip=round_trip)
+        rows = quant.fp8_dequant_1x128(d.expand_x, d.dynamic_scales, cfg.dtype) if cfg.fp8_dispatch and not round_trip else d.expand_x
         out = self.experts(rows, d.expert_token_nums) if self.w13 is not None else rows
         return ep.combine(self.comm, out, d, expert_scales=d.topk_weights)

@@ -52,7 +52,7 @@ def dispatch(comm, x: torch.Tensor, *, num_experts: int, top_k: int, expert_ids:
              max_recv_rows: Optional[int] = None, expand_x_out: Optional[torch.Tensor] = None,
              expert_scales: Optional[torch.Tensor] = None, dedup: Optional[bool] = None,
              scales: Optional[torch.Tensor] = None, shared_expert_num: int = 0,
-             shared_expert_rank_num: int = 0, tp_world_size: int = 1) -> DispatchResult:
+             shared_expert_rank_num: int = 0, tp_world_size: int = 1, round_trip: bool = False) -> DispatchResult:
     """``tp_world_size`` T > 1: tensor parallelism inside expert parallelism.  The ranks form ``world / T`` groups of T
     consecutive ranks that hold the same ``num_experts / (world / T)`` experts, each a slice of their weights; every
     route is written to all T ranks of its expert's group in one hop, so each of them receives all the group's rows
@@ -64,7 +64,10 @@ def dispatch(comm, x: torch.Tensor, *, num_experts: int, top_k: int, expert_ids:
     ``dedup`` (default: on when gate weights are known at dispatch time): a token with several experts on one
     remote rank crosses NVLink once in each direction; the expert rank replicates it after arrival and sums
     its outputs, gate-weighted in fp32, before sending them back.  The weights used for those sums are the ones
-    given here (fused routing or ``expert_scales``), so pass the same ones to ``combine``."""
+    given here (fused routing or ``expert_scales``), so pass the same ones to ``combine``.
+
+    ``round_trip`` (one rank, ``quant_mode=QUANT_FP8_1X128``): ``expand_x`` holds rows of x's type that have been through fp8, bit for
+    bit what ``quant.fp8_dequant_1x128`` makes of the 8-bit rows, in one pass; there are no ``dynamic_scales``."""
     bs = x.shape[0]
     if dedup is None:
         dedup = gate_logits is not None or expert_scales is not None
@@ -75,7 +78,7 @@ def dispatch(comm, x: torch.Tensor, *, num_experts: int, top_k: int, expert_ids:
         max_recv_rows = bs * comm.world_size * min(top_k, num_experts // (comm.world_size // tp_world_size - shared_expert_rank_num))
     out = _C.ep_dispatch(comm, x, expert_ids, gate_logits, selection_bias, active_mask, top_k, num_experts, quant_mode,
                          score_func, renormalize, routed_scale, token_nums_type, max_recv_rows, expand_x_out, expert_scales,
-                         bool(dedup), scales, shared_expert_num, shared_expert_rank_num, tp_world_size)
+                         bool(dedup), scales, shared_expert_num, shared_expert_rank_num, tp_world_size, bool(round_trip))
     res = DispatchResult(*out, bs=bs, top_k=top_k, num_experts=num_experts, dedup=bool(dedup),
                          shared_expert_num=shared_expert_num, shared_expert_rank_num=shared_expert_rank_num,
                          tp_world_size=tp_world_size)
