@@ -122,6 +122,29 @@ int IssueWorldLaunch(EmulatedWorld *world, std::vector<PendingLaunch *> &perRank
 
 } // namespace
 
+int LaunchOverlapped(const void *kernel, unsigned gridX, unsigned gridY, unsigned block, size_t smemBytes, unsigned cluster, void **params,
+                     TileXRStream stream)
+{
+    cudaLaunchAttribute attrs[2];
+    unsigned n = 0;
+    attrs[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[n++].val.programmaticStreamSerializationAllowed = 1;
+    if (cluster > 0) {
+        attrs[n].id = cudaLaunchAttributeClusterDimension;
+        attrs[n].val.clusterDim.x = cluster;
+        attrs[n].val.clusterDim.y = 1;
+        attrs[n++].val.clusterDim.z = 1;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(gridX, gridY, 1);
+    cfg.blockDim = dim3(block, 1, 1);
+    cfg.dynamicSmemBytes = smemBytes;
+    cfg.stream = static_cast<cudaStream_t>(stream);
+    cfg.attrs = attrs;
+    cfg.numAttrs = n;
+    return static_cast<int>(cudaLaunchKernelExC(&cfg, kernel, params));
+}
+
 uint64_t LaunchCount() { return g_launches.load(); }
 void NoteLaunch() { g_launches.fetch_add(1); }
 
@@ -153,6 +176,8 @@ int LaunchKernel(TileXRCommPtr commPtr, const KernelEntry &kernel, const void *a
     cudaError_t e;
     if (cfg.cooperative) {
         e = cudaLaunchCooperativeKernel(kernel.single, dim3(cfg.grid), dim3(cfg.block), params, cfg.smemBytes, stream);
+    } else if (cfg.overlap) {
+        e = static_cast<cudaError_t>(LaunchOverlapped(kernel.single, cfg.grid, 1, cfg.block, cfg.smemBytes, 0, params, stream));
     } else {
         e = cudaLaunchKernel(kernel.single, dim3(cfg.grid), dim3(cfg.block), params, cfg.smemBytes, stream);
     }

@@ -266,7 +266,7 @@ int LaunchCombineLocal(EpCombineArgs *a, const TileXREpCombineParams &p, TileXRC
     PerfLaunchInfo info{static_cast<uint32_t>(TILEXR_OP_EP_COMBINE), static_cast<uint32_t>(p.dtype), static_cast<uint32_t>(c.rank),
                         static_cast<uint32_t>(c.rankSize), grid, static_cast<uint64_t>(p.bs) * a->rowBytes};
     a->perfTrace = PerfTracePrepareLaunch(info, stream);
-    LaunchConfig cfg{grid, EP_LOCAL_THREADS, 0, false};
+    LaunchConfig cfg{grid, EP_LOCAL_THREADS, 0, false, true};
     return LaunchKernel(comm, EpCombineLocalKernelEntry(), a, cfg, stream);
 }
 

@@ -31,6 +31,7 @@
 
 #include <algorithm>
 #include <cstdio>
+#include <tuple>
 #include <cuda_runtime_api.h>
 
 #include "device/tilexr_data_as_flag.cuh"
@@ -1096,6 +1097,8 @@ __device__ void EpCombineLocalBody(const EpCombineArgs &a)
 {
     constexpr int KU = 8;              // routes whose columns are in flight together
     const int lane = threadIdx.x & 31;
+    StreamRelease();
+    StreamWait();
     Waiter w = MakeWaiter(a.comm, a.magic, blockIdx.x);
     PerfScope perf = PerfInit(threadIdx.x == 0 ? a.perfTrace : nullptr, static_cast<uint32_t>(a.comm->rank), blockIdx.x);
     PerfStageBegin(perf, TILEXR_PERF_KERNEL_TOTAL);
@@ -1202,6 +1205,8 @@ __device__ __forceinline__ void Fp8QuantStore16(const float *f, int64_t idx, uin
 
 __global__ void __launch_bounds__(256) Fp8Quant1x128Kernel(const uint8_t *x, int64_t vecs, int bf16, uint8_t *y, float *scales)
 {
+    StreamRelease();
+    StreamWait();
     const int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (idx >= vecs) return;          // vecs is a multiple of eight: the threads of a 128-element block leave together
     float f[16];
@@ -1225,6 +1230,8 @@ __device__ __forceinline__ void Swiglu8(const uint8_t *gate, const uint8_t *up, 
 
 __global__ void __launch_bounds__(256) SwigluKernel(const uint8_t *gateUp, int64_t vecs, int vecsPerRow, int bf16, uint8_t *y)
 {
+    StreamRelease();
+    StreamWait();
     const int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;     // a thread per 8 outputs
     if (idx >= vecs) return;
     const int64_t row = idx / vecsPerRow;
@@ -1236,6 +1243,8 @@ __global__ void __launch_bounds__(256) SwigluKernel(const uint8_t *gateUp, int64
 
 __global__ void __launch_bounds__(256) SwigluFp8Quant1x128Kernel(const uint8_t *gateUp, int64_t vecs, int vecsPerRow, int bf16, uint8_t *y, float *scales)
 {
+    StreamRelease();
+    StreamWait();
     const int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;     // a thread per 16 outputs
     if (idx >= vecs) return;
     const int64_t row = idx / vecsPerRow;
@@ -1255,6 +1264,8 @@ constexpr int DEQUANT_STEPS = 4;
 // Bound by memory: 32768 x 7168 reads 242 MB and writes 470 MB, 142 us with one step, a 64-bit division and a row index per thread, 107 us so (6.7 TB/s).
 __global__ void __launch_bounds__(256) Fp8Dequant1x128Kernel(const uint8_t *y, const float *scales, int64_t vecs, int bf16, uint8_t *x)
 {
+    StreamRelease();
+    StreamWait();
     // Eight elements per thread and step, DEQUANT_STEPS steps with all their loads first.  h is a multiple of 128, so the
     // matrix is one run of vectors and vector i has scale i / 16: no division by the row length.
     const int64_t base = static_cast<int64_t>(blockIdx.x) * (blockDim.x * DEQUANT_STEPS) + threadIdx.x;
@@ -1340,6 +1351,8 @@ __global__ void __launch_bounds__(256) Mxfp8DequantKernel(const uint8_t *y, cons
 __global__ void __launch_bounds__(256) Mxfp8Dequant8Kernel(const uint8_t *y, const uint8_t *scales, int64_t vecs, int vecsPerRow, int blocksPerRow, int e5m2,
                                                            int bf16, uint8_t *x)
 {
+    StreamRelease();
+    StreamWait();
     const int64_t base = static_cast<int64_t>(blockIdx.x) * (blockDim.x * DEQUANT_STEPS) + threadIdx.x;
     uint2 raw[DEQUANT_STEPS];
     int exponent[DEQUANT_STEPS];
@@ -1432,6 +1445,8 @@ __global__ void __launch_bounds__(256) CombineBackwardLocalKernel(const uint8_t 
                                                                   const int32_t *rowCount, int64_t routes, int topK, int64_t capacity, int vecsPerRow,
                                                                   int bf16, uint8_t *gradRows, float *gradWeights)
 {
+    StreamRelease();
+    StreamWait();
     const int64_t i = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (i >= *rowCount && i < capacity) {           // a row that no route fills
@@ -1529,6 +1544,18 @@ __global__ void __launch_bounds__(256) RmsNormKernel(const uint8_t *x, uint8_t *
     }
 }
 
+// A launch of 256-thread blocks of a kernel that calls StreamWait; CheckLaunch finds its error.
+template <typename... P, typename... A> void LaunchSimple(void (*kernel)(P...), unsigned grid, void *stream, A... args)
+{
+    std::tuple<P...> values(static_cast<P>(args)...);
+    std::apply(
+        [&](auto &...v) {
+            void *params[] = {const_cast<void *>(static_cast<const void *>(&v))...};
+            LaunchOverlapped(reinterpret_cast<const void *>(kernel), grid, 1, 256, 0, 0, params, stream);
+        },
+        values);
+}
+
 int CheckLaunch(const char *what)
 {
     const cudaError_t e = cudaGetLastError();
@@ -1572,8 +1599,8 @@ int LaunchRoutingTopK(const RoutingArgs &args, void *stream)
 int LaunchFp8Quant1x128(const void *x, int64_t rows, int64_t h, bool bf16, void *y, float *scales, void *stream)
 {
     const int64_t vecs = rows * (h / 16);
-    Fp8Quant1x128Kernel<<<static_cast<unsigned>((vecs + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const uint8_t *>(x), vecs, bf16 ? 1 : 0, static_cast<uint8_t *>(y), scales);
+    LaunchSimple(Fp8Quant1x128Kernel, static_cast<unsigned>((vecs + 255) / 256), stream,
+                 static_cast<const uint8_t *>(x), vecs, bf16 ? 1 : 0, static_cast<uint8_t *>(y), scales);
     return CheckLaunch("fp8 quant");
 }
 
@@ -1581,13 +1608,13 @@ int LaunchSwiglu(const void *gateUp, int64_t rows, int64_t f, bool bf16, void *y
 {
     if (scales != nullptr) {
         const int64_t vecs = rows * (f / 16);
-        SwigluFp8Quant1x128Kernel<<<static_cast<unsigned>((vecs + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-            static_cast<const uint8_t *>(gateUp), vecs, static_cast<int>(f / 16), bf16 ? 1 : 0, static_cast<uint8_t *>(y), scales);
+        LaunchSimple(SwigluFp8Quant1x128Kernel, static_cast<unsigned>((vecs + 255) / 256), stream,
+                     static_cast<const uint8_t *>(gateUp), vecs, static_cast<int>(f / 16), bf16 ? 1 : 0, static_cast<uint8_t *>(y), scales);
         return CheckLaunch("swiglu fp8 quant");
     }
     const int64_t vecs = rows * (f / 8);
-    SwigluKernel<<<static_cast<unsigned>((vecs + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const uint8_t *>(gateUp), vecs, static_cast<int>(f / 8), bf16 ? 1 : 0, static_cast<uint8_t *>(y));
+    LaunchSimple(SwigluKernel, static_cast<unsigned>((vecs + 255) / 256), stream,
+                 static_cast<const uint8_t *>(gateUp), vecs, static_cast<int>(f / 8), bf16 ? 1 : 0, static_cast<uint8_t *>(y));
     return CheckLaunch("swiglu");
 }
 
@@ -1595,8 +1622,7 @@ int LaunchFp8Dequant1x128(const void *y, const float *scales, int64_t rows, int6
 {
     const int64_t n = rows * (h / 8);
     const unsigned grid = static_cast<unsigned>((n + 256 * DEQUANT_STEPS - 1) / (256 * DEQUANT_STEPS));
-    Fp8Dequant1x128Kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const uint8_t *>(y), scales, n, bf16 ? 1 : 0,
-                                                                                static_cast<uint8_t *>(x));
+    LaunchSimple(Fp8Dequant1x128Kernel, grid, stream, static_cast<const uint8_t *>(y), scales, n, bf16 ? 1 : 0, static_cast<uint8_t *>(x));
     return CheckLaunch("fp8 dequant");
 }
 
@@ -1613,9 +1639,8 @@ int LaunchMxfp8Dequant(const void *y, const uint8_t *scales, int64_t rows, int64
 {
     if (h % 8 == 0 && ((reinterpret_cast<uintptr_t>(y) & 7u) | (reinterpret_cast<uintptr_t>(x) & 15u)) == 0) {
         const int64_t vecs = rows * (h / 8);
-        Mxfp8Dequant8Kernel<<<static_cast<unsigned>((vecs + 256 * DEQUANT_STEPS - 1) / (256 * DEQUANT_STEPS)), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-            static_cast<const uint8_t *>(y), scales, vecs, static_cast<int>(h / 8), static_cast<int>((h + 31) / 32), e5m2 ? 1 : 0, bf16 ? 1 : 0,
-            static_cast<uint8_t *>(x));
+        LaunchSimple(Mxfp8Dequant8Kernel, static_cast<unsigned>((vecs + 256 * DEQUANT_STEPS - 1) / (256 * DEQUANT_STEPS)), stream,
+                     static_cast<const uint8_t *>(y), scales, vecs, static_cast<int>(h / 8), static_cast<int>((h + 31) / 32), e5m2 ? 1 : 0, bf16 ? 1 : 0, static_cast<uint8_t *>(x));
         return CheckLaunch("mxfp8 dequant");
     }
     const int64_t n = rows * h;
@@ -1639,9 +1664,8 @@ int LaunchCombineBackwardLocal(const void *gradY, const float *weights, const vo
                                int64_t topK, int64_t capacity, int64_t h, bool bf16, void *gradRows, float *gradWeights, void *stream)
 {
     const int64_t warps = std::max(bs * topK, capacity);
-    CombineBackwardLocalKernel<<<static_cast<unsigned>((warps + 7) / 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const uint8_t *>(gradY), weights, static_cast<const uint8_t *>(rows), routeRows, rowCount, bs * topK, static_cast<int>(topK), capacity,
-        static_cast<int>(h / 8), bf16 ? 1 : 0, static_cast<uint8_t *>(gradRows), gradWeights);
+    LaunchSimple(CombineBackwardLocalKernel, static_cast<unsigned>((warps + 7) / 8), stream,
+                 static_cast<const uint8_t *>(gradY), weights, static_cast<const uint8_t *>(rows), routeRows, rowCount, bs * topK, static_cast<int>(topK), capacity, static_cast<int>(h / 8), bf16 ? 1 : 0, static_cast<uint8_t *>(gradRows), gradWeights);
     return CheckLaunch("combine backward on one rank");
 }
 

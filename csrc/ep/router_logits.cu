@@ -17,6 +17,7 @@
 
 #include <cuda_runtime_api.h>
 
+#include "device/tilexr_platform.cuh"
 #include "ep_kernels.cuh"
 #include "tilexr_types.h"
 
@@ -104,6 +105,8 @@ __global__ void __launch_bounds__(RL_THREADS, 1) RouterLogitsKernel(const Router
 #pragma unroll
         for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
     }
+    tilexr::StreamRelease();
+    tilexr::StreamWait();
     if (chunks > 0) LoadChunk<RL_TOKENS>(a, smemAddr, t0, e0, kBegin, kEnd, tid);
     for (int c = 0; c < chunks; ++c) {
         if (c + 1 < chunks) {
@@ -205,22 +208,13 @@ int LaunchRouterLogits(const void *x, const float *gate, int64_t tokens, int64_t
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     // one block per SM: K is split while the parts still fit beside one another and hold a chunk each
     while (a.split < RL_MAX_SPLIT && tiles * a.split * 2 <= sms && a.split * 2 * RL_CHUNK <= h + RL_CHUNK - 1) a.split *= 2;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = static_cast<unsigned>(a.split);
-    attr.val.clusterDim.y = 1;
-    attr.val.clusterDim.z = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(static_cast<unsigned>(tokenTiles * a.split), static_cast<unsigned>((experts + RL_EXPERTS - 1) / RL_EXPERTS));
-    cfg.blockDim = dim3(RL_THREADS);
-    cfg.dynamicSmemBytes = static_cast<size_t>(RlSmemBytes(perBlock));
-    cfg.stream = static_cast<cudaStream_t>(stream);
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
     void *params[] = {&a};
     // the limit belongs to the kernel on the current device: raised on every call, so that a second device of the process has it, too
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, RlSmemBytes(perBlock));
-    if (e == cudaSuccess) e = cudaLaunchKernelExC(&cfg, kernel, params);
+    if (e == cudaSuccess) {
+        e = static_cast<cudaError_t>(LaunchOverlapped(kernel, static_cast<unsigned>(tokenTiles * a.split), static_cast<unsigned>((experts + RL_EXPERTS - 1) / RL_EXPERTS),
+                                                      RL_THREADS, static_cast<size_t>(RlSmemBytes(perBlock)), static_cast<unsigned>(a.split), params, stream));
+    }
     if (e != cudaSuccess) {
         fprintf(stderr, "[TileXR] router logits launch failed: %s\n", cudaGetErrorString(e));
         cudaGetLastError();

@@ -155,23 +155,12 @@ int LaunchSkinny(const void *a, const void *b, const int64_t *groupRows, void *c
     std::call_once(once, [] {
         cudaFuncSetAttribute(GemmSkinnyKernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(GEMM_SKINNY_SMEM_BYTES));
     });
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = static_cast<unsigned>(g.split);
-    attr.val.clusterDim.y = 1;
-    attr.val.clusterDim.z = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(plan.grid);
-    cfg.blockDim = dim3(GEMM_SKINNY_THREADS);
-    cfg.dynamicSmemBytes = GEMM_SKINNY_SMEM_BYTES;
-    cfg.stream = static_cast<cudaStream_t>(stream);
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
     for (int64_t base = 0; base < groups; base += GEMM_SKINNY_MAX_GROUPS) {
         g.groupBase = static_cast<int32_t>(base);
         g.groups = static_cast<int32_t>(std::min<int64_t>(GEMM_SKINNY_MAX_GROUPS, groups - base));
         void *params[] = {&g};
-        const cudaError_t e = cudaLaunchKernelExC(&cfg, GemmSkinnyKernel(), params);
+        const cudaError_t e = static_cast<cudaError_t>(LaunchOverlapped(GemmSkinnyKernel(), plan.grid, 1, GEMM_SKINNY_THREADS, GEMM_SKINNY_SMEM_BYTES,
+                                                                        static_cast<unsigned>(g.split), params, stream));
         if (e != cudaSuccess) {
             TILEXR_LOG(ERROR) << "matmul (few rows) launch failed: " << cudaGetErrorString(e);
             cudaGetLastError();
@@ -236,8 +225,7 @@ int TileXRMatmul(const void *a, const void *b, void *c, int64_t m, int64_t n, in
             cudaFuncSetAttribute(GemmPairKernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(GEMM_PAIR_SMEM_BYTES));
         });
         void *pairParams[] = {&g};
-        const cudaError_t pe = cudaLaunchKernel(GemmPairKernel(), dim3(2 * pairs), dim3(GEMM_PAIR_THREADS), pairParams,
-                                                GEMM_PAIR_SMEM_BYTES, static_cast<cudaStream_t>(stream));
+        const cudaError_t pe = static_cast<cudaError_t>(LaunchOverlapped(GemmPairKernel(), 2 * pairs, 1, GEMM_PAIR_THREADS, GEMM_PAIR_SMEM_BYTES, 0, pairParams, stream));
         if (pe != cudaSuccess) {
             TILEXR_LOG(ERROR) << "matmul (CTA pairs) launch failed: " << cudaGetErrorString(pe);
             cudaGetLastError();
@@ -254,8 +242,7 @@ int TileXRMatmul(const void *a, const void *b, void *c, int64_t m, int64_t n, in
         cudaFuncSetAttribute(GemmKernelEmulated(), cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(GEMM_SMEM_BYTES));
     });
     void *params[] = {&g};
-    const cudaError_t e = cudaLaunchKernel(GemmKernelSingle(), dim3(grid), dim3(GEMM_THREADS), params, GEMM_SMEM_BYTES,
-                                           static_cast<cudaStream_t>(stream));
+    const cudaError_t e = static_cast<cudaError_t>(LaunchOverlapped(GemmKernelSingle(), grid, 1, GEMM_THREADS, GEMM_SMEM_BYTES, 0, params, stream));
     if (e != cudaSuccess) {
         TILEXR_LOG(ERROR) << "matmul launch failed: " << cudaGetErrorString(e);
         cudaGetLastError();
@@ -320,8 +307,7 @@ int TileXRGroupedMatmul(const void *a, const void *b, const int64_t *groupRows, 
         const int64_t tilesAtMost = ((maxRows + 2 * GEMM_BM - 1) / (2 * GEMM_BM) + g.groups) * g.nBlocks;
         const int pairs = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(tilesAtMost, EnvLong("TILEXR_GEMM_CTAS", sms) / 2)));
         void *params[] = {&g};
-        const cudaError_t e = cudaLaunchKernel(GemmPairKernel(), dim3(2 * pairs), dim3(GEMM_PAIR_THREADS), params, GEMM_PAIR_SMEM_BYTES,
-                                               static_cast<cudaStream_t>(stream));
+        const cudaError_t e = static_cast<cudaError_t>(LaunchOverlapped(GemmPairKernel(), 2 * pairs, 1, GEMM_PAIR_THREADS, GEMM_PAIR_SMEM_BYTES, 0, params, stream));
         if (e != cudaSuccess) {
             TILEXR_LOG(ERROR) << "grouped matmul launch failed: " << cudaGetErrorString(e);
             cudaGetLastError();
@@ -374,8 +360,7 @@ int TileXRMatmulFp8(const void *a, const void *b, void *c, int64_t m, int64_t n,
         cudaFuncSetAttribute(GemmPairKernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(GEMM_PAIR_SMEM_BYTES));
     });
     void *params[] = {&g};
-    const cudaError_t e = cudaLaunchKernel(GemmPairKernel(), dim3(2 * pairs), dim3(GEMM_PAIR_THREADS), params, GEMM_PAIR_SMEM_BYTES,
-                                           static_cast<cudaStream_t>(stream));
+    const cudaError_t e = static_cast<cudaError_t>(LaunchOverlapped(GemmPairKernel(), 2 * pairs, 1, GEMM_PAIR_THREADS, GEMM_PAIR_SMEM_BYTES, 0, params, stream));
     if (e != cudaSuccess) {
         TILEXR_LOG(ERROR) << "fp8 matmul launch failed: " << cudaGetErrorString(e);
         cudaGetLastError();
@@ -431,8 +416,8 @@ int TileXRMatmulFp8BlockScaled(const void *a, const float *scaleA, const void *b
         cudaFuncSetAttribute(GemmFp8BlockKernel(GEMM_PLAIN), cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(GEMM_FP8_BLOCK_SMEM_BYTES));
     });
     void *params[] = {&g};
-    const cudaError_t e = cudaLaunchKernel(GemmFp8BlockKernel(GEMM_PLAIN), dim3(2 * pairs), dim3(GEMM_FP8_BLOCK_THREADS), params, GEMM_FP8_BLOCK_SMEM_BYTES,
-                                           static_cast<cudaStream_t>(stream));
+    const cudaError_t e = static_cast<cudaError_t>(LaunchOverlapped(GemmFp8BlockKernel(GEMM_PLAIN), 2 * pairs, 1, GEMM_FP8_BLOCK_THREADS, GEMM_FP8_BLOCK_SMEM_BYTES, 0,
+                                                                    params, stream));
     if (e != cudaSuccess) {
         TILEXR_LOG(ERROR) << "block-scaled fp8 matmul launch failed: " << cudaGetErrorString(e);
         cudaGetLastError();

@@ -279,6 +279,8 @@ __device__ void GemmBody(const GemmArgs &a)
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(SmemAddr(&st->tmemBase)), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    StreamRelease();
+    StreamWait();
     TcFenceBefore();
     __syncthreads();
     TcFenceAfter();

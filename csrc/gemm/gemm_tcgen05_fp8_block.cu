@@ -408,6 +408,8 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(SmemAddr(&st->tmemBase)), "r"(FB_TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
+    StreamRelease();
+    StreamWait();
     FbFenceBefore();
     __syncthreads();
     FbClusterSync();

@@ -421,6 +421,8 @@ __device__ void PairBody(const GemmArgs &a)
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&a.tmapB)) : "memory");
         if (a.mode == GEMM_ALL_GATHER) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&a.tmapALocal)) : "memory");
     }
+    StreamRelease();
+    StreamWait();
     if (a.mode == GEMM_GROUPED && warp == 2) {
         BuildGroupTable(a.groupRows, a.groupBase, a.groups, a.M, 2 * GEMM_BM, lane, gt->rowStart, gt->blockStart);
     }

@@ -202,6 +202,8 @@ __global__ void __launch_bounds__(GEMM_SKINNY_THREADS, 2) TileXRGemmSkinny(const
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&a.tmapW)) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&a.tmapX)) : "memory");
     }
+    StreamRelease();
+    StreamWait();
     if (a.groupRows != nullptr && warp == 2) BuildGroupTable(a.groupRows, a.groupBase, a.groups, a.M, a.tn, lane, rowStart, chunkStart);
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(SmemAddr(&st->tmemBase)), "r"(tmemCols) : "memory");

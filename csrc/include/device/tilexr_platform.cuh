@@ -51,6 +51,14 @@ inline HostTraceHooks *&HostTraceSlot()
 }
 #endif
 
+#if defined(__CUDACC__)
+// A kernel launched with an overlap (tilexr_launch.h) may start while the kernel before it in its stream still runs.  StreamWait comes
+// before its first access to global memory, in every block: what came before in the stream has finished and can be seen.  StreamRelease lets
+// the kernel behind it start, so far as it was launched that way too, once every block has come here.
+__device__ __forceinline__ void StreamWait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void StreamRelease() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+#endif
+
 // ---- 64-bit flag words --------------------------------------------------------------------
 
 TXR_D void st_release_sys_u64(uint64_t *p, uint64_t v)
