@@ -5,6 +5,8 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <map>
+#include <mutex>
 
 #include <cuda_runtime_api.h>
 
@@ -245,6 +247,37 @@ int CombineWithTp(const TileXREpCombineParams *p, TileXRCommPtr comm, TileXRStre
     return TileXRMoeEpCombineFused(&q, comm, stream);
 }
 
+// Blocks of a cluster that `kernel` may have on the current device: EP_CLUSTER_BLOCKS, which a kernel has to be allowed, or the eight that every
+// kernel may have.  Asked of the driver once per kernel and device.
+int64_t ClusterBlocks(const void *kernel)
+{
+    static std::mutex mutex;
+    static std::map<std::pair<const void *, int>, int64_t> known;
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) return 0;
+    std::lock_guard<std::mutex> lock(mutex);
+    const auto it = known.find({kernel, device});
+    if (it != known.end()) return it->second;
+    int64_t blocks = 8;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = static_cast<unsigned>(EP_CLUSTER_BLOCKS);
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(static_cast<unsigned>(EP_CLUSTER_BLOCKS));
+        cfg.blockDim = dim3(EP_BLOCK_THREADS);
+        cfg.dynamicSmemBytes = 48 * 1024;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0) blocks = EP_CLUSTER_BLOCKS;
+    }
+    cudaGetLastError();
+    known[{kernel, device}] = blocks;
+    return blocks;
+}
+
 // Combine without peers (EpCombineLocalBody): (token, column part) items dealt out to the warps beforehand.
 int LaunchCombineLocal(EpCombineArgs *a, const TileXREpCombineParams &p, TileXRCommPtr comm, TileXRStream stream, const Ctx &c)
 {
@@ -391,9 +424,13 @@ int TileXR::EpDispatch(const TileXREpDispatchParams *p, int32_t *laneCountOut, b
     const bool aligned = (reinterpret_cast<uintptr_t>(p->expandXOut) & 15u) == 0;
     const bool local = c.rankSize == 1 && aligned;       // no peers: a kernel of its own
     const KernelEntry &kernel = local ? EpDispatchLocalKernelEntry(p->quantMode, round) : EpDispatchKernelEntry(p->quantMode);
+    const int64_t clusterMost = local && (c.hostArgs->extraFlag & TILEXR_FLAG_EMULATED) == 0 && p->bs <= EP_CLUSTER_TOKENS && capBlocks >= EP_CLUSTER_BLOCKS
+                                    ? ClusterBlocks(EpDispatchClusterKernel(p->quantMode, round)) : 0;
+    const bool cluster = clusterMost > 0;
     for (int64_t perBlock = c.rankSize == 1 ? 4 : 16;; perBlock = 16) {
         grid = static_cast<unsigned>(std::max<int64_t>(minBlocks, std::min<int64_t>((p->bs + perBlock - 1) / perBlock, capBlocks)));
         unsigned gridCap = 0;
+        if (cluster) grid = static_cast<unsigned>(std::min<int64_t>(p->bs, clusterMost));
         for (;;) {
             tokensPerBlock = static_cast<uint32_t>((p->bs + grid - 1) / grid);
             if (static_cast<int64_t>(tokensPerBlock) * routesPerToken > EP_MAX_ROUTES_PER_BLOCK) {
@@ -403,6 +440,7 @@ int TileXR::EpDispatch(const TileXREpDispatchParams *p, int32_t *laneCountOut, b
             }
             smem = local ? EpDispatchLocalSmemBytes(static_cast<int>(numCols), static_cast<int>(tokensPerBlock * routesPerToken))
                          : EpDispatchSmemBytes(static_cast<int>(smemCols), static_cast<int>(tokensPerBlock * routesPerToken));
+            if (cluster) break;
             unsigned maxGrid = 0;
             ret = MaxCooperativeGrid(comm, kernel, EP_BLOCK_THREADS, smem, ranksPerDevice, &maxGrid);
             if (ret != TILEXR_SUCCESS) return ret;
@@ -411,7 +449,7 @@ int TileXR::EpDispatch(const TileXREpDispatchParams *p, int32_t *laneCountOut, b
             if (grid <= maxGrid) break;
             grid = maxGrid;
         }
-        grid = static_cast<unsigned>(std::max<int64_t>((p->bs + tokensPerBlock - 1) / tokensPerBlock, std::min<int64_t>(minBlocks, gridCap)));
+        grid = static_cast<unsigned>(std::max<int64_t>((p->bs + tokensPerBlock - 1) / tokensPerBlock, cluster ? 0 : std::min<int64_t>(minBlocks, gridCap)));
         // (the table of the local kernel, one or two bytes per block in rows of 16 bytes, fits that of eight blocks' 32-bit counts)
         if (!DispatchLayout(p->h, numCols, c.rankSize, p->maxRecvRows, p->quantMode, elemSize, local ? std::max<int64_t>(grid, 8) : grid, zeroCopy, &a.win)) {
             return TILEXR_ERROR_PARA_CHECK_FAIL;
@@ -475,6 +513,18 @@ int TileXR::EpDispatch(const TileXREpDispatchParams *p, int32_t *laneCountOut, b
                             static_cast<uint32_t>(c.rank), static_cast<uint32_t>(c.rankSize), grid,
                             static_cast<uint64_t>(p->bs) * p->h * elemSize};
         a.perfTrace = PerfTracePrepareLaunch(info, stream);
+    }
+    if (cluster) {
+        void *params[] = {&a};
+        const cudaError_t e = static_cast<cudaError_t>(
+            LaunchOverlapped(EpDispatchClusterKernel(p->quantMode, round), grid, 1, EP_BLOCK_THREADS, smem, grid, params, stream));
+        if (e != cudaSuccess) {
+            TILEXR_LOG(ERROR) << "EP dispatch of " << p->bs << " tokens: launch failed: " << cudaGetErrorString(e);
+            cudaGetLastError();
+            return TILEXR_ERROR_RUNTIME;
+        }
+        NoteLaunch();
+        return TILEXR_SUCCESS;
     }
     LaunchConfig cfg{grid, EP_BLOCK_THREADS, smem, true};
     return LaunchKernel(comm, kernel, &a, cfg, stream);

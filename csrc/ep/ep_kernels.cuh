@@ -186,6 +186,10 @@ int LaunchRmsNorm(const void *x, void *residual, const void *gamma, float eps, i
                   void *stream);
 
 size_t EpDispatchSmemBytes(int numExperts, int routesPerBlock);
+// The form for few tokens: all its blocks are one cluster.
+const void *EpDispatchClusterKernel(int64_t quantMode, bool round);
+constexpr int64_t EP_CLUSTER_TOKENS = 64;
+constexpr int64_t EP_CLUSTER_BLOCKS = 16;
 size_t EpDispatchLocalSmemBytes(int numExperts, int routesPerBlock);
 
 } // namespace TileXR
