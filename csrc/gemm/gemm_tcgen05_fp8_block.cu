@@ -281,18 +281,19 @@ __device__ __forceinline__ uint32_t FbPackPair(float lo, float hi, bool bf16)
     return *reinterpret_cast<const uint32_t *>(&v);
 }
 
-// Two fp32 values as the operand of a packed instruction, and two multiply-adds, each rounded like fmaf.
-__device__ __forceinline__ uint64_t FbPair(uint32_t lo, uint32_t hi)
+// acc[0, 1] += x[0, 1] * f in one instruction, each rounded like fmaf.
+__device__ __forceinline__ void FbFma2(const uint32_t *x, float f, float *acc)
 {
-    uint64_t v;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(lo), "r"(hi));
-    return v;
-}
-__device__ __forceinline__ uint64_t FbFma2(uint64_t x, uint64_t y, uint64_t z)
-{
-    uint64_t v;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(x), "l"(y), "l"(z));
-    return v;
+    asm("{\n"
+        ".reg .b64 xx, ff, aa;\n"
+        "mov.b64 xx, {%2, %3};\n"
+        "mov.b64 ff, {%4, %4};\n"
+        "mov.b64 aa, {%0, %1};\n"
+        "fma.rn.f32x2 aa, xx, ff, aa;\n"
+        "mov.b64 {%0, %1}, aa;\n"
+        "}\n"
+        : "+f"(acc[0]), "+f"(acc[1])
+        : "r"(x[0]), "r"(x[1]), "f"(f));
 }
 
 // The grouped tile walk of the bf16 CTA-pair kernel: 256-row blocks advance fastest inside a group.
@@ -634,9 +635,9 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
                 }
                 __syncwarp();
             }
-            uint64_t acc[COLS / 2];                // pairs of columns
+            float acc[COLS];
 #pragma unroll
-            for (int j = 0; j < COLS / 2; ++j) acc[j] = 0;
+            for (int j = 0; j < COLS; ++j) acc[j] = 0.f;
             for (int kb0 = 0; kb0 < KB; kb0 += segBlocks, ++seg) {
                 // The scales go through shared memory: a lane reading its own row's scale from memory for every block touches 32 lines per warp
                 // and block.  Those of the next segment, of this item or the next one, come while this one is folded: fetched between
@@ -664,13 +665,15 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
                 // it is never stored (a test of the verdict in front of the release cost 2 %).
                 for (int kb = 0; kb < n; ++kb) {
                     const float f = sa[kb] * sb[kb];
-                    const uint64_t ff = FbPair(__float_as_uint(f), __float_as_uint(f));
                     const uint32_t p = kbAll & 1u;
                     FbWaitBarWarp(&st->scratchFull[p], (kbAll >> 1) & 1u, st, peerAbortAddr, budgetNs);
                     ++kbAll;
                     FbFenceAfter();
                     const uint32_t taddr = tmemBase + (static_cast<uint32_t>(quad * 32) << 16) + p * GEMM_BN + static_cast<uint32_t>(h * COLS);
-                    // Sixteen columns at a time, the next ones on their way while these are folded, two columns per multiply-add.
+                    // Sixteen columns at a time, the next ones on their way while these are folded.  In a whole tile one column per multiply-add:
+                    // two are quicker by themselves (285 clocks per block, 351 with one) but slow down beside the tensor cores, which read and
+                    // write the same memory (608 and 371): 8192^3 564 us and 514 to 548, 2048 x 14336 x 4096 128 and 120.  A narrow one leaves
+                    // the tensor cores idle anyway: 600 x 2048 x 8192 29.5 us and, one column at a time, 32.
                     uint32_t r[2][16];
                     FbTmemLoad16(taddr, r[0]);
 #pragma unroll
@@ -684,9 +687,13 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
                             __syncwarp();
                             if (lane == 0) FbArriveCluster(SmemAddr(&st->scratchEmpty[p]) & FB_PEER_BIT_MASK);
                         }
+                        float *to = acc + cc * 16;
+                        if constexpr (COLS == FB_HALF_N) {
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            acc[cc * 8 + j] = FbFma2(FbPair(r[cc & 1][2 * j], r[cc & 1][2 * j + 1]), ff, acc[cc * 8 + j]);
+                            for (int j = 0; j < 16; ++j) to[j] = fmaf(__uint_as_float(r[cc & 1][j]), f, to[j]);
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 16; j += 2) FbFma2(r[cc & 1] + j, f, to + j);
                         }
                     }
                 }
@@ -721,8 +728,7 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
                         uint32_t w[4];
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
-                            const uint64_t two = acc[(round * CHUNKS + v) * 4 + j];
-                            w[j] = FbPackPair(__uint_as_float(static_cast<uint32_t>(two)), __uint_as_float(static_cast<uint32_t>(two >> 32)), bf16);
+                            w[j] = FbPackPair(acc[(round * CHUNKS + v) * 8 + 2 * j], acc[(round * CHUNKS + v) * 8 + 2 * j + 1], bf16);
                         }
                         *reinterpret_cast<uint4 *>(myStage + lane * 128 + ((v ^ (lane & 7)) * 16)) = make_uint4(w[0], w[1], w[2], w[3]);
                     }
