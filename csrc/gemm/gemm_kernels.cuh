@@ -196,6 +196,7 @@ __device__ __forceinline__ void BuildGroupTable(const int64_t *groupRows, int gr
 }
 #endif
 
+const void *StageCopyKernel();                       // (dst0, src0, vecs0, dst1, src1, vecs1), 256 threads a block
 const void *GemmFp8BlockKernel(int mode);            // a kernel per GemmMode (plain, all-gather, reduce-scatter)
 const void *GemmFp8BlockKernelEmulated(int mode);    // all-gather, reduce-scatter
 const void *GemmKernelSingle();

@@ -857,8 +857,30 @@ template <int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_FP8_BLOCK_THREADS, 1)
 TileXRGemmFp8BlockScaled_emulated(const GemmBlockArgs *perRank) { FbBody<MODE>(perRank[blockIdx.y]); }
 
+// Two pieces of memory, 16-byte vectors, four in flight per thread.
+__global__ void __launch_bounds__(256) TileXRStageCopy(uint8_t *dst0, const uint8_t *src0, int64_t vecs0, uint8_t *dst1, const uint8_t *src1, int64_t vecs1)
+{
+    StreamRelease();
+    StreamWait();
+    const int64_t threads = static_cast<int64_t>(gridDim.x) * blockDim.x;
+    for (int64_t i0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i0 < vecs0 + vecs1; i0 += 4 * threads) {
+        Vec16 q[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int64_t i = i0 + u * threads;
+            if (i < vecs0 + vecs1) q[u] = ld_vec16_stream(i < vecs0 ? src0 + i * 16 : src1 + (i - vecs0) * 16);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int64_t i = i0 + u * threads;
+            if (i < vecs0 + vecs1) st_vec16(i < vecs0 ? dst0 + i * 16 : dst1 + (i - vecs0) * 16, q[u]);
+        }
+    }
+}
+
 } // namespace
 
+const void *StageCopyKernel() { return reinterpret_cast<const void *>(&TileXRStageCopy); }
 const void *GemmFp8BlockKernel(int mode)
 {
     return mode == GEMM_ALL_GATHER       ? reinterpret_cast<const void *>(&TileXRGemmFp8BlockScaled<GEMM_ALL_GATHER>)

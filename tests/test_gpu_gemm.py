@@ -326,6 +326,23 @@ def test_all_gather_matmul_fp8_block_exactly(txr, ranks, shard_rows, n, k):
         world.destroy()
 
 
+@pytest.mark.parametrize("rows,n,k", [(256, 136, 512), (512, 2568, 1536), (1280, 5128, 512)])
+def test_all_gather_matmul_fp8_block_on_one_rank(txr, port, rows, n, k):
+    """A rank without peers: the product of its own rows, exactly, and all rows and scales in the staging buffers; then of rows that are there already."""
+    comm = txr.init_process(0, 1, comm_id=f"127.0.0.1:{port}", buffer_mb=64, device=0)
+    try:
+        qa, sa, qw, sw = _exact_block_operands(rows, n, k, rows + n)
+        want = _exact_block_product(qa, sa, qw, sw).to(torch.bfloat16)
+        a_staging, s_staging = comm.symm_empty((rows, k), torch.float8_e4m3fn), comm.symm_empty((rows, k // 128), torch.float32)
+        for a, s in ((qa, sa), (a_staging, s_staging)):
+            got = txr.gemm.all_gather_matmul_fp8_block(comm, a, s, a_staging, s_staging, qw, sw)
+            assert torch.equal(got, want)
+            assert torch.equal(a_staging.view(torch.uint8), qa.view(torch.uint8)) and torch.equal(s_staging, sa)
+        assert comm.device_status() == 0
+    finally:
+        comm.destroy()
+
+
 @pytest.mark.parametrize("ranks,shard_rows,n,k", [(4, 256, 2568, 128 * 65), (2, 512, 2824, 128), (2, 256, 136, 128 * 129)])
 def test_matmul_reduce_scatter_fp8_block_exactly(txr, ranks, shard_rows, n, k):
     """Several tiles per CTA pair (a tile's staging shares its memory with the next tile's scales) and more blocks of K than a CTA holds
