@@ -76,15 +76,15 @@ __device__ __forceinline__ uint64_t *FlagB(const ArNormArgs &a, int owner, int s
 // Sums a row over all ranks in rank order (`srcOf(s)` gives rank s's copy), adds the residual, normalises.  Every 16-byte
 // column of the new residual goes to `putRes(v, column)` and of the result to `putY(v, column)`, straight from registers:
 // two-shot stores them to the own tensors and to every peer at once.
-template <typename SrcFn, typename ResFn, typename YFn>
+template <int NV, typename SrcFn, typename ResFn, typename YFn>
 __device__ __forceinline__ void ReduceNormRow(const ArNormArgs &a, SrcFn srcOf, int R, const uint8_t *resSrc, ResFn putRes, YFn putY, float *sPartial)
 {
     const bool bf16 = a.isBf16 != 0;
     const int vecs = a.rowBytes / 16;
-    float vals[ARN_MAX_VECS][8];
+    float vals[NV][8];
     float ss = 0.f;
 #pragma unroll
-    for (int i = 0; i < ARN_MAX_VECS; ++i) {
+    for (int i = 0; i < NV; ++i) {
         const int v = i * ARN_THREADS + threadIdx.x;
         if (v < vecs) {
             // Four ranks' copies of the column are fetched before the first is added (in rank order, so the sum does not
@@ -130,7 +130,7 @@ __device__ __forceinline__ void ReduceNormRow(const ArNormArgs &a, SrcFn srcOf, 
     for (int i = 0; i < static_cast<int>(ARN_THREADS / 32); ++i) tot += sPartial[i];
     const float rstd = rsqrtf(tot / static_cast<float>(a.h) + a.eps);
 #pragma unroll
-    for (int i = 0; i < ARN_MAX_VECS; ++i) {
+    for (int i = 0; i < NV; ++i) {
         const int v = i * ARN_THREADS + threadIdx.x;
         if (v < vecs) {
             float g[8], o[8];
@@ -148,26 +148,44 @@ __device__ __forceinline__ void ReduceNormRow(const ArNormArgs &a, SrcFn srcOf, 
 constexpr int ARN_GROUP = 8;
 constexpr int ARN_OWN_GROUP = 4;
 
-// Copies `rows` rows (at most ARN_GROUP) of `vecs` 16-byte columns; `srcRow(g)` and `dstRow(g)` give row g's ends.
+// Copies `rows` rows (at most ARN_GROUP) of `vecs` 16-byte columns; `srcRow(g)` and `dstRow(g)` give row g's ends.  Two rows at a time, two
+// columns of each per thread in flight; the ends of a row are worked out once (a division and a walk through the window's tables, per
+// column they were a third of the launch: 256 x 7168 on four emulated ranks 34.9 -> 26.4 us).
 template <typename SrcFn, typename DstFn>
 __device__ __forceinline__ void CopyRows(int rows, int vecs, SrcFn srcRow, DstFn dstRow)
 {
-    const int total = rows * vecs;
-    for (int i0 = static_cast<int>(threadIdx.x); i0 < total; i0 += 4 * static_cast<int>(ARN_THREADS)) {
-        Vec16 q[4];
+    for (int g0 = 0; g0 < rows; g0 += 2) {
+        const uint8_t *src[2];
+        uint8_t *dst[2];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int i = i0 + u * static_cast<int>(ARN_THREADS);
-            if (i < total) q[u] = ld_vec16_stream(srcRow(i / vecs) + static_cast<int64_t>(i % vecs) * 16);
+        for (int u = 0; u < 2; ++u) {
+            const int g = min(g0 + u, rows - 1);
+            src[u] = srcRow(g);
+            dst[u] = dstRow(g);
         }
+        for (int v0 = static_cast<int>(threadIdx.x); v0 < vecs; v0 += 2 * static_cast<int>(ARN_THREADS)) {
+            const int v1 = v0 + static_cast<int>(ARN_THREADS);
+            Vec16 q[2][2];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int i = i0 + u * static_cast<int>(ARN_THREADS);
-            if (i < total) st_vec16(dstRow(i / vecs) + static_cast<int64_t>(i % vecs) * 16, q[u]);
+            for (int u = 0; u < 2; ++u) {
+                if (g0 + u < rows) {
+                    q[u][0] = ld_vec16_stream(src[u] + static_cast<int64_t>(v0) * 16);
+                    if (v1 < vecs) q[u][1] = ld_vec16_stream(src[u] + static_cast<int64_t>(v1) * 16);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                if (g0 + u < rows) {
+                    st_vec16(dst[u] + static_cast<int64_t>(v0) * 16, q[u][0]);
+                    if (v1 < vecs) st_vec16(dst[u] + static_cast<int64_t>(v1) * 16, q[u][1]);
+                }
+            }
         }
     }
 }
 
+// `NV` 16-byte columns of a row per thread at most.
+template <int NV>
 __device__ void ArNormBody(const ArNormArgs &a)
 {
     __shared__ float sPartial[ARN_THREADS / 32];
@@ -210,7 +228,7 @@ __device__ void ArNormBody(const ArNormArgs &a)
             auto srcOf = [&](int s) -> const uint8_t * { return s == rank ? a.x + row * rb : PlaneA(a, rank, s, row, epoch); };
             uint8_t *res = a.residual != nullptr ? a.residual + row * rb : nullptr;
             uint8_t *yRow = a.y + row * rb;
-            ReduceNormRow(a, srcOf, R, res, [&](int v, const Vec16 &q) { st_vec16(res + v * 16, q); },
+            ReduceNormRow<NV>(a, srcOf, R, res, [&](int v, const Vec16 &q) { st_vec16(res + v * 16, q); },
                           [&](int v, const Vec16 &q) { st_vec16(yRow + v * 16, q); }, sPartial);
         }
     } else if (ok) {
@@ -256,7 +274,7 @@ __device__ void ArNormBody(const ArNormArgs &a)
                         st_vec16(dst + v * 16, q);
                     }
                 };
-                ReduceNormRow(a, srcOf, R, resRow, [&](int v, const Vec16 &q) { putAll(v, q, resRow, 1, a.resHandle, a.resOffset); },
+                ReduceNormRow<NV>(a, srcOf, R, resRow, [&](int v, const Vec16 &q) { putAll(v, q, resRow, 1, a.resHandle, a.resOffset); },
                               [&](int v, const Vec16 &q) { putAll(v, q, yRow, 0, a.yHandle, a.yOffset); }, sPartial);
             }
             if (!ok) break;
@@ -291,7 +309,9 @@ __device__ void ArNormBody(const ArNormArgs &a)
     KernelEpilogue(w, ok);
 }
 
-TILEXR_DEFINE_KERNEL(TileXRAllReduceRmsNormKernel, ArNormArgs, ArNormBody, ARN_THREADS)
+// Rows of up to 8192 columns leave room for two blocks on an SM.
+TILEXR_DEFINE_KERNEL_OCC(TileXRAllReduceRmsNormKernel, ArNormArgs, ArNormBody<2>, ARN_THREADS, 2)
+TILEXR_DEFINE_KERNEL(TileXRAllReduceRmsNormWideKernel, ArNormArgs, ArNormBody<ARN_MAX_VECS>, ARN_THREADS)
 
 long EnvLong(const char *name, long fallback)
 {
@@ -364,7 +384,8 @@ int TileXRAllReduceRmsNorm(const void *x, void *residualInOut, const void *gamma
     }
     const int ranksPerDevice = (hostArgs->extraFlag & TILEXR_FLAG_EMULATED) ? R : 1;
     unsigned maxGrid = 0;
-    ret = MaxCooperativeGrid(comm, TileXRAllReduceRmsNormKernelEntry, ARN_THREADS, 0, ranksPerDevice, &maxGrid);
+    const KernelEntry &kernel = h <= static_cast<int64_t>(ARN_THREADS) * 2 * 8 ? TileXRAllReduceRmsNormKernelEntry : TileXRAllReduceRmsNormWideKernelEntry;
+    ret = MaxCooperativeGrid(comm, kernel, ARN_THREADS, 0, ranksPerDevice, &maxGrid);
     if (ret != TILEXR_SUCCESS) return ret;
 
     for (int64_t done = 0; done < rows; done += maxRows) {
@@ -398,7 +419,7 @@ int TileXRAllReduceRmsNorm(const void *x, void *residualInOut, const void *gamma
         const unsigned want = static_cast<unsigned>(std::min<int64_t>(work, EnvLong("TILEXR_AR_NORM_BLOCKS", 64)));
         const unsigned grid = std::max(1u, std::min(want, maxGrid));
         LaunchConfig cfg{grid, ARN_THREADS, 0, true};
-        ret = LaunchKernel(comm, TileXRAllReduceRmsNormKernelEntry, &a, cfg, stream);
+        ret = LaunchKernel(comm, kernel, &a, cfg, stream);
         if (ret != TILEXR_SUCCESS) return ret;
     }
     return TILEXR_SUCCESS;

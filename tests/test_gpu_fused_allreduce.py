@@ -82,6 +82,15 @@ def test_all_reduce_rmsnorm_groups_of_rows(txr, ranks, rows, h, algo, with_res, 
     test_all_reduce_rmsnorm(txr, ranks, rows, h, algo, with_res, symmetric)
 
 
+@pytest.mark.parametrize("ranks,rows,h,algo,with_res,symmetric", [
+    (2, 9, 8192, 2, False, False),        # the longest rows of the kernel with two 16-byte columns per thread: all of them used
+    (2, 9, 8200, 2, True, False),         # the shortest of the other kernel
+    (3, 26, 4104, 1, True, False),        # one thread has a second column; an odd row after whole pairs
+])
+def test_all_reduce_rmsnorm_around_two_columns_per_thread(txr, ranks, rows, h, algo, with_res, symmetric):
+    test_all_reduce_rmsnorm(txr, ranks, rows, h, algo, with_res, symmetric)
+
+
 def test_emulated_world_of_more_ranks_than_travel_with_a_launch():
     """Argument blocks of more ranks than fit the launch's parameters come as a device array."""
     require_cuda()
