@@ -16,7 +16,9 @@
 // 16.2 us with the barrier in memory, 10.0 so; 64 tokens 17.8 and 14.8; 40 x 4096, top-6, 16 bits 11.5 and 8.9).
 //
 // Bound by the stores of step 4 for large batches; steps 1 to 3 are a chain of memory round trips that small batches wait for
-// (us, general kernel and this one: 16 x 7168 by 256 experts, fp8 18.3 14.6; 1009 x 4096, top-6, 16 bits 23.5 18.9; 4096 x 7168, fp8 91 84).
+// (us, general kernel and this one: 16 x 7168 by 256 experts, fp8 18.3 14.6; 1009 x 4096, top-6, 16 bits 23.5 18.9; 4096 x 7168, fp8 91 84, of
+// which the stores take 63: 3.9 TB/s of writes, what a plain fill of such a buffer reaches.  The reads of the tokens pass beside them; brought to
+// L2 during steps 1 to 3 they only delay the routes, 89).
 // The blocks wait for one another, so the launch is a cooperative one.
 #include <cuda_runtime_api.h>
 
@@ -189,15 +191,6 @@ __device__ void DispatchLocalBody(const EpDispatchArgs &a)
     const int nRoutes = nTok * K;
     const uint64_t inBytes = static_cast<uint64_t>(a.h) * a.elemSize;      // of a token
     const uint64_t rowBytes = a.win.rowBytes;                              // of a row of the output
-
-    // The block's tokens start on their way to L2 now: memory is idle while the routes are counted.
-    {
-        const uint8_t *rows = a.x + static_cast<int64_t>(t0) * inBytes;
-        const int64_t bytes = static_cast<int64_t>(nTok) * inBytes;
-        for (int64_t off = static_cast<int64_t>(tid) * 128; off < bytes; off += static_cast<int64_t>(EP_BLOCK_THREADS) * 128) {
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(rows + off));
-        }
-    }
 
     // ---- 1. route, rank, count ---------------------------------------------------------------------------------
     for (int e = tid; e < E; e += EP_BLOCK_THREADS) sm.hist[e] = 0;
