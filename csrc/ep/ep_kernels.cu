@@ -1218,17 +1218,20 @@ __global__ void __launch_bounds__(256) Fp8Quant1x128Kernel(const uint8_t *x, int
 // silu(gate) * up of rows [gate (f elements) | up (f elements)], computed in fp32 and rounded to the 16-bit type; with
 // `scales` the rounded values are then quantised as above, else they are stored.  One pass instead of the four to six
 // elementwise launches (and their fp32 copies of both halves) of the unfused form: 146 + 11 -> 21 us for 2048 rows of 2 x 7168.
-// Bound by the arithmetic (an exponential and a division per output; the SMs 79 % busy, DRAM 46 % at 8192 rows).
-__device__ __forceinline__ void Swiglu8(const uint8_t *gate, const uint8_t *up, bool bf16, float *o)
+// Bound by the arithmetic (an exponential and a division per output; the SMs 79 % busy, DRAM 46 % at 8192 rows).  A kernel per 16-bit type: with the
+// type read at run time the conversions of both are in the way (8192 rows of 2 x 7168: 69.3 us with fp8 output and 69.2 without, 66.4 and 67.5 so).
+template <bool BF16>
+__device__ __forceinline__ void Swiglu8(const uint8_t *gate, const uint8_t *up, float *o)
 {
     float g[8], u[8];
-    Unpack8(ld_vec16(gate), bf16, g);
-    Unpack8(ld_vec16(up), bf16, u);
+    Unpack8(ld_vec16(gate), BF16, g);
+    Unpack8(ld_vec16(up), BF16, u);
 #pragma unroll
     for (int j = 0; j < 8; ++j) o[j] = g[j] / (1.0f + expf(-g[j])) * u[j];
 }
 
-__global__ void __launch_bounds__(256) SwigluKernel(const uint8_t *gateUp, int64_t vecs, int vecsPerRow, int bf16, uint8_t *y)
+template <bool BF16>
+__global__ void __launch_bounds__(256) SwigluKernel(const uint8_t *gateUp, int64_t vecs, int vecsPerRow, uint8_t *y)
 {
     StreamRelease();
     StreamWait();
@@ -1237,11 +1240,12 @@ __global__ void __launch_bounds__(256) SwigluKernel(const uint8_t *gateUp, int64
     const int64_t row = idx / vecsPerRow;
     const uint8_t *gate = gateUp + (idx + row * vecsPerRow) * 16;                         // row r starts at vector 2 r vecsPerRow
     float o[8];
-    Swiglu8(gate, gate + static_cast<int64_t>(vecsPerRow) * 16, bf16 != 0, o);
-    st_vec16(y + idx * 16, Pack8(o, bf16 != 0));
+    Swiglu8<BF16>(gate, gate + static_cast<int64_t>(vecsPerRow) * 16, o);
+    st_vec16(y + idx * 16, Pack8(o, BF16));
 }
 
-__global__ void __launch_bounds__(256) SwigluFp8Quant1x128Kernel(const uint8_t *gateUp, int64_t vecs, int vecsPerRow, int bf16, uint8_t *y, float *scales)
+template <bool BF16>
+__global__ void __launch_bounds__(256) SwigluFp8Quant1x128Kernel(const uint8_t *gateUp, int64_t vecs, int vecsPerRow, uint8_t *y, float *scales)
 {
     StreamRelease();
     StreamWait();
@@ -1251,10 +1255,10 @@ __global__ void __launch_bounds__(256) SwigluFp8Quant1x128Kernel(const uint8_t *
     const uint8_t *gate = gateUp + (idx + row * vecsPerRow) * 32;
     const uint8_t *up = gate + static_cast<int64_t>(vecsPerRow) * 32;
     float f[16];
-    Swiglu8(gate, up, bf16 != 0, f);
-    Swiglu8(gate + 16, up + 16, bf16 != 0, f + 8);
-    Unpack8(Pack8(f, bf16 != 0), bf16 != 0, f);              // quantise what the unfused form stores
-    Unpack8(Pack8(f + 8, bf16 != 0), bf16 != 0, f + 8);
+    Swiglu8<BF16>(gate, up, f);
+    Swiglu8<BF16>(gate + 16, up + 16, f + 8);
+    Unpack8(Pack8(f, BF16), BF16, f);              // quantise what the unfused form stores
+    Unpack8(Pack8(f + 8, BF16), BF16, f + 8);
     Fp8QuantStore16(f, idx, 0xffu << (threadIdx.x & 24), y, scales);
 }
 
@@ -1347,9 +1351,10 @@ __global__ void __launch_bounds__(256) Mxfp8DequantKernel(const uint8_t *y, cons
 }
 
 // MXFP8 rows whose length is a multiple of eight (a group of eight elements then lies in one 32-element block and its 16
-// bytes of output are aligned): eight elements per thread instead of one.  32768 x 7168: 783 -> 140 us.
-__global__ void __launch_bounds__(256) Mxfp8Dequant8Kernel(const uint8_t *y, const uint8_t *scales, int64_t vecs, int vecsPerRow, int blocksPerRow, int e5m2,
-                                                           int bf16, uint8_t *x)
+// bytes of output are aligned): eight elements per thread instead of one.  32768 x 7168: 783 -> 139 us, 132 with a
+// kernel per pair of types and without a division per vector where rows are whole blocks.
+template <bool E5M2, bool BF16>
+__global__ void __launch_bounds__(256) Mxfp8Dequant8Kernel(const uint8_t *y, const uint8_t *scales, int64_t vecs, int vecsPerRow, int blocksPerRow, uint8_t *x)
 {
     StreamRelease();
     StreamWait();
@@ -1361,8 +1366,12 @@ __global__ void __launch_bounds__(256) Mxfp8Dequant8Kernel(const uint8_t *y, con
         const int64_t i = base + u * static_cast<int64_t>(blockDim.x);
         if (i < vecs) {
             raw[u] = __ldcs(reinterpret_cast<const uint2 *>(y) + i);
-            const int64_t row = i / vecsPerRow;
-            exponent[u] = static_cast<int>(__ldg(scales + row * blocksPerRow + (i - row * vecsPerRow) / 4)) - 127;
+            int64_t at = i >> 2;                                       // rows of whole 32-element blocks: vector i has scale i / 4
+            if (vecsPerRow != 4 * blocksPerRow) {
+                const int64_t row = i / vecsPerRow;
+                at = row * blocksPerRow + (i - row * vecsPerRow) / 4;
+            }
+            exponent[u] = static_cast<int>(__ldg(scales + at)) - 127;
         }
     }
 #pragma unroll
@@ -1370,8 +1379,8 @@ __global__ void __launch_bounds__(256) Mxfp8Dequant8Kernel(const uint8_t *y, con
         const int64_t i = base + u * static_cast<int64_t>(blockDim.x);
         if (i >= vecs) break;
         float f[8];
-        Fp8Unpack8(raw[u], e5m2 ? __NV_E5M2 : __NV_E4M3, exp2f(static_cast<float>(exponent[u])), f);
-        st_vec16(x + i * 16, Pack8(f, bf16 != 0));
+        Fp8Unpack8(raw[u], E5M2 ? __NV_E5M2 : __NV_E4M3, exp2f(static_cast<float>(exponent[u])), f);
+        st_vec16(x + i * 16, Pack8(f, BF16));
     }
 }
 
@@ -1608,13 +1617,13 @@ int LaunchSwiglu(const void *gateUp, int64_t rows, int64_t f, bool bf16, void *y
 {
     if (scales != nullptr) {
         const int64_t vecs = rows * (f / 16);
-        LaunchSimple(SwigluFp8Quant1x128Kernel, static_cast<unsigned>((vecs + 255) / 256), stream,
-                     static_cast<const uint8_t *>(gateUp), vecs, static_cast<int>(f / 16), bf16 ? 1 : 0, static_cast<uint8_t *>(y), scales);
+        LaunchSimple(bf16 ? SwigluFp8Quant1x128Kernel<true> : SwigluFp8Quant1x128Kernel<false>, static_cast<unsigned>((vecs + 255) / 256), stream,
+                     static_cast<const uint8_t *>(gateUp), vecs, static_cast<int>(f / 16), static_cast<uint8_t *>(y), scales);
         return CheckLaunch("swiglu fp8 quant");
     }
     const int64_t vecs = rows * (f / 8);
-    LaunchSimple(SwigluKernel, static_cast<unsigned>((vecs + 255) / 256), stream,
-                 static_cast<const uint8_t *>(gateUp), vecs, static_cast<int>(f / 8), bf16 ? 1 : 0, static_cast<uint8_t *>(y));
+    LaunchSimple(bf16 ? SwigluKernel<true> : SwigluKernel<false>, static_cast<unsigned>((vecs + 255) / 256), stream,
+                 static_cast<const uint8_t *>(gateUp), vecs, static_cast<int>(f / 8), static_cast<uint8_t *>(y));
     return CheckLaunch("swiglu");
 }
 
@@ -1639,8 +1648,10 @@ int LaunchMxfp8Dequant(const void *y, const uint8_t *scales, int64_t rows, int64
 {
     if (h % 8 == 0 && ((reinterpret_cast<uintptr_t>(y) & 7u) | (reinterpret_cast<uintptr_t>(x) & 15u)) == 0) {
         const int64_t vecs = rows * (h / 8);
-        LaunchSimple(Mxfp8Dequant8Kernel, static_cast<unsigned>((vecs + 256 * DEQUANT_STEPS - 1) / (256 * DEQUANT_STEPS)), stream,
-                     static_cast<const uint8_t *>(y), scales, vecs, static_cast<int>(h / 8), static_cast<int>((h + 31) / 32), e5m2 ? 1 : 0, bf16 ? 1 : 0, static_cast<uint8_t *>(x));
+        const auto kernel = e5m2 ? (bf16 ? Mxfp8Dequant8Kernel<true, true> : Mxfp8Dequant8Kernel<true, false>)
+                                 : (bf16 ? Mxfp8Dequant8Kernel<false, true> : Mxfp8Dequant8Kernel<false, false>);
+        LaunchSimple(kernel, static_cast<unsigned>((vecs + 256 * DEQUANT_STEPS - 1) / (256 * DEQUANT_STEPS)), stream,
+                     static_cast<const uint8_t *>(y), scales, vecs, static_cast<int>(h / 8), static_cast<int>((h + 31) / 32), static_cast<uint8_t *>(x));
         return CheckLaunch("mxfp8 dequant");
     }
     const int64_t n = rows * h;
