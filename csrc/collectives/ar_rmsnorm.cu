@@ -415,8 +415,11 @@ int TileXRAllReduceRmsNorm(const void *x, void *residualInOut, const void *gamma
         if (ret != TILEXR_SUCCESS) return ret;
         a.magic = magic;
         (void)rank;
-        const int64_t work = twoShot ? n : n;
-        const unsigned want = static_cast<unsigned>(std::min<int64_t>(work, EnvLong("TILEXR_AR_NORM_BLOCKS", 64)));
+        // With all ranks on this GPU every block that fits is taken: the launch is bound by this chip's memory, not by links (two ranks, 512 x 8192
+        // 47.5 us with 64 blocks each, 31.0 with 148; four ranks, 1024 x 4096 49.9 with 64 and 49.2 with 74; eight ranks no difference).  Ranks on GPUs of their
+        // own keep 64, which their links were measured with.
+        const long most = (hostArgs->extraFlag & TILEXR_FLAG_EMULATED) || R == 1 ? static_cast<long>(maxGrid) : 64;
+        const unsigned want = static_cast<unsigned>(std::min<int64_t>(n, EnvLong("TILEXR_AR_NORM_BLOCKS", most)));
         const unsigned grid = std::max(1u, std::min(want, maxGrid));
         LaunchConfig cfg{grid, ARN_THREADS, 0, true};
         ret = LaunchKernel(comm, kernel, &a, cfg, stream);
