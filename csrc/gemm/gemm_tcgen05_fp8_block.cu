@@ -24,9 +24,9 @@
 //
 // What bounds a block of K: the four instructions need 512 clocks at the tensor cores' rate, the fold 128 multiply-adds per thread
 // and its tensor-memory reads, and a scratch goes round through instruction, commit, fold and release, two of them in flight.
-// 8192^3 with all-zero operands, where power is no limit, takes 432 us at 1965 MHz: 947 clocks per block of K, the ends of the
+// 8192^3 with all-zero operands, where power is no limit, takes 421 us at 1965 MHz: 923 clocks per block of K, the ends of the
 // tiles included (767 us with an issuer of one diverged lane, two groups of N = 128 and a scale fetched per lane and block); with
-// random operands 511 us in a short loop, 570 at the power cap.
+// random operands 485 - 503 us in a short loop, 569 at the power cap.
 //
 // Fused with the collectives of a tensor-parallel layer (mode of GemmBlockArgs):
 //
@@ -37,7 +37,7 @@
 //                   communication.  The TMA warp of a CTA acquires the flag of its 128 rows before the first load of a
 //                   tile (TMA then reads LOCAL memory, without multicast); each promoter warp acquires it before it
 //                   reads the rows' scales.  Every rank walks the shards starting with its own, whose rows and scales it
-//                   reads where they are: waiting for its own copy of them cost 90 us at 2048 x 4096 on one rank.  That
+//                   reads where they are: waiting for its own copy of them cost 90 us at 2048 x 4096 on one rank (which now takes the plain kernel).  That
 //                   copy is made last, in slices of all CTAs, since nobody waits for it.
 //   GEMM -> reduce-scatter    the promoters store their 128 x 256 partial tile into the row owner's staging slot and
 //                   raise the tile's flag; when a CTA has run out of tiles its promoters add, in rank order, the
