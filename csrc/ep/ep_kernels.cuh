@@ -21,7 +21,7 @@ constexpr int EP_FP8_MAX_H = 8192;      // register-resident quantised row: 16 x
 constexpr uint32_t EP_COUNT_FLAG_SLOT = TILEXR_FLAGS_PER_PAIR - 1;   // blocks of a dispatch stay below this flag slot
 // Operator scratch of the control block (64-bit words from TILEXR_CTRL_SCRATCH_WORD) as the EP kernels use it.
 constexpr int EP_SCRATCH_CURSOR_WORD = 0;     // combine: two 32-bit work cursors
-constexpr int EP_SCRATCH_DONE_WORD = 1;       // dispatch: 32-bit count of blocks that have finished counting
+constexpr int EP_SCRATCH_DONE_WORD = 1;       // dispatch: 32-bit count of blocks that have finished counting; alone, see ep_dispatch_local.cu
 constexpr int EP_SCRATCH_BUCKET_WORD = 2;     // combine: 32-bit rows per bucket, EP_MAX_BUCKETS of them
 constexpr int EP_MAX_BUCKETS = 8;
 constexpr int EP_SCRATCH_TOTALS_WORD = 8;     // dispatch: 32-bit routes per column of this rank, EP_MAX_EXPERTS at most

@@ -794,3 +794,24 @@ def test_dispatch_through_fp8_and_back(txr, port, tokens, hidden, experts, dtype
             ep.dispatch(comm, x, round_trip=True, **dict(args, quant_mode=ep.QUANT_NONE))
     finally:
         comm.destroy()
+
+
+def test_dispatches_of_a_single_rank_in_turn(txr):
+    """The barrier's count runs on from launch to launch: large and small grids, and clusters, which do not use it, on one communicator."""
+    from conftest import free_port
+
+    ep, experts, top_k, g = txr.ep, 24, 4, torch.Generator().manual_seed(9)
+    comm = txr.init_process(0, 1, comm_id=f"127.0.0.1:{free_port()}", buffer_mb=64, device=0)
+    try:
+        for tokens in (3000, 65, 64, 300, 1, 3000, 129, 1009, 65):
+            x = torch.randn(tokens, 64, generator=g).to(torch.bfloat16).cuda()
+            ids = torch.randint(0, experts, (tokens, top_k), generator=g).to(torch.int32)
+            d = ep.dispatch(comm, x, num_experts=experts, top_k=top_k, expert_ids=ids.cuda(), expert_scales=torch.ones(tokens, top_k).cuda(),
+                            max_recv_rows=tokens * top_k)
+            flat = ids.reshape(-1).long()
+            order = torch.sort(flat, stable=True).indices
+            assert torch.equal(d.expert_token_nums.cpu(), torch.bincount(flat, minlength=experts))
+            assert torch.equal(d.expand_x[:tokens * top_k], x[(order // top_k).cuda()])
+        assert comm.device_status() == 0
+    finally:
+        comm.destroy()
