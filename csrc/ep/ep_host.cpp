@@ -427,6 +427,8 @@ int TileXR::EpDispatch(const TileXREpDispatchParams *p, int32_t *laneCountOut, b
     const int64_t clusterMost = local && (c.hostArgs->extraFlag & TILEXR_FLAG_EMULATED) == 0 && p->bs <= EP_CLUSTER_TOKENS && capBlocks >= EP_CLUSTER_BLOCKS
                                     ? ClusterBlocks(EpDispatchClusterKernel(p->quantMode, round)) : 0;
     const bool cluster = clusterMost > 0;
+    int device = 0, sms = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return TILEXR_ERROR_RUNTIME;
     for (int64_t perBlock = c.rankSize == 1 ? 4 : 16;; perBlock = 16) {
         grid = static_cast<unsigned>(std::max<int64_t>(minBlocks, std::min<int64_t>((p->bs + perBlock - 1) / perBlock, capBlocks)));
         unsigned gridCap = 0;
@@ -446,8 +448,16 @@ int TileXR::EpDispatch(const TileXREpDispatchParams *p, int32_t *laneCountOut, b
             if (ret != TILEXR_SUCCESS) return ret;
             if (maxGrid == 0) return TILEXR_ERROR_NOT_SUPPORT;
             gridCap = maxGrid;
-            if (grid <= maxGrid) break;
-            grid = maxGrid;
+            if (grid > maxGrid) {
+                grid = maxGrid;
+                continue;
+            }
+            // Alone, blocks that leave some SMs with two and others with one take as long as two: one block per SM where its share is an eighth smaller
+            // or more (1009 x 4096, 253 blocks of four tokens 18.4 us, 145 of seven 17.2; at 2048 tokens 38.3 and 38.2, at 4096 79.8 and 81.0).
+            const int64_t most = (p->bs + tokensPerBlock - 1) / tokensPerBlock;
+            const int64_t share = sms > 0 ? (p->bs + sms - 1) / sms : 0;
+            if (!local || perBlock != 4 || most <= sms || share * 8 > 2 * static_cast<int64_t>(tokensPerBlock) * 7) break;
+            grid = static_cast<unsigned>(sms);
         }
         grid = static_cast<unsigned>(std::max<int64_t>((p->bs + tokensPerBlock - 1) / tokensPerBlock, cluster ? 0 : std::min<int64_t>(minBlocks, gridCap)));
         // (the table of the local kernel, one or two bytes per block in rows of 16 bytes, fits that of eight blocks' 32-bit counts)

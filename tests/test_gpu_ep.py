@@ -803,7 +803,7 @@ def test_dispatches_of_a_single_rank_in_turn(txr):
     ep, experts, top_k, g = txr.ep, 24, 4, torch.Generator().manual_seed(9)
     comm = txr.init_process(0, 1, comm_id=f"127.0.0.1:{free_port()}", buffer_mb=64, device=0)
     try:
-        for tokens in (3000, 65, 64, 300, 1, 3000, 129, 1009, 65):
+        for tokens in (3000, 65, 64, 300, 1, 3000, 129, 1009, 65, 592, 593, 1036, 1037, 1184, 1185):
             x = torch.randn(tokens, 64, generator=g).to(torch.bfloat16).cuda()
             ids = torch.randint(0, experts, (tokens, top_k), generator=g).to(torch.int32)
             d = ep.dispatch(comm, x, num_experts=experts, top_k=top_k, expert_ids=ids.cuda(), expert_scales=torch.ones(tokens, top_k).cuda(),
