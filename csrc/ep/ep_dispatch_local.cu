@@ -16,7 +16,7 @@
 // 16.2 us with the barrier in memory, 10.0 so; 64 tokens 17.8 and 14.8; 40 x 4096, top-6, 16 bits 11.5 and 8.9).
 //
 // Bound by the stores of step 4 for large batches; steps 1 to 3 are a chain of memory round trips that small batches wait for
-// (us, general kernel and this one: 16 x 7168 by 256 experts, fp8 18.3 14.6; 1009 x 4096, top-6, 16 bits 23.5 18.4; 4096 x 7168, fp8 91 81, of
+// (us, general kernel and this one: 16 x 7168 by 256 experts, fp8 18.3 14.6; 1009 x 4096, top-6, 16 bits 23.5 17.2; 4096 x 7168, fp8 91 80, of
 // which the stores take 63: 3.9 TB/s of writes, what a plain fill of such a buffer reaches.  The reads of the tokens pass beside them; brought to
 // L2 during steps 1 to 3 they only delay the routes, 89).
 // The blocks wait for one another, so the launch is a cooperative one.
