@@ -179,7 +179,7 @@ __device__ void DispatchLocalBody(const EpDispatchArgs &a)
     uint8_t *table = DataHalf(comm, comm->rank, 0) + a.win.blockCountOff;
     // [0] blocks that have counted, over all launches; [1] how many that were before this one.  Block 0 moves [1] on once everybody has arrived, so
     // nothing is cleared at the end and no block has to be the last to leave (1009 x 4096, top-6, 16 bits 21.0 -> 18.4 us; 4096 x 7168, fp8 83.6 -> 80.9).
-    uint32_t *doneBlocks = reinterpret_cast<uint32_t *>(CtrlWord(comm, comm->rank, TILEXR_CTRL_SCRATCH_WORD + EP_SCRATCH_DONE_WORD));
+    uint32_t *doneBlocks = reinterpret_cast<uint32_t *>(CtrlWord(comm, comm->rank, TILEXR_CTRL_SCRATCH_WORD + EP_SCRATCH_LOCAL_DONE_WORD));
     const uint32_t doneBefore = !CLUSTER && tid == 0 ? __ldcg(doneBlocks + 1) : 0u;
 
     if (block == 0 && tid == 0) {

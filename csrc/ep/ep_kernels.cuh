@@ -21,11 +21,16 @@ constexpr int EP_FP8_MAX_H = 8192;      // register-resident quantised row: 16 x
 constexpr uint32_t EP_COUNT_FLAG_SLOT = TILEXR_FLAGS_PER_PAIR - 1;   // blocks of a dispatch stay below this flag slot
 // Operator scratch of the control block (64-bit words from TILEXR_CTRL_SCRATCH_WORD) as the EP kernels use it.
 constexpr int EP_SCRATCH_CURSOR_WORD = 0;     // combine: two 32-bit work cursors
-constexpr int EP_SCRATCH_DONE_WORD = 1;       // dispatch: 32-bit count of blocks that have finished counting; alone, see ep_dispatch_local.cu
+constexpr int EP_SCRATCH_DONE_WORD = 1;       // dispatch: 32-bit count of blocks that have finished counting
 constexpr int EP_SCRATCH_BUCKET_WORD = 2;     // combine: 32-bit rows per bucket, EP_MAX_BUCKETS of them
 constexpr int EP_MAX_BUCKETS = 8;
 constexpr int EP_SCRATCH_TOTALS_WORD = 8;     // dispatch: 32-bit routes per column of this rank, EP_MAX_EXPERTS at most
 constexpr int EP_SCRATCH_READY_WORD = 640;    // dispatch: per block, epoch of the launch whose histogram it has written
+// Dispatch on one rank (ep_dispatch_local.cu): its barrier's running count and the count before this launch, never cleared by a launch.
+// A word of its own: the kernels above expect theirs to be zero, and both kinds run on one communicator.
+constexpr int EP_SCRATCH_LOCAL_DONE_WORD = 1280;
+static_assert(EP_SCRATCH_READY_WORD + (EP_COUNT_FLAG_SLOT + 1) / 2 <= EP_SCRATCH_LOCAL_DONE_WORD && EP_SCRATCH_LOCAL_DONE_WORD < TILEXR_CTRL_SCRATCH_WORDS,
+              "the word lies behind those of every block");
 
 // Where a dispatch puts things inside one data half of the DESTINATION's window.  Identical
 // on every rank; computed by EpDispatchLayout() on the host.

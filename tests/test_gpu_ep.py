@@ -815,3 +815,46 @@ def test_dispatches_of_a_single_rank_in_turn(txr):
         assert comm.device_status() == 0
     finally:
         comm.destroy()
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("aligned_first", [True, False])
+def test_dispatches_of_a_single_rank_on_and_off_the_16_byte_grid_in_turn(txr, fp8, aligned_first):
+    """Outputs on and off the 16-byte grid take different kernels: on one communicator, in grids that grow and shrink, with a combine in
+    between and without, neither leaves anything behind that the other reads."""
+    from conftest import free_port
+
+    ep, h, experts, top_k, g = txr.ep, 512, 24, 4, torch.Generator().manual_seed(21)
+    comm = txr.init_process(0, 1, comm_id=f"127.0.0.1:{free_port()}", buffer_mb=64, device=0)
+    try:
+        aligned = aligned_first
+        for step, tokens in enumerate((65, 1009, 300, 3000, 65, 65, 3000, 1009, 1009, 300, 64, 3000, 16, 300)):
+            n = tokens * top_k
+            x = torch.randn(tokens, h, generator=g).to(torch.bfloat16).cuda()
+            ids = torch.stack([torch.randperm(experts, generator=g)[:top_k] for _ in range(tokens)]).to(torch.int32)
+            row_type = torch.float8_e4m3fn if fp8 else torch.bfloat16
+            out = torch.zeros(n * h + 16, dtype=row_type, device="cuda")[0 if aligned else 1:][:n * h].view(n, h)
+            assert (out.data_ptr() % 16 == 0) == aligned
+            d = ep.dispatch(comm, x, num_experts=experts, top_k=top_k, expert_ids=ids.cuda(), expert_scales=torch.ones(tokens, top_k).cuda(),
+                            quant_mode=ep.QUANT_FP8_1X128 if fp8 else ep.QUANT_NONE, max_recv_rows=n, expand_x_out=out)
+            torch.cuda.synchronize()
+            assert comm.device_status() == 0
+            flat = ids.reshape(-1).long()
+            order = torch.sort(flat, stable=True).indices
+            counts = torch.bincount(flat, minlength=experts)
+            assert int(d.recv_total) == n and torch.equal(d.expert_token_nums.cpu(), counts) and torch.equal(d.send_counts.cpu().long(), counts.cumsum(0))
+            assert torch.equal(d.route_rows.cpu().reshape(-1)[order].long(), torch.arange(n))
+            src = (order // top_k).cuda()
+            want = x[src]
+            if fp8:
+                want, scales = txr.quant.fp8_quant_1x128(want)
+                assert torch.equal(d.dynamic_scales, scales)
+            assert torch.equal(out.view(torch.uint8) if fp8 else out, want.view(torch.uint8) if fp8 else want)
+            if step % 3 == 1:
+                y = ep.combine(comm, x[src], d)
+                torch.cuda.synchronize()
+                # top_k equal rows with weight one: four times the value, exact in bf16
+                assert comm.device_status() == 0 and torch.equal(y, x * top_k)
+            aligned = not aligned
+    finally:
+        comm.destroy()
