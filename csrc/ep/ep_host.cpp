@@ -409,7 +409,12 @@ int TileXR::EpDispatch(const TileXREpDispatchParams *p, int32_t *laneCountOut, b
     const uint64_t outBytes = static_cast<uint64_t>(p->maxRecvRows) * (quant ? p->h : p->h * elemSize);
     TileXRUDMAMemHandle handle = 0;
     uint64_t regionOffset = 0;
-    const bool zeroCopy = EnvLong("TILEXR_EP_ZERO_COPY", 1) != 0 &&
+    const bool aligned = (reinterpret_cast<uintptr_t>(p->expandXOut) & 15u) == 0;
+    // per-expert smoothing makes the rows of one token differ from expert to expert: nothing to share
+    const bool dedup = p->dedup != 0 && c.rankSize > 1 && !(int8Mode && p->scales != nullptr);
+    // Rows that are quantised on the way, and rows that are copied on from the output, go in 16-byte pieces: into an output off that grid
+    // they take the way through the window, registered or not.
+    const bool zeroCopy = EnvLong("TILEXR_EP_ZERO_COPY", 1) != 0 && (aligned || !(quant || dedup)) &&
                           TileXRFindRegistration(comm, p->expandXOut, outBytes, &handle, &regionOffset) == TILEXR_SUCCESS;
 
     EpDispatchArgs a;
@@ -421,7 +426,6 @@ int TileXR::EpDispatch(const TileXREpDispatchParams *p, int32_t *laneCountOut, b
     // 148 SMs, and 4096 tokens left 40 of the 296 places empty.  With peers sixteen: every block raises a flag on every rank and every
     // block polls them all, and ranks whose batches differ a little launch grids of one size, as an emulated world requires.
     // Every block also takes a row of counts in the window: sixteen where the window is too small for the counts of more blocks.
-    const bool aligned = (reinterpret_cast<uintptr_t>(p->expandXOut) & 15u) == 0;
     const bool local = c.rankSize == 1 && aligned;       // no peers: a kernel of its own
     const KernelEntry &kernel = local ? EpDispatchLocalKernelEntry(p->quantMode, round) : EpDispatchKernelEntry(p->quantMode);
     const int64_t clusterMost = local && (c.hostArgs->extraFlag & TILEXR_FLAG_EMULATED) == 0 && p->bs <= EP_CLUSTER_TOKENS && capBlocks >= EP_CLUSTER_BLOCKS
@@ -512,8 +516,7 @@ int TileXR::EpDispatch(const TileXREpDispatchParams *p, int32_t *laneCountOut, b
     a.expandScalesOut = p->expandScalesOut;
     a.assistExtOut = p->assistExtOut;
     a.quantScales = int8Mode ? p->scales : nullptr;
-    // per-expert smoothing makes the rows of one token differ from expert to expert: nothing to share
-    a.dedup = (p->dedup != 0 && c.rankSize > 1 && a.quantScales == nullptr) ? 1u : 0u;
+    a.dedup = dedup ? 1u : 0u;
     int64_t magic = 0;
     ret = TileXRCommNextMagic(comm, &magic);
     if (ret != TILEXR_SUCCESS) return ret;

@@ -639,7 +639,7 @@ __device__ void EpDispatchBody(const EpDispatchArgs &a)
                     ++followers;
                     next = reinterpret_cast<const uint2 *>(winExt + f * 8)->x & EP_LINK_NEXT_MASK;
                 }
-                const int rowVecs16 = static_cast<int>(a.win.rowBytes / 16);
+                const int rowVecs16 = a.directOwn != 0 ? static_cast<int>(a.win.rowBytes / 16) : 0;     // an output off the 16-byte grid takes single bytes
                 for (int v0 = 0; v0 < rowVecs16; v0 += 128) {
                     Vec16 q[4];
 #pragma unroll
@@ -656,11 +656,9 @@ __device__ void EpDispatchBody(const EpDispatchArgs &a)
                         }
                     }
                 }
-                // a row whose length is not a multiple of 16 bytes keeps its tail
-                for (uint32_t bidx = static_cast<uint32_t>(rowVecs16) * 16 + lane; bidx < a.win.rowBytes; bidx += 32) {
-                    for (int j = 0; j < followers; ++j) {
-                        (a.expandXOut + __shfl_sync(0xffffffffu, myFollower, j) * a.win.rowBytes)[bidx] = src[bidx];
-                    }
+                for (int j = 0; j < followers; ++j) {
+                    uint8_t *dst = a.expandXOut + __shfl_sync(0xffffffffu, myFollower, j) * a.win.rowBytes;
+                    for (uint32_t i = static_cast<uint32_t>(rowVecs16) * 16 + lane; i < a.win.rowBytes; i += 32) dst[i] = src[i];
                 }
                 for (int j = 0; j < followers; ++j) {
                     const int64_t f = __shfl_sync(0xffffffffu, myFollower, j);

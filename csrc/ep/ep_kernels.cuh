@@ -111,7 +111,7 @@ struct EpDispatchArgs {
     float *expandScalesOut;          // [maxRecvRows] or null
     int32_t *assistExtOut;           // [maxRecvRows, 2] or null
     uint32_t dedup;
-    uint32_t directOwn;              // rows for this rank's own experts may be stored to expandXOut by the sender (16-byte aligned)
+    uint32_t directOwn;              // expandXOut is on the 16-byte grid: the sender stores rows for this rank's own experts there
 };
 
 struct EpCombineArgs {

@@ -858,3 +858,45 @@ def test_dispatches_of_a_single_rank_on_and_off_the_16_byte_grid_in_turn(txr, fp
             aligned = not aligned
     finally:
         comm.destroy()
+
+
+@pytest.mark.parametrize("registered", [False, True])
+@pytest.mark.parametrize("mode", ["none", "fp8", "mxfp8", "int8"])
+@pytest.mark.parametrize("ranks,dedup", [(1, False), (2, False), (3, True)])
+def test_dispatch_into_any_output_off_the_16_byte_grid(txr, ranks, dedup, mode, registered):
+    """Every transport, tokens with several experts on one rank, ordinary and registered memory: as into an output on the grid.  Rows of an odd number of
+    16-byte pieces where the transport allows it."""
+    ep = txr.ep
+    modes = {"none": ep.QUANT_NONE, "fp8": ep.QUANT_FP8_1X128, "mxfp8": ep.QUANT_MXFP8_E4M3, "int8": ep.QUANT_DYNAMIC_INT8}
+    row_type = {"none": torch.bfloat16, "fp8": torch.float8_e4m3fn, "mxfp8": torch.float8_e4m3fn, "int8": torch.int8}[mode]
+    h, tokens, experts, top_k = {"none": 1032, "fp8": 512, "mxfp8": 512, "int8": 1040}[mode], 75, 6, 4
+    g = torch.Generator().manual_seed(ranks)
+    xs = [torch.randn(tokens, h, generator=g).to(torch.bfloat16).cuda() for _ in range(ranks)]
+    ids = [torch.stack([torch.randperm(experts, generator=g)[:top_k] for _ in range(tokens)]).to(torch.int32).cuda() for _ in range(ranks)]
+    weights = torch.rand(tokens, top_k, generator=g).cuda()
+    cap = tokens * ranks * top_k
+    world = txr.init_emulated_world(ranks, device=0, buffer_mb=64)
+    try:
+        if registered:
+            memory = world.symm_empty((cap * h + 16,), row_type)
+        else:
+            memory = [torch.zeros(cap * h + 16, dtype=row_type, device="cuda") for _ in range(ranks)]
+        results = []
+        for offset in (0, 1):
+            outs = [m[offset:offset + cap * h].view(cap, h) for m in memory]
+            results.append(world.run(lambda c, r: ep.dispatch(c, xs[r], expert_ids=ids[r], expert_scales=weights, num_experts=experts, top_k=top_k,
+                                                              quant_mode=modes[mode], max_recv_rows=cap, expand_x_out=outs[r], dedup=dedup)))
+            world.check()
+            if offset == 0:
+                rows = [d.expand_x[:int(d.recv_total)].clone() for d in results[0]]
+                for m in memory:
+                    m.view(torch.uint8).zero_()
+        for d, e, want in zip(*results, rows):
+            n = int(d.recv_total)
+            assert e.expand_x.data_ptr() % 16 != 0 and int(e.recv_total) == n > 0
+            assert torch.equal(e.expand_x[:n].view(torch.uint8) if mode != "none" else e.expand_x[:n], want.view(torch.uint8) if mode != "none" else want)
+            assert torch.equal(e.assist[:n], d.assist[:n]) and torch.equal(e.route_rows, d.route_rows)
+            if mode != "none":
+                assert torch.equal(e.dynamic_scales[:n], d.dynamic_scales[:n])
+    finally:
+        world.destroy()
