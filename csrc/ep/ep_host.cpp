@@ -390,6 +390,10 @@ int TileXR::EpDispatch(const TileXREpDispatchParams *p, int32_t *laneCountOut, b
             return TILEXR_ERROR_PARA_CHECK_FAIL;
         }
     }
+    if ((fp8Mode || int8Mode) && (reinterpret_cast<uintptr_t>(p->x) & 15u) != 0) {
+        TILEXR_LOG(ERROR) << "EP dispatch: tokens that are quantised on the way must be 16-byte aligned";
+        return TILEXR_ERROR_PARA_CHECK_FAIL;
+    }
     if (p->activeMaskType != TILEXR_EP_ACTIVE_MASK_NONE && p->xActiveMask == nullptr) return TILEXR_ERROR_PARA_CHECK_FAIL;
     if (p->activeMaskType < 0 || p->activeMaskType > TILEXR_EP_ACTIVE_MASK_EXPERT) return TILEXR_ERROR_PARA_CHECK_FAIL;
     if (p->maxRecvRows <= 0) return TILEXR_ERROR_PARA_CHECK_FAIL;
@@ -553,6 +557,10 @@ int TileXRMoeEpCombineFused(const TileXREpCombineParams *p, TileXRCommPtr comm, 
     if (p == nullptr || p->expertOut == nullptr || p->assistInfoForCombine == nullptr || p->sendCounts == nullptr ||
         p->yOut == nullptr) {
         TILEXR_LOG(ERROR) << "EP combine: null tensor";
+        return TILEXR_ERROR_PARA_CHECK_FAIL;
+    }
+    if (((reinterpret_cast<uintptr_t>(p->expertOut) | reinterpret_cast<uintptr_t>(p->sharedExpertX) | reinterpret_cast<uintptr_t>(p->yOut)) & 15u) != 0) {
+        TILEXR_LOG(ERROR) << "EP combine: expertOut, sharedExpertX and yOut must be 16-byte aligned";
         return TILEXR_ERROR_PARA_CHECK_FAIL;
     }
     if (p->tpWorldSize > 1) return CombineWithTp(p, comm, stream, c);

@@ -900,3 +900,29 @@ def test_dispatch_into_any_output_off_the_16_byte_grid(txr, ranks, dedup, mode, 
                 assert torch.equal(e.dynamic_scales[:n], d.dynamic_scales[:n])
     finally:
         world.destroy()
+
+
+def test_tensors_off_the_16_byte_grid_that_the_kernels_read_in_16_byte_pieces(txr, port):
+    """Refused on the host, before a launch; tokens that are only copied may start anywhere."""
+    ep, h, tokens, experts, top_k = txr.ep, 512, 9, 8, 2
+    comm = txr.init_process(0, 1, comm_id=f"127.0.0.1:{port}", buffer_mb=16, device=0)
+    try:
+        def off(rows):
+            return torch.randn(rows * h + 8, generator=torch.Generator().manual_seed(rows)).to(torch.bfloat16).cuda()[1:1 + rows * h].view(rows, h)
+
+        ids = (torch.arange(tokens * top_k, dtype=torch.int32).view(tokens, top_k) % experts).cuda()
+        x = off(tokens)
+        args = dict(num_experts=experts, top_k=top_k, expert_ids=ids)
+        for mode in (ep.QUANT_FP8_1X128, ep.QUANT_MXFP8_E5M2, ep.QUANT_DYNAMIC_INT8):
+            with pytest.raises(RuntimeError):
+                ep.dispatch(comm, x, quant_mode=mode, **args)
+        d = ep.dispatch(comm, x, **args)
+        n = int(d.recv_total)
+        assert n == tokens * top_k and torch.equal(d.expand_x[:n], x[d.assist[:n, 1].long()])
+        rows = d.expand_x.shape[0]
+        for kw in (dict(expert_out=off(rows)), dict(shared_expert_x=x)):
+            with pytest.raises(RuntimeError):
+                ep.combine(comm, kw.pop("expert_out", d.expand_x), d, **kw)
+        assert torch.equal(ep.combine(comm, d.expand_x, d), x * top_k) and comm.device_status() == 0
+    finally:
+        comm.destroy()
