@@ -1278,7 +1278,7 @@ __global__ void __launch_bounds__(256) Fp8Dequant1x128Kernel(const uint8_t *y, c
         const int64_t i = base + u * static_cast<int64_t>(blockDim.x);
         if (i < vecs) {
             raw[u] = __ldcs(reinterpret_cast<const uint2 *>(y) + i);
-            s[u] = __ldg(scales + (i >> 4));
+            s[u] = scales[i >> 4];
         }
     }
 #pragma unroll
@@ -1369,7 +1369,7 @@ __global__ void __launch_bounds__(256) Mxfp8Dequant8Kernel(const uint8_t *y, con
                 const int64_t row = i / vecsPerRow;
                 at = row * blocksPerRow + (i - row * vecsPerRow) / 4;
             }
-            exponent[u] = static_cast<int>(__ldg(scales + at)) - 127;
+            exponent[u] = static_cast<int>(scales[at]) - 127;
         }
     }
 #pragma unroll

@@ -54,7 +54,8 @@ inline HostTraceHooks *&HostTraceSlot()
 #if defined(__CUDACC__)
 // A kernel launched with an overlap (tilexr_launch.h) may start while the kernel before it in its stream still runs.  StreamWait comes
 // before its first access to global memory, in every block: what came before in the stream has finished and can be seen.  StreamRelease lets
-// the kernel behind it start, so far as it was launched that way too, once every block has come here.
+// the kernel behind it start, so far as it was launched that way too, once every block has come here.  What a kernel before it has written is
+// not read with ld.global.nc or __ldg behind the wait: such a load may be served as if the data had not changed since the kernel started.
 __device__ __forceinline__ void StreamWait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void StreamRelease() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 #endif
