@@ -188,6 +188,15 @@ TXR_D uint64_t atom_cas_sys_u64(uint64_t *p, uint64_t expected, uint64_t desired
 #endif
 }
 
+TXR_D void fence_acq_rel_gpu()
+{
+#if TXR_ON_DEVICE
+    asm volatile("fence.acq_rel.gpu;" ::: "memory");
+#else
+    __atomic_thread_fence(__ATOMIC_SEQ_CST);
+#endif
+}
+
 TXR_D void fence_acq_rel_sys()
 {
 #if TXR_ON_DEVICE

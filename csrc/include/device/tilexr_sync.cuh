@@ -253,7 +253,8 @@ TXR_D void PublishDone(const Waiter &w)
     CommArgs *a = w.args;
     // One fence orders everything this rank did before all of the stores below; a release store per peer would
     // wait for the previous peer's store to be acknowledged over NVLink, rankSize - 1 round trips in a row.
-    if (!OneGpu(a)) fence_acq_rel_sys();      // else the exit counter has ordered it
+    if (OneGpu(a)) fence_acq_rel_gpu();
+    else fence_acq_rel_sys();
     for (int i = 0; i < a->rankSize; ++i) {
         const int r = (a->rank + i) % a->rankSize;
         st_relaxed_sys_u64(CtrlWord(a, r, TILEXR_CTRL_DONE_WORD + a->rank), MakeFlag(w.epoch, 0));
@@ -297,8 +298,8 @@ __device__ __forceinline__ void KernelEpilogue(Waiter &w, bool ok, int scratchWo
     __shared__ int sLastToLeave;
     __syncthreads();
     CommArgs *a = w.args;
-    // Without a reader on another GPU the counter's acquire and release order all there is to keep: the system-wide fence of every
-    // block cost about 3 us in a launch of 32 small blocks.
+    // Without a reader on another GPU the counter's acquire and release order what the blocks did before what its last one publishes:
+    // the system-wide fence of every block cost about 3 us in a launch of 32 small blocks.
     const bool oneGpu = OneGpu(a);
     if (threadIdx.x == 0) {
         if (!oneGpu) fence_acq_rel_sys();
