@@ -157,11 +157,10 @@ __device__ __forceinline__ int RouteToken(const float *logits, const float *bias
     return RouteTokenN<EP_MAX_EXPERTS / 32>(logits, bias, numExperts, topK, scoreFunc, renormalize, routedScale, lane, idsOut, weightsOut, picked);
 }
 
-// The end of a launch whose blocks read neither the epoch nor the counters of the control block: what KernelEpilogue keeps, by one thread.
+// What KernelEpilogue keeps but for the status, by one thread and without waiting for the other blocks.
 __device__ __forceinline__ void EndLocalLaunch(CommArgs *c, const Waiter &w)
 {
     c->dfx[TILEXR_DFX_LAUNCHES] += 1;
-    if (c->dfx[TILEXR_DFX_FAIL_CODE] == 0) c->dfx[TILEXR_DFX_RUN_STATUS] = TILEXR_RUN_FINISHED;
     st_relaxed_sys_u64(CtrlWord(c, c->rank, TILEXR_CTRL_DONE_WORD + c->rank), MakeFlag(w.epoch, 0));
     *CtrlWord(c, c->rank, TILEXR_CTRL_EPOCH_WORD) = w.epoch;
 }

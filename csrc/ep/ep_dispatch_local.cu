@@ -474,6 +474,7 @@ __device__ void DispatchLocalBody(const EpDispatchArgs &a)
     // All blocks have passed the barrier: none of them reads these words any more.
     if (block == 0 && tid == 0) {
         if (!CLUSTER) doneBlocks[1] = doneBefore + static_cast<uint32_t>(G);
+        if (comm->dfx[TILEXR_DFX_FAIL_CODE] == 0) comm->dfx[TILEXR_DFX_RUN_STATUS] = TILEXR_RUN_FINISHED;       // a failure is every block's
         EndLocalLaunch(comm, w);
     }
     if (!CLUSTER) return;

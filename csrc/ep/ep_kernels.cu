@@ -1159,12 +1159,18 @@ __device__ void EpCombineLocalBody(const EpCombineArgs &a)
     }
     PerfStageEnd(perf, TILEXR_PERF_PEER_IPC_TO_OUTPUT);
     PerfStageEnd(perf, TILEXR_PERF_KERNEL_TOTAL);
-    // The launch counts like the others; no other block of it reads these words, so one thread keeps them without waiting for anybody.
+    // The launch counts like the others; one thread keeps the record without waiting for anybody.  Other blocks may still run: one that fails after this
+    // overwrites the status, one that failed before is not overwritten.  (A block that only starts now would tag the abort word with the next
+    // epoch; nothing but its being set is read.)  The last block to leave would know, but a counter that every block adds to behind its
+    // stores takes 2.6 us of 1009 x 4096 tokens.
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         CommArgs *c = a.comm;
         c->dfx[TILEXR_DFX_MAGIC] = w.epoch;
         c->dfx[TILEXR_DFX_OP] = TILEXR_OP_EP_COMBINE;
         c->dfx[TILEXR_DFX_COUNT_ARG] = a.bs;
+        auto *status = reinterpret_cast<unsigned long long *>(&c->dfx[TILEXR_DFX_RUN_STATUS]);
+        atomicCAS(status, 0ull, static_cast<unsigned long long>(TILEXR_RUN_FINISHED));
+        atomicCAS(status, static_cast<unsigned long long>(TILEXR_RUN_STARTED), static_cast<unsigned long long>(TILEXR_RUN_FINISHED));
         EndLocalLaunch(c, w);
     }
 }

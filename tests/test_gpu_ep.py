@@ -760,10 +760,13 @@ def test_combine_of_a_route_that_the_dispatch_did_not_place(txr, port):
         y = ep.combine(comm, d.expand_x, d)
         torch.cuda.synchronize()
         assert comm.device_status() == 0 and torch.equal(y, torch.where((ids >= 0), x, torch.zeros_like(x)))
+        run_status, launch_count, finished, failed = 3, 10, 0x0D0E, 0xDEAD         # words of the failure record, two values
+        assert comm.dfx()[run_status] == finished
+        launches = comm.dfx()[launch_count]
         d.topk_ids = ids.clone().fill_(1)
         ep.combine(comm, d.expand_x, d)
         torch.cuda.synchronize()
-        assert comm.device_status() != 0
+        assert comm.device_status() != 0 and comm.dfx()[run_status] == failed and comm.dfx()[launch_count] == launches + 1
         comm.reset_status()
         d.topk_ids = ids
         assert torch.equal(ep.combine(comm, d.expand_x, d), y) and comm.device_status() == 0
