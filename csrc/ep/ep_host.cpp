@@ -285,6 +285,7 @@ int LaunchCombineLocal(EpCombineArgs *a, const TileXREpCombineParams &p, TileXRC
     int ret = MaxCooperativeGrid(comm, EpCombineLocalKernelEntry(), EP_LOCAL_THREADS, 0, 1, &places);
     if (ret != TILEXR_SUCCESS) return ret;
     if (places == 0) return TILEXR_ERROR_NOT_SUPPORT;
+    places = static_cast<unsigned>(std::min<int64_t>(places, std::max<int64_t>(1, EnvLong("TILEXR_EP_BLOCKS", places))));
     // A part is 32 vectors (a column of 16 bytes per lane, one round trip) until every warp has eight of them: then longer parts, for
     // fewer looks at the routes, and still enough items that the last round of them is short.  (2 to 32 of them, or no longer parts: within
     // 2 % at 1009 and 4096 tokens.)

@@ -929,3 +929,30 @@ def test_tensors_off_the_16_byte_grid_that_the_kernels_read_in_16_byte_pieces(tx
         assert torch.equal(ep.combine(comm, d.expand_x, d), x * top_k) and comm.device_status() == 0
     finally:
         comm.destroy()
+
+
+@pytest.mark.parametrize("cap", [1, 20, None])
+def test_blocks_of_a_single_rank_under_the_switch(txr, monkeypatch, tmp_path, cap):
+    """TILEXR_EP_BLOCKS caps the blocks of a dispatch and of a combine, whichever kernel they take; the results are the same."""
+    import json
+
+    from conftest import free_port
+
+    from tilexr_b200.utils.stage_profile import stage_profile
+
+    ep, h, tokens, experts, top_k = txr.ep, 512, 400, 16, 2
+    g = torch.Generator().manual_seed(3)
+    x = torch.randn(tokens, h, generator=g).to(torch.bfloat16).cuda()
+    ids = torch.stack([torch.randperm(experts, generator=g)[:top_k] for _ in range(tokens)]).to(torch.int32).cuda()
+    if cap is not None:
+        monkeypatch.setenv("TILEXR_EP_BLOCKS", str(cap))
+    comm = txr.init_process(0, 1, comm_id=f"127.0.0.1:{free_port()}", buffer_mb=64, device=0)
+    try:
+        with stage_profile(str(tmp_path)):
+            d = ep.dispatch(comm, x, num_experts=experts, top_k=top_k, expert_ids=ids)
+            y = ep.combine(comm, d.expand_x, d)
+        assert comm.device_status() == 0 and torch.equal(y, x * top_k)
+        blocks = [json.loads(p.read_text())["blocks"] for p in sorted(tmp_path.rglob("trace.json"))]
+        assert len(blocks) == 2 and (min(blocks) > 20 if cap is None else max(blocks) <= cap), blocks
+    finally:
+        comm.destroy()
