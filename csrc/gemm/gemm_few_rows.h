@@ -95,6 +95,13 @@ inline Fp8Slices PlanFp8Slices(int64_t tiles, int64_t pairs)
     return best;
 }
 
+// Blocks of the copy in front of a gathered product on one rank: four 16-byte vectors per thread until there are four blocks to an SM, and no more
+// than `ctas`, the caller's cap (0: none).
+inline int64_t StageCopyBlocks(int64_t vecs, int64_t sms, int64_t ctas)
+{
+    return std::min((vecs + 1023) / 1024, ctas > 0 ? std::min(ctas, 4 * sms) : 4 * sms);
+}
+
 } // namespace TileXR
 
 #endif // TILEXR_GEMM_FEW_ROWS_H

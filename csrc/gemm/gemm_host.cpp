@@ -725,7 +725,7 @@ int TileXRAllGatherMatmulFp8Block(const void *aShard, const float *scaleAShard, 
         int sms = 0;
         ret = SmCount(&sms);
         if (ret != TILEXR_SUCCESS) return ret;
-        const int64_t blocks = std::min<int64_t>(4 * sms, (vecs0 + vecs1 + 1023) / 1024);
+        const int64_t blocks = StageCopyBlocks(vecs0 + vecs1, sms, EnvLong("TILEXR_GEMM_CTAS", 0));
         if (blocks > 0) {
             const cudaError_t e = static_cast<cudaError_t>(LaunchOverlapped(StageCopyKernel(), static_cast<unsigned>(blocks), 1, 256, 0, 0, params, stream));
             if (e != cudaSuccess) {

@@ -232,3 +232,24 @@ int main()
 def test_few_rows_line_lies_where_it_was_measured(tmp_path):
     """The choice between the wide and the few-rows GEMM takes the slower one nowhere by more than the measurements' spread."""
     _run_host_program(tmp_path, FEW_ROWS_LINE_PROGRAM, ROOT / "csrc" / "gemm")
+
+
+STAGE_COPY_PROGRAM = r'''
+#include <cstdio>
+#include "gemm_few_rows.h"
+int main()
+{
+    const int64_t counts[] = {0, 1, 1023, 1024, 1025, 100000, 606208, 606209, 10000000};
+    for (int64_t vecs : counts) for (int64_t cap : {0, 1, 2, 20, 148, 592, 1000}) {
+        const int64_t blocks = TileXR::StageCopyBlocks(vecs, 148, cap);
+        if ((blocks == 0) != (vecs == 0) || blocks > 592 || (cap > 0 && blocks > cap) || (blocks - 1) * 1024 >= vecs + (vecs == 0)) return 1;
+        if (cap == 0 && blocks < 592 && blocks * 1024 < vecs) return 2;
+    }
+    std::puts("ok");
+    return 0;
+}
+'''
+
+
+def test_copy_in_front_of_a_gathered_product_keeps_to_the_callers_ctas(tmp_path):
+    _run_host_program(tmp_path, STAGE_COPY_PROGRAM, ROOT / "csrc" / "gemm")

@@ -326,9 +326,11 @@ def test_all_gather_matmul_fp8_block_exactly(txr, ranks, shard_rows, n, k):
         world.destroy()
 
 
-@pytest.mark.parametrize("rows,n,k", [(256, 136, 512), (512, 2568, 1536), (1280, 5128, 512)])
-def test_all_gather_matmul_fp8_block_on_one_rank(txr, port, rows, n, k):
+@pytest.mark.parametrize("rows,n,k,ctas", [(256, 136, 512, None), (512, 2568, 1536, None), (1280, 5128, 512, None), (512, 520, 1536, "3")])
+def test_all_gather_matmul_fp8_block_on_one_rank(txr, port, monkeypatch, rows, n, k, ctas):
     """A rank without peers: the product of its own rows, exactly, and all rows and scales in the staging buffers; then of rows that are there already."""
+    if ctas is not None:
+        monkeypatch.setenv("TILEXR_GEMM_CTAS", ctas)
     comm = txr.init_process(0, 1, comm_id=f"127.0.0.1:{port}", buffer_mb=64, device=0)
     try:
         qa, sa, qw, sw = _exact_block_operands(rows, n, k, rows + n)
