@@ -570,8 +570,8 @@ int TileXRMatmulReduceScatter(const void *a, const void *b, void *partialStaging
     const int64_t m = shardRows * R;
     ret = CheckShape(a, b, out, m, n, k, dtype);
     if (ret != TILEXR_SUCCESS) return ret;
-    if (partialStaging == nullptr || shardRows % GEMM_BM != 0) {
-        TILEXR_LOG(ERROR) << "matmul reduce-scatter: shardRows must be a multiple of " << GEMM_BM << " and a staging buffer is required";
+    if (partialStaging == nullptr || (reinterpret_cast<uintptr_t>(partialStaging) & 15u) != 0 || shardRows % GEMM_BM != 0) {
+        TILEXR_LOG(ERROR) << "matmul reduce-scatter: shardRows must be a multiple of " << GEMM_BM << " and a 16-byte aligned staging buffer is required";
         return TILEXR_ERROR_PARA_CHECK_FAIL;
     }
     TileXRUDMAMemHandle handle = 0;
@@ -690,7 +690,8 @@ int TileXRAllGatherMatmulFp8Block(const void *aShard, const float *scaleAShard, 
     const int64_t m = shardRows * R;
     if (aShard == nullptr || scaleAShard == nullptr || aStaging == nullptr || scaleStaging == nullptr || b == nullptr || c == nullptr ||
         shardRows <= 0 || n <= 0 || k <= 0 ||
-        ((reinterpret_cast<uintptr_t>(aShard) | reinterpret_cast<uintptr_t>(scaleAShard) | reinterpret_cast<uintptr_t>(c)) & 15u) != 0) {
+        ((reinterpret_cast<uintptr_t>(aShard) | reinterpret_cast<uintptr_t>(scaleAShard) | reinterpret_cast<uintptr_t>(scaleStaging) |
+          reinterpret_cast<uintptr_t>(c)) & 15u) != 0) {
         TILEXR_LOG(ERROR) << "all-gather block-scaled matmul: null or misaligned tensor";
         return TILEXR_ERROR_PARA_CHECK_FAIL;
     }
@@ -794,6 +795,10 @@ int TileXRMatmulReduceScatterFp8Block(const void *a, const float *scaleA, const 
     if (Alone(hostArgs)) {
         // The sum over one rank is its own partial product: no staging, no flags, no second pass over it.
         return TileXRMatmulFp8BlockScaled(a, scaleA, b, scaleB, out, m, n, k, inDtype, outDtype, FailWord(devArgs), stream);
+    }
+    if ((reinterpret_cast<uintptr_t>(partialStaging) & 15u) != 0) {
+        TILEXR_LOG(ERROR) << "block-scaled matmul reduce-scatter: the staging buffer must be 16-byte aligned";
+        return TILEXR_ERROR_PARA_CHECK_FAIL;
     }
     ret = MakeMap8(&g.tmapA, a, m, k, GEMM_BM);
     if (ret != TILEXR_SUCCESS) return ret;

@@ -340,6 +340,10 @@ def test_all_gather_matmul_fp8_block_on_one_rank(txr, port, monkeypatch, rows, n
             got = txr.gemm.all_gather_matmul_fp8_block(comm, a, s, a_staging, s_staging, qw, sw)
             assert torch.equal(got, want)
             assert torch.equal(a_staging.view(torch.uint8), qa.view(torch.uint8)) and torch.equal(s_staging, sa)
+        if k % 512 == 0:
+            off = comm.symm_empty((rows * (k // 128) + 4,), torch.float32)[1:1 + rows * (k // 128)].view(rows, k // 128)
+            with pytest.raises(RuntimeError):                  # the scales travel in 16-byte pieces
+                txr.gemm.all_gather_matmul_fp8_block(comm, qa, sa, a_staging, off, qw, sw)
         assert comm.device_status() == 0
     finally:
         comm.destroy()
@@ -439,3 +443,20 @@ def test_matmul_fp8_block_slices_exactly(txr, m, n, k):
     128 and of 64 columns)."""
     ops = _exact_block_operands(m, n, k, k + m)
     assert torch.equal(txr.gemm.matmul_fp8_block(*ops), _exact_block_product(*ops).to(torch.bfloat16))
+
+
+def test_staging_buffers_off_the_16_byte_grid(txr):
+    """Partial tiles travel in 16-byte pieces: refused on the host, before a launch."""
+    rows, n, k, ranks = 256, 136, 512, 2
+    world = txr.init_emulated_world(ranks, device=0, buffer_mb=16)
+    try:
+        a, b = torch.zeros(ranks * rows, k, dtype=torch.bfloat16, device="cuda"), torch.zeros(n, k, dtype=torch.bfloat16, device="cuda")
+        qa, sa, qw, sw = _exact_block_operands(ranks * rows, n, k, 1)
+        stagings = [s[1:1 + ranks * rows * n].view(ranks * rows, n) for s in world.symm_empty((ranks * rows * n + 8,), torch.bfloat16)]
+        with pytest.raises(RuntimeError):
+            world.run(lambda c, r: txr.gemm.matmul_reduce_scatter(c, a, b, stagings[r]))
+        with pytest.raises(RuntimeError):
+            world.run(lambda c, r: txr.gemm.matmul_reduce_scatter_fp8_block(c, qa, sa, qw, sw, stagings[r]))
+        world.check()
+    finally:
+        world.destroy()
