@@ -309,7 +309,7 @@ __device__ void ArNormBody(const ArNormArgs &a)
     KernelEpilogue(w, ok);
 }
 
-// Rows of up to 8192 columns leave room for two blocks on an SM.
+// Rows of up to 8192 columns can have two blocks on an SM.
 TILEXR_DEFINE_KERNEL_OCC(TileXRAllReduceRmsNormKernel, ArNormArgs, ArNormBody<2>, ARN_THREADS, 2)
 TILEXR_DEFINE_KERNEL(TileXRAllReduceRmsNormWideKernel, ArNormArgs, ArNormBody<ARN_MAX_VECS>, ARN_THREADS)
 
@@ -383,10 +383,19 @@ int TileXRAllReduceRmsNorm(const void *x, void *residualInOut, const void *gamma
         zeroCopy = TileXRFindRegistration(comm, residualInOut, totalBytes, &resHandle, &resOffset) == TILEXR_SUCCESS;
     }
     const int ranksPerDevice = (hostArgs->extraFlag & TILEXR_FLAG_EMULATED) ? R : 1;
-    unsigned maxGrid = 0;
-    const KernelEntry &kernel = h <= static_cast<int64_t>(ARN_THREADS) * 2 * 8 ? TileXRAllReduceRmsNormKernelEntry : TileXRAllReduceRmsNormWideKernelEntry;
-    ret = MaxCooperativeGrid(comm, kernel, ARN_THREADS, 0, ranksPerDevice, &maxGrid);
+    unsigned maxWide = 0, maxTwo = 0;
+    ret = MaxCooperativeGrid(comm, TileXRAllReduceRmsNormWideKernelEntry, ARN_THREADS, 0, ranksPerDevice, &maxWide);
     if (ret != TILEXR_SUCCESS) return ret;
+    if (h <= static_cast<int64_t>(ARN_THREADS) * 2 * 8) {
+        ret = MaxCooperativeGrid(comm, TileXRAllReduceRmsNormKernelEntry, ARN_THREADS, 0, ranksPerDevice, &maxTwo);
+        if (ret != TILEXR_SUCCESS) return ret;
+    }
+    // Where a GPU has this rank alone and peers, 64 blocks, which the links were measured with.  Else every block that fits: the launch is bound
+    // by this chip's memory, not by links (two ranks, 512 x 8192 47.5 us with 64 blocks each, 31.0 with 148; four ranks, 1024 x 4096
+    // 49.9 with 64 and 49.2 with 74; eight ranks no difference).
+    const bool peers = R > 1 && (hostArgs->extraFlag & TILEXR_FLAG_EMULATED) == 0;
+    const long most = peers ? 64 : static_cast<long>(std::max(maxWide, maxTwo));
+    const int64_t wantMost = EnvLong("TILEXR_AR_NORM_BLOCKS", most);
 
     for (int64_t done = 0; done < rows; done += maxRows) {
         const int64_t n = std::min<int64_t>(maxRows, rows - done);
@@ -415,12 +424,11 @@ int TileXRAllReduceRmsNorm(const void *x, void *residualInOut, const void *gamma
         if (ret != TILEXR_SUCCESS) return ret;
         a.magic = magic;
         (void)rank;
-        // With all ranks on this GPU every block that fits is taken: the launch is bound by this chip's memory, not by links (two ranks, 512 x 8192
-        // 47.5 us with 64 blocks each, 31.0 with 148; four ranks, 1024 x 4096 49.9 with 64 and 49.2 with 74; eight ranks no difference).  Ranks on GPUs of their
-        // own keep 64, which their links were measured with.
-        const long most = (hostArgs->extraFlag & TILEXR_FLAG_EMULATED) || R == 1 ? static_cast<long>(maxGrid) : 64;
-        const unsigned want = static_cast<unsigned>(std::min<int64_t>(n, EnvLong("TILEXR_AR_NORM_BLOCKS", most)));
-        const unsigned grid = std::max(1u, std::min(want, maxGrid));
+        const int64_t want = std::max<int64_t>(1, std::min(n, wantMost));
+        // The form with two blocks to an SM spills at its 64 registers: only for a grid that needs the second one.
+        const bool two = want > static_cast<int64_t>(maxWide) && maxTwo > maxWide;
+        const KernelEntry &kernel = two ? TileXRAllReduceRmsNormKernelEntry : TileXRAllReduceRmsNormWideKernelEntry;
+        const unsigned grid = static_cast<unsigned>(std::min<int64_t>(want, std::max(1u, two ? maxTwo : maxWide)));
         LaunchConfig cfg{grid, ARN_THREADS, 0, true};
         ret = LaunchKernel(comm, kernel, &a, cfg, stream);
         if (ret != TILEXR_SUCCESS) return ret;

@@ -113,3 +113,19 @@ def test_emulated_world_of_more_ranks_than_travel_with_a_launch():
             assert torch.allclose(y.float(), want, rtol=2 ** -7, atol=2 ** -7) and torch.equal(y, ys[0])
     finally:
         world.destroy()
+
+
+@pytest.mark.parametrize("ranks,rows,h,algo,with_res,symmetric", [
+    (2, 75, 8192, 1, True, False),        # one row more than there are places with one block to an SM: the form with two, all its columns used
+    (2, 74, 8192, 1, True, False),        # the last grid of the other
+    (3, 51, 4104, 2, True, True),         # 49 blocks per rank fit one to an SM; one thread has a second column
+    (2, 160, 8200, 1, False, False),      # too long for two columns per thread, whatever the grid
+])
+def test_all_reduce_rmsnorm_around_one_block_per_sm(txr, ranks, rows, h, algo, with_res, symmetric):
+    test_all_reduce_rmsnorm(txr, ranks, rows, h, algo, with_res, symmetric)
+
+
+@pytest.mark.parametrize("blocks", ["1", "9", "100"])
+def test_all_reduce_rmsnorm_under_the_switch(txr, monkeypatch, blocks):
+    monkeypatch.setenv("TILEXR_AR_NORM_BLOCKS", blocks)
+    test_all_reduce_rmsnorm(txr, 2, 130, 2048, 1, True, False)
