@@ -65,7 +65,7 @@ inline FewRowsLaunch PlanFewRows(int64_t m, int64_t n, int64_t k, int64_t groups
     return {split, static_cast<unsigned>(split > 1 ? items * split : std::max<int64_t>(1, std::min(items, places)))};
 }
 
-// How the 256 x 256 tiles of a block-scaled fp8 product are dealt out to CTA pairs: the first `wide` whole, the others in slices of
+// How the 256 x 256 tiles of a plain block-scaled fp8 product (the fused forms keep to whole ones: with peers slices were not measured) are dealt out to CTA pairs: the first `wide` whole, the others in slices of
 // `width` columns, so that a last wave of a few tiles, or a product of a few tiles, does not leave most pairs without work.  Every slice
 // reads its tile's rows of A again and waits for the same round trips per block of K, so the narrow ones are not cheap.
 // us, whole tiles and the choice: 2048 x 7168 x 4096 (224 tiles on 74 pairs, the last two in slices of 32) 86.7 78.4; 4096 x 7168 x 4096

@@ -753,8 +753,6 @@ int TileXRAllGatherMatmulFp8Block(const void *aShard, const float *scaleAShard, 
     unsigned grid = 0;
     ret = Fp8BlockFusedGrid(comm, hostArgs, g.mode, &grid);
     if (ret != TILEXR_SUCCESS) return ret;
-    ret = Fp8Slicing(&g, b, grid / 2);
-    if (ret != TILEXR_SUCCESS) return ret;
     int64_t magic = 0;
     ret = TileXRCommNextMagic(comm, &magic);
     if (ret != TILEXR_SUCCESS) return ret;

@@ -328,14 +328,14 @@ struct FbItem {
     int col0, width;     // columns of C
 };
 
-// Item `i` of the launch: a whole tile or a slice of one.  A slice may lie past the last column (col0 >= N): nobody works on it.
+// Item `i` of the launch: a whole tile or, in the plain mode, a slice of one.  A slice may lie past the last column (col0 >= N): nobody works on it.
 template <int MODE>
 __device__ __forceinline__ FbItem FbItemOf(const GemmBlockArgs &a, int i, int mTiles, int rank)
 {
     FbItem it;
     int t = i, slice = 0;
     it.width = GEMM_BN;
-    if (MODE != GEMM_REDUCE_SCATTER && i >= a.wideTiles) {
+    if (MODE == GEMM_PLAIN && i >= a.wideTiles) {
         const int per = GEMM_BN / a.sliceWidth;
         const int u = i - a.wideTiles;
         t = a.wideTiles + u / per;
@@ -467,7 +467,7 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
                     uint8_t *sb = sa + GEMM_STAGE_A_BYTES;
                     if (leader) MbarExpectTx(&st->full[stage], 2 * stageBytes);
                     FbTmaLoad(sa, mapA, kb * 128, yA, &st->full[stage]);       // x in bytes = elements: a multiple of 128
-                    if (MODE == GEMM_REDUCE_SCATTER || it.width == GEMM_BN) {
+                    if (MODE != GEMM_PLAIN || it.width == GEMM_BN) {
                         FbTmaLoad(sb, &a.tmapB, kb * 128, rowB, &st->full[stage]);
                     } else {
                         for (int r = 0; r < it.width / 2; r += GEMM_FP8_SLICE_BOX) FbTmaLoad(sb + r * 128, &a.tmapBSlice, kb * 128, rowB + r, &st->full[stage]);
@@ -760,7 +760,7 @@ __device__ __forceinline__ void FbBody(const GemmBlockArgs &a)
         findItem();
         for (bool go = true; go && nextT < items;) {
             const FbItem it = nextItem;
-            if (MODE == GEMM_REDUCE_SCATTER || it.width == GEMM_BN) go = foldItem(FbCols<FB_HALF_N>{}, it);
+            if (MODE != GEMM_PLAIN || it.width == GEMM_BN) go = foldItem(FbCols<FB_HALF_N>{}, it);
             else if (it.width == 128) go = foldItem(FbCols<64>{}, it);
             else if (it.width == 64) go = foldItem(FbCols<32>{}, it);
             else go = foldItem(FbCols<16>{}, it);
