@@ -65,34 +65,25 @@ inline FewRowsLaunch PlanFewRows(int64_t m, int64_t n, int64_t k, int64_t groups
     return {split, static_cast<unsigned>(split > 1 ? items * split : std::max<int64_t>(1, std::min(items, places)))};
 }
 
-// How the 256 x 256 tiles of a plain block-scaled fp8 product (the fused forms keep to whole ones: with peers slices were not measured) are dealt out to CTA pairs: the first `wide` whole, the others in slices of
-// `width` columns, so that a last wave of a few tiles, or a product of a few tiles, does not leave most pairs without work.  Every slice
-// reads its tile's rows of A again and waits for the same round trips per block of K, so the narrow ones are not cheap.
-// us, whole tiles and the choice: 2048 x 7168 x 4096 (224 tiles on 74 pairs, the last two in slices of 32) 86.7 78.4; 4096 x 7168 x 4096
-// (448, the last four so) 149 139; 16 x 7168 x 2048 (28, slices of 128) 14.6 12.6; 100 x 4096 x 4096 (16, slices of 64) 21.7 17.6.
+// How the 256 x 256 tiles of a plain block-scaled fp8 product are dealt out to CTA pairs (the fused forms keep to whole ones: with peers slices were
+// not measured): the first `wide` whole, the others in slices of `width` columns, so that a last wave of a few tiles, or a product of a
+// few tiles, does not leave most pairs without work.  A slice reads its tile's rows of A again and waits for the same round trips per
+// block of K, so a narrow one takes about 0.70 (32 columns), 0.72 or 0.77 (128) of a whole tile at any K from 512 to 8192: the narrowest slices
+// that all find a pair at once, and whole tiles where not even those of 128 columns do.
+// us at K 2048 on 74 pairs, whole tiles, slices of 128, 64 and 32 columns: 2 tiles 12.1 9.7 9.2 8.8; 16 12.5 10.0 9.4 14.9; 28 12.9 10.3 15.5 26.2;
+// 40 13.3 16.7 21.4 31.9; 76 22.4 20.2 19.6 19.5; 224 41.7 39.2 38.7 38.6.  At K 4096, 224 and 448 tiles: 70.3 whole and 64.9 in
+// slices of 32, 122.3 and 119.6.
 struct Fp8Slices {
     int wide, width, items;
 };
 inline Fp8Slices PlanFp8Slices(int64_t tiles, int64_t pairs)
 {
-    constexpr int WIDTHS[] = {128, 64, 32};
-    constexpr int COST[] = {56, 36, 30};             // of a slice, a whole tile 100
-    Fp8Slices best = {static_cast<int>(tiles), 256, static_cast<int>(tiles)};
-    int64_t bestCost = (tiles + pairs - 1) / pairs * 100;
-    const int64_t rounds = tiles / pairs;
-    for (int64_t keep = rounds; keep >= std::max<int64_t>(0, rounds - 1); --keep) {
-        const int64_t rest = tiles - keep * pairs;
-        if (rest == 0) continue;
-        for (int i = 0; i < 3; ++i) {
-            const int64_t slices = rest * (256 / WIDTHS[i]);
-            const int64_t cost = keep * 100 + (slices + pairs - 1) / pairs * COST[i];
-            if (cost < bestCost) {
-                bestCost = cost;
-                best = {static_cast<int>(keep * pairs), WIDTHS[i], static_cast<int>(keep * pairs + slices)};
-            }
-        }
+    const int64_t wide = tiles / pairs * pairs, rest = tiles - wide;
+    for (int width = 32; rest > 0 && width <= 128; width *= 2) {
+        const int64_t slices = rest * (256 / width);
+        if (slices <= pairs) return {static_cast<int>(wide), width, static_cast<int>(wide + slices)};
     }
-    return best;
+    return {static_cast<int>(tiles), 256, static_cast<int>(tiles)};
 }
 
 // Blocks of the copy in front of a gathered product on one rank: four 16-byte vectors per thread until there are four blocks to an SM, and no more
