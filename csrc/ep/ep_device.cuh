@@ -1,4 +1,4 @@
-// Device code that the expert-parallel kernels share: routing of a token, block quantisation.
+// Device code that the expert-parallel kernels share: routing of a token, ranking of a block's routes, quantisation of rows.
 #ifndef TILEXR_EP_DEVICE_CUH
 #define TILEXR_EP_DEVICE_CUH
 
@@ -241,6 +241,56 @@ __device__ __forceinline__ Vec16 QuantMx16(const float *f, bool e5m2, int lane, 
         q.w = Fp8x4(f[12] * inv, f[13] * inv, f[14] * inv, f[15] * inv);
     }
     return q;
+}
+
+// Rank of each of a block's routes among its routes to the same column (expert[] -1: none), in (token, k) order, and the routes per column in hist[],
+// which is zero before: one warp walks the routes 32 at a time; lanes with the same column find one another with a match and the last
+// of them moves the column's running count on.
+__device__ __forceinline__ void RankBlockRoutes(int routes, const int32_t *expert, int32_t *rank, int32_t *hist, int lane)
+{
+    for (int base = 0; base < routes; base += 32) {
+        const int i = base + lane;
+        const int e = i < routes ? expert[i] : -1;
+        const uint32_t same = __match_any_sync(0xffffffffu, e);
+        int r = 0;
+        if (e >= 0) r = hist[e] + __popc(same & ((1u << lane) - 1u));
+        __syncwarp();
+        if (e >= 0 && (same & ~((2u << lane) - 1u)) == 0) hist[e] += __popc(same);
+        __syncwarp();
+        if (i < routes) rank[i] = r;
+    }
+}
+
+// int8 rows with optional per-expert smoothing scales `sc` (null: none): the largest magnitude of a row of `chunks` 16-element pieces, the same in all
+// lanes, and every `parts`-th 512 elements of it from `part` on, times `inv`, rounded and clamped.  Called by a whole warp.
+__device__ __forceinline__ float Int8RowAmax(const uint8_t *row, const float *sc, int chunks, bool bf16, int lane)
+{
+    float amax = 0.f;
+    for (int c = lane; c < chunks; c += 32) {
+        float f[16];
+        Unpack8(ld_vec16(row + static_cast<int64_t>(c) * 32), bf16, f);
+        Unpack8(ld_vec16(row + static_cast<int64_t>(c) * 32 + 16), bf16, f + 8);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) amax = fmaxf(amax, fabsf(sc != nullptr ? f[j] * sc[c * 16 + j] : f[j]));
+    }
+    return WarpMax(amax);
+}
+
+__device__ __forceinline__ void Int8RowStore(const uint8_t *row, const float *sc, float inv, int chunks, bool bf16, int part, int parts, int lane, uint8_t *to)
+{
+    for (int c = part * 32 + lane; c < chunks; c += parts * 32) {
+        float f[16];
+        Unpack8(ld_vec16(row + static_cast<int64_t>(c) * 32), bf16, f);
+        Unpack8(ld_vec16(row + static_cast<int64_t>(c) * 32 + 16), bf16, f + 8);
+        uint32_t wds[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            const float v = (sc != nullptr ? f[j] * sc[c * 16 + j] : f[j]) * inv;
+            const int q = max(-128, min(127, __float2int_rn(v)));
+            wds[j >> 2] |= static_cast<uint32_t>(q & 0xff) << (8 * (j & 3));
+        }
+        st_vec16(to + static_cast<int64_t>(c) * 16, Vec16{wds[0], wds[1], wds[2], wds[3]});
+    }
 }
 
 } // namespace

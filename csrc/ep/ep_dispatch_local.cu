@@ -219,20 +219,7 @@ __device__ void DispatchLocalBody(const EpDispatchArgs &a)
         }
     }
     __syncthreads();
-    // Rank of each route among the block's routes to the same expert, in (token, k) order (as in the general kernel).
-    if (warp == 0) {
-        for (int base = 0; base < nRoutes; base += 32) {
-            const int i = base + lane;
-            const int e = i < nRoutes ? sm.routeExpert[i] : -1;
-            const uint32_t same = __match_any_sync(0xffffffffu, e);
-            int r = 0;
-            if (e >= 0) r = sm.hist[e] + __popc(same & ((1u << lane) - 1u));
-            __syncwarp();
-            if (e >= 0 && (same & ~((2u << lane) - 1u)) == 0) sm.hist[e] += __popc(same);
-            __syncwarp();
-            if (i < nRoutes) sm.routeRank[i] = r;
-        }
-    }
+    if (warp == 0) RankBlockRoutes(nRoutes, sm.routeExpert, sm.routeRank, sm.hist, lane);
     __syncthreads();
     if (!CLUSTER) {
         if (wide) StoreCounts<uint16_t>(table, pitch, E, block, sm.hist, tid);
@@ -354,36 +341,11 @@ __device__ void DispatchLocalBody(const EpDispatchArgs &a)
                     const float *sc = a.quantScales != nullptr ? a.quantScales + static_cast<int64_t>(e) * a.h : nullptr;
                     float inv = 1.0f;
                     if (int8Dynamic) {
-                        float amax = 0.f;
-                        for (int it = 0; it < iters; ++it) {
-                            const int c = it * 32 + lane;
-                            if (c < chunks) {
-                                float f[16];
-                                Unpack8(ld_vec16(row + static_cast<int64_t>(c) * 32), bf16, f);
-                                Unpack8(ld_vec16(row + static_cast<int64_t>(c) * 32 + 16), bf16, f + 8);
-#pragma unroll
-                                for (int j = 0; j < 16; ++j) amax = fmaxf(amax, fabsf(sc != nullptr ? f[j] * sc[c * 16 + j] : f[j]));
-                            }
-                        }
-                        amax = WarpMax(amax);
+                        const float amax = Int8RowAmax(row, sc, chunks, bf16, lane);
                         if (amax > 0.f) inv = 127.0f / amax;
                         if (part == 0 && lane == 0) a.dynamicScalesOut[rr] = amax > 0.f ? amax / 127.0f : 1.0f;
                     }
-                    for (int it = part; it < iters; it += parts) {
-                        const int c = it * 32 + lane;
-                        if (c >= chunks) continue;
-                        float f[16];
-                        Unpack8(ld_vec16(row + static_cast<int64_t>(c) * 32), bf16, f);
-                        Unpack8(ld_vec16(row + static_cast<int64_t>(c) * 32 + 16), bf16, f + 8);
-                        uint32_t wds[4] = {0u, 0u, 0u, 0u};
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) {
-                            const float v = (sc != nullptr ? f[j] * sc[c * 16 + j] : f[j]) * inv;
-                            const int q = max(-128, min(127, __float2int_rn(v)));
-                            wds[j >> 2] |= static_cast<uint32_t>(q & 0xff) << (8 * (j & 3));
-                        }
-                        st_vec16(p + static_cast<int64_t>(c) * 16, Vec16{wds[0], wds[1], wds[2], wds[3]});
-                    }
+                    Int8RowStore(row, sc, inv, chunks, bf16, part, parts, lane, p);
                 }
             } else if (quant) {
                 // each 512-element chunk is quantised once and stored to every destination right away
