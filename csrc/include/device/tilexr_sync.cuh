@@ -317,10 +317,9 @@ __device__ __forceinline__ void KernelEpilogue(Waiter &w, bool ok, int scratchWo
     }
     if (threadIdx.x == 0) {
         if (sLastToLeave != 0) {
-            uint32_t *exitCounter =
-                reinterpret_cast<uint32_t *>(CtrlWord(a, a->rank, TILEXR_CTRL_GRIDBAR_WORD + TILEXR_CTRL_GRIDBAR_COUNT));
-            st_release_gpu_u32(exitCounter, 0);
             PublishDone(w);
+            // read by the next launch only: an ordinary store (a release is a second fence in a row, 1 us of four emulated ranks' 256 x 7168)
+            *reinterpret_cast<uint32_t *>(CtrlWord(a, a->rank, TILEXR_CTRL_GRIDBAR_WORD + TILEXR_CTRL_GRIDBAR_COUNT)) = 0;
             *CtrlWord(a, a->rank, TILEXR_CTRL_EPOCH_WORD) = w.epoch;
             if (a->dfx[TileXR::TILEXR_DFX_FAIL_CODE] == 0 && ok) {
                 a->dfx[TileXR::TILEXR_DFX_RUN_STATUS] = TILEXR_RUN_FINISHED;
