@@ -83,8 +83,8 @@ def test_all_reduce_rmsnorm_groups_of_rows(txr, ranks, rows, h, algo, with_res, 
 
 
 @pytest.mark.parametrize("ranks,rows,h,algo,with_res,symmetric", [
-    (2, 9, 8192, 2, False, False),        # the longest rows of the kernel with two 16-byte columns per thread: all of them used
-    (2, 9, 8200, 2, True, False),         # the shortest of the other kernel
+    (2, 9, 8192, 2, False, False),        # the longest rows for two 16-byte columns per thread: all of them used (a grid this small takes the other kernel)
+    (2, 9, 8200, 2, True, False),         # the shortest with a third
     (3, 26, 4104, 1, True, False),        # one thread has a second column; an odd row after whole pairs
 ])
 def test_all_reduce_rmsnorm_around_two_columns_per_thread(txr, ranks, rows, h, algo, with_res, symmetric):
